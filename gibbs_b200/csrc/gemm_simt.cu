@@ -3,28 +3,64 @@
 // the tensor-core kernel does not take (a weight kept in 32-bit beside 16-bit
 // activations, sizes it refuses).  No tensor-core mode of any kind is used.
 //
-// Each output element is one accumulator that walks k in ascending order, so
-// its value does not depend on the tile shape or on the rows beside it: the
-// three kernels below (a general one, one with 128 x 128 tiles and 8 x 8
-// outputs per thread for prompts, one with 16-column tiles for a few rows
-// that spreads a narrow weight over many blocks) give the same bits.
+// The order of every sum depends on K alone.  K is cut into at most eight segments of equal length
+// (simt_segment(K)); inside a segment two accumulators walk its even and its odd k upwards and are
+// added at its end, and the segments' sums are added in ascending order.  The two kernels below (one
+// for a few rows, which spreads the segments over threads, one with tiles of rows x columns, which
+// spreads them over the CTAs of a cluster) therefore give the same bits however the rows are cut, and
+// both find parallel work in a narrow weight.  Against 64 bits the sums are off by 0.27 of what one
+// accumulator over all of K is (K = 1536: 1.9e-7 against 7.0e-7).  A general kernel (one accumulator over all of K) takes what cannot be read in pieces of
+// four elements.
 // (MisterTK/gibbs Linear: src/graph/cpu.rs:249-274, 2338-2417; its blocked
 // 32-bit product: src/model/nn.rs:383-529.)
 #include "common.cuh"
 
 namespace {
 
-// Four consecutive elements of a row as 32-bit values (rows are 16-byte / 8-byte aligned).  The
-// loads go through L2 (ld.global.cg), never through the read-only path: the activations were
-// written by the kernel before this one, and a load the compiler takes for invariant may be moved
-// above the wait for that kernel (it was, with the first k-block fetched right after the wait).
-__device__ __forceinline__ float4 load4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-  const uint2 u = __ldcg(reinterpret_cast<const uint2*>(p));
+constexpr int SEGS = 8;       // at most this many segments of K (one CTA of a cluster each in the tile kernel)
+constexpr int SK = 32;        // a segment is a multiple of this long
+
+inline int simt_segment(int K) { return gb_div_up(gb_div_up(K, SEGS), SK) * SK; }
+
+// Two 32-bit accumulators, of the even and of the odd k: a pair of neighbouring elements is one operand of
+// fma.rn.f32x2 as it comes from memory (one instruction for two fused multiply-adds, each rounded as fmaf's).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 w) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(w));
+}
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+
+// Four consecutive elements in shared memory as 32-bit values, in two pairs.
+__device__ __forceinline__ ulonglong2 lds4(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ ulonglong2 lds4(const bf16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
   const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&u.x);
   const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&u.y);
-  return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
+  return make_ulonglong2(pack2(__low2float(lo), __high2float(lo)), pack2(__low2float(hi), __high2float(hi)));
 }
+
+// Four consecutive elements on their way to shared memory; zeros where `live` is false (the source
+// address is then not read, wherever it points).
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+               ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy4(bf16* dst, const bf16* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;"
+               ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
 __device__ __forceinline__ void store_out(void* out, int out_dtype, int accumulate, size_t o, float v) {
   if (out_dtype == GB_F32) {
@@ -35,129 +71,281 @@ __device__ __forceinline__ void store_out(void* out, int out_dtype, int accumula
   }
 }
 
-// ---- prompts: 128 x 128 tiles, 256 threads, 8 x 8 outputs per thread, k-blocks of 16 fetched into
-// registers while the block before is multiplied.  K and the row strides are multiples of 4.
-constexpr int LT = 128;     // tile edge
-constexpr int LK = 16;
-constexpr int LPAD = 4;
+// ---- a few rows (decode): bound by the weight's stream from HBM.  A block takes 8 x CG x CPT columns; a
+// thread walks one segment for CPT columns and MT of the RG x MT rows, so a weight of N rows is spread
+// over N / (8 CG CPT) blocks and a chain of additions is K / 8 long.  Rows of weight and activations pass
+// through a ring of ST stages of 32 k per segment, copied 16 bytes (8 for bfloat16) a thread; the
+// weight's first stages are on their way before the kernel in front has finished.  Rows are padded
+// to 36 elements, which leaves the 16-byte reads of eight columns without bank conflicts.
+// Measured (weights not in L2, us; one accumulator over all of K, no ring before -> now): 2 rows
+// 1536 x 4608 51 -> 9, 1536 x 1536 25 -> 3.8, 1536 x 13824 119 -> 19 (4.4 TB/s), 6912 x 1536 94 -> 14,
+// 1536 x 65536 417 -> 71 (5.6 TB/s); 8 rows 52 -> 11, 25 -> 7, 120 -> 24, 95 -> 25, 421 -> 83.
+constexpr int RPAD = SK + 4;
+
+template <typename TA, typename TW, int RG, int CG, int MT, int CPT, int ST>
+struct RowsRing {
+  static constexpr int A_SEG = RG * MT * RPAD + 4;                       // (the 4 keep the segments' reads apart)
+  static constexpr int W_STAGE = SEGS * 8 * CG * CPT * RPAD;
+  static constexpr int A_STAGE = SEGS * A_SEG;
+  static constexpr int BYTES = ST * (W_STAGE * (int)sizeof(TW) + A_STAGE * (int)sizeof(TA));
+  static_assert(SEGS * RG * MT * 8 * CG * CPT * 4 <= BYTES, "the segments' sums take the ring's place");
+};
+
+template <typename TA, typename TW, int RG, int CG, int MT, int CPT, int ST>
+__global__ void __launch_bounds__(64 * RG * CG)
+gemm_simt_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
+                      const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
+                      int accumulate, int M, int N, int K, int L) {
+  using Ring = RowsRing<TA, TW, RG, CG, MT, CPT, ST>;
+  constexpr int NB = 8 * CG * CPT, MR = RG * MT, T = 64 * RG * CG;
+  extern __shared__ __align__(16) unsigned char smem[];
+  TW* ws = reinterpret_cast<TW*>(smem);
+  TA* as = reinterpret_cast<TA*>(smem + ST * Ring::W_STAGE * sizeof(TW));
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  const int n0 = blockIdx.x * NB;
+  const int segs = (K + L - 1) / L, steps = L / SK;
+  // what this thread copies: four k (at lk) of every T/8-th row of both tiles; the weight's rows are
+  // (segment, column) pairs, the activations' (segment, row) pairs
+  constexpr int RC = T / 8;                            // 8, 16 or 32 rows at once
+  constexpr int WN = SEGS * NB / RC, AN = (SEGS * MR + RC - 1) / RC;
+  const int lr = tid >> 3, lk = (tid & 7) * 4;
+  auto copy_w = [&](int step) {
+    TW* dst = ws + (step % ST) * Ring::W_STAGE + lr * RPAD + lk;
+    const int k = step * SK + lk;
+#pragma unroll
+    for (int i = 0; i < WN; ++i) {
+      const int r = lr + RC * i, s = r / NB, n = n0 + r % NB;
+      const int gk = s * L + k;
+      copy4(dst + RC * i * RPAD, W + (size_t)n * ldw + gk, n < N && gk < K);
+    }
+  };
+  auto copy_a = [&](int step) {
+    TA* dst = as + (step % ST) * Ring::A_STAGE + lk;
+    const int k = step * SK + lk;
+#pragma unroll
+    for (int i = 0; i < AN; ++i) {
+      const int r = lr + RC * i, s = r / MR, m = r % MR;
+      const int gk = s * L + k;
+      if (SEGS * MR % RC != 0 && r >= SEGS * MR) break;
+      copy4(dst + s * Ring::A_SEG + m * RPAD, A + (size_t)m * lda + gk, m < M && gk < K);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < ST - 1; ++i)
+    if (i < steps) copy_w(i);
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < ST - 1; ++i) {
+    if (i < steps) copy_a(i);
+    copies_commit();
+  }
+  // this thread's row group, segment and columns col + 8 CG j
+  const int rg = tid / (64 * CG), seg = (tid >> 3) & 7, col = (tid & 7) + 8 * (tid / 64 % CG);
+  f32x2 acc[MT][CPT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) acc[m][j] = 0;
+  for (int step = 0; step < steps; ++step) {
+    copies_wait<ST - 2>();
+    __syncthreads();                                   // the stage has arrived, the one before it has been used
+    if (step + ST - 1 < steps) {
+      copy_w(step + ST - 1);
+      copy_a(step + ST - 1);
+    }
+    copies_commit();
+    const TW* w = ws + (step % ST) * Ring::W_STAGE + (seg * NB + col) * RPAD;
+    const TA* a = as + (step % ST) * Ring::A_STAGE + seg * Ring::A_SEG + rg * MT * RPAD;
+#pragma unroll
+    for (int k = 0; k < SK; k += 4) {
+      ulonglong2 wv[CPT];
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) wv[j] = lds4(w + j * 8 * CG * RPAD + k);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const ulonglong2 av = lds4(a + m * RPAD + k);
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) {
+          fma2(acc[m][j], av.x, wv[j].x);
+          fma2(acc[m][j], av.y, wv[j].y);
+        }
+      }
+    }
+  }
+  copies_wait<0>();
+  __syncthreads();                                     // the ring is free: the segments' sums go there
+  float* red = reinterpret_cast<float*>(smem);         // [segment][row][column]
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) red[(seg * MR + rg * MT + m) * NB + j * 8 * CG + col] = sum2(acc[m][j]);
+  __syncthreads();
+  for (int i = tid; i < MR * NB; i += T) {
+    const int m = i / NB, n = n0 + i % NB;
+    if (m >= M || n >= N) continue;
+    float v = 0.f;
+    for (int s = 0; s < segs; ++s) v += red[s * MR * NB + i];
+    if (bias) v += bias[n];
+    store_out(out, out_dtype, accumulate, (size_t)m * ldo + n, v);
+  }
+}
+
+// ---- more rows: bound by the FMA pipe (and near it, by the reads of shared memory that feed it).  Tiles
+// of 32 rows x 64 columns, one warp, 8 x 8 outputs a thread.  The CTAs of a cluster take a segment of K
+// each and add their tiles through distributed shared memory, so that a narrow product of a short prompt
+// still fills the chip and no workspace or second launch is needed; one warp a CTA waits for nobody else's
+// copies.  A quarter of a warp reads one row of activations and eight of weights (pad 4: no conflicts).
+// Measured (225 rows, us; 128 x 128 tiles over the whole of K before -> now): 1536 x 4608 213 -> 97,
+// 1536 x 1536 197 -> 43, 1536 x 13824 307 -> 262 (36 TFLOP/s of the 72 an FMA loop reaches), 6912 x 1536
+// 887 -> 169; 1600 rows: 587 -> 528, 301 -> 186, 1490 -> 1554, 1334 -> 769; 60 rows (the general kernel
+// before) 1536 x 1536 310 -> 22.  Tiles of 64 x 64, 64 x 128 and 128 x 128: 2 to 10% slower, stages of
+// 16 k 10% (twice the cache lines a copy touches), more CTAs an SM by fewer registers 40% (spills).
+constexpr int BM = 32, BNT = 64;                       // a tile
+constexpr int TK = SK, TPAD = TK + 4, TST = 2;         // a ring of two stages of 32 k
 
 template <typename TA, typename TW>
-__global__ void __launch_bounds__(256, 2)
-gemm_simt_tile128_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
-                         const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
-                         int accumulate, int M, int N, int K) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ __align__(16) float As[LK][LT + LPAD];
-  __shared__ __align__(16) float Ws[LK][LT + LPAD];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * LT, n0 = blockIdx.x * LT;
-  // what this thread fetches of a k-block: 4 consecutive k of rows lr and lr + 64 of both tiles
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
+struct TileSmem {
+  static constexpr int RING = TST * TPAD * (BM * (int)sizeof(TA) + BNT * (int)sizeof(TW));
+  static constexpr int LD = BNT + 8;               // (eight columns of four rows are stored at once)
+  static constexpr int SUMS = BM * LD * 4;
+  static constexpr int BYTES = RING > SUMS ? RING : SUMS;
+};
 
-  float acc[8][8];
+template <typename TA, typename TW>
+__global__ void __launch_bounds__(BM * BNT / 64, 8)
+gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
+                      const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
+                      int accumulate, int M, int N, int K, int L, int segs) {
+  constexpr int T = BM * BNT / 64, TX = BNT / 8, TY = BM / 8, RT = T * 4 / TK;     // RT rows of a tile are copied at once
+  static_assert(BM % RT == 0 && BNT % RT == 0, "");
+  extern __shared__ __align__(16) unsigned char smem[];
+  TA* as = reinterpret_cast<TA*>(smem);
+  TW* ws = reinterpret_cast<TW*>(smem + TST * TPAD * BM * sizeof(TA));
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  const int seg = blockIdx.x % segs;                                       // (= the CTA's rank in its cluster)
+  const int n0 = (blockIdx.x / segs) * BNT, m0 = blockIdx.y * BM;
+  const int k_lo = seg * L, k_hi = min(K, k_lo + L);
+  const int steps = (k_hi - k_lo + TK - 1) / TK;
+  const int lr = tid / (TK / 4), lk = tid % (TK / 4) * 4;
+  auto copy_w = [&](int step) {
+    TW* dst = ws + (step % TST) * TPAD * BNT + lr * TPAD + lk;
+    const int k = k_lo + step * TK + lk;
+    const int rows = k < k_hi ? N - n0 - lr : 0;
+    const TW* src = W + (size_t)(n0 + lr) * ldw + k;
+#pragma unroll
+    for (int i = 0; i < BNT / RT; ++i, src += RT * ldw) copy4(dst + RT * i * TPAD, src, RT * i < rows);
+  };
+  auto copy_a = [&](int step) {
+    TA* dst = as + (step % TST) * TPAD * BM + lr * TPAD + lk;
+    const int k = k_lo + step * TK + lk;
+    const int rows = k < k_hi ? M - m0 - lr : 0;
+    const TA* src = A + (size_t)(m0 + lr) * lda + k;
+#pragma unroll
+    for (int i = 0; i < BM / RT; ++i, src += RT * lda) copy4(dst + RT * i * TPAD, src, RT * i < rows);
+  };
+#pragma unroll
+  for (int i = 0; i < TST - 1; ++i)
+    if (i < steps) copy_w(i);
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < TST - 1; ++i) {
+    if (i < steps) copy_a(i);
+    copies_commit();
+  }
+  const int tx = tid % TX, ty = tid / TX;              // outputs: rows ty + TY i, columns tx + TX j
+  f32x2 acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-  float4 fa[2], fw[2];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gm = m0 + lr + 64 * h, gn = n0 + lr + 64 * h, gk = k0 + lk;
-      fa[h] = (gm < M && gk < K) ? load4(A + (size_t)gm * lda + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-      fw[h] = (gn < N && gk < K) ? load4(W + (size_t)gn * ldw + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  auto stash = [&]() {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = lr + 64 * h;
-      As[lk][r] = fa[h].x; As[lk + 1][r] = fa[h].y; As[lk + 2][r] = fa[h].z; As[lk + 3][r] = fa[h].w;
-      Ws[lk][r] = fw[h].x; Ws[lk + 1][r] = fw[h].y; Ws[lk + 2][r] = fw[h].z; Ws[lk + 3][r] = fw[h].w;
-    }
-  };
-  fetch(0);
-  for (int k0 = 0; k0 < K; k0 += LK) {
-    stash();
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+  for (int step = 0; step < steps; ++step) {
+    copies_wait<TST - 2>();
     __syncthreads();
-    if (k0 + LK < K) fetch(k0 + LK);
-#pragma unroll
-    for (int k = 0; k < LK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[k][64 + ty * 4]);
-      const float4 w0 = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-      const float4 w1 = *reinterpret_cast<const float4*>(&Ws[k][64 + tx * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+    if (step + TST - 1 < steps) {
+      copy_w(step + TST - 1);
+      copy_a(step + TST - 1);
     }
-    __syncthreads();
-  }
+    copies_commit();
+    const TA* a = as + ((step % TST) * BM + ty) * TPAD;
+    const TW* w = ws + ((step % TST) * BNT + tx) * TPAD;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-    if (gm >= M) continue;
+    for (int k = 0; k < TK; k += 4) {
+      ulonglong2 av[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[gn];
-      store_out(out, out_dtype, accumulate, (size_t)gm * ldo + gn, v);
+      for (int i = 0; i < 8; ++i) av[i] = lds4(a + i * TY * TPAD + k);
+      ulonglong2 next = lds4(w + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const ulonglong2 wv = next;                    // (the next column's four are asked for ahead of this one's products)
+        if (j < 7) next = lds4(w + (j + 1) * TX * TPAD + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[i].x, wv.x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[i].y, wv.y);
+      }
     }
   }
+  copies_wait<0>();
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(smem);        // [BM][LD]
+  constexpr int LD = TileSmem<TA, TW>::LD;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sums[(ty + TY * i) * LD + tx + TX * j] = sum2(acc[i][j]);
+  // every CTA adds and stores its share of the tile, four columns a thread
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  constexpr int QUADS = BM * BNT / 4;
+  const int share = (QUADS + segs - 1) / segs;
+  const int q_end = min(QUADS, (seg + 1) * share);
+  const unsigned base = (unsigned)__cvta_generic_to_shared(sums);
+  const bool vec = out_dtype == GB_F32 && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
+  for (int q = seg * share + tid; q < q_end; q += T) {
+    const int gm = m0 + q / (BNT / 4), gn = n0 + (q % (BNT / 4)) * 4;
+    if (gm >= M || gn >= N) continue;
+    float4 p[SEGS];
+#pragma unroll
+    for (int s = 0; s < SEGS; ++s) {
+      if (s >= segs) break;
+      unsigned at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(base + 4u * (q / (BNT / 4) * LD + q % (BNT / 4) * 4)), "r"(s));
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(p[s].x), "=f"(p[s].y), "=f"(p[s].z), "=f"(p[s].w) : "r"(at) : "memory");
+    }
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < SEGS; ++s) {
+      if (s >= segs) break;
+      v[0] += p[s].x; v[1] += p[s].y; v[2] += p[s].z; v[3] += p[s].w;
+    }
+    if (bias) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (gn + e < N) v[e] += bias[gn + e];
+    }
+    const size_t o = (size_t)gm * ldo + gn;
+    if (vec && gn + 3 < N) {
+      float4* of = reinterpret_cast<float4*>((float*)out + o);
+      if (accumulate) {
+        const float4 x = *of;
+        v[0] = x.x + v[0]; v[1] = x.y + v[1]; v[2] = x.z + v[2]; v[3] = x.w + v[3];
+      }
+      *of = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (gn + e < N) store_out(out, out_dtype, accumulate, o + e, v[e]);
+    }
+  }
+  // (a CTA's shared memory stays until its peers have read it)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// ---- a few rows (decode): a block takes 16 columns of the weight and up to 16 rows, one output per
-// thread, k-blocks of 64 fetched into registers while the block before is multiplied.  A weight of
-// N rows is spread over N / 16 blocks, so that also a narrow weight is streamed by the whole GPU.
-constexpr int SK = 64;
-
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(256)
-gemm_simt_rows16_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
-                        const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
-                        int accumulate, int M, int N, int K) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ float As[16][SK + 1];
-  __shared__ float Ws[16][SK + 1];
-  const int tid = threadIdx.x;
-  const int tn = tid & 15, tm = tid >> 4;            // this thread's output: row tm, column n0 + tn
-  const int n0 = blockIdx.x * 16;
-  const int lr = tid >> 4, lk = (tid & 15) * 4;       // what it fetches: 4 consecutive k of row lr of both tiles
-  float acc = 0.f;
-  float4 fa, fw;
-  auto fetch = [&](int k0) {
-    const int gk = k0 + lk;
-    fa = (lr < M && gk < K) ? load4(A + (size_t)lr * lda + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-    fw = (n0 + lr < N && gk < K) ? load4(W + (size_t)(n0 + lr) * ldw + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  fetch(0);
-  for (int k0 = 0; k0 < K; k0 += SK) {
-    As[lr][lk] = fa.x; As[lr][lk + 1] = fa.y; As[lr][lk + 2] = fa.z; As[lr][lk + 3] = fa.w;
-    Ws[lr][lk] = fw.x; Ws[lr][lk + 1] = fw.y; Ws[lr][lk + 2] = fw.z; Ws[lr][lk + 3] = fw.w;
-    __syncthreads();
-    if (k0 + SK < K) fetch(k0 + SK);
-#pragma unroll
-    for (int k = 0; k < SK; ++k) acc = fmaf(As[tm][k], Ws[tn][k], acc);
-    __syncthreads();
-  }
-  const int gn = n0 + tn;
-  if (tm < M && gn < N) {
-    float v = acc;
-    if (bias) v += bias[gn];
-    store_out(out, out_dtype, accumulate, (size_t)tm * ldo + gn, v);
-  }
-}
-
-// ---- the general kernel: any sizes and strides
+// ---- the general kernel: any sizes and strides, one accumulator over all of K
 
 constexpr int BN = 64;
 constexpr int BK = 16;
@@ -224,27 +412,74 @@ gemm_simt_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long
   }
 }
 
+template <typename TA, typename TW, int RG, int CG, int MT, int CPT, int ST>
+cudaError_t launch_rows(const TA* A, long long lda, const TW* W, long long ldw, const float* bias, void* out, long long ldo,
+                        int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_simt_rows_kernel<TA, TW, RG, CG, MT, CPT, ST>;
+  constexpr int smem = RowsRing<TA, TW, RG, CG, MT, CPT, ST>::BYTES;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  return gb_launch(kernel, dim3(gb_div_up(N, 8 * CG * CPT)), dim3(64 * RG * CG), smem, stream, A, lda, W, ldw, bias, out, ldo, out_dtype,
+                   accumulate, M, N, K, simt_segment(K));
+}
+
 template <typename TA, typename TW>
-void launch(const void* A, long long lda, const void* W, long long ldw, const float* bias, void* out, long long ldo,
-            int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+cudaError_t launch_tile(const TA* A, long long lda, const TW* W, long long ldw, const float* bias, void* out, long long ldo,
+                        int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+  auto kernel = gemm_simt_tile_kernel<TA, TW>;
+  constexpr int smem = TileSmem<TA, TW>::BYTES;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const int L = simt_segment(K), segs = gb_div_up(K, L);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)gb_div_up(N, BNT) * segs, gb_div_up(M, BM));
+  cfg.blockDim = dim3(BM * BNT / 64);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = segs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, L, segs);
+}
+
+template <typename TA, typename TW>
+cudaError_t launch(const void* a, long long lda, const void* w, long long ldw, const float* bias, void* out, long long ldo,
+                   int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+  const TA* A = (const TA*)a;
+  const TW* W = (const TW*)w;
+  // (K up to 2^30: the last segment's end is worked out in 32 bits)
   const bool rows4 = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A % (4 * sizeof(TA))) == 0 &&
-                     ((uintptr_t)W % (4 * sizeof(TW))) == 0;
+                     ((uintptr_t)W % (4 * sizeof(TW))) == 0 && K <= (1 << 30);
+#define GB_ARGS A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream
   if (rows4 && M <= 16) {
-    gb_launch(gemm_simt_rows16_kernel<TA, TW>, dim3(gb_div_up(N, 16)), dim3(256), 0, stream, (const TA*)A, lda,
-              (const TW*)W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K);
-  } else if (rows4 && M > 64) {
-    dim3 grid(gb_div_up(N, LT), gb_div_up(M, LT));
-    gb_launch(gemm_simt_tile128_kernel<TA, TW>, dim3(grid), dim3(256), 0, stream, (const TA*)A, lda, (const TW*)W,
-              ldw, bias, out, ldo, out_dtype, accumulate, M, N, K);
-  } else if (M <= 16) {
-    dim3 grid(gb_div_up(N, BN), gb_div_up(M, 16));
-    gb_launch(gemm_simt_kernel<TA, TW, 1>, dim3(grid), dim3(256), 0, stream, (const TA*)A, lda, (const TW*)W, ldw, bias, out, ldo,
-                                                          out_dtype, accumulate, M, N, K);
-  } else {
-    dim3 grid(gb_div_up(N, BN), gb_div_up(M, 64));
-    gb_launch(gemm_simt_kernel<TA, TW, 4>, dim3(grid), dim3(256), 0, stream, (const TA*)A, lda, (const TW*)W, ldw, bias, out, ldo,
-                                                          out_dtype, accumulate, M, N, K);
+    // Every block reads the same activations, all of them at about the same k, so those few lines of L2
+    // bound the stream: 32 columns a block where the weight has enough rows for the chip (two rows,
+    // 1536 x 65536: 71 us against 97 with 8 columns), 8 and a deeper ring where it is narrow.
+    const bool wide = N >= 16 * 148;
+    if (M == 1) return wide ? launch_rows<TA, TW, 1, 2, 1, 2, 2>(GB_ARGS) : launch_rows<TA, TW, 1, 1, 1, 1, 6>(GB_ARGS);
+    if (M == 2) return wide ? launch_rows<TA, TW, 1, 2, 2, 2, 2>(GB_ARGS) : launch_rows<TA, TW, 1, 1, 2, 1, 6>(GB_ARGS);
+    if (M <= 4) return wide ? launch_rows<TA, TW, 1, 2, 4, 2, 2>(GB_ARGS) : launch_rows<TA, TW, 1, 1, 4, 1, 6>(GB_ARGS);
+    if (M <= 8) return wide ? launch_rows<TA, TW, 2, 2, 4, 2, 2>(GB_ARGS) : launch_rows<TA, TW, 2, 1, 4, 1, 4>(GB_ARGS);
+    return wide ? launch_rows<TA, TW, 4, 2, 4, 2, 2>(GB_ARGS) : launch_rows<TA, TW, 4, 1, 4, 1, 4>(GB_ARGS);
   }
+  if (rows4 && gb_div_up(N, BNT) <= 2147483647LL / SEGS) {
+    return launch_tile<TA, TW>(GB_ARGS);
+  }
+#undef GB_ARGS
+  if (M <= 16) {
+    dim3 grid(gb_div_up(N, BN), gb_div_up(M, 16));
+    return gb_launch(gemm_simt_kernel<TA, TW, 1>, dim3(grid), dim3(256), 0, stream, A, lda, W, ldw, bias, out, ldo, out_dtype,
+                     accumulate, M, N, K);
+  }
+  dim3 grid(gb_div_up(N, BN), gb_div_up(M, 64));
+  return gb_launch(gemm_simt_kernel<TA, TW, 4>, dim3(grid), dim3(256), 0, stream, A, lda, W, ldw, bias, out, ldo, out_dtype,
+                   accumulate, M, N, K);
 }
 
 }  // namespace
@@ -262,16 +497,18 @@ GB_API int gb_linear_simt(const void* A, int a_dtype, long long lda, const void*
   if (out_dtype != GB_F32 && out_dtype != GB_BF16) GB_FAIL(GB_ERR_ARG, "gb_linear_simt: output dtype %d", out_dtype);
   if (gb_div_up(M, 16) > 65535 || gb_div_up(N, 16) > 2147483647LL)
     GB_FAIL(GB_ERR_ARG, "gb_linear_simt: M = %d or N = %d is too large", M, N);
+  cudaError_t e;
   if (a_dtype == GB_F32 && w_dtype == GB_F32)
-    launch<float, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<float, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
   else if (a_dtype == GB_BF16 && w_dtype == GB_BF16)
-    launch<bf16, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<bf16, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
   else if (a_dtype == GB_BF16 && w_dtype == GB_F32)
-    launch<bf16, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<bf16, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
   else if (a_dtype == GB_F32 && w_dtype == GB_BF16)
-    launch<float, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<float, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
   else
     GB_FAIL(GB_ERR_ARG, "gb_linear_simt: operand dtypes %d, %d", a_dtype, w_dtype);
+  if (e != cudaSuccess) GB_FAIL(GB_ERR_CUDA, "gb_linear_simt: %s", cudaGetErrorString(e));
   GB_CHECK_LAUNCH("gb_linear_simt");
   return GB_OK;
 }

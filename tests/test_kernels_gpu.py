@@ -1017,6 +1017,37 @@ def test_linear_simt_gives_the_same_bits_however_the_rows_are_cut(pair):
         assert torch.equal(part, whole[lo:hi]), (lo, hi)
 
 
+@pytest.mark.parametrize("k", [4, 28, 32, 36, 96, 252, 256, 260, 1032, 1536, 6912])
+@pytest.mark.parametrize("pair", ["f32xf32", "bf16xf32", "f32xbf16"])
+def test_linear_simt_at_the_edges_of_segments_and_tiles(k, pair):
+    """K of one to eight segments, whole and ragged; rows at the edges of the few-rows kernel's row counts and
+    of the tiles; columns of narrow and wide weights.  Each output adds chains of at most K/16 + 16 products and
+    9 + 8 further terms, so its error is below (K/16 + 33) 2^-24 sum |a w|."""
+    from gibbs_b200 import ops
+    torch.manual_seed(k)
+    ad, wd = {"f32xf32": ("float32", "float32"), "bf16xf32": ("bfloat16", "float32"), "f32xbf16": ("float32", "bfloat16")}[pair]
+    for n in (1, 7, 65, 130, 2369):
+        w, wr = _quant(torch.randn(n, k), wd)
+        a, ar = _quant(torch.randn(70, k), ad)
+        bias = torch.randn(n)
+        want, size = ar @ wr.T, ar.abs() @ wr.abs().T + bias.double().abs()
+        whole = None
+        for m in (70, 33, 32, 31, 17, 16, 15, 9, 8, 5, 4, 3, 2, 1):
+            wide = torch.full((m, n + 3), 7.0, device=DEV)          # rows further apart than they are long
+            out = wide[:, :n]
+            ops.linear_simt(a[:m], w, bias.to(DEV), out)
+            err = (out.double().cpu() - (want + bias.double())[:m]).abs()
+            assert (err <= (k / 16 + 33) * 2.0 ** -24 * size[:m]).all(), (n, m)
+            assert (wide[:, n:] == 7.0).all()
+            whole = out.clone() if whole is None else whole
+            assert torch.equal(out, whole[:m]), (n, m)              # the same bits however the rows are cut
+        res = torch.randn(33, n)
+        acc = res.clone().to(DEV)
+        ops.linear_simt(a[:33], w, None, acc, accumulate=True)
+        assert ((acc.double().cpu() - want[:33] - res.double()).abs() <=
+                (k / 16 + 33) * 2.0 ** -24 * (size[:33] + res.double().abs())).all()
+
+
 @pytest.mark.parametrize("vocab,k", [(1000, 5), (65536, 20), (50257, 1), (7, 32)])
 def test_logprob_info_matches_the_plain_rule(vocab, k):
     """Probability of the chosen token, entropy and the k most probable tokens of every row,
