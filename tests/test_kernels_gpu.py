@@ -1048,6 +1048,48 @@ def test_linear_simt_at_the_edges_of_segments_and_tiles(k, pair):
                 (k / 16 + 33) * 2.0 ** -24 * (size[:33] + res.double().abs())).all()
 
 
+@pytest.mark.parametrize("hd,group", [(4, 1), (12, 3), (32, 5), (36, 4), (64, 3), (100, 2), (128, 1), (192, 8), (256, 9)])
+def test_float32_attention_at_the_edges_of_tiles_and_warps(hd, group):
+    """Contexts at the edges of key tiles and of a round of all warps' tiles, windows and soft caps.  A score is off
+    by at most d = (hd + 4) 2^-24 scale |q|.|k|, so a weight by a factor of exp(2 d + 2^-21) at most (expf: 2 units
+    in the last place, twice); the weighted sum adds (keys/8 + 40) 2^-24."""
+    from gibbs_b200 import ops
+    torch.manual_seed(hd)
+    kvh, ps, n_pages = 2, 16, 140
+    heads = kvh * group
+    kp, vp = torch.randn(n_pages, kvh, ps, hd), torch.randn(n_pages, kvh, ps, hd)
+    pages = torch.randperm(n_pages)[:130]
+    pos = [0, 1, 30, 31, 32, 33, 127, 128, 255, 256, 257, 511, 700, 2049]
+    q = torch.randn(len(pos), heads * hd)
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    bt = pages.to(torch.int32)[None, :].to(DEV)
+    scale = hd ** -0.5
+    for window, cap in ((0, 0.0), (33, 0.0), (300, 0.0), (0, 2.0)):
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        out = torch.empty(len(pos), heads * hd, device=DEV)
+        kpd, vpd, qd = kp.to(DEV), vp.to(DEV), q.to(DEV)
+        ops.paged_attention(qd, heads, kvh, hd, kpd, vpd, bt, t([0] * len(pos)), t(pos), scale, window, out, status, softcap=cap)
+        assert int(status.item()) == 0
+        for i, p in enumerate(pos):
+            lo = max(0, p - window + 1) if window else 0
+            j = torch.arange(lo, p + 1)
+            keys, vals = kp[pages[j // ps], :, j % ps].double(), vp[pages[j // ps], :, j % ps].double()      # [L, kvh, hd]
+            qi = q[i].double().reshape(kvh, group, hd)
+            sc = torch.einsum("ghd,lgd->ghl", qi, keys) * scale
+            d = (hd + 4) * 2.0 ** -24 * scale * torch.einsum("ghd,lgd->ghl", qi.abs(), keys.abs()).amax(-1)
+            if cap:
+                sc, d = cap * torch.tanh(sc / cap), d + 2.0 ** -21 * cap
+            w = torch.softmax(sc, -1)
+            want = torch.einsum("ghl,lgd->ghd", w, vals)
+            size = torch.einsum("ghl,lgd->ghd", w, vals.abs())
+            tol = (2 * (2 * d[..., None] + 2.0 ** -21) + (len(j) / 8 + 40) * 2.0 ** -24) * size
+            got = out[i].double().cpu().reshape(kvh, group, hd)
+            assert ((got - want).abs() <= tol).all(), (window, cap, p)
+            alone = torch.empty(1, heads * hd, device=DEV)
+            ops.paged_attention(qd[i:i + 1], heads, kvh, hd, kpd, vpd, bt, t([0]), t([p]), scale, window, alone, status, softcap=cap)
+            assert torch.equal(alone[0], out[i])
+
+
 @pytest.mark.parametrize("vocab,k", [(1000, 5), (65536, 20), (50257, 1), (7, 32)])
 def test_logprob_info_matches_the_plain_rule(vocab, k):
     """Probability of the chosen token, entropy and the k most probable tokens of every row,
