@@ -209,14 +209,15 @@ struct TileSmem {
   static constexpr int RING = TST * TPAD * (BM * (int)sizeof(TA) + BNT * (int)sizeof(TW));
   static constexpr int LD = BNT + 8;               // (eight columns of four rows are stored at once)
   static constexpr int SUMS = BM * LD * 4;
-  static constexpr int BYTES = RING > SUMS ? RING : SUMS;
+  static constexpr int BYTES = RING > SUMS ? RING : SUMS;      // a CTA a segment: the sums take the ring's place
+  static constexpr int BYTES_WHOLE = RING + SUMS;              // a CTA takes all segments
 };
 
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(BM * BNT / 64, 8)
 gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
                       const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
-                      int accumulate, int M, int N, int K, int L, int segs) {
+                      int accumulate, int M, int N, int K, int L, int segs, int whole) {
   constexpr int T = BM * BNT / 64, TX = BNT / 8, TY = BM / 8, RT = T * 4 / TK;     // RT rows of a tile are copied at once
   static_assert(BM % RT == 0 && BNT % RT == 0, "");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -226,7 +227,7 @@ gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long
   const int tid = threadIdx.x;
   const int seg = blockIdx.x % segs;                                       // (= the CTA's rank in its cluster)
   const int n0 = (blockIdx.x / segs) * BNT, m0 = blockIdx.y * BM;
-  const int k_lo = seg * L, k_hi = min(K, k_lo + L);
+  const int k_lo = seg * L, k_hi = whole ? K : min(K, k_lo + L);
   const int steps = (k_hi - k_lo + TK - 1) / TK;
   const int lr = tid / (TK / 4), lk = tid % (TK / 4) * 4;
   auto copy_w = [&](int step) {
@@ -254,6 +255,8 @@ gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long
     if (i < steps) copy_a(i);
     copies_commit();
   }
+  constexpr int LD = TileSmem<TA, TW>::LD;
+  float* sums = reinterpret_cast<float*>(smem + (whole ? TileSmem<TA, TW>::RING : 0));      // [BM][LD]
   const int tx = tid % TX, ty = tid / TX;              // outputs: rows ty + TY i, columns tx + TX j
   f32x2 acc[8][8];
 #pragma unroll
@@ -286,15 +289,27 @@ gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long
         for (int i = 0; i < 8; ++i) fma2(acc[i][j], av[i].y, wv.y);
       }
     }
+    if (whole && ((step + 1) % (L / TK) == 0 || step + 1 == steps)) {
+      // a segment's end: every thread adds its outputs to its own sums
+      const bool first = step < L / TK;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float* at = sums + (ty + TY * i) * LD + tx + TX * j;
+          *at = (first ? 0.f : *at) + sum2(acc[i][j]);
+          acc[i][j] = 0;
+        }
+    }
   }
   copies_wait<0>();
   __syncthreads();
-  float* sums = reinterpret_cast<float*>(smem);        // [BM][LD]
-  constexpr int LD = TileSmem<TA, TW>::LD;
+  if (!whole) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sums[(ty + TY * i) * LD + tx + TX * j] = sum2(acc[i][j]);
+      for (int j = 0; j < 8; ++j) sums[(ty + TY * i) * LD + tx + TX * j] = sum2(acc[i][j]);
+  }
   // every CTA adds and stores its share of the tile, four columns a thread
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -427,14 +442,17 @@ template <typename TA, typename TW>
 cudaError_t launch_tile(const TA* A, long long lda, const TW* W, long long ldw, const float* bias, void* out, long long ldo,
                         int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
   auto kernel = gemm_simt_tile_kernel<TA, TW>;
-  constexpr int smem = TileSmem<TA, TW>::BYTES;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  const int L = simt_segment(K), segs = gb_div_up(K, L);
+  using Smem = TileSmem<TA, TW>;
+  static_assert(Smem::BYTES_WHOLE <= 48 * 1024, "no more shared memory than every launch may have");
+  const int L = simt_segment(K);
+  // Segments of less than 128 are over before their CTA has started and ended: one CTA takes them all where
+  // the tiles alone fill the chip (2134 rows, 128 x 2048, bfloat16 weights: 55 us against 72).
+  const int whole = L < 128 && (long long)gb_div_up(M, BM) * gb_div_up(N, BNT) >= 4 * 148;
+  const int segs = whole ? 1 : gb_div_up(K, L);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)gb_div_up(N, BNT) * segs, gb_div_up(M, BM));
   cfg.blockDim = dim3(BM * BNT / 64);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = whole ? Smem::BYTES_WHOLE : Smem::BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -445,7 +463,7 @@ cudaError_t launch_tile(const TA* A, long long lda, const TW* W, long long ldw, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, L, segs);
+  return cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, L, segs, whole);
 }
 
 template <typename TA, typename TW>

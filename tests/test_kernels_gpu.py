@@ -1041,6 +1041,10 @@ def test_linear_simt_at_the_edges_of_segments_and_tiles(k, pair):
             assert (wide[:, n:] == 7.0).all()
             whole = out.clone() if whole is None else whole
             assert torch.equal(out, whole[:m]), (n, m)              # the same bits however the rows are cut
+        if k == 260 and n == 2369:                                  # enough tiles for a CTA to take all (short) segments itself
+            many = torch.empty(540, n, device=DEV)
+            ops.linear_simt(torch.cat([a] * 7 + [a[:50]]), w, bias.to(DEV), many)
+            assert torch.equal(many[:70], whole) and torch.equal(many[490:], whole[:50])
         res = torch.randn(33, n)
         acc = res.clone().to(DEV)
         ops.linear_simt(a[:33], w, None, acc, accumulate=True)
