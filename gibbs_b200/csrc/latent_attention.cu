@@ -364,54 +364,50 @@ latent_attention_kernel(const float* qp, const TC* pages, const int* block_table
   }
 }
 
-// One warp per (token, head): the chunks' partial results, merged in chunk order.
+// One block per (token, head): the chunks' partial results, merged in chunk order.  The chunks' weights
+// exp(m_s - M) are worked out once into shared memory; then every thread has its columns and asks for
+// sixteen chunks' values at a time.  Bound by the trips to L2 (weights, then sums).  Measured, 2 tokens x 16 heads,
+// 32 chunks of 512: 6 us in a decode step, 37 to 40 with a warp per (token, head) that took one chunk after the other.
+constexpr int LM_CHUNKS = 64;                              // (gb_latent_attention_chunks gives no more)
+
 __global__ void latent_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate,
-                                              float* out, long long ldo, int n, int H, int r,
-                                              const float* __restrict__ sink) {
+                                              float* out, long long ldo, int H, int r, const float* __restrict__ sink) {
+  __shared__ float es[LM_CHUNKS];
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
-  const long long idx = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (idx >= (long long)n * H) return;
+  const long long idx = blockIdx.x;
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
-  const float* w = ws + (size_t)idx * splits * (r + 2);
-  // the chunks' weights exp(m_s - M) once (lane s for chunk s, 32 chunks at a time), then the columns
-  float M = -INFINITY;
-  for (int s = lane; s < splits; s += 32) M = fmaxf(M, w[(size_t)s * (r + 2)]);
-  M = warp_max(M);
+  const size_t ld = (size_t)r + 2;
+  const float* w = ws + (size_t)idx * splits * ld;
+  // (every warp takes the maxima and denominators for itself: lane s has chunks s and s + 32)
+  const float m0 = lane < splits ? w[lane * ld] : -INFINITY, m1 = lane + 32 < splits ? w[(lane + 32) * ld] : -INFINITY;
+  const float l0 = lane < splits ? w[lane * ld + 1] : 0.f, l1 = lane + 32 < splits ? w[(lane + 32) * ld + 1] : 0.f;
+  float M = warp_max(fmaxf(m0, m1));
   if (sink) M = fmaxf(M, sink[h]);
+  const float e0 = m0 > -INFINITY ? expf(m0 - M) : 0.f, e1 = m1 > -INFINITY ? expf(m1 - M) : 0.f;
+  const float el0 = e0 * l0, el1 = e1 * l1;
   float L = sink ? expf(sink[h] - M) : 0.f;
-  for (int s0 = 0; s0 < splits; s0 += 32) {                // in chunk order
-    const int s = s0 + lane;
-    const float m = s < splits ? w[(size_t)s * (r + 2)] : -INFINITY;
-    const float e = m > -INFINITY ? expf(m - M) : 0.f;
-    const float el = s < splits ? e * w[(size_t)s * (r + 2) + 1] : 0.f;
-    for (int u = 0; u < 32 && s0 + u < splits; ++u) L += __shfl_sync(0xffffffffu, el, u);
+  for (int s = 0; s < splits; ++s) L += __shfl_sync(0xffffffffu, s < 32 ? el0 : el1, s & 31);      // in chunk order
+  if (threadIdx.x < 32) {
+    es[lane] = e0;
+    es[lane + 32] = e1;
   }
+  __syncthreads();
   const float g = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + h]) : 1.f;
   const float inv = g / L;
-  for (int d0 = 0; d0 < r; d0 += 128) {                    // four columns per lane at a time
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s0 = 0; s0 < splits; s0 += 32) {
-      const int s = s0 + lane;
-      const float m = s < splits ? w[(size_t)s * (r + 2)] : -INFINITY;
-      const float e = m > -INFINITY ? expf(m - M) : 0.f;
-      for (int u = 0; u < 32 && s0 + u < splits; ++u) {
-        const float eu = __shfl_sync(0xffffffffu, e, u);
-        if (eu == 0.f) continue;                             // a chunk without keys (the whole warp together)
-        const float* wu = w + (size_t)(s0 + u) * (r + 2) + 2;
+  float* dst = out + (size_t)t * ldo + (size_t)h * r;
+  for (int d = threadIdx.x; d < r; d += blockDim.x) {
+    float a = 0.f;
+    for (int s0 = 0; s0 < splits; s0 += 16) {
+      float v[16];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int d = d0 + lane + 32 * v;
-          if (d < r) a[v] = fmaf(eu, wu[d], a[v]);
-        }
-      }
-    }
+      for (int u = 0; u < 16; ++u) v[u] = s0 + u < splits && es[s0 + u] != 0.f ? ldcg_now(w + (s0 + u) * ld + 2 + d) : 0.f;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int d = d0 + lane + 32 * v;
-      if (d < r) out[(size_t)t * ldo + (size_t)h * r + d] = a[v] * inv;
+      for (int u = 0; u < 16; ++u)
+        if (s0 + u < splits && es[s0 + u] != 0.f) a = fmaf(es[s0 + u], v[u], a);      // (a chunk without keys left no sum)
     }
+    dst[d] = a * inv;
   }
 }
 
@@ -428,6 +424,24 @@ int gb_latent_attention_tc_launch(const float* qp, const bf16* pages, const int*
                                   const float* gate, long long ld_gate, float* out, long long ldo, int n, int R, int H, int r,
                                   int dr, float scale, const float* sink, float* ws, long long ws_rows, int* status,
                                   cudaStream_t stream);
+
+bool gb_latent_attention_split_takes(int n, int R, int H, int r, int dr, bool pages_bf16, const void* pages, const void* qp,
+                                     const void* out, long long ldo);
+cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages, const int* block_table, int bt_stride,
+                                             int page_size, int n_pages, const int* tok_req, const int* tok_pos,
+                                             const int* q_start, const float* gate, long long ld_gate, float* out,
+                                             long long ldo, int n, int R, int H, int r, int dr, float scale, int window,
+                                             const float* sink, float* ws, int splits, int chunk, int* status,
+                                             cudaStream_t stream);
+
+// The second of a launch's two kernels where the keys were cut: 2 (kernels launched), or a failure's code.
+static int launch_merge(const float* ws, int splits, const float* gate, long long ld_gate, float* out, long long ldo, int n,
+                        int H, int r, const float* sink, cudaStream_t stream) {
+  gb_launch(latent_attention_merge_kernel, dim3((unsigned)((long long)n * H)), dim3(r <= 128 ? 128 : r <= 256 ? 256 : 512), 0,
+            stream, ws, splits, gate, ld_gate, out, ldo, H, r, sink);
+  GB_CHECK_LAUNCH("latent_attention_merge");
+  return 2;
+}
 
 // How the visible keys of a launch are cut into chunks of whole key tiles: (chunks, keys per chunk).
 // Few tokens (decoding) get many chunks, so that the GPU is occupied; a launch with enough (token, head
@@ -533,11 +547,8 @@ GB_OP(gb_op_latent_attention) {
     if (parts >= 1) {
       GB_CHECK_LAUNCH("latent_attention (tensor cores)");
       if (parts == 1) return 1;
-      gb_launch(latent_attention_merge_kernel, dim3(gb_div_up((long long)n * H, 4)), dim3(128), 0, ctx->stream,
-                op_ptr<const float>(a[19]), parts, op_ptr<const float>(a[9]), a[10], op_ptr<float>(a[11]), a[12], n, H, r,
-                op_ptr<const float>(a[20]));
-      GB_CHECK_LAUNCH("latent_attention_merge");
-      return 2;
+      return launch_merge(op_ptr<const float>(a[19]), parts, op_ptr<const float>(a[9]), a[10], op_ptr<float>(a[11]), a[12], n,
+                          H, r, op_ptr<const float>(a[20]), ctx->stream);
     }
   }
   if (r > 512) GB_FAIL(GB_ERR_ARG, "latent_attention: latent size %d (at most 512)", r);
@@ -548,6 +559,28 @@ GB_OP(gb_op_latent_attention) {
   int splits = gb_latent_attention_chunks(n, H, (int)a[17], (int)a[18], &chunk);
   float* ws = op_ptr<float>(a[19]);
   if (ws == nullptr || (long long)n * H * splits > gb_latent_attention_workspace_rows()) splits = 1;
+  // bfloat16 pages, a window or single tokens: tensor cores with whole queries and weights (latent_attention_tc.cu).
+  // Measured at 16 heads, 512 + 64 entries, window 1024, portions of 1801 and 333 tokens: 0.9 ms against 4.5 on the kernel
+  // below; one token each: 14 us against 38.
+  if (a[22] && gb_latent_attention_split_takes(n, (int)a[21], H, r, dr, a[2] == GB_BF16, op_ptr<const void>(a[1]),
+                                               op_ptr<const void>(a[0]), op_ptr<const void>(a[11]), a[12])) {
+    if (n > (int)a[21] && splits > 1) {
+      // portions: a row tile's keys span its tokens' positions and the window in front of the first
+      const int span = a[17] > 0 ? (int)(a[17] < a[18] ? a[17] : a[18]) + gb_div_up(32, H) : (int)a[18];
+      chunk = 32 * gb_div_up(gb_div_up(span, splits), 32);
+      splits = gb_div_up(span, chunk);
+    }
+    const cudaError_t e = gb_latent_attention_split_launch(
+        op_ptr<const float>(a[0]), op_ptr<const bf16>(a[1]), op_ptr<const int>(a[3]), (int)a[4], (int)a[5], (int)a[6],
+        op_ptr<const int>(a[7]), op_ptr<const int>(a[8]), op_ptr<const int>(a[22]), op_ptr<const float>(a[9]), a[10],
+        op_ptr<float>(a[11]), a[12], n, (int)a[21], H, r, dr, (float)f[0], (int)a[17], op_ptr<const float>(a[20]), ws, splits,
+        chunk, ctx->status, ctx->stream);
+    if (e != cudaSuccess) GB_FAIL(GB_ERR_CUDA, "latent_attention: %s", cudaGetErrorString(e));
+    GB_CHECK_LAUNCH("latent_attention (tensor cores, whole weights)");
+    if (splits == 1) return 1;
+    return launch_merge(ws, splits, op_ptr<const float>(a[9]), a[10], op_ptr<float>(a[11]), a[12], n, H, r,
+                        op_ptr<const float>(a[20]), ctx->stream);
+  }
   // (fewer heads than a block has room for: fewer warps, so that none idles through the key tiles)
   const int warps = H >= LA_HB ? LA_WARPS : (gb_div_up(H, LA_HW) < 2 ? 2 : gb_div_up(H, LA_HW));
   const dim3 grid(n, gb_div_up(H, LA_HB), splits), block(32 * warps);
@@ -573,8 +606,6 @@ GB_OP(gb_op_latent_attention) {
 #undef LA
   GB_CHECK_LAUNCH("latent_attention");
   if (splits == 1) return 1;
-  gb_launch(latent_attention_merge_kernel, dim3(gb_div_up((long long)n * H, 4)), dim3(128), 0, ctx->stream, ws, splits,
-            op_ptr<const float>(a[9]), a[10], op_ptr<float>(a[11]), a[12], n, H, r, op_ptr<const float>(a[20]));
-  GB_CHECK_LAUNCH("latent_attention_merge");
-  return 2;
+  return launch_merge(ws, splits, op_ptr<const float>(a[9]), a[10], op_ptr<float>(a[11]), a[12], n, H, r,
+                      op_ptr<const float>(a[20]), ctx->stream);
 }

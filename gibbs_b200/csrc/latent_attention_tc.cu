@@ -15,8 +15,8 @@
 //  (p = hi + lo), so 16 bits of every weight count.  A learned sink per head joins the denominator at the end; an
 //  optional gate multiplies the result.  With `splits` 2 (a step of few tiles: one long prompt) the key tiles of
 //  every row tile are cut in two halves for two CTAs, which leave (maximum, sum, weighted sum) per row for the merge
-//  kernel of latent_attention.cu, and the row tiles with the most keys are launched first.  Causal, no window: what has one runs on the generic kernel, as do 32-bit
-//  pages and steps of single tokens.  Rows in shared memory lie `stride` entries apart: the row's length rounded up
+//  kernel of latent_attention.cu, and the row tiles with the most keys are launched first.  Causal, no window: what has one runs
+//  on the second kernel below, as do steps of single tokens; 32-bit pages run on the generic kernel.  Rows in shared memory lie `stride` entries apart: the row's length rounded up
 //  to 16, plus 8 (an odd number of 16-byte pieces, so that ldmatrix meets no bank twice).
 #include "hybrid.cuh"
 
@@ -313,6 +313,339 @@ template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStrea
   return 0;
 }
 
+// The same for windows and for steps of single tokens, with the queries and the softmax weights kept whole: each is
+// cut into THREE bfloat16 terms (truncated, so 8 + 8 + 8 bits hold all 24), the cached rows are bfloat16 as they lie,
+// every product of two terms is exact and the sums are 32-bit, as on the generic kernel.  The tensor cores truncate
+// where they add, so a sum runs there over 16 or 32 products only, the smallest terms first, and goes on in rounded
+// 32-bit additions (with chains over whole rows and all keys the error was 1.2 to 1.9 times the generic kernel's).
+//
+//  CTA: 32 consecutive (token, head) rows of one request, whatever the number of heads; 8 warps = 2 groups of 16 rows x
+//  4 slices.  Key tiles of 32 rows by cp.async into two buffers.  For S a slice is a quarter of the row's entries: a
+//  warp takes 16 rows x 32 keys over its quarter (the queries' three terms would otherwise be read from shared memory
+//  by every warp: 3 x 37 KB a tile), the four partial scores are added in shared memory, eight threads a row keep the
+//  maximum and the sum in 32-bit and leave the weights' three terms there.  For O a slice is a quarter of the latent's
+//  columns.  With `splits`, blockIdx.y takes `chunk` keys counted from the tile's first visible one and leaves
+//  (maximum, sum, weighted sum) per row for the merge kernel.
+//  Bound by the shared-memory reads of the tensor operands (about 2,700 cycles a tile of 32 x 32 at 512 + 64 entries
+//  against 1,600 of mma.sync).
+constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLD = 36, LTX_PLD = 40;
+
+struct LtxParams {
+  const float* qp;          // [tokens * heads][dk]
+  const bf16* pages;        // [n_pages][page_size][dk]
+  const int* block_table;
+  int bt_stride, page_size, n_pages;
+  const int* tok_req;
+  const int* tok_pos;
+  const int* q_start;
+  int n, R, H, r, dk, stride, window, splits, chunk;
+  const float* gate;
+  long long ld_gate;
+  float* out;
+  long long ldo;
+  float* ws;                // [tokens * heads][splits][r + 2] partial results (splits > 1)
+  float scale_log2;
+  const float* sink;
+  int* status;
+};
+
+size_t ltx_smem(int stride) {
+  return sizeof(bf16) * (3 * LTX_ROWS + 2 * LTX_KEYS) * (size_t)stride + sizeof(float) * 4 * LTX_ROWS * LTX_SLD +
+         sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 2 * LTX_ROWS;
+}
+
+// x = t0 + t1 + t2, each a bfloat16 (the upper half of a 32-bit number)
+__device__ __forceinline__ void ltx_split(float x, unsigned short (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const unsigned u = __float_as_uint(x) & 0xffff0000u;
+    t[i] = (unsigned short)(u >> 16);
+    x -= __uint_as_float(u);
+  }
+}
+
+template <int OC>                                          // columns of the latent a warp takes
+__global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const LtxParams p) {
+  extern __shared__ __align__(16) unsigned char ltc_smem[];
+  const int STRIDE = p.stride, dk = p.dk, H = p.H, r = p.r;
+  bf16* Qs = reinterpret_cast<bf16*>(ltc_smem);            // [3][32][STRIDE]
+  bf16* Cs = Qs + 3 * LTX_ROWS * STRIDE;                   // [2][32][STRIDE]
+  float* Sp = reinterpret_cast<float*>(Cs + 2 * LTX_KEYS * STRIDE);      // [4][32][LTX_SLD]
+  bf16* Pt = reinterpret_cast<bf16*>(Sp + 4 * LTX_ROWS * LTX_SLD);       // [3][32][LTX_PLD]
+  float* corr = reinterpret_cast<float*>(Pt + 3 * LTX_ROWS * LTX_PLD);   // [32], [32]
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wr = warp & 1, wk = warp >> 1, g = lane >> 2, t4 = lane & 3;
+  // which request's which tile: requests have ceil(rows / 32) tiles each, one after the other
+  int req = -1, tile = 0, first = 0, len = 0, before = 0;
+  for (int r0 = 0; r0 < p.R && req < 0; r0 += 32) {
+    const int mine = r0 + lane;
+    const int b = mine < p.R ? p.q_start[mine] : 0, e = mine + 1 < p.R ? p.q_start[mine + 1] : p.n;
+    const int tiles = mine < p.R ? (int)(((long long)(e - b) * H + LTX_ROWS - 1) / LTX_ROWS) : 0;
+    int upto = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.x);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      req = r0 + src;
+      first = __shfl_sync(0xffffffffu, b, src);
+      len = __shfl_sync(0xffffffffu, e - b, src);
+      tile = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - tiles, src);
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  if (req < 0) return;
+  const int row0 = tile * LTX_ROWS;                        // (rows of the request)
+  const int rows_live = min(LTX_ROWS, len * H - row0);
+  const int pos_req = p.tok_pos[first];                    // the request's tokens have consecutive positions
+  const int pos0 = pos_req + row0 / H, kmax = pos_req + (row0 + rows_live - 1) / H;
+  const int* table = p.block_table + (size_t)p.tok_req[first] * p.bt_stride;
+  const int base = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+  const int k_begin = p.splits > 1 ? base + (int)blockIdx.y * p.chunk : base;
+  const int k_end = p.splits > 1 ? min(kmax, k_begin + p.chunk - 1) : kmax;          // (the last key)
+  // zeros where nothing is copied: columns dk .. stride
+  const int pad = (STRIDE - dk) >> 3;
+  for (int i = tid; i < (3 * LTX_ROWS + 2 * LTX_KEYS) * pad; i += 256)
+    *reinterpret_cast<uint4*>(Qs + (size_t)(i / pad) * STRIDE + dk + 8 * (i % pad)) = make_uint4(0u, 0u, 0u, 0u);
+
+  const int pieces = dk >> 3;                              // 16-byte pieces of a cached row
+  auto stage = [&](int k0, int b) {
+    bf16* dst = Cs + (size_t)b * LTX_KEYS * STRIDE;
+#pragma unroll
+    for (int u = 0; u < LTX_KEYS / 8; ++u) {
+      const int j = warp + 8 * u, key = min(k0 + j, k_end);               // (rows behind the last key are masked)
+      const int page = table[key / p.page_size];
+      const bool bad = page < 0 || page >= p.n_pages;
+      if (bad && lane == 0) atomicExch(p.status, LTC_BAD_PAGE_READ);
+      const bf16* src = p.pages + ((size_t)(bad ? 0 : page) * p.page_size + key % p.page_size) * dk;
+      for (int c = lane; c < pieces; c += 32) {
+        if (bad) *reinterpret_cast<uint4*>(dst + j * STRIDE + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
+        else gb_cp_async_16(dst + j * STRIDE + 8 * c, src + 8 * c);
+      }
+    }
+    ltc_commit();
+  };
+  pdl_wait();
+  if (k_begin <= k_end) stage(k_begin, 0);
+  {
+    // (a warp asks for two rows at once: up to ten trips to L2 side by side)
+    const float* src = p.qp + ((size_t)first * H + row0) * dk;
+    constexpr int QL = 5;                                  // quads a lane takes of a row: 32 * 5 >= 576 / 4
+    const int quads = dk >> 2;
+#pragma unroll
+    for (int rr = 0; rr < LTX_ROWS / 8; rr += 2) {
+      float4 v[2][QL];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = warp + 8 * (rr + u);
+#pragma unroll
+        for (int i = 0; i < QL; ++i)
+          v[u][i] = row < rows_live && lane + 32 * i < quads
+                        ? ldcg_now(reinterpret_cast<const float4*>(src + (size_t)row * dk) + lane + 32 * i)
+                        : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = warp + 8 * (rr + u);
+#pragma unroll
+        for (int i = 0; i < QL; ++i) {
+          if (lane + 32 * i >= quads) break;
+          unsigned short a[3], b[3], d[3], e[3];
+          ltx_split(v[u][i].x, a);
+          ltx_split(v[u][i].y, b);
+          ltx_split(v[u][i].z, d);
+          ltx_split(v[u][i].w, e);
+#pragma unroll
+          for (int t = 0; t < 3; ++t)
+            *reinterpret_cast<uint2*>(Qs + ((size_t)t * LTX_ROWS + row) * STRIDE + 4 * (lane + 32 * i)) =
+                make_uint2(a[t] | (unsigned)b[t] << 16, d[t] | (unsigned)e[t] << 16);
+        }
+      }
+    }
+  }
+  // the softmax's view: eight threads a row, four keys each
+  const int srow = tid >> 3, scol = (tid & 7) * 4;
+  const int spos = pos_req + (row0 + srow) / H, slo = p.window > 0 ? spos - p.window + 1 : 0;
+  float m = -INFINITY, l = 0.f;
+  float o[OC / 8][4];
+#pragma unroll
+  for (int j = 0; j < OC / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  const int ksteps = (dk + 15) >> 4, per = (ksteps + 3) >> 2;
+  const int ks_begin = wk * per, ks_end = min(ksteps, ks_begin + per);
+  const int npairs = min(OC / 16, max(0, (r - wk * OC + 15) >> 4));       // pairs of 8 output columns that hold anything
+  const bool warp_live = wr * 16 < rows_live;
+
+  int b = 0;
+  for (int k0 = k_begin; k0 <= k_end; k0 += LTX_KEYS, b ^= 1) {
+    ltc_wait<0>();
+    __syncthreads();                                       // this tile is there, the one before it has been used
+    if (k0 + LTX_KEYS <= k_end) stage(k0 + LTX_KEYS, b ^ 1);
+    const bf16* C = Cs + (size_t)b * LTX_KEYS * STRIDE;
+    if (warp_live) {
+      float s[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+      const bf16* qa = Qs + (wr * 16 + (lane & 15)) * STRIDE + (lane >> 4) * 8;
+      const bf16* cb = C + ((lane & 7) + (lane >> 4) * 8) * STRIDE + ((lane >> 3) & 1) * 8;
+#pragma unroll 3
+      for (int ks = ks_begin; ks < ks_end; ++ks) {
+        unsigned bb[2][4], a[3][4];
+        ltc_ldmatrix(bb[0], cb + ks * 16);
+        ltc_ldmatrix(bb[1], cb + 16 * STRIDE + ks * 16);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) ltc_ldmatrix(a[t], qa + (size_t)t * LTX_ROWS * STRIDE + ks * 16);
+        float part[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[j][0] = part[j][1] = part[j][2] = part[j][3] = 0.f;
+#pragma unroll
+        for (int t = 2; t >= 0; --t) {
+#pragma unroll
+          for (int np = 0; np < 2; ++np) {
+            ltc_mma(part[2 * np], a[t], bb[np][0], bb[np][1]);
+            ltc_mma(part[2 * np + 1], a[t], bb[np][2], bb[np][3]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[j][e] += part[j][e];
+      }
+      float* dst = Sp + (wk * LTX_ROWS + wr * 16 + g) * LTX_SLD + 2 * t4;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(s[j][0], s[j][1]);
+        *reinterpret_cast<float2*>(dst + 8 * LTX_SLD + 8 * j) = make_float2(s[j][2], s[j][3]);
+      }
+    }
+    __syncthreads();
+    {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float4 v = *reinterpret_cast<const float4*>(Sp + (w * LTX_ROWS + srow) * LTX_SLD + scol);
+        s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+      }
+      float mx = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = k0 + scol + e;
+        s[e] = (srow < rows_live && k <= min(spos, k_end) && k >= slo) ? s[e] * p.scale_log2 : -INFINITY;
+        mx = fmaxf(mx, s[e]);
+      }
+#pragma unroll
+      for (int x = 1; x < 8; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+      const float mn = fmaxf(m, mx), ref = mn == -INFINITY ? 0.f : mn;    // (a row may see no key of this tile)
+      const float c = exp2f(m - ref);
+      m = mn;
+      unsigned short t[4][3];
+      float sum = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[e] = exp2f(s[e] - ref);
+        sum += s[e];
+        ltx_split(s[e], t[e]);
+      }
+      l = l * c + sum;                                     // (this thread's share; the row is added at the end)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        *reinterpret_cast<uint2*>(Pt + (i * LTX_ROWS + srow) * LTX_PLD + scol) =
+            make_uint2(t[0][i] | (unsigned)t[1][i] << 16, t[2][i] | (unsigned)t[3][i] << 16);
+      if ((tid & 7) == 0) corr[srow] = c;
+    }
+    __syncthreads();
+    if (warp_live) {
+      const float c_a = corr[wr * 16 + g], c_b = corr[wr * 16 + g + 8];
+      const bf16* ct = C + ((lane & 7) + ((lane >> 3) & 1) * 8) * STRIDE + wk * OC + (lane >> 4) * 8;
+      const bf16* pa = Pt + (wr * 16 + (lane & 15)) * LTX_PLD + (lane >> 4) * 8;
+      unsigned a[2][3][4];
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+        for (int t = 0; t < 3; ++t) ltc_ldmatrix(a[kk][t], pa + t * LTX_ROWS * LTX_PLD + kk * 16);
+#pragma unroll
+      for (int np = 0; np < OC / 16; ++np) {
+        if (np < npairs) {
+          float part[2][4];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) part[j][0] = part[j][1] = part[j][2] = part[j][3] = 0.f;
+          unsigned bb[2][4];
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) ltc_ldmatrix_t(bb[kk], ct + kk * 16 * STRIDE + np * 16);
+#pragma unroll
+          for (int t = 2; t >= 0; --t)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              ltc_mma(part[0], a[kk][t], bb[kk][0], bb[kk][1]);
+              ltc_mma(part[1], a[kk][t], bb[kk][2], bb[kk][3]);
+            }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            o[2 * np + j][0] = fmaf(o[2 * np + j][0], c_a, part[j][0]);
+            o[2 * np + j][1] = fmaf(o[2 * np + j][1], c_a, part[j][1]);
+            o[2 * np + j][2] = fmaf(o[2 * np + j][2], c_b, part[j][2]);
+            o[2 * np + j][3] = fmaf(o[2 * np + j][3], c_b, part[j][3]);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int x = 1; x < 8; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+  const size_t flat0 = (size_t)first * H + row0;           // this tile's first (token, head) row of the step
+  if (p.splits > 1) {
+    if ((tid & 7) == 0 && srow < rows_live) {
+      float* w = p.ws + ((flat0 + srow) * p.splits + blockIdx.y) * (size_t)(r + 2);
+      w[0] = m * 0.6931471805599453f;                      // (natural units; -inf stays -inf: a chunk without keys)
+      w[1] = l;
+    }
+    if (k_begin > k_end) return;                           // (the merge does not read a sum without keys)
+  } else if ((tid & 7) == 0 && srow < rows_live) {
+    constexpr float LOG2E = 1.4426950408889634f;
+    const size_t flat = flat0 + srow, t = flat / H;
+    const int h = (int)(flat - t * H);
+    float f = 1.f / l;
+    if (p.sink) {
+      const float s2 = p.sink[h] * LOG2E, top = fmaxf(m, s2), e = exp2f(m - top);
+      f = e / (exp2f(s2 - top) + e * l);
+    }
+    if (p.gate) f *= hy_sigmoid(p.gate[t * p.ld_gate + h]);
+    corr[LTX_ROWS + srow] = f;
+  }
+  __syncthreads();
+  if (!warp_live) return;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int row = wr * 16 + g + 8 * half;
+    if (row >= rows_live) continue;
+    const size_t flat = flat0 + row;
+    float* dst;
+    float f = 1.f;
+    if (p.splits > 1) {
+      dst = p.ws + (flat * p.splits + blockIdx.y) * (size_t)(r + 2) + 2;
+    } else {
+      dst = p.out + (flat / H) * p.ldo + (flat % H) * (size_t)r;
+      f = corr[LTX_ROWS + row];
+    }
+    dst += wk * OC + 2 * t4;
+#pragma unroll
+    for (int j = 0; j < OC / 8; ++j)
+      if (wk * OC + 8 * j < r) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(o[j][2 * half] * f, o[j][2 * half + 1] * f);
+  }
+}
+
+template <int OC> cudaError_t ltx_launch(const LtxParams& p, cudaStream_t stream) {
+  const size_t smem = ltx_smem(p.stride);
+  const cudaError_t e = cudaFuncSetAttribute(latent_attention_split_kernel<OC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // (every request's last tile may be partly filled: at most R tiles beside the whole ones)
+  const unsigned tiles = (unsigned)((long long)p.n * p.H / LTX_ROWS + p.R);
+  return gb_launch(latent_attention_split_kernel<OC>, dim3(tiles, p.splits), dim3(256), smem, stream, p);
+}
+
 // out[t, h, :] = x[t, h, :] W[h]^T on tensor cores, for the two per-head products around the attention (W_uk^T on the
 // queries, W_uv on the weighted latents) when a step has rows enough.  A CTA takes 64 rows x 64 outputs of one head
 // in steps of 32 inputs; x is 32-bit and rounded to bfloat16 on its way into shared memory, as the framework's other
@@ -462,4 +795,32 @@ int gb_latent_attention_tc_launch(const float* qp, const bf16* pages, const int*
   else if (r <= 256) rc = ltc_launch<256>(p, tiles, R, stream);
   else rc = ltc_launch<512>(p, tiles, R, stream);
   return rc < 0 ? rc : p.splits;
+}
+
+// Whether the second kernel takes a launch the first does not: bfloat16 pages whose rows can be copied in 16-byte
+// pieces, a latent of at most 512 entries and a row of at most 576.
+bool gb_latent_attention_split_takes(int n, int R, int H, int r, int dr, bool pages_bf16, const void* pages, const void* qp,
+                                     const void* out, long long ldo) {
+  return pages_bf16 && dr >= 0 && dr % 8 == 0 && r + dr <= 576 && H >= 1 && r % 8 == 0 && r >= 8 && r <= 512 && R >= 1 &&
+         (long long)n * H <= (1 << 30) && ((uintptr_t)pages & 15) == 0 && ((uintptr_t)qp & 15) == 0 &&
+         ((uintptr_t)out & 7) == 0 && ldo % 2 == 0;
+}
+
+// The keys are cut into `splits` chunks of `chunk` (a multiple of the key tile) counted from a tile's first visible key.
+cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages, const int* block_table, int bt_stride,
+                                             int page_size, int n_pages, const int* tok_req, const int* tok_pos,
+                                             const int* q_start, const float* gate, long long ld_gate, float* out,
+                                             long long ldo, int n, int R, int H, int r, int dr, float scale, int window,
+                                             const float* sink, float* ws, int splits, int chunk, int* status,
+                                             cudaStream_t stream) {
+  LtxParams p;
+  p.qp = qp; p.pages = pages; p.block_table = block_table; p.bt_stride = bt_stride; p.page_size = page_size;
+  p.n_pages = n_pages; p.tok_req = tok_req; p.tok_pos = tok_pos; p.q_start = q_start; p.n = n; p.R = R; p.H = H; p.r = r;
+  p.dk = r + dr; p.stride = 16 * ((p.dk + 15) / 16) + 8; p.window = window; p.splits = splits; p.chunk = chunk;
+  p.gate = gate; p.ld_gate = ld_gate; p.out = out; p.ldo = ldo; p.ws = ws; p.scale_log2 = scale * 1.4426950408889634f;
+  p.sink = sink; p.status = status;
+  if (r <= 64) return ltx_launch<16>(p, stream);
+  if (r <= 128) return ltx_launch<32>(p, stream);
+  if (r <= 256) return ltx_launch<64>(p, stream);
+  return ltx_launch<128>(p, stream);
 }

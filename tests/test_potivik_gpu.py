@@ -118,6 +118,61 @@ def test_latent_attention_alone_whole_cut_and_decoded(cfg, layer, dtype):
         hz.close(rid)
 
 
+@pytest.mark.parametrize("H,r,dr", [(1, 8, 0), (3, 24, 8), (8, 64, 40), (5, 136, 8), (16, 256, 32), (33, 320, 0), (16, 512, 64)])
+@pytest.mark.parametrize("window", [0, 1, 31, 33, 200])
+def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H, r, dr, window):
+    """The tensor-core kernel for windows and single tokens against 64-bit arithmetic on the same pages: portions that
+    end inside row tiles, key tiles and pages, single tokens, both in one step, chunked and not.  A score is off by at
+    most d = (r + dr + 16) 2^-24 scale |q|.|c| (its sum is cut into terms of three sizes and four quarters), a weight
+    by exp(2 d + 2^-20), the weighted sum by (keys + 64) 2^-24."""
+    from gibbs_b200.ops import hybrid, library
+    torch.manual_seed(r + window)
+    Dk, ps, R = r + dr, 16, 3
+    n_pages = 64
+    pages = torch.randn(n_pages, ps, Dk).to(torch.bfloat16)
+    perm = torch.randperm(n_pages)[:60].reshape(3, 20)
+    scale, sink = 0.7 * Dk ** -0.5, torch.randn(H)
+    lens_of = {"portions": [(0, 70), (30, 33), (250, 1)], "single": [(299, 1), (31, 1), (0, 1)], "mixed": [(100, 1), (0, 40), (200, 17)]}
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    rows = library("hybrid").gb_latent_attention_workspace_rows()
+    ws = torch.full((rows, r + 2), float("nan"), device=DEV)
+    for what, spans in lens_of.items():
+        if window == 0 and what != "single":
+            continue                                        # (such steps run on the kernel without windows)
+        tok_req = [i for i, (p, k) in enumerate(spans) for _ in range(k)]
+        tok_pos = [p + j for p, k in spans for j in range(k)]
+        n = len(tok_req)
+        starts = [sum(k for _, k in spans[:i]) for i in range(R)]
+        q, gate = torch.randn(n, H, Dk), torch.randn(n, H)
+        dev = {k: v.to(DEV).contiguous() for k, v in dict(q=q, pages=pages, gate=gate, sink=sink).items()}
+        table, tr, tp, qs = i32(perm.tolist()), i32(tok_req), i32(tok_pos), i32(starts)
+        got = {}
+        for tc in (True, False):
+            out = torch.full((n, H * r), float("nan"), device=DEV)
+            hybrid.call("latent_attention", [dev["q"].data_ptr(), dev["pages"].data_ptr(), 1, table.data_ptr(), 20, ps, n_pages,
+                                             tr.data_ptr(), tp.data_ptr(), dev["gate"].data_ptr(), H, out.data_ptr(), H * r, n, H,
+                                             r, dr, window, 320, ws.data_ptr(), dev["sink"].data_ptr(), R if tc else 0,
+                                             qs.data_ptr() if tc else 0], [scale])
+            got[tc] = out.double().cpu().reshape(n, H, r)
+        off = {True: 0.0, False: 0.0}
+        for t in range(n):
+            lo = max(0, tok_pos[t] - window + 1) if window else 0
+            j = torch.arange(lo, tok_pos[t] + 1)
+            c = pages[perm[tok_req[t]][j // ps], j % ps].double()
+            sc = q[t].double() @ c.T * scale
+            w = torch.softmax(torch.cat([sc, sink.double()[:, None]], 1), 1)[:, :-1]
+            f = torch.sigmoid(gate[t].double())[:, None]
+            want, size = (w @ c[:, :r]) * f, (w @ c[:, :r].abs()) * f
+            d = (Dk + 16) * 2.0 ** -24 * scale * (q[t].double().abs() @ c.T.abs()).amax(1)
+            tol = (2 * d[:, None] + 2.0 ** -20 + (len(j) + 64) * 2.0 ** -24) * size + 2.0 ** -22 * want.abs()
+            assert ((got[True][t] - want).abs() <= tol).all(), (what, t)
+            for tc in off:
+                off[tc] += float((got[tc][t] - want).pow(2).sum())
+        assert not torch.equal(got[True], got[False])                # (two kernels did run)
+        if what == "portions":                              # (rows enough for the two errors to be compared: measured 0.4 to 1.1)
+            assert off[True] <= 1.25 ** 2 * off[False], (off[True] / off[False]) ** 0.5
+
+
 def _pointed_attention(window, T, hot_key, query, d=64, seed=7):
     """Weights and inputs for which the query position's score against ``hot_key`` stands far
     above all others (when that key is visible), and whose values tell keys apart.  The latent is
