@@ -253,51 +253,81 @@ __global__ void ssm_scan_kernel(const float* xbc, long long ld, const float* dt_
     }
 }
 
-// The same recurrence with the state in registers and (almost) no exchange between lanes: SPLIT neighbouring
-// lanes share a column p of a head, each with 32 of the column's state values (N up to 32 * SPLIT), so a token
-// costs a thread 64 multiply-adds and the column log2(SPLIT) shuffles; B_t and C_t are read from shared memory
-// four values an instruction.  The inputs of SCOL_TOKENS tokens at a time arrive by asynchronous copies into
-// one of two buffers while the tokens of the other are consumed.
-constexpr int SCOL_TOKENS = 16, SCOL_THREADS = 64;
+// The same recurrence with the state in registers and little exchange between lanes: SPLIT neighbouring
+// lanes share SCOL_CP columns of a head, each with 16 of a column's state values (N up to 16 * SPLIT); B_t
+// and C_t are read from shared memory four values an instruction, once for both columns, and those of the
+// token behind are asked for ahead of a token's multiply-adds (packed in pairs: fma.rn.f32x2).  Tokens are
+// taken SPLIT at a time: the SPLIT partial read-outs are added by exchanging halves, so that lane q ends with
+// token q's sum (SPLIT - 1 shuffles a column for SPLIT tokens).  The inputs of SCOL_TOKENS tokens at a time
+// arrive by asynchronous copies into one of two buffers while the tokens of the other are consumed.
+// Bound by the chain of a token: a long prompt is one sequence of tokens for few warps.  Measured at 64 heads of 64
+// columns, 128 state values, portions of 1801 and 333 tokens: 443 us; with one column and 32 values a thread, its
+// reads of shared memory waited for one by one, 1028 us; with one column and 16 values a thread 640 us.
+constexpr int SCOL_TOKENS = 16, SCOL_NV = 16, SCOL_CP = 2;
 
 __device__ __forceinline__ void scol_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int LEFT> __device__ __forceinline__ void scol_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+typedef unsigned long long scol_f2;
+__device__ __forceinline__ scol_f2 scol_pack(float lo, float hi) {
+  scol_f2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 scol_unpack(scol_f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ scol_f2 scol_mul(scol_f2 a, scol_f2 b) {
+  scol_f2 v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ scol_f2 scol_fma(scol_f2 a, scol_f2 b, scol_f2 c) {
+  scol_f2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+
 template <int SPLIT>
-__global__ void ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long long ld_dt,
-                                     const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                                     const float* __restrict__ dskip, float* state, long long slot_stride,
-                                     const int* slot_ids, const int* q_start, const int* q_len, float* y, long long ldy,
-                                     int H, int P, int N, int G) {
-  constexpr int NR = 32 * SPLIT, COLS = SCOL_THREADS / SPLIT;
+__global__ void __launch_bounds__(128)
+ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long long ld_dt, const float* __restrict__ dt_bias,
+                     const float* __restrict__ a_log, const float* __restrict__ dskip, float* state, long long slot_stride,
+                     const int* slot_ids, const int* q_start, const int* q_len, float* y, long long ldy, int H, int P, int N,
+                     int G) {
+  constexpr int NR = SCOL_NV * SPLIT, NQ = SCOL_NV / 4;
   extern __shared__ __align__(16) float scol[];
-  constexpr int PER = SCOL_TOKENS * (2 * NR + COLS);      // one buffer: B [T][NR] | C [T][NR] | x [T][COLS]
+  const int COLS = SCOL_CP * (int)blockDim.x / SPLIT, half = COLS / SCOL_CP;
+  const int PER = SCOL_TOKENS * (2 * NR + COLS);           // one buffer: B [T][NR] | C [T][NR] | x [T][COLS]
   float* sRaw = scol + 2 * PER;                            // [2][T] dt before the bias
-  float* sDt = sRaw + 2 * SCOL_TOKENS;                     // [T] step size, [T] decay
-  float* sDecay = sDt + SCOL_TOKENS;
+  float2* sDt = reinterpret_cast<float2*>(sRaw + 2 * SCOL_TOKENS);         // [T] (step size, decay)
   pdl_trigger();
-  const int col = threadIdx.x / SPLIT, q = threadIdx.x % SPLIT;
-  const int r = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * COLS, p = p0 + col;
-  const bool active = p < P;
+  const int col = threadIdx.x / SPLIT, q = threadIdx.x % SPLIT;            // columns col and col + half
+  const int r = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * COLS;
   const int g = h / (H / G);
   const int inner = H * P;
   const float bias = dt_bias[h], neg_a = -expf(a_log[h]), dsk = dskip[h];
   const int first = q_start[r], len = q_len[r];
   // (this kernel keeps a head's state as [state][head_dim], so that neighbouring columns lie side by side)
-  float* S = state + (size_t)slot_ids[r] * slot_stride + (size_t)h * P * N + (active ? p : 0);
-  if (N < NR)                                              // the padding N .. NR of B and C stays zero
+  float* S = state + (size_t)slot_ids[r] * slot_stride + (size_t)h * P * N;
+  bool active[SCOL_CP];
+#pragma unroll
+  for (int c = 0; c < SCOL_CP; ++c) active[c] = p0 + col + c * half < P;
+  // (the padding N .. NR of B and C and the columns beyond P stay zero)
+  if (N < NR || p0 + COLS > P)
     for (int i = threadIdx.x; i < 2 * PER; i += blockDim.x) scol[i] = 0.f;
   pdl_wait();
-  // this thread's state values: n = 4 (q + SPLIT i) + e, i < 8, e < 4
-  float s[32];
+  // this thread's state values: n = 4 (q + SPLIT i) + e, i < NQ, e < 4, in pairs (N is a multiple of 4)
+  scol_f2 s[SCOL_CP][2 * NQ];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int c = 0; c < SCOL_CP; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int n = 4 * (q + SPLIT * i) + e;
-      s[4 * i + e] = (active && n < N) ? S[(size_t)n * P] : 0.f;
+    for (int i = 0; i < 2 * NQ; ++i) {
+      const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1), at = p0 + col + c * half;
+      s[c][i] = scol_pack(active[c] && n < N ? S[(size_t)n * P + at] : 0.f, active[c] && n < N ? S[(size_t)(n + 1) * P + at] : 0.f);
     }
   __syncthreads();
 
@@ -307,11 +337,11 @@ __global__ void ssm_scan_cols_kernel(const float* xbc, long long ld, const float
     float* B = scol + b * PER;
     float* C = B + SCOL_TOKENS * NR;
     float* X = C + SCOL_TOKENS * NR;
-    for (int i = threadIdx.x; i < 2 * nt * pieces; i += blockDim.x) {
-      const int which = i / (nt * pieces), rem = i - which * nt * pieces;
-      const int tt = rem / pieces, c4 = rem - tt * pieces;
-      const float* src = xbc + (size_t)(first + t0 + tt) * ld + inner + (which ? G + g : g) * N + 4 * c4;
-      gb_cp_async_16((which ? C : B) + tt * NR + 4 * c4, src);
+    for (int i = threadIdx.x; i < nt * pieces; i += blockDim.x) {
+      const int tt = i / pieces, c4 = i - tt * pieces;
+      const float* src = xbc + (size_t)(first + t0 + tt) * ld + inner + g * N + 4 * c4;
+      gb_cp_async_16(B + tt * NR + 4 * c4, src);
+      gb_cp_async_16(C + tt * NR + 4 * c4, src + G * N);
     }
     for (int i = threadIdx.x; i < nt * xpieces; i += blockDim.x) {
       const int tt = i / xpieces, c4 = i - tt * xpieces;
@@ -335,45 +365,97 @@ __global__ void ssm_scan_cols_kernel(const float* xbc, long long ld, const float
     __syncthreads();
     if ((int)threadIdx.x < nt) {
       const float dt = hy_softplus(sRaw[b * SCOL_TOKENS + threadIdx.x] + bias);
-      sDt[threadIdx.x] = dt;
-      sDecay[threadIdx.x] = expf(neg_a * dt);
+      sDt[threadIdx.x] = make_float2(dt, expf(neg_a * dt));
     }
     __syncthreads();
-    const float* B = scol + b * PER;
+    const float* B = scol + b * PER + 4 * q;
     const float* C = B + SCOL_TOKENS * NR;
-    const float* X = C + SCOL_TOKENS * NR;
-    for (int tt = 0; tt < nt; ++tt) {                      // (every lane, also of a column beyond P: the shuffles below)
-      const float decay = sDecay[tt], xv = active ? X[tt * COLS + col] : 0.f, dx = sDt[tt] * xv;
-      float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;        // four chains; added in a fixed order
+    const float* X = scol + b * PER + 2 * SCOL_TOKENS * NR + col;
+    struct Inputs {
+      ulonglong2 b[NQ], c[NQ];
+      float x[SCOL_CP];
+      float2 dt;
+    };
+    auto load = [&](int tt, Inputs& in) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 b4 = *reinterpret_cast<const float4*>(B + tt * NR + 4 * (q + SPLIT * i));
-        const float4 c4 = *reinterpret_cast<const float4*>(C + tt * NR + 4 * (q + SPLIT * i));
-        s[4 * i] = fmaf(decay, s[4 * i], b4.x * dx);
-        y0 = fmaf(s[4 * i], c4.x, y0);
-        s[4 * i + 1] = fmaf(decay, s[4 * i + 1], b4.y * dx);
-        y1 = fmaf(s[4 * i + 1], c4.y, y1);
-        s[4 * i + 2] = fmaf(decay, s[4 * i + 2], b4.z * dx);
-        y2 = fmaf(s[4 * i + 2], c4.z, y2);
-        s[4 * i + 3] = fmaf(decay, s[4 * i + 3], b4.w * dx);
-        y3 = fmaf(s[4 * i + 3], c4.w, y3);
+      for (int i = 0; i < NQ; ++i) {
+        in.b[i] = *reinterpret_cast<const ulonglong2*>(B + tt * NR + 4 * SPLIT * i);
+        in.c[i] = *reinterpret_cast<const ulonglong2*>(C + tt * NR + 4 * SPLIT * i);
       }
-      float ys = (y0 + y1) + (y2 + y3);
+      in.dt = sDt[tt];
 #pragma unroll
-      for (int o = 1; o < SPLIT; o <<= 1) ys += __shfl_xor_sync(0xffffffffu, ys, o);
-      if (active && q == 0) y[(size_t)(first + t0 + tt) * ldy + h * P + p] = ys + dsk * xv;
+      for (int c = 0; c < SCOL_CP; ++c) in.x[c] = X[tt * COLS + c * half];
+    };
+    // a token's step: this thread's share of its read-outs
+    auto token = [&](const Inputs& in, float (&ys)[SCOL_CP]) {
+      const scol_f2 decay = scol_pack(in.dt.y, in.dt.y);
+#pragma unroll
+      for (int c = 0; c < SCOL_CP; ++c) {
+        const float dxv = in.dt.x * in.x[c];
+        const scol_f2 dx = scol_pack(dxv, dxv);
+        scol_f2 y0 = 0, y1 = 0;                            // four chains in pairs; added in a fixed order
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          s[c][2 * i] = scol_fma(decay, s[c][2 * i], scol_mul(in.b[i].x, dx));
+          y0 = scol_fma(s[c][2 * i], in.c[i].x, y0);
+          s[c][2 * i + 1] = scol_fma(decay, s[c][2 * i + 1], scol_mul(in.b[i].y, dx));
+          y1 = scol_fma(s[c][2 * i + 1], in.c[i].y, y1);
+        }
+        const float2 ya = scol_unpack(y0), yb = scol_unpack(y1);
+        ys[c] = (ya.x + ya.y) + (yb.x + yb.y);
+      }
+    };
+    // (every lane takes part, also of a column beyond P: the shuffles)
+    int tt = 0;
+    Inputs in[2];
+    load(0, in[0]);
+    for (; tt + SPLIT <= nt; tt += SPLIT) {
+      float ys[SPLIT][SCOL_CP];
+#pragma unroll
+      for (int u = 0; u < SPLIT; ++u) {
+        load(min(tt + u + 1, SCOL_TOKENS - 1), in[(u + 1) & 1]);           // (behind the chunk's last token: read, not used)
+        token(in[u & 1], ys[u]);
+      }
+#pragma unroll
+      for (int c = 0; c < SCOL_CP; ++c) {
+#pragma unroll
+        for (int o = 1, left = SPLIT / 2; o < SPLIT; o <<= 1, left >>= 1) {
+          const bool up = (q & o) != 0;
+#pragma unroll
+          for (int u = 0; u < SPLIT / 2; ++u) {
+            if (u >= left) break;
+            const float keep = up ? ys[2 * u + 1][c] : ys[2 * u][c], give = up ? ys[2 * u][c] : ys[2 * u + 1][c];
+            ys[u][c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        if (active[c])
+          y[(size_t)(first + t0 + tt + q) * ldy + h * P + p0 + col + c * half] = ys[0][c] + dsk * X[(tt + q) * COLS + c * half];
+      }
+    }
+    for (; tt < nt; ++tt) {
+      float ys[SCOL_CP];
+      load(tt, in[0]);
+      token(in[0], ys);
+#pragma unroll
+      for (int c = 0; c < SCOL_CP; ++c) {
+#pragma unroll
+        for (int o = 1; o < SPLIT; o <<= 1) ys[c] += __shfl_xor_sync(0xffffffffu, ys[c], o);
+        if (active[c] && q == 0)
+          y[(size_t)(first + t0 + tt) * ldy + h * P + p0 + col + c * half] = ys[c] + dsk * X[tt * COLS + c * half];
+      }
     }
     __syncthreads();                                       // before the copies of the chunk after next land here
   }
-  if (active) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+  for (int c = 0; c < SCOL_CP; ++c)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int n = 4 * (q + SPLIT * i) + e;
-        if (n < N) S[(size_t)n * P] = s[4 * i + e];
-      }
-  }
+    for (int i = 0; i < 2 * NQ; ++i) {
+      const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1), at = p0 + col + c * half;
+      if (!active[c] || n >= N) continue;
+      const float2 v = scol_unpack(s[c][i]);
+      S[(size_t)n * P + at] = v.x;
+      S[(size_t)(n + 1) * P + at] = v.y;
+    }
 }
 
 }  // namespace
@@ -428,18 +510,20 @@ GB_OP(gb_op_ssm_scan) {
   if (R <= 0) return 0;
   if (G <= 0 || H % G) GB_FAIL(GB_ERR_ARG, "ssm_scan: %d heads in %d groups", H, G);
   if (N > 256) GB_FAIL(GB_ERR_ARG, "ssm_scan: state size %d (at most 256)", N);
-  // states of up to 128 values whose rows can be copied in 16-byte pieces: state in registers, 32 values a thread
+  // states of up to 128 values whose rows can be copied in 16-byte pieces: state in registers, 16 values of two columns a thread
   if (N <= 128 && N % 4 == 0 && P % 4 == 0 && a[1] % 4 == 0 && (a[0] & 15) == 0) {
-    const int split = N <= 32 ? 1 : (N <= 64 ? 2 : 4);
-    const int cols = SCOL_THREADS / split;
-    const size_t smem_cols = sizeof(float) * (2 * (size_t)SCOL_TOKENS * (2 * 32 * split + cols) + 4 * SCOL_TOKENS);
+    const int split = N <= 32 ? 2 : (N <= 64 ? 4 : 8);
+    // four warps a block (they share the copies of B and C), two where that leaves SMs without a block
+    const int threads = (long long)R * H * gb_div_up(P, SCOL_CP * 128 / split) >= 148 ? 128 : 64;
+    const int cols = SCOL_CP * threads / split;
+    const size_t smem_cols = sizeof(float) * (2 * (size_t)SCOL_TOKENS * (2 * SCOL_NV * split + cols) + 4 * SCOL_TOKENS);
     const dim3 grid_cols(R, H, gb_div_up(P, cols));
 #define SCOL_LAUNCH(SP)                                                                                               \
-    gb_launch(ssm_scan_cols_kernel<SP>, grid_cols, dim3(SCOL_THREADS), smem_cols, ctx->stream, op_ptr<const float>(a[0]), \
+    gb_launch(ssm_scan_cols_kernel<SP>, grid_cols, dim3(threads), smem_cols, ctx->stream, op_ptr<const float>(a[0]), \
               a[1], op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<const float>(a[5]),              \
               op_ptr<const float>(a[6]), op_ptr<float>(a[7]), a[8], op_ptr<const int>(a[9]), op_ptr<const int>(a[10]),   \
               op_ptr<const int>(a[11]), op_ptr<float>(a[12]), a[13], H, P, N, G)
-    if (split == 1) SCOL_LAUNCH(1); else if (split == 2) SCOL_LAUNCH(2); else SCOL_LAUNCH(4);
+    if (split == 2) SCOL_LAUNCH(2); else if (split == 4) SCOL_LAUNCH(4); else SCOL_LAUNCH(8);
 #undef SCOL_LAUNCH
     GB_CHECK_LAUNCH("ssm_scan (columns)");
     return 1;

@@ -173,6 +173,46 @@ def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H
             assert off[True] <= 1.25 ** 2 * off[False], (off[True] / off[False]) ** 0.5
 
 
+@pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
+def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
+    """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
+    do not, against the recurrence in 64 bits.  The state is a sum of decayed products whose errors decay with it: each
+    token adds 4 roundings to what is kept and exp and softplus a few units in the last place; the read-out adds N
+    terms.  With decays of at most exp(-0.5) per token the kept errors add up to less than 2.6 tokens' worth."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(N)
+    for lens in ([1, 2, 7], [8, 9, 15], [16, 17, 33, 1, 130]):
+        R, n = len(lens), sum(lens)
+        ld = H * P + 2 * G * N
+        xbc, dt = torch.randn(n, ld), torch.rand(n, H)
+        bias, alog, D = torch.rand(H), torch.rand(H), torch.randn(H)
+        slot, S0 = H * P * N, torch.randn(R + 2, H, N, P)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        ids, starts = list(range(R, 0, -1)), [sum(lens[:i]) for i in range(R)]
+        dev = [t.to(DEV) for t in (xbc, dt, bias, alog, D)]
+        state, y = S0.clone().to(DEV), torch.full((n, H * P), float("nan"), device=DEV)
+        i = [i32(ids), i32(starts), i32(lens)]
+        p = [t.data_ptr() for t in dev]
+        hybrid.call("ssm_scan", [p[0], ld, p[1], H, p[2], p[3], p[4], state.data_ptr(), slot, i[0].data_ptr(), i[1].data_ptr(),
+                                 i[2].data_ptr(), y.data_ptr(), H * P, R, H, P, N, G])
+        step = torch.nn.functional.softplus(dt.double() + bias.double())
+        decay = torch.exp(-torch.exp(alog.double()) * step)
+        assert decay.max() <= math.exp(-0.5)
+        x, B, C = xbc[:, :H * P].double().reshape(n, H, P), xbc[:, H * P:H * P + G * N].double(), xbc[:, H * P + G * N:].double()
+        B, C = (t.reshape(n, G, N).repeat_interleave(H // G, 1) for t in (B, C))
+        for r in range(R):
+            S, size = S0[ids[r]].double(), S0[ids[r]].double().abs()
+            for t in range(starts[r], starts[r] + lens[r]):
+                add = B[t][:, :, None] * (step[t][:, None] * x[t])[:, None]
+                S, size = decay[t][:, None, None] * S + add, decay[t][:, None, None] * size + add.abs()
+                want = (S * C[t][:, :, None]).sum(1) + D.double()[:, None] * x[t]
+                bound = (size * C[t].abs()[:, :, None]).sum(1) + (D.double()[:, None] * x[t]).abs()
+                err = (y[t].double().cpu().reshape(H, P) - want).abs()
+                assert (err <= (N / 4 + 40) * 2.0 ** -24 * bound).all(), (lens, r, t - starts[r])
+            assert ((state[ids[r]].double().cpu() - S).abs() <= 40 * 2.0 ** -24 * size).all()
+        assert torch.equal(state[0].cpu(), S0[0]) and torch.equal(state[R + 1].cpu(), S0[R + 1])
+
+
 def _pointed_attention(window, T, hot_key, query, d=64, seed=7):
     """Weights and inputs for which the query position's score against ``hot_key`` stands far
     above all others (when that key is visible), and whose values tell keys apart.  The latent is
