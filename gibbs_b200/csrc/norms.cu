@@ -181,9 +181,21 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
                                 int dim, int kind, float eps, bf16* copy, ThenNorm then) {
   __shared__ float scratch[32];
   pdl_trigger();
-  pdl_wait();
   const float* row = y + (size_t)blockIdx.x * ldy;
   float* o = x + (size_t)blockIdx.x * ldx;
+  // The gains are on hand before the kernel in front has finished (pinned, see gb_pin): read behind the sums, each was
+  // a trip to L2 of its own (2 rows of 2048 in a decode step: 6.3 us; 2.8 so).
+  const bool whole = dim <= NORM_CACHE * (int)blockDim.x, second = then.gain != nullptr;
+  float g1[NORM_CACHE], g2[NORM_CACHE];
+#pragma unroll
+  for (int i = 0; i < NORM_CACHE; ++i) {
+    const int d = threadIdx.x + i * blockDim.x;
+    g1[i] = whole && d < dim ? gain[d] : 0.f;
+    g2[i] = whole && second && d < dim ? then.gain[d] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < NORM_CACHE; ++i) { gb_pin(g1[i]); gb_pin(g2[i]); }
+  pdl_wait();
   RowCache c;
   row_load(row, dim, c);
   float old[NORM_CACHE];
@@ -201,7 +213,7 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
     for (int i = 0; i < NORM_CACHE; ++i) {
       const int d = threadIdx.x + i * blockDim.x;
       if (d < dim) {
-        const float v = old[i] + (c.v[i] - mean) * rstd * gain[d];
+        const float v = old[i] + (c.v[i] - mean) * rstd * g1[i];
         o[d] = v;
         if (copy) copy[(size_t)blockIdx.x * dim + d] = __float2bfloat16_rn(v);
         c.v[i] = v;
@@ -216,7 +228,7 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
       for (int i = 0; i < NORM_CACHE; ++i) {
         const int d = threadIdx.x + i * blockDim.x;
         if (d < dim) {
-          const float h = (c.v[i] - mean2) * rstd2 * then.gain[d];
+          const float h = (c.v[i] - mean2) * rstd2 * g2[i];
           if (then.out_dtype == GB_BF16) ((bf16*)then.out)[(size_t)blockIdx.x * dim + d] = __float2bfloat16_rn(h);
           else ((float*)then.out)[(size_t)blockIdx.x * dim + d] = h;
         }
