@@ -213,6 +213,32 @@ def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
         assert torch.equal(state[0].cpu(), S0[0]) and torch.equal(state[R + 1].cpu(), S0[R + 1])
 
 
+@pytest.mark.parametrize("weights,result", [("float32", "float32"), ("bfloat16", "float32"), ("bfloat16", "bfloat16")])
+@pytest.mark.parametrize("H,O,I", [(1, 1, 8), (3, 5, 24), (16, 128, 512), (2, 17, 1024), (2, 18, 1032), (4, 512, 128), (2, 9, 20)])
+def test_head_products_of_a_few_rows(H, O, I, weights, result):
+    """Rows 1 to 17 (the few-rows kernel ends at 16), outputs that do not fill a warp's four, inputs at and beyond what
+    its registers hold and no whole pieces (the other kernels): a lane adds I / 32 + 8 products, then five levels.
+    From 64 rows on bfloat16 weights round their inputs; these stay below."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(I)
+    W = torch.randn(H, O, I).to(DTYPES[weights])
+    Wd = W.to(DEV)
+    for n in (1, 2, 3, 16, 17):
+        x, gate = torch.randn(n, H * I + 4), torch.randn(n, H * O)
+        xd, gd = x.to(DEV), gate.to(DEV)
+        for gated in (False, True):
+            out = torch.full((n, H * O), float("nan"), dtype=DTYPES[result], device=DEV)
+            hybrid.call("head_linear", [xd.data_ptr(), H * I + 4, I, Wd.data_ptr(), 1 if weights == "bfloat16" else 0, out.data_ptr(),
+                                        1 if result == "bfloat16" else 0, H * O, O, n, H, O, I] +
+                        ([gd.data_ptr(), H * O] if gated else []))
+            xs = x[:, :H * I].double().reshape(n, H, I)
+            f = torch.sigmoid(gate.double()).reshape(n, H, O) if gated else torch.ones(n, H, O, dtype=torch.float64)
+            want = torch.einsum("nhi,hoi->nho", xs, W.double()) * f
+            size = torch.einsum("nhi,hoi->nho", xs.abs(), W.double().abs()) * f
+            tol = (I / 8 + 24) * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if result == "bfloat16" else 0)
+            assert ((out.double().cpu().reshape(n, H, O) - want).abs() <= tol).all(), (n, gated)
+
+
 def _pointed_attention(window, T, hot_key, query, d=64, seed=7):
     """Weights and inputs for which the query position's score against ``hot_key`` stands far
     above all others (when that key is visible), and whose values tell keys apart.  The latent is
