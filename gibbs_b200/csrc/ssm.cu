@@ -253,15 +253,15 @@ __global__ void ssm_scan_kernel(const float* xbc, long long ld, const float* dt_
     }
 }
 
-// The same recurrence with the state in registers and little exchange between lanes: SPLIT neighbouring
-// lanes share SCOL_CP columns of a head, each with 16 of a column's state values (N up to 16 * SPLIT); B_t
+// The same recurrence with the state in registers and little exchange between lanes: SPLIT lanes
+// share SCOL_CP columns of a head, each with 16 of a column's state values (N up to 16 * SPLIT); B_t
 // and C_t are read from shared memory four values an instruction, once for both columns, and those of the
 // token behind are asked for ahead of a token's multiply-adds (packed in pairs: fma.rn.f32x2).  Tokens are
 // taken SPLIT at a time: the SPLIT partial read-outs are added by exchanging halves, so that lane q ends with
 // token q's sum (SPLIT - 1 shuffles a column for SPLIT tokens).  The inputs of SCOL_TOKENS tokens at a time
 // arrive by asynchronous copies into one of two buffers while the tokens of the other are consumed.
 // Bound by the chain of a token: a long prompt is one sequence of tokens for few warps.  Measured at 64 heads of 64
-// columns, 128 state values, portions of 1801 and 333 tokens: 443 us; with one column and 32 values a thread, its
+// columns, 128 state values, portions of 1801 and 333 tokens: 430 us; with one column and 32 values a thread, its
 // reads of shared memory waited for one by one, 1028 us; with one column and 16 values a thread 640 us.
 constexpr int SCOL_TOKENS = 16, SCOL_NV = 16, SCOL_CP = 2;
 
@@ -305,8 +305,11 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
   float* sRaw = scol + 2 * PER;                            // [2][T] dt before the bias
   float2* sDt = reinterpret_cast<float2*>(sRaw + 2 * SCOL_TOKENS);         // [T] (step size, decay)
   pdl_trigger();
-  const int col = threadIdx.x / SPLIT, q = threadIdx.x % SPLIT;            // columns col and col + half
-  const int r = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * COLS;
+  // columns col and col + half, the column's share q.  (Neighbouring lanes have neighbouring columns and the SAME share: a
+  // quarter of a warp then reads one or two pieces of B or C, which cost shared memory one pass and not four.)
+  constexpr int CPW = 32 / SPLIT;
+  const int lane = threadIdx.x & 31, col = (threadIdx.x >> 5) * CPW + lane % CPW, q = lane / CPW;
+  const int pb = (P + COLS - 1) / COLS, hp = blockIdx.x % (H * pb), r = blockIdx.x / (H * pb), h = hp % H, p0 = hp / H * COLS;
   const int g = h / (H / G);
   const int inner = H * P;
   const float bias = dt_bias[h], neg_a = -expf(a_log[h]), dsk = dskip[h];
@@ -425,7 +428,7 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
           for (int u = 0; u < SPLIT / 2; ++u) {
             if (u >= left) break;
             const float keep = up ? ys[2 * u + 1][c] : ys[2 * u][c], give = up ? ys[2 * u][c] : ys[2 * u + 1][c];
-            ys[u][c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            ys[u][c] = keep + __shfl_xor_sync(0xffffffffu, give, o * CPW);
           }
         }
         if (active[c])
@@ -439,7 +442,7 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
 #pragma unroll
       for (int c = 0; c < SCOL_CP; ++c) {
 #pragma unroll
-        for (int o = 1; o < SPLIT; o <<= 1) ys[c] += __shfl_xor_sync(0xffffffffu, ys[c], o);
+        for (int o = 1; o < SPLIT; o <<= 1) ys[c] += __shfl_xor_sync(0xffffffffu, ys[c], o * CPW);
         if (active[c] && q == 0)
           y[(size_t)(first + t0 + tt) * ldy + h * P + p0 + col + c * half] = ys[c] + dsk * X[tt * COLS + c * half];
       }
@@ -517,7 +520,9 @@ GB_OP(gb_op_ssm_scan) {
     const int threads = (long long)R * H * gb_div_up(P, SCOL_CP * 128 / split) >= 148 ? 128 : 64;
     const int cols = SCOL_CP * threads / split;
     const size_t smem_cols = sizeof(float) * (2 * (size_t)SCOL_TOKENS * (2 * SCOL_NV * split + cols) + 4 * SCOL_TOKENS);
-    const dim3 grid_cols(R, H, gb_div_up(P, cols));
+    // (a request's blocks follow one another, so that a long portion's are spread over all SMs: with the requests as the
+    // fastest dimension every other SM got all of a long portion's blocks and the rest those of a short one)
+    const dim3 grid_cols((unsigned)((long long)R * H * gb_div_up(P, cols)));
 #define SCOL_LAUNCH(SP)                                                                                               \
     gb_launch(ssm_scan_cols_kernel<SP>, grid_cols, dim3(threads), smem_cols, ctx->stream, op_ptr<const float>(a[0]), \
               a[1], op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<const float>(a[5]),              \
