@@ -97,10 +97,25 @@ __global__ void stream_kernel(StreamParams p, int streams) {
       for (int i = 0; i < S * S; ++i) m[i] = w_mix[i];
     }
   }
+  const int pieces = p.dim / VEC;
+  // (the gain of the pieces a thread keeps: on hand before the sublayer has finished, pinned, see gb_pin)
+  float gain[STREAM_CACHE][VEC];
+#pragma unroll
+  for (int c = 0; c < STREAM_CACHE; ++c) {
+    const int i = threadIdx.x + c * blockDim.x;
+    Piece<VEC> g;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) g.v[e] = 0.f;
+    if (p.gain && i < pieces) g.load(p.gain + (size_t)i * VEC);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      gain[c][e] = g.v[e];
+      gb_pin(gain[c][e]);
+    }
+  }
   pdl_wait();
   float* x = p.x + (size_t)src * p.ldx;
   const float* y = MIX ? p.y + (size_t)r * p.ldy : nullptr;
-  const int pieces = p.dim / VEC;
   float cache[STREAM_CACHE][VEC];
   float ss = 0.f;
   auto read = [&](const Piece<VEC>* v, float* u) {
@@ -128,12 +143,12 @@ __global__ void stream_kernel(StreamParams p, int streams) {
         const float* at = p.part + (size_t)r * p.dim + (size_t)i * VEC;
 #pragma unroll
         for (int e = 0; e < VEC; ++e) yy.v[e] = 0.f;
-        for (int s0 = 0; s0 < p.splits; s0 += 4) {         // (four requested together, added in order)
-          Piece<VEC> t[4];
+        for (int s0 = 0; s0 < p.splits; s0 += 8) {         // (eight requested together, added in order)
+          Piece<VEC> t[8];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) t[u].load(at + (size_t)min(s0 + u, p.splits - 1) * p.part_stride);
+          for (int u = 0; u < 8; ++u) t[u].load(at + (size_t)min(s0 + u, p.splits - 1) * p.part_stride);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
+          for (int u = 0; u < 8; ++u)
             if (s0 + u < p.splits) {
 #pragma unroll
               for (int e = 0; e < VEC; ++e) yy.v[e] += t[u].v[e];
@@ -192,9 +207,7 @@ __global__ void stream_kernel(StreamParams p, int streams) {
   for (int c = 0; c < STREAM_CACHE; ++c) {
     const int i = threadIdx.x + c * blockDim.x;
     if (i >= pieces) continue;
-    Piece<VEC> g;
-    g.load(p.gain + (size_t)i * VEC);
-    store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, cache[c], rstd, g.v);
+    store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, cache[c], rstd, gain[c]);
   }
   // (a row too long for the registers: what this thread wrote is read again)
   for (int i = threadIdx.x + STREAM_CACHE * blockDim.x; i < pieces; i += blockDim.x) {
@@ -216,7 +229,12 @@ int launch_streams(const StreamParams& p, int n, int streams, cudaStream_t strea
   const bool vec = p.dim % 4 == 0 && p.ldx % 4 == 0 && p.ldy % 4 == 0 && (bits & 15) == 0 &&
                    ((uintptr_t)p.out & (p.out_dtype == GB_BF16 ? 7 : 15)) == 0;
   const int pieces = vec ? p.dim / 4 : p.dim;
-  const dim3 block(pieces <= 64 ? 64 : pieces <= 256 ? 128 : 256);
+  // A few rows (fewer than half of the SMs) of up to four streams: a piece a thread, so that all of a row is asked for at once
+  // (a thread's second piece waits behind the stores of its first); 2 rows of 4 x 2048 in a decode step, with the gain
+  // read ahead: 4.4 us against 5.3 with two pieces a thread.  With many rows the wider blocks are slower (2134 rows: 61 us
+  // against 39), and more streams need more registers than 512 threads have.
+  const bool few = n <= 74 && streams <= 4 && vec;
+  const dim3 block(pieces <= 64 ? 64 : few ? 32 * (pieces < 512 ? gb_div_up(pieces, 32) : 16) : pieces <= 256 ? 128 : 256);
 #define STREAMS(S)                                                                                       \
   do {                                                                                                   \
     if (MIX && p.part) {                                                                                 \
