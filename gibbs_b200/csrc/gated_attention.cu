@@ -87,7 +87,8 @@ enum { PREP_NORM_WHOLE = 1, PREP_Q_BF16 = 2, PREP_PAGES_BF16 = 4, PREP_NORM_HEAD
 // (2i, 2i+1) or, with `halves`, in pairs (i, i + rot_dims/2); cosines and sines are multiplied by mscale.
 __device__ __forceinline__ float prep_element(const float* x, const float* __restrict__ gain, bool gain_per_head,
                                               float rstd, int base, int d, int rot_dims, bool halves,
-                                              const float* __restrict__ inv_freq, int pos, float mscale) {
+                                              const float* __restrict__ inv_freq, int pos, float mscale,
+                                              const float2* trig = nullptr) {
   const int gb = gain_per_head ? 0 : base;
   const float own = x[base + d] * rstd * (gain ? gain[gb + d] : 1.f);
   if (d >= rot_dims) return own;
@@ -96,8 +97,15 @@ __device__ __forceinline__ float prep_element(const float* x, const float* __res
   const int partner = halves ? (second ? d - half : d + half) : (d ^ 1);
   const int fi = halves ? (second ? d - half : d) : (d >> 1);
   const float other = x[base + partner] * rstd * (gain ? gain[gb + partner] : 1.f);
-  const float ang = (float)pos * inv_freq[fi];
-  const float c = cosf(ang) * mscale, s = sinf(ang) * mscale;
+  float c, s;
+  if (trig != nullptr) {
+    c = trig[fi].x;
+    s = trig[fi].y;
+  } else {
+    const float ang = (float)pos * inv_freq[fi];
+    c = cosf(ang) * mscale;
+    s = sinf(ang) * mscale;
+  }
   // the pair (u, v) becomes (u c - v s, v c + u s)
   return second ? own * c + other * s : own * c - other * s;
 }
@@ -105,7 +113,13 @@ __device__ __forceinline__ float prep_element(const float* x, const float* __res
 // One block per token.  A query head is `maps` heads of `dim` entries side by side (one for an ordinary
 // attention), and so is a key head: a key row in the pages holds them all.  A warp takes one head of `dim`
 // entries at a time: its norm (when heads are normed one by one), then its elements.
-template <typename TC, typename TQ>
+// FEW (steps of a few tokens): gridDim.y blocks share a token's heads, and the angles' cosines and sines (up to
+// PREP_PAIRS) are in shared memory before the product in front has finished.  Measured, 2 tokens of 32 + 8 heads of 64:
+// 6.1 us a launch in a decode step against 7.7 with one block a token.  (With many tokens a table per block was slower than
+// angles worked out by every head: the blocks that wait for it hold the SM.)
+constexpr int PREP_PAIRS = 128, PREP_FEW = 64;
+
+template <typename TC, typename TQ, bool FEW>
 __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, long long ld, int k_col, int v_col, const float* __restrict__ q_gain,
                                const float* __restrict__ k_gain, const float* __restrict__ inv_freq, int rot_dims,
                                const int* tok_req, const int* tok_pos, const int* block_table, int bt_stride,
@@ -126,6 +140,19 @@ __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, lon
   const float mscale = rot_dims > 0 ? inv_freq[rot_dims >> 1] : 1.f;
   int page = -1;
   if (writes) page = block_table[(size_t)tok_req[t] * bt_stride + pos / page_size];
+  __shared__ float2 trig_table[FEW ? PREP_PAIRS : 1];
+  const float2* trig = nullptr;
+  if constexpr (FEW) {
+    if ((rot_dims >> 1) <= PREP_PAIRS) {
+      for (int i = threadIdx.x; i < (rot_dims >> 1); i += blockDim.x) {
+        const float ang = (float)pos * inv_freq[i];
+        trig_table[i] = make_float2(cosf(ang) * mscale, sinf(ang) * mscale);
+      }
+      __syncthreads();
+      trig = trig_table;
+    }
+  }
+  const int part = FEW ? blockIdx.y : 0, parts = FEW ? gridDim.y : 1;
   pdl_wait();
   const float* row = fused + (size_t)t * ld;
   const int nq = H * maps * dim, nk = G * maps * dim;
@@ -141,7 +168,7 @@ __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, lon
     }
   }
   const bool normed = whole || per_head;
-  for (int h = warp; h < H * maps; h += warps) {
+  for (int h = warp + part * warps; h < H * maps; h += warps * parts) {
     float rstd = q_rstd;
     if (per_head) {
       float ss = 0.f;
@@ -152,14 +179,16 @@ __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, lon
     if (after) {
       float ss = 0.f;
       for (int d = lane; d < dim; d += 32) {
-        const float v = prep_element(row, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale);
+        const float v = prep_element(row, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
+                                     trig);
         ss += v * v;
       }
       post = temp / sqrtf(warp_sum(ss) / (float)dim + eps);
     }
     for (int d = lane; d < dim; d += 32)
       q_out[(size_t)t * ldq + h * dim + d] = from_f32<TQ>(post * prep_element(row, normed ? q_gain : nullptr, per_head, rstd,
-                                                                              h * dim, d, rot_dims, halves, inv_freq, pos, mscale));
+                                                                              h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
+                                                                              trig));
   }
   if (!writes) return;
   if (page < 0 || page >= n_pages) {
@@ -167,7 +196,7 @@ __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, lon
     return;
   }
   const int slot = pos % page_size;
-  for (int h = warp; h < G * maps; h += warps) {
+  for (int h = warp + part * warps; h < G * maps; h += warps * parts) {
     const int g = h / maps, m = h - g * maps;
     float rstd = k_rstd;
     if (per_head) {
@@ -180,16 +209,17 @@ __global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, lon
     if (after) {
       float ss = 0.f;
       for (int d = lane; d < dim; d += 32) {
-        const float v = prep_element(row + k_col, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale);
+        const float v = prep_element(row + k_col, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
+                                     trig);
         ss += v * v;
       }
       post = 1.0f / sqrtf(warp_sum(ss) / (float)dim + eps);
     }
     for (int d = lane; d < dim; d += 32)
       dst[d] = from_f32<TC>(post * prep_element(row + k_col, normed ? k_gain : nullptr, per_head, rstd, h * dim, d, rot_dims,
-                                                halves, inv_freq, pos, mscale));
+                                                halves, inv_freq, pos, mscale, trig));
   }
-  for (int i = threadIdx.x; i < G * vdim; i += blockDim.x) {
+  for (int i = threadIdx.x + part * blockDim.x; i < G * vdim; i += blockDim.x * parts) {
     const int g = i / vdim, d = i - g * vdim;
     v_pages[(((size_t)page * G + g) * page_size + slot) * vdim + d] = from_f32<TC>(row[v_col + i]);
   }
@@ -536,8 +566,12 @@ GB_OP(gb_op_qk_prep) {
   const int threads = H * maps * dim >= 2048 ? 512 : 256;
   const long long ldq = (long long)H * maps * dim;
   const int mode = flags & (PREP_NORM_WHOLE | PREP_NORM_HEAD | PREP_ROT_HALVES | PREP_NORM_AFTER);
+  const bool few = n <= PREP_FEW;
+  // (a warp a query head or two; the key heads and values come on top)
+  const int parts = H * maps >= 4 * (threads / 32) ? 4 : gb_div_up(H * maps, threads / 32);
 #define PREP(TC, TQ)                                                                                                     \
-  gb_launch(qk_prep_kernel<TC, TQ>, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2],    \
+  gb_launch(few ? qk_prep_kernel<TC, TQ, true> : qk_prep_kernel<TC, TQ, false>, few ? dim3(n, parts) : dim3(n),           \
+            dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2],                                     \
             (int)a[3], op_ptr<const float>(a[4]), op_ptr<const float>(a[5]), op_ptr<const float>(a[6]), (int)a[7],        \
             op_ptr<const int>(a[8]), op_ptr<const int>(a[9]), op_ptr<const int>(a[10]), (int)a[11], (int)a[12],           \
             op_ptr<TC>(a[13]), op_ptr<TC>(a[14]), (int)a[15], H, G, dim, vdim, maps, mode, (float)f[0], (float)f[1], \
