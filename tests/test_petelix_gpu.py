@@ -487,3 +487,42 @@ def test_tensor_core_attention_against_the_generic_kernel(cfg, layer, monkeypatc
         outs[on] = hz.run_cut("r", h, [150, 3, 1, 1, 90, 1, 64, 2, 1])
         check_rows(outs[on], want, "bfloat16", what=f"tensor cores {on}")
     assert rel_rows(outs[True], outs[False]).max() < 1.5e-2
+
+
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("longest,vdim", [(300, 40), (4100, 33), (20000, 64), (20000, 256)])
+def test_chunks_of_keys_are_merged_whatever_their_number(longest, vdim, sink):
+    """Contexts that fill one chunk, some or nearly all of 2 to 79 (an upper bound on the context decides), the others
+    empty, against 64 bits: a score is off by (dim + 4) 2^-24 scale |q|.|k| at most, a weight by exp of twice that and
+    2^-20, the sums by (keys + chunks + 64) 2^-24."""
+    from gibbs_b200.ops import hybrid, library
+    torch.manual_seed(longest + vdim)
+    H, G, dim, ps, pos = 4, 2, 16, 16, [0, 299, 255 if longest == 300 else 2500]
+    n, blocks = len(pos), max(pos) // 16 + 1
+    kp, vp = torch.randn(n * blocks, G, ps, dim), torch.randn(n * blocks, G, ps, vdim)
+    table = torch.randperm(n * blocks).reshape(n, blocks)
+    q, gate = torch.randn(n, H * dim), torch.randn(n, H * vdim)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    lib = library("hybrid")
+    ws = torch.full((lib.gb_sink_attention_workspace_rows(), vdim + 2), float("nan"), device=DEV)
+    dev = [t.to(DEV) for t in (q, kp, vp, gate)]
+    ints = [i32(table.tolist()), i32(list(range(n))), i32(pos)]
+    out = torch.full((n, H * vdim), float("nan"), device=DEV)
+    scale = dim ** -0.5
+    launched = hybrid.call("sink_attention", [dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), ints[0].data_ptr(), blocks, ps,
+                                              n * blocks, ints[1].data_ptr(), ints[2].data_ptr(), dev[3].data_ptr(), H * vdim,
+                                              out.data_ptr(), H * vdim, n, H, G, dim, vdim, 0, longest, ws.data_ptr()],
+                           [scale, 0.0, 0.0], flags=1 if sink else 0)
+    assert launched == 2                                 # (the attention and the merge)
+    for t in range(n):
+        j = torch.arange(pos[t] + 1)
+        for h in range(H):
+            k, v = kp[table[t][j // ps], h // 2, j % ps].double(), vp[table[t][j // ps], h // 2, j % ps].double()
+            qh = q[t, h * dim:(h + 1) * dim].double()
+            sc = k @ qh * scale
+            w = torch.softmax(torch.cat([sc, torch.zeros(1, dtype=F64)]) if sink else sc, 0)[:len(j)]
+            f = torch.sigmoid(gate[t, h * vdim:(h + 1) * vdim].double())
+            d = (dim + 4) * 2.0 ** -24 * scale * float((k.abs() @ qh.abs()).max())
+            tol = (2 * (2 * d + 2.0 ** -20) + (len(j) + 79 + 64) * 2.0 ** -24) * (w @ v.abs()) * f
+            err = (out[t, h * vdim:(h + 1) * vdim].double().cpu() - (w @ v) * f).abs()
+            assert (err <= tol).all(), (t, h)
