@@ -437,44 +437,60 @@ paged_attention_kernel(const T* q, long long ldq, const T* k_pages,
 // warp i mod warps) and their states are merged in order at the end, so a result depends on the query's
 // position only, however the batch was cut.  A tile's keys and values are requested together, row by row in
 // 16-byte pieces; lane j takes key j's scores for all the heads, then the lanes spread over the dimensions
-// for the weighted sum.  Bound by the trip to memory and the chain behind it: a warp per head with a lane
-// walking whole rows of its own keys (the kernel above, still the one for other row lengths) waited for one
-// trip after the other.  Measured in steps of 2 tokens at contexts of 75 to 158 and one prompt of 225 tokens,
-// 24 heads of 64 over 8: 83 -> 19 us a launch on average; 3 tokens, 3 heads of 32 over 1: 13 -> 6 us.
-constexpr int AF_HEADS = 4, AF_KT = 32;
+// for the weighted sum.  Up to one, two or four heads a block by the group's size, so that a group of one does not pay for four.
+// Bound by the trip to memory and the chain behind it: a warp per head with a lane walking whole rows of its own keys (the
+// kernel above, still the one for other row lengths) waited for one trip after the other.  Measured (us, that kernel -> this
+// one), 24 heads of 64 over 8: 2 tokens of 110 keys 44 -> 8.0, 8 of 1024 331 -> 29, a prompt of 225 447 -> 95, of 2048 23,720 ->
+// 3,389; 3 heads of 32 over 1, 2 tokens of 110: 23 -> 6.1; a prompt of 64, 8 heads of 64 over 8: 27.9 -> 24.8.
+// A score is added in four chains and every AF_KG keys have a sum of their own: against 64 bits the results are off by 0.62
+// of what that kernel's are (mean over 187 steps of 1 to 2048 tokens and 11 layer sizes; the largest 1.01).  With one chain a
+// score and one over all of a warp's keys it was 1.05 to 2.1 times.
+constexpr int AF_KT = 32, AF_KG = 8;
 
 inline int af_warps(int hd) { return hd <= 64 ? 8 : (hd <= 128 ? 4 : 2); }        // (as many tiles as shared memory takes)
-inline int af_warp_floats(int hd) { return AF_KT * (hd + 4) + AF_KT * hd + AF_KT * AF_HEADS; }
+inline int af_warp_floats(int hd, int heads) { return AF_KT * (hd + 4) + AF_KT * hd + AF_KT * heads; }
 
-template <int DL>                                      // dimensions a lane: head sizes up to 32 * DL
-__global__ void __launch_bounds__(256)
+// Two 32-bit multiply-adds side by side, each rounded as fmaf's.
+typedef unsigned long long af_f2;
+__device__ __forceinline__ void af_fma2(af_f2& acc, af_f2 a, af_f2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float af_sum2(af_f2 v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+
+template <int DL, int HEADS>                           // dimensions a lane (head sizes up to 32 * DL), heads a block
+__global__ void __launch_bounds__(256, DL == 1 ? 3 : 1)
 paged_attention_f32_kernel(const float* q, long long ldq, const float* k_pages, const float* v_pages, const int* block_table,
                            int bt_stride, int page_size, int n_pages, const int* tok_req, const int* tok_pos,
                            float* __restrict__ out, long long ldo, int group, int kv_heads, int hd, float scale,
                            float softcap, int window, int* __restrict__ status) {
+  struct alignas(4 * HEADS) Weights { float v[HEADS]; };
   extern __shared__ __align__(16) float sm[];
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int t = blockIdx.x, kvh = blockIdx.y, g0 = blockIdx.z * AF_HEADS;
-  const int live_heads = min(AF_HEADS, group - g0), h0 = kvh * group + g0;
-  float* qs = sm;                                                            // [AF_HEADS][hd]
-  const int warp_floats = AF_KT * (hd + 4) + AF_KT * hd + AF_KT * AF_HEADS;
-  float* ks = sm + AF_HEADS * hd + warp * warp_floats;                       // [AF_KT][hd + 4]: this warp's
+  const int t = blockIdx.x, kvh = blockIdx.y, g0 = blockIdx.z * HEADS;
+  const int live_heads = min(HEADS, group - g0), h0 = kvh * group + g0;
+  float* qs = sm;                                                            // [HEADS][hd]
+  const int warp_floats = AF_KT * (hd + 4) + AF_KT * hd + AF_KT * HEADS;
+  float* ks = sm + HEADS * hd + warp * warp_floats;                       // [AF_KT][hd + 4]: this warp's
   float* vs = ks + AF_KT * (hd + 4);                                         // [AF_KT][hd]
-  float* ps = vs + AF_KT * hd;                                               // [AF_KT][AF_HEADS]
+  float* ps = vs + AF_KT * hd;                                               // [AF_KT][HEADS]
   const int pos = tok_pos[t];
   const int* bt = block_table + (size_t)tok_req[t] * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   const int pieces = hd >> 2;
   pdl_wait();
-  for (int i = threadIdx.x; i < AF_HEADS * hd; i += blockDim.x) {
+  for (int i = threadIdx.x; i < HEADS * hd; i += blockDim.x) {
     const int g = i / hd;
     qs[i] = g < live_heads ? q[(size_t)t * ldq + (size_t)(h0 + g) * hd + (i - g * hd)] : 0.f;
   }
   __syncthreads();
-  float m[AF_HEADS], l[AF_HEADS], o[AF_HEADS][DL];
+  float m[HEADS], l[HEADS], o[HEADS][DL];
 #pragma unroll
-  for (int g = 0; g < AF_HEADS; ++g) {
+  for (int g = 0; g < HEADS; ++g) {
     m[g] = -INFINITY;
     l[g] = 0.f;
 #pragma unroll
@@ -507,24 +523,25 @@ paged_attention_f32_kernel(const float* q, long long ldq, const float* k_pages, 
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    float s[AF_HEADS];
+    float s[HEADS];
+    af_f2 dot[HEADS][2];                                 // four chains a score
 #pragma unroll
-    for (int g = 0; g < AF_HEADS; ++g) s[g] = 0.f;
+    for (int g = 0; g < HEADS; ++g) dot[g][0] = dot[g][1] = 0;
     const float* kr = ks + lane * (hd + 4);
 #pragma unroll 4
     for (int c = 0; c < pieces; ++c) {
-      const float4 kv = *reinterpret_cast<const float4*>(kr + 4 * c);
+      const ulonglong2 kv = *reinterpret_cast<const ulonglong2*>(kr + 4 * c);
 #pragma unroll
-      for (int g = 0; g < AF_HEADS; ++g) {
-        const float4 qv = *reinterpret_cast<const float4*>(qs + g * hd + 4 * c);
-        s[g] = fmaf(qv.x, kv.x, s[g]);
-        s[g] = fmaf(qv.y, kv.y, s[g]);
-        s[g] = fmaf(qv.z, kv.z, s[g]);
-        s[g] = fmaf(qv.w, kv.w, s[g]);
+      for (int g = 0; g < HEADS; ++g) {
+        const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qs + g * hd + 4 * c);
+        af_fma2(dot[g][0], qv.x, kv.x);
+        af_fma2(dot[g][1], qv.y, kv.y);
       }
     }
 #pragma unroll
-    for (int g = 0; g < AF_HEADS; ++g) {
+    for (int g = 0; g < HEADS; ++g) s[g] = af_sum2(dot[g][0]) + af_sum2(dot[g][1]);
+#pragma unroll
+    for (int g = 0; g < HEADS; ++g) {
       float v = s[g] * scale;
       if (softcap > 0.f) v = softcap * tanhf(v / softcap);         // scores squashed into (-cap, cap)
       const float m_new = fmaxf(m[g], warp_max(row >= 0 ? v : -INFINITY));
@@ -536,48 +553,61 @@ paged_attention_f32_kernel(const float* q, long long ldq, const float* k_pages, 
       for (int e = 0; e < DL; ++e) o[g][e] *= corr;
       s[g] = p;
     }
-    *reinterpret_cast<float4*>(ps + lane * AF_HEADS) = make_float4(s[0], s[1], s[2], s[3]);
+    Weights mine;
+#pragma unroll
+    for (int g = 0; g < HEADS; ++g) mine.v[g] = s[g];
+    *reinterpret_cast<Weights*>(ps + lane * HEADS) = mine;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
     const int n = min(AF_KT, pos - k0 + 1);
-#pragma unroll 4
-    for (int j = 0; j < n; ++j) {
-      const float4 p = *reinterpret_cast<const float4*>(ps + j * AF_HEADS);
+    for (int j0 = 0; j0 < n; j0 += AF_KG) {              // AF_KG keys have a sum of their own
+      float part[HEADS][DL];
 #pragma unroll
-      for (int e = 0; e < DL; ++e) {
-        const int d = lane + 32 * e;
-        const float v = d < hd ? vs[j * hd + d] : 0.f;
-        o[0][e] = fmaf(p.x, v, o[0][e]);
-        o[1][e] = fmaf(p.y, v, o[1][e]);
-        o[2][e] = fmaf(p.z, v, o[2][e]);
-        o[3][e] = fmaf(p.w, v, o[3][e]);
+      for (int g = 0; g < HEADS; ++g)
+#pragma unroll
+        for (int e = 0; e < DL; ++e) part[g][e] = 0.f;
+#pragma unroll
+      for (int u = 0; u < AF_KG; ++u) {
+        if (j0 + u >= n) break;
+        const Weights w = *reinterpret_cast<const Weights*>(ps + (j0 + u) * HEADS);
+#pragma unroll
+        for (int e = 0; e < DL; ++e) {
+          const int d = lane + 32 * e;
+          const float v = d < hd ? vs[(j0 + u) * hd + d] : 0.f;
+#pragma unroll
+          for (int g = 0; g < HEADS; ++g) part[g][e] = fmaf(w.v[g], v, part[g][e]);
+        }
       }
+#pragma unroll
+      for (int g = 0; g < HEADS; ++g)
+#pragma unroll
+        for (int e = 0; e < DL; ++e) o[g][e] += part[g][e];
     }
   }
-  // every warp leaves its state where its keys were: [AF_HEADS][hd] sums, then maxima and denominators
+  // every warp leaves its state where its keys were: [HEADS][hd] sums, then maxima and denominators
   __syncwarp();
 #pragma unroll
-  for (int g = 0; g < AF_HEADS; ++g) {
+  for (int g = 0; g < HEADS; ++g) {
     const float total = warp_sum(l[g]);
 #pragma unroll
     for (int e = 0; e < DL; ++e)
       if (lane + 32 * e < hd) ks[g * hd + lane + 32 * e] = o[g][e];
     if (lane == 0) {
-      ks[AF_HEADS * hd + g] = m[g];
-      ks[AF_HEADS * (hd + 1) + g] = total;
+      ks[HEADS * hd + g] = m[g];
+      ks[HEADS * (hd + 1) + g] = total;
     }
   }
   __syncthreads();
-  const float* states = sm + AF_HEADS * hd;
+  const float* states = sm + HEADS * hd;
   for (int i = threadIdx.x; i < live_heads * hd; i += blockDim.x) {
     const int g = i / hd, d = i - g * hd;
     float m_all = -INFINITY;
-    for (int w = 0; w < warps; ++w) m_all = fmaxf(m_all, states[(size_t)w * warp_floats + AF_HEADS * hd + g]);
+    for (int w = 0; w < warps; ++w) m_all = fmaxf(m_all, states[(size_t)w * warp_floats + HEADS * hd + g]);
     float sum = 0.f, v = 0.f;
     for (int w = 0; w < warps; ++w) {
       const float* st = states + (size_t)w * warp_floats;
-      const float mw = st[AF_HEADS * hd + g], f = mw == -INFINITY ? 0.f : expf(mw - m_all);
-      sum += st[AF_HEADS * (hd + 1) + g] * f;
+      const float mw = st[HEADS * hd + g], f = mw == -INFINITY ? 0.f : expf(mw - m_all);
+      sum += st[HEADS * (hd + 1) + g] * f;
       v += st[g * hd + d] * f;
     }
     const float inv = sum > 0.f ? 1.0f / sum : 0.f;
@@ -585,17 +615,17 @@ paged_attention_f32_kernel(const float* q, long long ldq, const float* k_pages, 
   }
 }
 
-template <int DL>
+template <int DL, int HEADS>
 cudaError_t launch_attention_f32(const float* q, long long ldq, const float* k_pages, const float* v_pages, const int* block_table,
                                  int bt_stride, int page_size, int n_pages, const int* tok_req, const int* tok_pos, float* out,
                                  long long ldo, int n_tokens, int heads, int kv_heads, int hd, float scale, float softcap,
                                  int window, int* status, cudaStream_t stream) {
   const int warps = af_warps(hd), group = heads / kv_heads;
-  const int smem = (AF_HEADS * hd + warps * af_warp_floats(hd)) * (int)sizeof(float);
-  auto kernel = paged_attention_f32_kernel<DL>;
+  const int smem = (HEADS * hd + warps * af_warp_floats(hd, HEADS)) * (int)sizeof(float);
+  auto kernel = paged_attention_f32_kernel<DL, HEADS>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  return gb_launch(kernel, dim3(n_tokens, kv_heads, gb_div_up(group, AF_HEADS)), dim3(32 * warps), smem, stream, q, ldq,
+  return gb_launch(kernel, dim3(n_tokens, kv_heads, gb_div_up(group, HEADS)), dim3(32 * warps), smem, stream, q, ldq,
                    k_pages, v_pages, block_table, bt_stride, page_size, n_pages, tok_req, tok_pos, out, ldo, group,
                    kv_heads, hd, scale, softcap, window, status);
 }
@@ -703,8 +733,12 @@ GB_API int gb_paged_attention(const void* q, int dtype, long long ldq, const voi
   // (rows of whole 16-byte pieces; the grid's limits hold for any pool that fits the card)
   if (dtype == GB_F32 && hd % 4 == 0 && ((uintptr_t)k_pages & 15) == 0 && ((uintptr_t)v_pages & 15) == 0 &&
       kv_heads <= 65535 && heads / kv_heads <= 65535) {
-    auto launch = hd <= 32 ? launch_attention_f32<1> : hd <= 64 ? launch_attention_f32<2> : hd <= 128 ? launch_attention_f32<4>
-                                                                                                       : launch_attention_f32<8>;
+#define AF_LAUNCH(HEADS)                                                                                   \
+  (hd <= 32 ? launch_attention_f32<1, HEADS> : hd <= 64 ? launch_attention_f32<2, HEADS>                    \
+   : hd <= 128 ? launch_attention_f32<4, HEADS> : launch_attention_f32<8, HEADS>)
+    const int group = heads / kv_heads;
+    auto launch = group == 1 ? AF_LAUNCH(1) : group == 2 ? AF_LAUNCH(2) : AF_LAUNCH(4);
+#undef AF_LAUNCH
     const cudaError_t e = launch((const float*)q, ldq, (const float*)k_pages, (const float*)v_pages, block_table, bt_stride,
                                  page_size, n_pages, tok_req, tok_pos, (float*)out, ldo, n_tokens, heads, kv_heads, hd, scale,
                                  softcap, window, status, stream);

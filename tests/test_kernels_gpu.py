@@ -1094,6 +1094,32 @@ def test_float32_attention_at_the_edges_of_tiles_and_warps(hd, group):
             assert torch.equal(alone[0], out[i])
 
 
+@pytest.mark.parametrize("hd,group", [(16, 2), (32, 3), (64, 1), (64, 4), (128, 2), (256, 8)])
+def test_float32_attention_is_as_exact_as_the_general_kernel(hd, group):
+    """Both kernels against 64 bits over short and long contexts: the root of the summed squares of all errors.  (Pages
+    that do not lie on a 16-byte boundary run on the general kernel, which has 32 chains of keys a head.)"""
+    from gibbs_b200 import ops
+    torch.manual_seed(hd + group)
+    kvh, ps, n_pages = 2, 16, 512
+    heads, pos = kvh * group, [15, 63, 255, 256, 1000, 2047, 4095, 8191]
+    size = n_pages * kvh * ps * hd
+    store = [torch.randn(size + 1, device=DEV) for _ in range(2)]
+    q = torch.randn(len(pos), heads * hd, device=DEV)
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    bt, off = torch.randperm(n_pages).to(torch.int32)[None, :].to(DEV), {}
+    for first in (0, 1):
+        kp, vp = (s[first:first + size].view(n_pages, kvh, ps, hd) for s in store)
+        out, status = torch.empty_like(q), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.paged_attention(q, heads, kvh, hd, kp, vp, bt, t([0] * len(pos)), t(pos), hd ** -0.5, 0, out, status)
+        keys, vals = (p[bt[0].long()].transpose(1, 2).reshape(-1, kvh, hd).double() for p in (kp, vp))
+        off[first] = 0.0
+        for i, last in enumerate(pos):
+            sc = torch.einsum("ghd,lgd->ghl", q[i].double().reshape(kvh, group, hd), keys[:last + 1]) * hd ** -0.5
+            want = torch.einsum("ghl,lgd->ghd", torch.softmax(sc, -1), vals[:last + 1])
+            off[first] += float((out[i].double().reshape(kvh, group, hd) - want).pow(2).sum() / want.pow(2).sum())
+    assert off[0] <= off[1], (off[0] / off[1]) ** 0.5
+
+
 @pytest.mark.parametrize("vocab,k", [(1000, 5), (65536, 20), (50257, 1), (7, 32)])
 def test_logprob_info_matches_the_plain_rule(vocab, k):
     """Probability of the chosen token, entropy and the k most probable tokens of every row,
