@@ -173,6 +173,45 @@ def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H
             assert off[True] <= 1.25 ** 2 * off[False], (off[True] / off[False]) ** 0.5
 
 
+@pytest.mark.parametrize("H,r,dr", [(1, 32, 0), (2, 64, 0), (4, 64, 16), (16, 128, 0), (16, 128, 32), (8, 256, 32), (16, 512, 0), (16, 512, 64)])
+def test_latent_attention_with_whole_weights_is_no_further_off_than_the_generic_kernel(H, r, dr):
+    """Single tokens at short and long contexts and a short portion, with and without a window, on both kernels against
+    64 bits: the root of the summed squares of all errors."""
+    from gibbs_b200.ops import hybrid, library
+    torch.manual_seed(r + dr)
+    Dk, ps, blocks = r + dr, 16, 128
+    pages = torch.randn(3 * blocks, ps, Dk, device=DEV).to(torch.bfloat16)
+    table = torch.randperm(3 * blocks, device=DEV).reshape(3, blocks)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ws = torch.empty(library("hybrid").gb_latent_attention_workspace_rows(), r + 2, device=DEV)
+    scale, bt, off = 0.7 * Dk ** -0.5, table.to(torch.int32), {True: 0.0, False: 0.0}
+    for spans in ([(2000, 1), (900, 1), (299, 1)], [(0, 7), (300, 9), (1500, 5)]):
+        tok_req = [i for i, (p, k) in enumerate(spans) for _ in range(k)]
+        tok_pos = [p + j for p, k in spans for j in range(k)]
+        n = len(tok_req)
+        starts = i32([sum(k for _, k in spans[:i]) for i in range(3)])
+        tr, tp = i32(tok_req), i32(tok_pos)
+        for window in (0, 128, 1024):
+            for _ in range(4 if H < 8 else 1):
+                q, gate, sink = (torch.randn(*s, device=DEV) for s in ((n, H, Dk), (n, H), (H,)))
+                got = {}
+                for tc in (True, False):
+                    got[tc] = torch.empty(n, H * r, device=DEV)
+                    hybrid.call("latent_attention", [q.data_ptr(), pages.data_ptr(), 1, bt.data_ptr(), blocks, ps, 3 * blocks,
+                                                     tr.data_ptr(), tp.data_ptr(), gate.data_ptr(), H, got[tc].data_ptr(), H * r, n,
+                                                     H, r, dr, window, 2001, ws.data_ptr(), sink.data_ptr(), 3 if tc else 0,
+                                                     starts.data_ptr() if tc else 0], [scale])
+                assert not torch.equal(got[True], got[False])                # (two kernels did run)
+                for t in range(n):
+                    j = torch.arange(max(0, tok_pos[t] - window + 1) if window else 0, tok_pos[t] + 1, device=DEV)
+                    c = pages[table[tok_req[t]][j // ps], j % ps].double()
+                    sc = torch.cat([q[t].double() @ c.T * scale, sink.double()[:, None]], 1)
+                    want = (torch.softmax(sc, 1)[:, :-1] @ c[:, :r]) * torch.sigmoid(gate[t].double())[:, None]
+                    for tc in off:
+                        off[tc] += float((got[tc][t].double().view(H, r) - want).pow(2).sum() / want.pow(2).sum())
+    assert off[True] <= off[False], (off[True] / off[False]) ** 0.5
+
+
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
 def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
     """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
