@@ -463,7 +463,7 @@ latent_attention_kernel(const float* qp, const TC* pages, const int* block_table
 // exp(m_s - M) are worked out once into shared memory; then every thread has its columns and asks for
 // sixteen chunks' values at a time.  Bound by the trips to L2 (weights, then sums).  Measured, 2 tokens x 16 heads,
 // 32 chunks of 512: 6 us in a decode step, 37 to 40 with a warp per (token, head) that took one chunk after the other.
-constexpr int LM_CHUNKS = 64;                              // (gb_latent_attention_chunks gives no more)
+constexpr int LM_CHUNKS = 96;                              // (the cuts give 64 at most, and with a window up to three more)
 
 __global__ void latent_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate,
                                               float* out, long long ldo, int H, int r, const float* __restrict__ sink) {
@@ -475,18 +475,23 @@ __global__ void latent_attention_merge_kernel(const float* ws, int splits, const
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
   const size_t ld = (size_t)r + 2;
   const float* w = ws + (size_t)idx * splits * ld;
-  // (every warp takes the maxima and denominators for itself: lane s has chunks s and s + 32)
-  const float m0 = lane < splits ? w[lane * ld] : -INFINITY, m1 = lane + 32 < splits ? w[(lane + 32) * ld] : -INFINITY;
-  const float l0 = lane < splits ? w[lane * ld + 1] : 0.f, l1 = lane + 32 < splits ? w[(lane + 32) * ld + 1] : 0.f;
-  float M = warp_max(fmaxf(m0, m1));
+  // (every warp takes the maxima and denominators for itself: lane s has chunks s, s + 32 and s + 64)
+  float m[LM_CHUNKS / 32], l[LM_CHUNKS / 32], M = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < LM_CHUNKS / 32; ++i) {
+    const int s = lane + 32 * i;
+    m[i] = s < splits ? w[s * ld] : -INFINITY;
+    l[i] = s < splits ? w[s * ld + 1] : 0.f;
+    M = fmaxf(M, m[i]);
+  }
+  M = warp_max(M);
   if (sink) M = fmaxf(M, sink[h]);
-  const float e0 = m0 > -INFINITY ? expf(m0 - M) : 0.f, e1 = m1 > -INFINITY ? expf(m1 - M) : 0.f;
-  const float el0 = e0 * l0, el1 = e1 * l1;
   float L = sink ? expf(sink[h] - M) : 0.f;
-  for (int s = 0; s < splits; ++s) L += __shfl_sync(0xffffffffu, s < 32 ? el0 : el1, s & 31);      // in chunk order
-  if (threadIdx.x < 32) {
-    es[lane] = e0;
-    es[lane + 32] = e1;
+#pragma unroll
+  for (int i = 0; i < LM_CHUNKS / 32; ++i) {
+    const float e = m[i] > -INFINITY ? expf(m[i] - M) : 0.f, el = e * l[i];
+    for (int s = 32 * i; s < splits && s < 32 * i + 32; ++s) L += __shfl_sync(0xffffffffu, el, s & 31);      // in chunk order
+    if (threadIdx.x < 32) es[lane + 32 * i] = e;
   }
   __syncthreads();
   const float g = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + h]) : 1.f;
@@ -532,6 +537,7 @@ cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages,
 // The second of a launch's two kernels where the keys were cut: 2 (kernels launched), or a failure's code.
 static int launch_merge(const float* ws, int splits, const float* gate, long long ld_gate, float* out, long long ldo, int n,
                         int H, int r, const float* sink, cudaStream_t stream) {
+  if (splits > LM_CHUNKS) GB_FAIL(GB_ERR_ARG, "latent_attention_merge: %d chunks", splits);
   gb_launch(latent_attention_merge_kernel, dim3((unsigned)((long long)n * H)), dim3(r <= 128 ? 128 : r <= 256 ? 256 : 512), 0,
             stream, ws, splits, gate, ld_gate, out, ldo, H, r, sink);
   GB_CHECK_LAUNCH("latent_attention_merge");
@@ -559,6 +565,27 @@ GB_API int gb_latent_attention_chunks(int n, int H, int window, int max_ctx, int
   }
   *chunk_out = chunk;
   return gb_div_up(span, chunk);
+}
+// The same for the kernel with whole weights on tensor cores, which has one CTA an SM and row tiles of 32 rows: about two rounds
+// of CTAs.  It takes the rows of several tokens together, so its chunks lie at multiples of their length: a row tile's keys
+// (its tokens' positions and the window in front of the first) may begin and end inside one; none lies behind the longest
+// context.
+static int split_chunks(int n, int H, int window, int max_ctx, int* chunk_out) {
+  const long long tiles = (long long)n * gb_div_up(H, 32);
+  const int wanted = tiles <= 4 ? 64 : (int)(296 / tiles), longest = max_ctx > 0 ? max_ctx : 1;
+  if (wanted <= 1 || (window > 0 ? window : longest) <= 32) { *chunk_out = 32; return 1; }
+  int chunk, splits;
+  if (window > 0) {
+    chunk = 32 * gb_div_up(gb_div_up((long long)window + 31, wanted), 32);
+    splits = gb_div_up((long long)window + gb_div_up(31, H) + chunk - 1, chunk);
+    if (max_ctx > 0 && splits > gb_div_up(longest, chunk)) splits = gb_div_up(longest, chunk);
+  } else {
+    chunk = 64;
+    while (gb_div_up(longest, chunk) > wanted) chunk *= 2;
+    splits = gb_div_up(longest, chunk);
+  }
+  *chunk_out = chunk;
+  return splits;
 }
 // Rows of (latent size + 2) floats a launch's partial results may need, whatever its sizes.
 // (also: two partial results a row for a prompt of up to 2,048 tokens and 16 heads on the tensor-core kernel)
@@ -672,12 +699,8 @@ GB_OP(gb_op_latent_attention) {
   // below; one token each: 14 us against 38.
   if (a[22] && gb_latent_attention_split_takes(n, (int)a[21], H, r, dr, a[2] == GB_BF16, op_ptr<const void>(a[1]),
                                                op_ptr<const void>(a[0]), op_ptr<const void>(a[11]), a[12])) {
-    if (n > (int)a[21] && splits > 1) {
-      // portions: a row tile's keys span its tokens' positions and the window in front of the first
-      const int span = a[17] > 0 ? (int)(a[17] < a[18] ? a[17] : a[18]) + gb_div_up(32, H) : (int)a[18];
-      chunk = 32 * gb_div_up(gb_div_up(span, splits), 32);
-      splits = gb_div_up(span, chunk);
-    }
+    splits = split_chunks(n, H, (int)a[17], (int)a[18], &chunk);
+    if (ws == nullptr || (long long)n * H * splits > gb_latent_attention_workspace_rows()) splits = 1;
     const cudaError_t e = gb_latent_attention_split_launch(
         op_ptr<const float>(a[0]), op_ptr<const bf16>(a[1]), op_ptr<const int>(a[3]), (int)a[4], (int)a[5], (int)a[6],
         op_ptr<const int>(a[7]), op_ptr<const int>(a[8]), op_ptr<const int>(a[22]), op_ptr<const float>(a[9]), a[10],

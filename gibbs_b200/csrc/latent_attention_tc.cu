@@ -327,8 +327,9 @@ template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStrea
 //  warp takes 16 rows x 32 keys over its quarter (the queries' three terms would otherwise be read from shared memory
 //  by every warp: 3 x 37 KB a tile), the four partial scores are added in shared memory, eight threads a row keep the
 //  maximum and the sum in 32-bit and leave the weights' three terms there.  For O a slice is a quarter of the latent's
-//  columns.  With `splits`, blockIdx.y takes `chunk` keys counted from the tile's first visible one and leaves
-//  (maximum, sum, weighted sum) per row for the merge kernel.
+//  columns.  Key tiles lie at multiples of 32, so a row's sums are grouped by its position alone, whatever the rows
+//  beside it.  With `splits`, blockIdx.y takes a chunk of keys, a multiple of `chunk` from position 0, and leaves (maximum,
+//  sum, weighted sum) per row for the merge kernel.
 //  Bound by the shared-memory reads of the tensor operands (about 2,700 cycles a tile of 32 x 32 at 512 + 64 entries
 //  against 1,600 of mma.sync).
 constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLD = 36, LTX_PLD = 40;
@@ -408,8 +409,20 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
   const int pos0 = pos_req + row0 / H, kmax = pos_req + (row0 + rows_live - 1) / H;
   const int* table = p.block_table + (size_t)p.tok_req[first] * p.bt_stride;
   const int base = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
-  const int k_begin = p.splits > 1 ? base + (int)blockIdx.y * p.chunk : base;
-  const int k_end = p.splits > 1 ? min(kmax, k_begin + p.chunk - 1) : kmax;          // (the last key)
+  // (key tiles lie at multiples of 32 and chunks at multiples of `chunk`, whatever row the tile begins with; the last chunk
+  // takes what is left)
+  const int origin = p.splits > 1 ? base / p.chunk * p.chunk + (int)blockIdx.y * p.chunk : 0;
+  const int k_begin = max(origin, base / LTX_KEYS * LTX_KEYS);
+  const int k_end = (int)blockIdx.y + 1 < p.splits ? min(kmax, origin + p.chunk - 1) : kmax;      // (the last key)
+  if (k_begin > k_end) {                                   // (splits > 1) no row sees a key of this chunk: the merge skips it
+    pdl_wait();
+    if (tid < rows_live) {
+      float* w = p.ws + (((size_t)first * H + row0 + tid) * p.splits + blockIdx.y) * (size_t)(r + 2);
+      w[0] = -INFINITY;
+      w[1] = 0.f;
+    }
+    return;
+  }
   // zeros where nothing is copied: columns dk .. stride
   const int pad = (STRIDE - dk) >> 3;
   for (int i = tid; i < (3 * LTX_ROWS + 2 * LTX_KEYS) * pad; i += 256)
@@ -420,7 +433,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     bf16* dst = Cs + (size_t)b * LTX_KEYS * STRIDE;
 #pragma unroll
     for (int u = 0; u < LTX_KEYS / 8; ++u) {
-      const int j = warp + 8 * u, key = min(k0 + j, k_end);               // (rows behind the last key are masked)
+      const int j = warp + 8 * u, key = min(max(k0 + j, base), k_end);    // (rows in front of the first key and behind the last are masked)
       const int page = table[key / p.page_size];
       const bool bad = page < 0 || page >= p.n_pages;
       if (bad && lane == 0) atomicExch(p.status, LTC_BAD_PAGE_READ);
@@ -433,7 +446,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     ltc_commit();
   };
   pdl_wait();
-  if (k_begin <= k_end) stage(k_begin, 0);
+  stage(k_begin, 0);
   {
     // (a warp asks for two rows at once: up to ten trips to L2 side by side)
     const float* src = p.qp + ((size_t)first * H + row0) * dk;
@@ -620,7 +633,6 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
       w[0] = m;                                            // (-inf: a chunk without keys)
       w[1] = l;
     }
-    if (k_begin > k_end) return;                           // (the merge does not read a sum without keys)
   } else if ((tid & 7) == 0 && srow < rows_live) {
     const size_t flat = flat0 + srow, t = flat / H;
     const int h = (int)(flat - t * H);
@@ -823,7 +835,8 @@ bool gb_latent_attention_split_takes(int n, int R, int H, int r, int dr, bool pa
          ((uintptr_t)out & 7) == 0 && ldo % 2 == 0;
 }
 
-// The keys are cut into `splits` chunks of `chunk` (a multiple of the key tile) counted from a tile's first visible key.
+// `splits` chunks of `chunk` keys (a multiple of the key tile), from the one that holds a row tile's first visible key on; the
+// last takes all that follow.
 cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages, const int* block_table, int bt_stride,
                                              int page_size, int n_pages, const int* tok_req, const int* tok_pos,
                                              const int* q_start, const float* gate, long long ld_gate, float* out,

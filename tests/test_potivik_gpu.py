@@ -212,6 +212,59 @@ def test_latent_attention_with_whole_weights_is_no_further_off_than_the_generic_
     assert off[True] <= off[False], (off[True] / off[False]) ** 0.5
 
 
+class LatentCalls:
+    """Single calls of the latent attention on bfloat16 pages of random rows."""
+    def __init__(self, H, r, dr, blocks=64, ps=16, seed=0):
+        from gibbs_b200.ops import library
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        self.H, self.r, self.dr, self.blocks, self.ps = H, r, dr, blocks, ps
+        self.pages = torch.randn(blocks, ps, r + dr, generator=g, device=DEV).to(torch.bfloat16)
+        self.table = torch.randperm(blocks, generator=g, device=DEV).to(torch.int32)
+        self.rows = library("hybrid").gb_latent_attention_workspace_rows()
+        self.ws = torch.full((self.rows, r + 2), float("nan"), device=DEV)
+
+    def __call__(self, q, gate, sink, spans, window, longest, chunks=True):
+        """q [tokens, H, r + dr], gate [tokens, H]; spans: (first position, tokens) of each request (all read the same
+        pages); `chunks` False: no workspace, one chunk."""
+        from gibbs_b200.ops import hybrid
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        R, n = len(spans), sum(k for _, k in spans)
+        req, pos = i32([i for i, (p, k) in enumerate(spans) for _ in range(k)]), i32([p + j for p, k in spans for j in range(k)])
+        start, bt = i32([sum(k for _, k in spans[:i]) for i in range(R)]), self.table.expand(R, -1).contiguous()
+        out = torch.full((n, self.H * self.r), float("nan"), device=DEV)
+        q, gate = q.contiguous(), gate.contiguous()
+        hybrid.call("latent_attention", [q.data_ptr(), self.pages.data_ptr(), 1, bt.data_ptr(), self.blocks, self.ps, self.blocks,
+                                         req.data_ptr(), pos.data_ptr(), gate.data_ptr(), self.H, out.data_ptr(), self.H * self.r, n,
+                                         self.H, self.r, self.dr, window, longest, self.ws.data_ptr() if chunks else 0,
+                                         0 if sink is None else sink.data_ptr(), R, start.data_ptr()], [(self.r + self.dr) ** -0.5])
+        return out
+
+
+@pytest.mark.parametrize("H,r,dr", [(3, 40, 8), (5, 128, 0), (16, 256, 32)])
+@pytest.mark.parametrize("window", [32, 33, 200])
+def test_latent_attention_with_whole_weights_does_not_depend_on_the_rows_beside_a_token(H, r, dr, window):
+    """A token's bits are the same however the portion is cut, alone and beside another request, with one chunk and with
+    chunks of the same length (as many tokens in the step), and where a request brings no token."""
+    call = LatentCalls(H, r, dr)
+    torch.manual_seed(window)
+    n, first = 37, 250
+    q, gate, sink = (torch.randn(*s, device=DEV) for s in ((n, H, r + dr), (n, H), (H,)))
+    whole = call(q, gate, sink, [(first, n)], window, 300, chunks=False)
+    for cuts in ([0, 1, n], [0, 16, 18, n], [0, 5, 7, 30, n]):
+        for a, b in zip(cuts, cuts[1:]):
+            assert torch.equal(call(q[a:b], gate[a:b], sink, [(first + a, b - a)], window, 300, chunks=False), whole[a:b]), (a, b)
+    some = call(q[:6], gate[:6], sink, [(first, 6)], window, 300)
+    for spans in ([(first, 1), (first + 1, 5)], [(first, 3), (first + 3, 0), (first + 3, 3)], [(first, 6)] + [(0, 0)] * 5,
+                  [(first + i, 1) for i in range(6)]):
+        assert torch.equal(call(q[:6], gate[:6], sink, spans, window, 300), some), spans
+    sc = torch.einsum("nhd,ld->nhl", q[:6].double(), call.pages[call.table.long()].reshape(-1, r + dr).double()) * (r + dr) ** -0.5
+    i, j = torch.arange(first, first + 6, device=DEV)[:, None], torch.arange(sc.shape[2], device=DEV)
+    sc.masked_fill_(~((j <= i) & (j > i - window))[:, None], -math.inf)
+    w = torch.softmax(torch.cat([sc, sink.double()[None, :, None].expand(6, H, 1)], 2), 2)[:, :, :-1]
+    want = (w @ call.pages[call.table.long()].reshape(-1, r + dr)[:, :r].double()) * torch.sigmoid(gate[:6].double())[..., None]
+    assert rel_rows(some.cpu(), want.reshape(6, -1).cpu()).max() < 2e-6
+
+
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
 def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
     """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
