@@ -355,7 +355,7 @@ struct LtxParams {
 
 size_t ltx_smem(int stride) {
   return sizeof(bf16) * (3 * LTX_ROWS + 2 * LTX_KEYS) * (size_t)stride + sizeof(float) * 4 * LTX_ROWS * LTX_SLD +
-         sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 2 * LTX_ROWS;
+         sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 3 * LTX_ROWS;
 }
 
 // x = t0 + t1 + t2, each a bfloat16 (the upper half of a 32-bit number)
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
   bf16* Cs = Qs + 3 * LTX_ROWS * STRIDE;                   // [2][32][STRIDE]
   float* Sp = reinterpret_cast<float*>(Cs + 2 * LTX_KEYS * STRIDE);      // [4][32][LTX_SLD]
   bf16* Pt = reinterpret_cast<bf16*>(Sp + 4 * LTX_ROWS * LTX_SLD);       // [3][32][LTX_PLD]
-  float* corr = reinterpret_cast<float*>(Pt + 3 * LTX_ROWS * LTX_PLD);   // [32], [32]
+  float* corr = reinterpret_cast<float*>(Pt + 3 * LTX_ROWS * LTX_PLD);   // [3][32]
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = warp & 1, wk = warp >> 1, g = lane >> 2, t4 = lane & 3;
@@ -636,13 +636,11 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
   } else if ((tid & 7) == 0 && srow < rows_live) {
     const size_t flat = flat0 + srow, t = flat / H;
     const int h = (int)(flat - t * H);
-    float f = 1.f / l;
-    if (p.sink) {
-      const float z = p.sink[h], top = fmaxf(m, z), e = expf(m - top);
-      f = e / (expf(z - top) + e * l);
-    }
-    if (p.gate) f *= hy_sigmoid(p.gate[t * p.ld_gate + h]);
-    corr[LTX_ROWS + srow] = f;
+    // (by the merge kernel's arithmetic, so that one chunk and several of which one holds keys give the same bits)
+    const float top = p.sink ? fmaxf(m, p.sink[h]) : m, e = expf(m - top);
+    const float open = p.gate ? hy_sigmoid(p.gate[t * p.ld_gate + h]) : 1.f;
+    corr[LTX_ROWS + srow] = e;
+    corr[2 * LTX_ROWS + srow] = open / __fadd_rn(p.sink ? expf(p.sink[h] - top) : 0.f, __fmul_rn(e, l));
   }
   __syncthreads();
   if (!warp_live) return;
@@ -652,17 +650,20 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     if (row >= rows_live) continue;
     const size_t flat = flat0 + row;
     float* dst;
-    float f = 1.f;
+    float e = 1.f, inv = 1.f;
     if (p.splits > 1) {
       dst = p.ws + (flat * p.splits + blockIdx.y) * (size_t)(r + 2) + 2;
     } else {
       dst = p.out + (flat / H) * p.ldo + (flat % H) * (size_t)r;
-      f = corr[LTX_ROWS + row];
+      e = corr[LTX_ROWS + row];
+      inv = corr[2 * LTX_ROWS + row];
     }
     dst += wk * OC + 2 * t4;
 #pragma unroll
     for (int j = 0; j < OC / 8; ++j)
-      if (wk * OC + 8 * j < r) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(o[j][2 * half] * f, o[j][2 * half + 1] * f);
+      if (wk * OC + 8 * j < r)
+        *reinterpret_cast<float2*>(dst + 8 * j) =
+            make_float2(__fmul_rn(__fmul_rn(e, o[j][2 * half]), inv), __fmul_rn(__fmul_rn(e, o[j][2 * half + 1]), inv));
   }
 }
 

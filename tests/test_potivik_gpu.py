@@ -168,7 +168,8 @@ def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H
             assert ((got[True][t] - want).abs() <= tol).all(), (what, t)
             for tc in off:
                 off[tc] += float((got[tc][t] - want).pow(2).sum())
-        assert not torch.equal(got[True], got[False])                # (two kernels did run)
+        # (two kernels did run; one key of few entries gives both the same sums, and both end by the merge's arithmetic)
+        assert window == 1 or not torch.equal(got[True], got[False])
         if what == "portions":                              # (rows enough for the two errors to be compared: measured 0.4 to 1.1)
             assert off[True] <= 1.25 ** 2 * off[False], (off[True] / off[False]) ** 0.5
 
@@ -263,6 +264,22 @@ def test_latent_attention_with_whole_weights_does_not_depend_on_the_rows_beside_
     w = torch.softmax(torch.cat([sc, sink.double()[None, :, None].expand(6, H, 1)], 2), 2)[:, :, :-1]
     want = (w @ call.pages[call.table.long()].reshape(-1, r + dr)[:, :r].double()) * torch.sigmoid(gate[:6].double())[..., None]
     assert rel_rows(some.cpu(), want.reshape(6, -1).cpu()).max() < 2e-6
+
+
+@pytest.mark.parametrize("H,r,dr,window", [(3, 40, 8, 0), (16, 256, 32, 0), (16, 512, 64, 0), (16, 512, 64, 40), (5, 128, 0, 512)])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_latent_attention_with_whole_weights_has_the_same_bits_in_one_chunk_and_in_several(H, r, dr, window, with_sink):
+    """Contexts that fit one chunk: without a workspace, with an upper bound that gives one chunk, and with one that gives
+    many, all others empty."""
+    call = LatentCalls(H, r, dr)
+    torch.manual_seed(r + window)
+    spans = [(20, 1), (5, 1), (31, 1)]
+    q, gate = torch.randn(3, H, r + dr, device=DEV), torch.randn(3, H, device=DEV)
+    sink = torch.randn(H, device=DEV) if with_sink else None
+    one = call(q, gate, sink, spans, window, 64, chunks=False)
+    assert not one.isnan().any()
+    for longest in (33, 64, 300, 1000):
+        assert torch.equal(call(q, gate, sink, spans, window, longest), one), longest
 
 
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
