@@ -355,7 +355,7 @@ struct LtxParams {
 
 size_t ltx_smem(int stride) {
   return sizeof(bf16) * (3 * LTX_ROWS + 2 * LTX_KEYS) * (size_t)stride + sizeof(float) * 4 * LTX_ROWS * LTX_SLD +
-         sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 3 * LTX_ROWS;
+         sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 3 * LTX_ROWS + 2 * sizeof(int);
 }
 
 // x = t0 + t1 + t2, each a bfloat16 (the upper half of a 32-bit number)
@@ -368,6 +368,18 @@ __device__ __forceinline__ void ltx_split(float x, unsigned short (&t)[3]) {
   }
 }
 
+// The score of a row and a key of the tile without tensor cores, for what is not finite: the terms of an infinite number
+// are no numbers, and an infinite entry is lost on a term that is 0.
+__device__ __noinline__ float ltx_score(const bf16* Qs, const bf16* C, int row, int key, int stride, int dk) {
+  float s = 0.f;
+  for (int d = 0; d < dk; ++d) {
+    float q = 0.f;
+    for (int t = 0; t < 3; ++t) q += __bfloat162float(Qs[((size_t)t * LTX_ROWS + row) * stride + d]);
+    s = fmaf(q, __bfloat162float(C[key * stride + d]), s);
+  }
+  return s;
+}
+
 template <int OC>                                          // columns of the latent a warp takes
 __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const LtxParams p) {
   extern __shared__ __align__(16) unsigned char ltc_smem[];
@@ -377,6 +389,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
   float* Sp = reinterpret_cast<float*>(Cs + 2 * LTX_KEYS * STRIDE);      // [4][32][LTX_SLD]
   bf16* Pt = reinterpret_cast<bf16*>(Sp + 4 * LTX_ROWS * LTX_SLD);       // [3][32][LTX_PLD]
   float* corr = reinterpret_cast<float*>(Pt + 3 * LTX_ROWS * LTX_PLD);   // [3][32]
+  volatile int* odd = reinterpret_cast<int*>(corr + 3 * LTX_ROWS);       // [2]: whether a tile holds what is not finite
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = warp & 1, wk = warp >> 1, g = lane >> 2, t4 = lane & 3;
@@ -483,6 +496,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
       }
     }
   }
+  if (tid < 2) odd[tid] = 0;
   // the softmax's view: eight threads a row, four keys each
   const int srow = tid >> 3, scol = (tid & 7) * 4;
   const int spos = pos_req + (row0 + srow) / H, slo = p.window > 0 ? spos - p.window + 1 : 0;
@@ -559,6 +573,14 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
         s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
       }
       float mx = -INFINITY;
+      if (srow < rows_live && !(fabsf(s[0]) + fabsf(s[1]) + fabsf(s[2]) + fabsf(s[3]) < INFINITY)) {
+        odd[b] = 1;                                        // (a query or a cached row is not finite, or a sum)
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+          const float x = ltx_score(Qs, C, srow, scol + e, STRIDE, dk);
+          if (e == 0) s[0] = x; else if (e == 1) s[1] = x; else if (e == 2) s[2] = x; else s[3] = x;
+        }
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int k = k0 + scol + e;
@@ -585,8 +607,34 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
             make_uint2(t[0][i] | (unsigned)t[1][i] << 16, t[2][i] | (unsigned)t[3][i] << 16);
       if ((tid & 7) == 0) corr[srow] = c;
     }
+    // A weight of 0 does not keep what is not finite out of a product, so a tile that holds any such thing takes only the keys
+    // each row sees.
     __syncthreads();
-    if (warp_live) {
+    if (tid == 0) odd[b ^ 1] = 0;                          // (the next tile's; this one's is read behind this barrier only)
+    if (odd[b] && warp_live) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int row = wr * 16 + g + 8 * half, pos = pos_req + (row0 + row) / H;
+        const float c = corr[row];
+#pragma unroll
+        for (int j = 0; j < OC / 8; ++j) {
+          o[j][2 * half] *= c;
+          o[j][2 * half + 1] *= c;
+        }
+        for (int k = 0; k < LTX_KEYS; ++k) {
+          if (k0 + k > min(pos, k_end) || (p.window > 0 && k0 + k <= pos - p.window)) continue;
+          const bf16* w = Pt + row * LTX_PLD + k;
+          const float weight = __bfloat162float(w[0]) + __bfloat162float(w[LTX_ROWS * LTX_PLD]) + __bfloat162float(w[2 * LTX_ROWS * LTX_PLD]);
+          const bf16* v = C + k * STRIDE + wk * OC + 2 * t4;
+#pragma unroll
+          for (int j = 0; j < OC / 8; ++j)
+            if (j < 2 * npairs) {
+              o[j][2 * half] = fmaf(weight, __bfloat162float(v[8 * j]), o[j][2 * half]);
+              o[j][2 * half + 1] = fmaf(weight, __bfloat162float(v[8 * j + 1]), o[j][2 * half + 1]);
+            }
+        }
+      }
+    } else if (warp_live) {
       const float c_a = corr[wr * 16 + g], c_b = corr[wr * 16 + g + 8];
       const bf16* ct = C + ((lane & 7) + ((lane >> 3) & 1) * 8) * STRIDE + wk * OC + (lane >> 4) * 8;
       const bf16* pa = Pt + (wr * 16 + (lane & 15)) * LTX_PLD + (lane >> 4) * 8;

@@ -282,6 +282,49 @@ def test_latent_attention_with_whole_weights_has_the_same_bits_in_one_chunk_and_
         assert torch.equal(call(q, gate, sink, spans, window, longest), one), longest
 
 
+@pytest.mark.parametrize("H,r,dr", [(3, 40, 8), (16, 320, 0), (16, 512, 64)])
+@pytest.mark.parametrize("window", [0, 40])
+def test_latent_attention_with_whole_weights_keeps_what_is_not_finite_to_the_rows_that_see_it(H, r, dr, window):
+    """Cached rows that hold no numbers or infinite ones (one behind some tokens, one in front of some windows), a query
+    that does: what is no number is what is none in 64 bits, all else as there, and rows that do not see it as without it."""
+    call = LatentCalls(H, r, dr)
+    torch.manual_seed(r)
+    spans, n = [(98, 7), (50, 1), (70, 1)], 9
+    q, gate, sink = (torch.randn(*s, device=DEV) for s in ((n, H, r + dr), (n, H), (H,)))
+    clean, pos, tok = call(q, gate, sink, spans, window, 128), [98 + i for i in range(7)] + [50, 70], torch.arange(n)
+
+    def exact(q):
+        out = []
+        for t in range(n):
+            c = call.pages[call.table.long()].reshape(-1, r + dr)[max(0, pos[t] - window + 1) if window else 0:pos[t] + 1].double()
+            sc = torch.cat([q[t].double() @ c.T * (r + dr) ** -0.5, sink.double()[:, None]], 1)
+            w = torch.softmax(sc, 1)[:, :-1]
+            out.append(((w[:, :, None] * c[None, :, :r]).sum(1) * torch.sigmoid(gate[t].double())[:, None]).reshape(-1))
+        return torch.stack(out).cpu()
+
+    def same(got, want, what):
+        assert torch.equal(got.isnan().cpu(), want.isnan()), what
+        assert rel_rows(got.nan_to_num(0.0).cpu() + 1e-30, want.nan_to_num(0.0) + 1e-30).max() < 1e-5, what
+
+    sound = call.pages.clone()
+    for value in (float("nan"), float("inf"), -float("inf")):
+        for at, entry in ((102, 3), (61, r - 1), (61, 0)):
+            call.pages.copy_(sound)
+            call.pages[call.table[at // 16].long(), at % 16, entry] = value
+            got = call(q, gate, sink, spans, window, 128)
+            same(got, exact(q), (value, at, entry))
+            blind = [t for t in tok.tolist() if at > pos[t] or (window and at <= pos[t] - window)]
+            assert blind and len(blind) < n
+            assert rel_rows(got[blind].cpu(), clean[blind].cpu()).max() < 1e-5
+            assert got[[t for t in range(n) if t not in blind]].isnan().any()
+        call.pages.copy_(sound)
+        bad = q.clone()
+        bad[2, H - 1, 5] = value
+        got = call(bad, gate, sink, spans, window, 128)
+        same(got, exact(bad), value)
+        assert torch.equal(got.isnan().any(1).cpu(), tok == 2)
+
+
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
 def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
     """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
