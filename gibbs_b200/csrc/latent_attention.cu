@@ -511,6 +511,48 @@ __global__ void latent_attention_merge_kernel(const float* ws, int splits, const
   }
 }
 
+// The same with a warp per (token, head), four to a block, for the few chunks of many rows (a prompt cut in two): the additions
+// in the same order, so the same bits.  Blocks of their own for rows of two chunks are mostly prologue.
+__global__ void __launch_bounds__(128)
+latent_attention_merge_rows_kernel(const float* ws, int splits, const float* gate, long long ld_gate, float* out, long long ldo,
+                                   long long rows, int H, int r, const float* __restrict__ sink) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long long idx = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (idx >= rows) return;
+  const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
+  const size_t ld = (size_t)r + 2;
+  const float* w = ws + (size_t)idx * splits * ld;
+  const float m = lane < splits ? w[lane * ld] : -INFINITY, l = lane < splits ? w[lane * ld + 1] : 0.f;
+  float M = warp_max(m);
+  if (sink) M = fmaxf(M, sink[h]);
+  const float e = m > -INFINITY ? expf(m - M) : 0.f, el = e * l;
+  float L = sink ? expf(sink[h] - M) : 0.f;
+  for (int s = 0; s < splits; ++s) L += __shfl_sync(0xffffffffu, el, s);
+  const float g = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + h]) : 1.f;
+  const float inv = g / L;
+  float* dst = out + (size_t)t * ldo + (size_t)h * r;
+  for (int d0 = 0; d0 < r; d0 += 256) {                    // eight columns a lane at a time
+    float a[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) a[v] = 0.f;
+    for (int s = 0; s < splits; ++s) {
+      const float es = __shfl_sync(0xffffffffu, e, s);
+      if (es == 0.f) continue;                             // (the whole warp together)
+      const float* ws_s = w + s * ld + 2;
+      float x[8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v) x[v] = d0 + lane + 32 * v < r ? ldcg_now(ws_s + d0 + lane + 32 * v) : 0.f;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) a[v] = fmaf(es, x[v], a[v]);
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      if (d0 + lane + 32 * v < r) dst[d0 + lane + 32 * v] = a[v] * inv;
+  }
+}
+
 }  // namespace
 
 bool gb_head_linear_tc_takes(int n, int I, long long ldx, long long xh, const void* x, const void* W);
@@ -538,7 +580,13 @@ cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages,
 static int launch_merge(const float* ws, int splits, const float* gate, long long ld_gate, float* out, long long ldo, int n,
                         int H, int r, const float* sink, cudaStream_t stream) {
   if (splits > LM_CHUNKS) GB_FAIL(GB_ERR_ARG, "latent_attention_merge: %d chunks", splits);
-  gb_launch(latent_attention_merge_kernel, dim3((unsigned)((long long)n * H)), dim3(r <= 128 ? 128 : r <= 256 ? 256 : 512), 0,
+  // (us of a block and of a warp a row: 2 chunks of 512, 256 rows 3.1 and 3.1, 1024 8.8 and 3.4, 8192 63 and 7.4; 8 chunks, 512 rows
+  // 6.3 and 7.6, 1024 10.6 and 7.7; 4 chunks of 64, 512 rows 2.8 and 2.5)
+  if (splits <= 8 && (long long)n * H >= 128 * splits)
+    gb_launch(latent_attention_merge_rows_kernel, dim3(gb_div_up((long long)n * H, 4)), dim3(128), 0, stream, ws, splits, gate,
+              ld_gate, out, ldo, (long long)n * H, H, r, sink);
+  else
+    gb_launch(latent_attention_merge_kernel, dim3((unsigned)((long long)n * H)), dim3(r <= 128 ? 128 : r <= 256 ? 256 : 512), 0,
             stream, ws, splits, gate, ld_gate, out, ldo, H, r, sink);
   GB_CHECK_LAUNCH("latent_attention_merge");
   return 2;

@@ -325,6 +325,36 @@ def test_latent_attention_with_whole_weights_keeps_what_is_not_finite_to_the_row
         assert torch.equal(got.isnan().any(1).cpu(), tok == 2)
 
 
+@pytest.mark.parametrize("splits,r", [(2, 8), (2, 512), (3, 264), (5, 40), (8, 512)])
+def test_latent_merge_has_the_same_bits_by_a_block_and_by_a_warp_a_row(splits, r):
+    """Steps of single tokens on both sides of the number of rows (128 a chunk) from which a warp takes a row: the first
+    tokens are the same, and so are their bits."""
+    H, n = 16, 8 * splits                                    # (n * H = 128 * splits is the first launch by warps)
+    call = LatentCalls(H, r, 0)
+    torch.manual_seed(r)
+    gate, sink = torch.randn(n, H, device=DEV), torch.randn(H, device=DEV)
+    by_blocks, by_warps = (_merge_alone(call, k, H, r, splits, sink, gate) for k in (n - 1, n))
+    assert torch.equal(by_blocks, by_warps[:n - 1])
+
+
+def _merge_alone(call, n, H, r, splits, sink, gate):
+    """The generic kernel on 32-bit pages of one chunk of 64 keys after the other: `splits` of them by the context."""
+    from gibbs_b200.ops import hybrid
+    g = torch.Generator(device=DEV).manual_seed(7)
+    blocks, ps, longest = 4 * splits, 16, 64 * splits
+    pages = torch.randn(blocks, ps, r, generator=g, device=DEV)
+    q = torch.randn(n, H, r, generator=g, device=DEV)
+    bt = torch.arange(blocks, dtype=torch.int32, device=DEV)[None].expand(n, -1).contiguous()
+    req = torch.arange(n, dtype=torch.int32, device=DEV)
+    pos = (torch.arange(n, device=DEV) * 37 % longest).to(torch.int32)
+    out = torch.full((n, H * r), float("nan"), device=DEV)
+    launched = hybrid.call("latent_attention", [q.data_ptr(), pages.data_ptr(), 0, bt.data_ptr(), blocks, ps, blocks, req.data_ptr(),
+                                                pos.data_ptr(), gate.data_ptr(), H, out.data_ptr(), H * r, n, H, r, 0, 0, longest,
+                                                call.ws.data_ptr(), sink.data_ptr(), 0, 0], [r ** -0.5])
+    assert launched == 2 and not out.isnan().any()
+    return out
+
+
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
 def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
     """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
