@@ -67,12 +67,17 @@ struct StreamParams {
 
 constexpr int STREAM_CACHE = 4;            // pieces of u a thread keeps between the sum of squares and the norm
 
-// S streams (0: any number up to MAX_STREAMS, taken from `streams`); PART: y comes as partial tiles.
-template <int S, int VEC, bool MIX, bool PART>
-__global__ void stream_kernel(StreamParams p, int streams) {
+// S streams (0: any number up to MAX_STREAMS, taken from `streams`); PART: y comes as partial tiles.  FEW: as many threads
+// as pieces (up to 512), the gain on hand before the sublayer has finished (pinned, see gb_pin); `lanes` is the number of threads a
+// row's sum of squares is spread over whatever the block's size, so that a row has the same bits in a step of few rows and of many.
+constexpr int STREAM_FEW = 512 * STREAM_CACHE;             // the most pieces of such a row
+
+template <int S, int VEC, bool MIX, bool PART, bool FEW>
+__device__ __forceinline__ void stream_rows(const StreamParams& p, int streams, int lanes) {
   constexpr int CAP = S > 0 ? S : MAX_STREAMS;
   __shared__ float scratch[32];
   __shared__ float w_mix[MIX ? CAP * CAP : 1], w_out[MIX ? CAP : 1], w_in[CAP];
+  extern __shared__ float4 all[];                          // (FEW) what every piece gives the next reader
   pdl_trigger();
   const int n_s = S > 0 ? S : streams;
   // (weights: nothing writes them while a model runs)
@@ -98,19 +103,16 @@ __global__ void stream_kernel(StreamParams p, int streams) {
     }
   }
   const int pieces = p.dim / VEC;
-  // (the gain of the pieces a thread keeps: on hand before the sublayer has finished, pinned, see gb_pin)
-  float gain[STREAM_CACHE][VEC];
+  Piece<VEC> gain[FEW ? STREAM_CACHE : 1];
+  if constexpr (FEW) {
 #pragma unroll
-  for (int c = 0; c < STREAM_CACHE; ++c) {
-    const int i = threadIdx.x + c * blockDim.x;
-    Piece<VEC> g;
+    for (int c = 0; c < STREAM_CACHE; ++c) {
+      const int i = threadIdx.x + c * blockDim.x;
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) g.v[e] = 0.f;
-    if (p.gain && i < pieces) g.load(p.gain + (size_t)i * VEC);
+      for (int e = 0; e < VEC; ++e) gain[c].v[e] = 0.f;
+      if (p.gain && i < pieces) gain[c].load(p.gain + (size_t)i * VEC);
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      gain[c][e] = g.v[e];
-      gb_pin(gain[c][e]);
+      for (int e = 0; e < VEC; ++e) gb_pin(gain[c].v[e]);
     }
   }
   pdl_wait();
@@ -143,12 +145,13 @@ __global__ void stream_kernel(StreamParams p, int streams) {
         const float* at = p.part + (size_t)r * p.dim + (size_t)i * VEC;
 #pragma unroll
         for (int e = 0; e < VEC; ++e) yy.v[e] = 0.f;
-        for (int s0 = 0; s0 < p.splits; s0 += 8) {         // (eight requested together, added in order)
-          Piece<VEC> t[8];
+        constexpr int AT_ONCE = FEW ? 8 : 4;               // (requested together, added in order)
+        for (int s0 = 0; s0 < p.splits; s0 += AT_ONCE) {
+          Piece<VEC> t[AT_ONCE];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) t[u].load(at + (size_t)min(s0 + u, p.splits - 1) * p.part_stride);
+          for (int u = 0; u < AT_ONCE; ++u) t[u].load(at + (size_t)min(s0 + u, p.splits - 1) * p.part_stride);
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
+          for (int u = 0; u < AT_ONCE; ++u)
             if (s0 + u < p.splits) {
 #pragma unroll
               for (int e = 0; e < VEC; ++e) yy.v[e] += t[u].v[e];
@@ -184,43 +187,75 @@ __global__ void stream_kernel(StreamParams p, int streams) {
       read(old, u);
     }
   };
+  if constexpr (FEW) {
+    // the sum of squares as `lanes` threads that walk the pieces would take it
 #pragma unroll
-  for (int c = 0; c < STREAM_CACHE; ++c) {
-    const int i = threadIdx.x + c * blockDim.x;
+    for (int c = 0; c < STREAM_CACHE; ++c) {
+      const int i = threadIdx.x + c * blockDim.x;
+      if (i >= pieces) break;
+      step(i, cache[c]);
+      if (p.gain) all[i] = make_float4(cache[c][0], cache[c][1], cache[c][2], cache[c][3]);
+    }
+    if (p.gain == nullptr) return;
+    __syncthreads();
+    if ((int)threadIdx.x < lanes)
+      for (int j = threadIdx.x; j < pieces; j += lanes) {
+        const float4 u = all[j];
+        ss = fmaf(u.w, u.w, fmaf(u.z, u.z, fmaf(u.y, u.y, fmaf(u.x, u.x, ss))));
+      }
+    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)p.dim + p.eps);
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) cache[c][e] = 0.f;
-    if (i < pieces) step(i, cache[c]);
+    for (int c = 0; c < STREAM_CACHE; ++c) {
+      const int i = threadIdx.x + c * blockDim.x;
+      if (i < pieces) store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, cache[c], rstd, gain[c].v);
+    }
+  } else {
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) ss = fmaf(cache[c][e], cache[c][e], ss);
-  }
-  for (int i = threadIdx.x + STREAM_CACHE * blockDim.x; i < pieces; i += blockDim.x) {
-    float u[VEC];
+    for (int c = 0; c < STREAM_CACHE; ++c) {
+      const int i = threadIdx.x + c * blockDim.x;
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) u[e] = 0.f;
-    step(i, u);
+      for (int e = 0; e < VEC; ++e) cache[c][e] = 0.f;
+      if (i < pieces) step(i, cache[c]);
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) ss = fmaf(u[e], u[e], ss);
-  }
-  if (p.gain == nullptr) return;
-  const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)p.dim + p.eps);
+      for (int e = 0; e < VEC; ++e) ss = fmaf(cache[c][e], cache[c][e], ss);
+    }
+    for (int i = threadIdx.x + STREAM_CACHE * blockDim.x; i < pieces; i += blockDim.x) {
+      float u[VEC];
 #pragma unroll
-  for (int c = 0; c < STREAM_CACHE; ++c) {
-    const int i = threadIdx.x + c * blockDim.x;
-    if (i >= pieces) continue;
-    store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, cache[c], rstd, gain[c]);
-  }
-  // (a row too long for the registers: what this thread wrote is read again)
-  for (int i = threadIdx.x + STREAM_CACHE * blockDim.x; i < pieces; i += blockDim.x) {
-    Piece<VEC> v[CAP], g;
-    float u[VEC];
+      for (int e = 0; e < VEC; ++e) u[e] = 0.f;
+      step(i, u);
 #pragma unroll
-    for (int s = 0; s < CAP; ++s)
-      if (S > 0 || s < n_s) v[s].load(x + (size_t)s * p.dim + (size_t)i * VEC);
-    read(v, u);
-    g.load(p.gain + (size_t)i * VEC);
-    store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, u, rstd, g.v);
+      for (int e = 0; e < VEC; ++e) ss = fmaf(u[e], u[e], ss);
+    }
+    if (p.gain == nullptr) return;
+    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)p.dim + p.eps);
+#pragma unroll
+    for (int c = 0; c < STREAM_CACHE; ++c) {
+      const int i = threadIdx.x + c * blockDim.x;
+      if (i >= pieces) continue;
+      Piece<VEC> g;
+      g.load(p.gain + (size_t)i * VEC);
+      store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, cache[c], rstd, g.v);
+    }
+    // (a row too long for the registers: what this thread wrote is read again)
+    for (int i = threadIdx.x + STREAM_CACHE * blockDim.x; i < pieces; i += blockDim.x) {
+      Piece<VEC> v[CAP], g;
+      float u[VEC];
+#pragma unroll
+      for (int s = 0; s < CAP; ++s)
+        if (S > 0 || s < n_s) v[s].load(x + (size_t)s * p.dim + (size_t)i * VEC);
+      read(v, u);
+      g.load(p.gain + (size_t)i * VEC);
+      store_normed<VEC>(p.out, p.out_dtype, (size_t)r * p.dim + (size_t)i * VEC, u, rstd, g.v);
+    }
   }
 }
+
+template <int S, int VEC, bool MIX, bool PART>
+__global__ void stream_kernel(StreamParams p, int streams) { stream_rows<S, VEC, MIX, PART, false>(p, streams, 0); }
+
+template <int S, bool MIX, bool PART>
+__global__ void __launch_bounds__(512) stream_few_kernel(StreamParams p, int lanes) { stream_rows<S, 4, MIX, PART, true>(p, S, lanes); }
 
 template <bool MIX>
 int launch_streams(const StreamParams& p, int n, int streams, cudaStream_t stream, const char* what) {
@@ -229,22 +264,19 @@ int launch_streams(const StreamParams& p, int n, int streams, cudaStream_t strea
   const bool vec = p.dim % 4 == 0 && p.ldx % 4 == 0 && p.ldy % 4 == 0 && (bits & 15) == 0 &&
                    ((uintptr_t)p.out & (p.out_dtype == GB_BF16 ? 7 : 15)) == 0;
   const int pieces = vec ? p.dim / 4 : p.dim;
-  // A few rows (fewer than half of the SMs) of up to four streams: a piece a thread, so that all of a row is asked for at once
-  // (a thread's second piece waits behind the stores of its first); 2 rows of 4 x 2048 in a decode step, with the gain
-  // read ahead: 4.4 us against 5.3 with two pieces a thread.  With many rows the wider blocks are slower (2134 rows: 61 us
-  // against 39), and more streams need more registers than 512 threads have.
-  const bool few = n <= 74 && streams <= 4 && vec;
-  const dim3 block(pieces <= 64 ? 64 : few ? 32 * (pieces < 512 ? gb_div_up(pieces, 32) : 16) : pieces <= 256 ? 128 : 256);
-#define STREAMS(S)                                                                                       \
-  do {                                                                                                   \
-    if (MIX && p.part) {                                                                                 \
-      if (vec) gb_launch(stream_kernel<S, 4, MIX, MIX>, dim3(n), block, 0, stream, p, streams);          \
-      else gb_launch(stream_kernel<S, 1, MIX, MIX>, dim3(n), block, 0, stream, p, streams);              \
-    } else {                                                                                             \
-      if (vec) gb_launch(stream_kernel<S, 4, MIX, false>, dim3(n), block, 0, stream, p, streams);        \
-      else gb_launch(stream_kernel<S, 1, MIX, false>, dim3(n), block, 0, stream, p, streams);            \
-    }                                                                                                    \
+  const int lanes = pieces <= 64 ? 64 : pieces <= 256 ? 128 : 256;
+  // A few rows (fewer than half of the SMs) of up to four streams: more threads, so that all of a row is asked for at once (a
+  // thread's second piece waits behind the stores of its first; more streams need more registers than 512 threads have); 2 rows of 4 x 2048 in a decode step: SM_TIMES
+  const bool few = n <= 74 && streams <= 4 && vec && pieces > lanes && pieces <= STREAM_FEW;
+  const dim3 block(!few ? lanes : pieces < 512 ? 32 * gb_div_up(pieces, 32) : 512);
+  const size_t smem = few ? sizeof(float4) * (size_t)pieces : 0;
+#define STREAMS_OF(S, PART)                                                                                            \
+  do {                                                                                                                 \
+    if (few) gb_launch(stream_few_kernel<(S >= 1 && S <= 4 ? S : 1), MIX, PART>, dim3(n), block, smem, stream, p, lanes); \
+    else if (vec) gb_launch(stream_kernel<S, 4, MIX, PART>, dim3(n), block, 0, stream, p, streams);                     \
+    else gb_launch(stream_kernel<S, 1, MIX, PART>, dim3(n), block, 0, stream, p, streams);                              \
   } while (0)
+#define STREAMS(S) do { if (MIX && p.part) STREAMS_OF(S, MIX); else STREAMS_OF(S, false); } while (0)
   switch (streams) {
     case 1: STREAMS(1); break;
     case 2: STREAMS(2); break;
@@ -254,6 +286,7 @@ int launch_streams(const StreamParams& p, int n, int streams, cudaStream_t strea
     default: STREAMS(0);
   }
 #undef STREAMS
+#undef STREAMS_OF
   GB_CHECK_LAUNCH(what);
   return 1;
 }

@@ -114,13 +114,14 @@ def eager(n, dtype="float32"):
 # mechanisms alone
 # ---------------------------------------------------------------------------
 
-@pytest.mark.parametrize("streams,d", [(1, 44), (2, 46), (3, 336), (4, 1536), (5, 45), (8, 64), (16, 40), (4, 5000), (3, 3001), (7, 1100)])
+@pytest.mark.parametrize("streams,d", [(1, 44), (2, 46), (3, 336), (4, 1536), (5, 45), (8, 64), (16, 40), (4, 5000), (3, 3001), (7, 1100), (2, 8196)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-def test_streams_are_mixed_and_read(streams, d, dtype):
-    """Several tokens: what a sublayer reads as a kernel of its own, the mixing alone, the mixing together with what the
+@pytest.mark.parametrize("n", [9, 74, 75, 200])
+def test_streams_are_mixed_and_read(streams, d, dtype, n):
+    """Steps of a few tokens and of many (74 is the last with more threads a row): what a sublayer reads as a kernel of its own, the mixing alone, the mixing together with what the
     next sublayer reads, and the norm in front of the head for gathered rows."""
     g = gen(streams * 1000 + d)
-    n, eps = 9, 1e-5
+    eps = 1e-5
     def connection():
         return {"in": torch.randn(streams, generator=g), "out": torch.randn(streams, generator=g),
                 "mix": torch.randn(streams, streams, generator=g)}
@@ -152,6 +153,25 @@ def test_streams_are_mixed_and_read(streams, d, dtype):
     rows = torch.tensor([7, 0, 7, 3], dtype=torch.int32, device=DEV)
     got = head.forward(xs, rows=rows).float().cpu()
     assert rel_rows(got, (plain.rms(want.sum(0), eps) * gain.double())[[7, 0, 7, 3]]).max() < tol
+
+
+@pytest.mark.parametrize("streams,d", [(1, 1024), (2, 260), (3, 336), (4, 1024), (4, 2048), (4, 5000), (2, 8192), (4, 8196), (8, 1024)])
+def test_streams_have_the_same_bits_in_a_step_of_few_rows_and_of_many(streams, d):
+    """One row, 74 and 75 of them (the last step with more threads a row and the first without), 200: mixed, read behind
+    the mixing and read alone."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(d)
+    x0, y = torch.randn(200, streams * d, device=DEV), torch.randn(200, d, device=DEV)
+    mix, out_w, in_w, gain = (torch.randn(*s, device=DEV) for s in ((streams, streams), (streams,), (streams,), (d,)))
+    whole = None
+    for n in (200, 75, 74, 1):
+        x, mixed, read = x0[:n].clone(), torch.empty(n, d, device=DEV), torch.empty(n, d, device=DEV)
+        hybrid.call("stream_read", [x.data_ptr(), streams * d, in_w.data_ptr(), gain.data_ptr(), read.data_ptr(), 0, 0, n, d, streams], [1e-5])
+        hybrid.call("stream_mix", [x.data_ptr(), streams * d, y.data_ptr(), d, mix.data_ptr(), out_w.data_ptr(), n, d, streams,
+                                   in_w.data_ptr(), gain.data_ptr(), mixed.data_ptr(), 0], [1e-5])
+        got = torch.cat([x, mixed, read], 1)
+        whole = got if whole is None else whole
+        assert torch.equal(got, whole[:n]), n
 
 
 @pytest.mark.parametrize("d", [45, 64, 300])
