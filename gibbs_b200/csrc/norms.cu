@@ -177,24 +177,28 @@ row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ ga
   }
 }
 
+// AHEAD: the gains are on hand before the kernel in front has finished (pinned, see gb_pin): read behind the sums, each was a
+// trip to L2 of its own (2 rows of 2048 in a decode step: 6.3 us; 2.8 so).  They cost registers, so blocks an SM, which a launch
+// of many rows needs more.
+template <bool AHEAD>
 __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long long ldy, const float* __restrict__ gain,
                                 int dim, int kind, float eps, bf16* copy, ThenNorm then) {
   __shared__ float scratch[32];
   pdl_trigger();
   const float* row = y + (size_t)blockIdx.x * ldy;
   float* o = x + (size_t)blockIdx.x * ldx;
-  // The gains are on hand before the kernel in front has finished (pinned, see gb_pin): read behind the sums, each was
-  // a trip to L2 of its own (2 rows of 2048 in a decode step: 6.3 us; 2.8 so).
-  const bool whole = dim <= NORM_CACHE * (int)blockDim.x, second = then.gain != nullptr;
-  float g1[NORM_CACHE], g2[NORM_CACHE];
+  float g1[AHEAD ? NORM_CACHE : 1], g2[AHEAD ? NORM_CACHE : 1];
+  if constexpr (AHEAD) {
+    const bool second = then.gain != nullptr;
 #pragma unroll
-  for (int i = 0; i < NORM_CACHE; ++i) {
-    const int d = threadIdx.x + i * blockDim.x;
-    g1[i] = whole && d < dim ? gain[d] : 0.f;
-    g2[i] = whole && second && d < dim ? then.gain[d] : 0.f;
+    for (int i = 0; i < NORM_CACHE; ++i) {
+      const int d = threadIdx.x + i * blockDim.x;
+      g1[i] = d < dim ? gain[d] : 0.f;
+      g2[i] = second && d < dim ? then.gain[d] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < NORM_CACHE; ++i) { gb_pin(g1[i]); gb_pin(g2[i]); }
   }
-#pragma unroll
-  for (int i = 0; i < NORM_CACHE; ++i) { gb_pin(g1[i]); gb_pin(g2[i]); }
   pdl_wait();
   RowCache c;
   row_load(row, dim, c);
@@ -213,7 +217,7 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
     for (int i = 0; i < NORM_CACHE; ++i) {
       const int d = threadIdx.x + i * blockDim.x;
       if (d < dim) {
-        const float v = old[i] + (c.v[i] - mean) * rstd * g1[i];
+        const float v = old[i] + (c.v[i] - mean) * rstd * (AHEAD ? g1[AHEAD ? i : 0] : gain[d]);
         o[d] = v;
         if (copy) copy[(size_t)blockIdx.x * dim + d] = __float2bfloat16_rn(v);
         c.v[i] = v;
@@ -228,7 +232,7 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
       for (int i = 0; i < NORM_CACHE; ++i) {
         const int d = threadIdx.x + i * blockDim.x;
         if (d < dim) {
-          const float h = (c.v[i] - mean2) * rstd2 * g2[i];
+          const float h = (c.v[i] - mean2) * rstd2 * (AHEAD ? g2[AHEAD ? i : 0] : then.gain[d]);
           if (then.out_dtype == GB_BF16) ((bf16*)then.out)[(size_t)blockIdx.x * dim + d] = __float2bfloat16_rn(h);
           else ((float*)then.out)[(size_t)blockIdx.x * dim + d] = h;
         }
@@ -696,7 +700,10 @@ GB_OP(gb_op_norm_add) {
   if (second && then.kind != NORM_LAYER && then.kind != NORM_RMS) GB_FAIL(GB_ERR_ARG, "norm_add: second kind %d", then.kind);
   const bool fused = second && dim <= NORM_CACHE * threads;   // the row fits the registers
   ThenNorm none = {nullptr, nullptr, 0, 0, 0.f};
-  gb_launch(norm_add_kernel, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<float>(a[0]), a[1],
+  // (us with the gains ahead and without, rows of 2048: 200 rows 3.2 and 4.2, 512 5.0 and 4.7, 2134 13.9 and 11.6; rows too long
+  // for the registers read them at the end either way)
+  const bool ahead = n <= 296 && dim <= NORM_CACHE * threads;
+  gb_launch(ahead ? norm_add_kernel<true> : norm_add_kernel<false>, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<float>(a[0]), a[1],
             op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]),
             fused ? then : none);
   GB_CHECK_LAUNCH("norm_add");

@@ -355,6 +355,32 @@ def _merge_alone(call, n, H, r, splits, sink, gate):
     return out
 
 
+@pytest.mark.parametrize("d", [40, 64, 300, 2048, 2049, 4096])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_norm_behind_a_sublayer_in_steps_of_few_rows_and_of_many(d, kind):
+    """296 rows (the last step whose gains are read ahead) and 297, with the next sublayer's norm and without: against 64
+    bits, and the rows they share have the same bits."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(d)
+    x0, y, gain, then = torch.randn(297, d), torch.randn(297, d), torch.randn(d), torch.randn(d)
+    dev = [t.to(DEV) for t in (y, gain, then)]
+    def norm(v, g):
+        v = v.double() - (v.double().mean(1, keepdim=True) if kind == 0 else 0.0)
+        return v / (v.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * g.double()
+    new = x0.double() + norm(y, gain)
+    for second in (False, True):
+        got = {}
+        for n in (297, 296):
+            x, h = x0[:n].to(DEV), torch.zeros(n, d, device=DEV)
+            hybrid.call("norm_add", [x.data_ptr(), d, dev[0].data_ptr(), d, dev[1].data_ptr(), n, d, kind, 0, dev[2].data_ptr() if second else 0,
+                                     h.data_ptr() if second else 0, 0, kind], [1e-5, 1e-5])
+            got[n] = torch.cat([x, h], 1)
+        assert torch.equal(got[296], got[297][:296])
+        assert rel_rows(got[297][:, :d].cpu(), new).max() < 1e-6
+        if second:
+            assert rel_rows(got[297][:, d:].cpu(), norm(new, then)).max() < 2e-6
+
+
 @pytest.mark.parametrize("H,P,N,G", [(2, 4, 4, 1), (3, 32, 32, 3), (4, 68, 36, 2), (2, 64, 64, 2), (64, 64, 128, 8), (5, 36, 124, 1)])
 def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
     """Lengths around the groups of 2 to 8 tokens and the chunks of 16, widths that fill a block's columns and lanes or
