@@ -146,12 +146,14 @@ __global__ void head_linear_small_kernel(const float* x, long long ldx, long lon
   }
 }
 
-// The same where the weight's rows are whole 16-byte pieces, at most HLF_PIECES a lane: a warp takes HLF_OUT outputs of
-// a head, its weights are in registers before the kernel in front has finished, and the inputs of HLF_ROWS rows at a
-// time are read once for all of them.  Bound by the trip to L2 for the inputs.  Measured, 2 rows of 16 heads in a decode
-// step: 512 -> 128 4.1 us (14.3 with a scalar load of 16 bits a lane and a block's inputs through shared memory), 128 -> 512
-// 4.9 us (8.5).
-constexpr int HLF_OUT = 4, HLF_ROWS = 2, HLF_PIECES = 4;
+// The same where the weight's rows are whole 16-byte pieces, at most PIECES (1, 2 or 4) a lane: a warp takes HLF_OUT outputs of
+// a head, its weights are in registers before the kernel in front has finished, and the inputs of 8 / PIECES rows at a
+// time are read once for all of them.  A lane adds its even and its odd inputs in two chains (one of all of a piece was 1.05 to 1.2
+// times as far off as the kernel above).  Bound by the trip to L2 for the inputs, one for every 8 / PIECES rows.
+// Measured (us, the kernel above -> this one; weights of 8 launches, not all in L2): 16 heads 512 -> 128, 2 rows 12.0 -> 2.6, 16 rows
+// 24.6 -> 8.4 (12.0 with two rows at a time whatever the pieces); 128 -> 512, 2 rows 7.0 -> 4.6, 16 rows 16.0 -> 10.4 (20.1); 8
+// heads 64 -> 64, 16 rows 5.4 -> 4.9 (8.1).
+constexpr int HLF_OUT = 4, HLF_PIECES = 4;
 
 // Eight bfloat16 or four 32-bit weights.
 __device__ __forceinline__ void hlf_unpack(const uint4& u, float (&v)[8]) {
@@ -170,32 +172,33 @@ __device__ __forceinline__ void hlf_unpack(const uint4& u, float (&v)[4]) {
   v[3] = __uint_as_float(u.w);
 }
 
-template <typename TW, typename TO>
+template <typename TW, typename TO, int PIECES>
 __global__ void __launch_bounds__(128)
 head_linear_few_kernel(const float* x, long long ldx, long long xh, const TW* __restrict__ W, TO* out, long long ldo,
                        long long oh, int n, int O, int I, const float* gate, long long ld_gate) {
-  constexpr int E = 16 / (int)sizeof(TW);
+  constexpr int E = 16 / (int)sizeof(TW), ROWS = 8 / PIECES;
   pdl_trigger();
   const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int o0 = (blockIdx.x * 4 + warp) * HLF_OUT;
   if (o0 >= O) return;                                     // (whole warps; nothing below meets the block)
-  uint4 w[HLF_OUT][HLF_PIECES];
+  uint4 w[HLF_OUT][PIECES];
 #pragma unroll
   for (int j = 0; j < HLF_OUT; ++j)
 #pragma unroll
-    for (int i = 0; i < HLF_PIECES; ++i) {
+    for (int i = 0; i < PIECES; ++i) {
       const int c = E * (lane + 32 * i);
       w[j][i] = o0 + j < O && c < I ? *reinterpret_cast<const uint4*>(W + ((size_t)h * O + o0 + j) * I + c) : make_uint4(0u, 0u, 0u, 0u);
       asm volatile("" : "+r"(w[j][i].x), "+r"(w[j][i].y), "+r"(w[j][i].z), "+r"(w[j][i].w));      // (stays here, see gb_pin)
     }
   pdl_wait();
-  for (int t0 = 0; t0 < n; t0 += HLF_ROWS) {
-    float acc[HLF_ROWS][HLF_OUT];
-    float4 xv[HLF_ROWS][HLF_PIECES][E / 4];
+  for (int t0 = 0; t0 < n; t0 += ROWS) {
+    const int live = n - t0;                               // (the first two rows are worked out whether there or not)
+    float acc[ROWS][HLF_OUT], odd[ROWS][HLF_OUT];
+    float4 xv[ROWS][PIECES][E / 4];
 #pragma unroll
-    for (int u = 0; u < HLF_ROWS; ++u)
+    for (int u = 0; u < ROWS; ++u)
 #pragma unroll
-      for (int i = 0; i < HLF_PIECES; ++i) {
+      for (int i = 0; i < PIECES; ++i) {
         const int c = E * (lane + 32 * i);
 #pragma unroll
         for (int e = 0; e < E / 4; ++e)
@@ -203,34 +206,43 @@ head_linear_few_kernel(const float* x, long long ldx, long long xh, const TW* __
                                             : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-    for (int u = 0; u < HLF_ROWS; ++u)
+    for (int u = 0; u < ROWS; ++u)
 #pragma unroll
-      for (int j = 0; j < HLF_OUT; ++j) acc[u][j] = 0.f;
+      for (int j = 0; j < HLF_OUT; ++j) acc[u][j] = odd[u][j] = 0.f;
 #pragma unroll
-    for (int i = 0; i < HLF_PIECES; ++i)
+    for (int i = 0; i < PIECES; ++i)
 #pragma unroll
       for (int j = 0; j < HLF_OUT; ++j) {
         float wv[E];
         hlf_unpack(w[j][i], wv);
 #pragma unroll
-        for (int u = 0; u < HLF_ROWS; ++u)
+        for (int u = 0; u < ROWS; ++u) {
+          if (u >= 2 && u >= live) break;
 #pragma unroll
           for (int e = 0; e < E / 4; ++e) {
             acc[u][j] = fmaf(xv[u][i][e].x, wv[4 * e], acc[u][j]);
-            acc[u][j] = fmaf(xv[u][i][e].y, wv[4 * e + 1], acc[u][j]);
+            odd[u][j] = fmaf(xv[u][i][e].y, wv[4 * e + 1], odd[u][j]);
             acc[u][j] = fmaf(xv[u][i][e].z, wv[4 * e + 2], acc[u][j]);
-            acc[u][j] = fmaf(xv[u][i][e].w, wv[4 * e + 3], acc[u][j]);
+            odd[u][j] = fmaf(xv[u][i][e].w, wv[4 * e + 3], odd[u][j]);
           }
+        }
       }
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
+    for (int u = 0; u < ROWS; ++u)
 #pragma unroll
-      for (int u = 0; u < HLF_ROWS; ++u)
+      for (int j = 0; j < HLF_OUT; ++j) acc[u][j] += odd[u][j];
 #pragma unroll
-        for (int j = 0; j < HLF_OUT; ++j) acc[u][j] += __shfl_xor_sync(0xffffffffu, acc[u][j], s);
+    for (int u = 0; u < ROWS; u += 2) {
+      if (u >= 2 && u >= live) break;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+        for (int j = 0; j < 2 * HLF_OUT; ++j)
+          acc[u + j / HLF_OUT][j % HLF_OUT] += __shfl_xor_sync(0xffffffffu, acc[u + j / HLF_OUT][j % HLF_OUT], s);
+    }
     // lane (u, j) stores its output
 #pragma unroll
-    for (int u = 0; u < HLF_ROWS; ++u)
+    for (int u = 0; u < ROWS; ++u)
 #pragma unroll
       for (int j = 0; j < HLF_OUT; ++j)
         if (lane == u * HLF_OUT + j && t0 + u < n && o0 + j < O) {
@@ -680,7 +692,9 @@ GB_OP(gb_op_head_linear) {
   if (n <= HL_SMALL_ROWS && I % (a[4] == GB_BF16 ? 8 : 4) == 0 && I <= 32 * HLF_PIECES * (a[4] == GB_BF16 ? 8 : 4) &&
       a[1] % 4 == 0 && a[2] % 4 == 0 && ((a[0] | a[3]) & 15) == 0) {
 #define HLF(TW, TO)                                                                                                       \
-    gb_launch(head_linear_few_kernel<TW, TO>, dim3(gb_div_up(O, 4 * HLF_OUT), H), dim3(128), 0, ctx->stream,              \
+    gb_launch(I <= 512 / (int)sizeof(TW)    ? head_linear_few_kernel<TW, TO, 1>                                           \
+              : I <= 1024 / (int)sizeof(TW) ? head_linear_few_kernel<TW, TO, 2> : head_linear_few_kernel<TW, TO, 4>,      \
+              dim3(gb_div_up(O, 4 * HLF_OUT), H), dim3(128), 0, ctx->stream,                                              \
               op_ptr<const float>(a[0]), a[1], a[2], op_ptr<const TW>(a[3]), op_ptr<TO>(a[5]), a[7], a[8], n, O, I,       \
               op_ptr<const float>(a[13]), a[14])
     if (a[4] == GB_BF16) { if (a[6] == GB_BF16) { HLF(bf16, bf16); } else { HLF(bf16, float); } }

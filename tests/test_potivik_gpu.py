@@ -447,6 +447,31 @@ def test_head_products_of_a_few_rows(H, O, I, weights, result):
             assert ((out.double().cpu().reshape(n, H, O) - want).abs() <= tol).all(), (n, gated)
 
 
+@pytest.mark.parametrize("weights", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,O,I", [(16, 16, 32), (16, 64, 64), (16, 128, 128), (16, 64, 256), (4, 64, 512), (2, 64, 1024)])
+def test_head_products_of_a_few_rows_are_no_further_off_than_the_other_kernel(H, O, I, weights):
+    """Rows from 1 to 16 on both kernels (inputs that are not 16-byte aligned run on the other) against 64 bits, the bits
+    of a row whatever the rows beside it."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(I)
+    W = torch.randn(H, O, I, device=DEV).to(DTYPES[weights])
+    if weights == "float32" and I > 512:
+        pytest.skip("more pieces than a lane keeps: the other kernel in both cases")
+    store, off, first = torch.randn(16 * H * I + 1, device=DEV), {0: 0.0, 1: 0.0}, None
+    for shift in (0, 1):
+        x = store[shift:shift + 16 * H * I].view(16, H * I)
+        want = torch.einsum("nhi,hoi->nho", x.double().view(16, H, I), W.double())
+        whole = None
+        for n in (16, 9, 8, 5, 4, 3, 2, 1):
+            out = torch.empty(n, H * O, device=DEV)
+            hybrid.call("head_linear", [x.data_ptr(), H * I, I, W.data_ptr(), 1 if weights == "bfloat16" else 0, out.data_ptr(), 0, H * O, O,
+                                        n, H, O, I])
+            whole = out if whole is None else whole
+            assert shift or torch.equal(out, whole[:n]), n
+            off[shift] += float((out.double().view(n, H, O) - want[:n]).pow(2).sum())
+    assert off[0] <= 1.05 ** 2 * off[1], (off[0] / off[1]) ** 0.5        # (other inputs: the two sums are each within 2%)
+
+
 def _pointed_attention(window, T, hot_key, query, d=64, seed=7):
     """Weights and inputs for which the query position's score against ``hot_key`` stands far
     above all others (when that key is visible), and whose values tell keys apart.  The latent is
