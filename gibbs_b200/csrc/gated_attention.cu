@@ -376,19 +376,19 @@ sink_attention_kernel(const TQ* q, long long ldq, const TC* k_pages, const TC* v
 }
 
 // One column of a (token, head)'s chunks: factor[s] * w[s][dv] over the chunks in order, sixteen requested at a time.
-// A chunk with factor 0 left no sum and is not read.
+// A chunk without keys (a negative factor) left no sum and is not read; one whose factor has become 0 is added all the same.
 template <bool WEIGHTED>
 __device__ __forceinline__ float sa_add_chunks(const float* w, size_t ld, int splits, const float* factor) {
   float a = 0.f;
   for (int s0 = 0; s0 < splits; s0 += 16) {
     float v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = s0 + u < splits && (!WEIGHTED || factor[s0 + u] != 0.f) ? ldcg_now(w + (s0 + u) * ld) : 0.f;
+    for (int u = 0; u < 16; ++u) v[u] = s0 + u < splits && (!WEIGHTED || !(factor[s0 + u] < 0.f)) ? ldcg_now(w + (s0 + u) * ld) : 0.f;
 #pragma unroll
     for (int u = 0; u < 16; ++u)
       if (s0 + u < splits) {
         if (!WEIGHTED) a += v[u];
-        else if (factor[s0 + u] != 0.f) a = fmaf(factor[s0 + u], v[u], a);
+        else if (!(factor[s0 + u] < 0.f)) a = fmaf(factor[s0 + u], v[u], a);
       }
   }
   return a;
@@ -425,12 +425,12 @@ __global__ void sink_attention_merge_kernel(const float* ws, int splits, const f
   __syncthreads();                                         // (every warp has read the maxima)
   for (int s = threadIdx.x; s < splits; s += blockDim.x) {
     const float ms = chunk_factor[s];
-    chunk_factor[s] = ms > -INFINITY ? expf(ms - M) : 0.f;
+    chunk_factor[s] = ms > -INFINITY ? expf(ms - M) : -1.f;
   }
   __syncthreads();
   float L = sa_sink_weight(M, sink, z);
   for (int s = 0; s < splits; ++s)
-    if (chunk_factor[s] != 0.f) L = fmaf(chunk_factor[s], chunk_sum[s], L);
+    if (!(chunk_factor[s] < 0.f)) L = fmaf(chunk_factor[s], chunk_sum[s], L);
   const float inv = 1.0f / L;
   for (int dv = threadIdx.x; dv < vdim; dv += blockDim.x) {
     const float a = sa_add_chunks<true>(w + 2 + dv, ld, splits, chunk_factor);

@@ -526,3 +526,29 @@ def test_chunks_of_keys_are_merged_whatever_their_number(longest, vdim, sink):
             tol = (2 * (2 * d + 2.0 ** -20) + (len(j) + 79 + 64) * 2.0 ** -24) * (w @ v.abs()) * f
             err = (out[t, h * vdim:(h + 1) * vdim].double().cpu() - (w @ v) * f).abs()
             assert (err <= tol).all(), (t, h)
+
+
+def test_a_chunk_whose_factor_is_zero_still_counts_where_its_sum_is_no_number():
+    """The last key's score is 200 above all others, so the first chunks' factors are 0 in 32 bits; a value that is no
+    number (or infinite) in one of them makes its column none, as in one chunk and in 64 bits."""
+    from gibbs_b200.ops import hybrid, library
+    H, G, dim, vdim, ps, L = 4, 2, 16, 40, 16, 4100
+    blocks = L // ps + 1
+    q = torch.zeros(1, H * dim, device=DEV)
+    q[:, ::dim] = 20.0
+    kp, vp = torch.randn(blocks, G, ps, dim, device=DEV), torch.randn(blocks, G, ps, vdim, device=DEV)
+    kp[..., 0] = 0.0
+    kp[(L - 1) // ps, :, (L - 1) % ps, 0] = 10.0
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    lib = library("hybrid")
+    ws = torch.empty(lib.gb_sink_attention_workspace_rows(), vdim + 2, device=DEV)
+    table, req, pos = i32([list(range(blocks))]), i32([0]), i32([L - 1])
+    for value in (float("nan"), float("inf")):
+        vp[3, :, 5, 7] = value
+        out = torch.zeros(1, H * vdim, device=DEV)
+        launched = hybrid.call("sink_attention", [q.data_ptr(), kp.data_ptr(), vp.data_ptr(), table.data_ptr(), blocks, ps, blocks, req.data_ptr(),
+                                                  pos.data_ptr(), 0, 0, out.data_ptr(), H * vdim, 1, H, G, dim, vdim, 0, L, ws.data_ptr()],
+                               [1.0, 0.0, 0.0])
+        assert launched == 2
+        bad = out.view(H, vdim).isnan()
+        assert bad[:, 7].all() and int(bad.sum()) == H
