@@ -552,3 +552,42 @@ def test_a_chunk_whose_factor_is_zero_still_counts_where_its_sum_is_no_number():
         assert launched == 2
         bad = out.view(H, vdim).isnan()
         assert bad[:, 7].all() and int(bad.sum()) == H
+
+
+@pytest.mark.parametrize("H,G,dim,vdim,maps", [(1, 1, 16, 8, 1), (4, 2, 40, 24, 1), (32, 8, 64, 64, 1), (9, 3, 64, 96, 2), (70, 7, 32, 32, 1), (8, 8, 300, 64, 1)])
+@pytest.mark.parametrize("flags", [0, 1, 8, 8 | 16, 32])
+def test_queries_and_keys_have_the_same_bits_in_a_step_of_few_tokens_and_of_many(H, G, dim, vdim, maps, flags):
+    """One token, 64 (the last step with several blocks a token and a table of angles) and 65: queries, keys and values, with
+    every norm and both ways of pairing; more angles than the table holds; and the first token against 64 bits."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(dim + flags)
+    ps, ld = 16, (H + G) * maps * dim + G * vdim
+    rot = dim // 2 * 2
+    x, qg, kg = torch.randn(65, ld, device=DEV), torch.randn(H * maps * dim, device=DEV), torch.randn(G * maps * dim, device=DEV)
+    inv = torch.rand(rot // 2 + 1, device=DEV)
+    inv[-1] = 1.25
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table, pos, whole = i32([[i] for i in range(65)]), [(7 * i + 3) % ps for i in range(65)], None
+    for n in (65, 64, 1):
+        kp, vp = torch.zeros(65, G, ps, maps * dim, device=DEV), torch.zeros(65, G, ps, vdim, device=DEV)
+        out, req, at = torch.empty(n, H * maps * dim, device=DEV), i32(list(range(n))), i32(pos[:n])
+        hybrid.call("qk_prep", [x.data_ptr(), ld, H * maps * dim, (H + G) * maps * dim, qg.data_ptr(), kg.data_ptr(), inv.data_ptr(), rot,
+                                req.data_ptr(), at.data_ptr(), table.data_ptr(), 1, ps, kp.data_ptr(), vp.data_ptr(), 65, n, H, G, dim, vdim,
+                                out.data_ptr(), maps], [1e-5, 0.0, 0.0], flags=flags)
+        got = torch.cat([out, kp[:n].flatten(1), vp[:n].flatten(1)], 1)
+        whole = got if whole is None else whole
+        assert torch.equal(got, whole[:n]), n
+    v = x[0, :H * maps * dim].double().view(H * maps, dim)
+    if flags & 1:
+        v = (v / (v.pow(2).mean() + 1e-5).sqrt()) * qg.double().view_as(v)
+    if flags & 8:
+        v = v / (v.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * qg[:dim].double()
+    ang = (pos[0] * inv[:-1]).double()                       # (the angle is formed in 32 bits)
+    c, s = torch.cos(ang) * 1.25, torch.sin(ang) * 1.25
+    a, b = (v[:, :rot // 2], v[:, rot // 2:rot]) if flags & 16 else (v[:, 0:rot:2], v[:, 1:rot:2])
+    u, w = a * c - b * s, b * c + a * s
+    turned = torch.cat([u, w], 1) if flags & 16 else torch.stack([u, w], 2).flatten(1)
+    turned = torch.cat([turned, v[:, rot:]], 1)
+    if flags & 32:
+        turned = turned / (turned.pow(2).mean(1, keepdim=True) + 1e-5).sqrt()
+    assert rel_rows(whole[0, :H * maps * dim].double().view(H * maps, dim).cpu(), turned.cpu()).max() < 2e-6
