@@ -261,7 +261,7 @@ __global__ void ssm_scan_kernel(const float* xbc, long long ld, const float* dt_
 // token q's sum (SPLIT - 1 shuffles a column for SPLIT tokens).  The inputs of SCOL_TOKENS tokens at a time
 // arrive by asynchronous copies into one of two buffers while the tokens of the other are consumed.
 // Bound by the chain of a token: a long prompt is one sequence of tokens for few warps.  Measured at 64 heads of 64
-// columns, 128 state values, portions of 1801 and 333 tokens: 430 us; with one column and 32 values a thread, its
+// columns, 128 state values, portions of 1801 and 333 tokens: 418 us; with one column and 32 values a thread, its
 // reads of shared memory waited for one by one, 1028 us; with one column and 16 values a thread 640 us.
 constexpr int SCOL_TOKENS = 16, SCOL_NV = 16, SCOL_CP = 2;
 
@@ -292,7 +292,124 @@ __device__ __forceinline__ scol_f2 scol_fma(scol_f2 a, scol_f2 b, scol_f2 c) {
   return v;
 }
 
-template <int SPLIT>
+// States of up to 32 values: a thread has a whole column of a head, so a token costs no exchange.  Measured (us) beside two columns and
+// 16 values a thread, 64 columns: 32 heads of 32, 64 requests of one token 7.7 and 19.3, one of 512 tokens 117 and 129;
+// 80 heads of 16, 64 requests 15.9 and 46.0.
+constexpr int SNAR_THREADS = 64, SNAR_N = 32;
+
+__global__ void
+ssm_scan_narrow_kernel(const float* xbc, long long ld, const float* dt_raw, long long ld_dt, const float* __restrict__ dt_bias,
+                       const float* __restrict__ a_log, const float* __restrict__ dskip, float* state, long long slot_stride,
+                       const int* slot_ids, const int* q_start, const int* q_len, float* y, long long ldy, int H, int P, int N,
+                       int G) {
+  constexpr int NR = SNAR_N, COLS = SNAR_THREADS;
+  extern __shared__ __align__(16) float scol[];
+  constexpr int PER = SCOL_TOKENS * (2 * NR + COLS);      // one buffer: B [T][NR] | C [T][NR] | x [T][COLS]
+  float* sRaw = scol + 2 * PER;                            // [2][T] dt before the bias
+  float* sDt = sRaw + 2 * SCOL_TOKENS;                     // [T] step size, [T] decay
+  float* sDecay = sDt + SCOL_TOKENS;
+  pdl_trigger();
+  // (head and columns from a flat block index make this 128 registers for 74, and a portion a third slower)
+  const int col = threadIdx.x, r = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * COLS, p = p0 + col;
+  const bool active = p < P;
+  const int g = h / (H / G);
+  const int inner = H * P;
+  const float bias = dt_bias[h], neg_a = -expf(a_log[h]), dsk = dskip[h];
+  const int first = q_start[r], len = q_len[r];
+  // (this kernel keeps a head's state as [state][head_dim], so that neighbouring columns lie side by side)
+  float* S = state + (size_t)slot_ids[r] * slot_stride + (size_t)h * P * N + (active ? p : 0);
+  if (N < NR)                                              // the padding N .. NR of B and C stays zero
+    for (int i = threadIdx.x; i < 2 * PER; i += blockDim.x) scol[i] = 0.f;
+  pdl_wait();
+  float s[32];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int n = 4 * i + e;
+      s[n] = (active && n < N) ? S[(size_t)n * P] : 0.f;
+    }
+  __syncthreads();
+
+  const int pieces = N >> 2, xpieces = min(COLS, P - p0) >> 2;
+  auto stage = [&](int t0, int b) {
+    const int nt = min(SCOL_TOKENS, len - t0);
+    float* B = scol + b * PER;
+    float* C = B + SCOL_TOKENS * NR;
+    float* X = C + SCOL_TOKENS * NR;
+    for (int i = threadIdx.x; i < 2 * nt * pieces; i += blockDim.x) {
+      const int which = i / (nt * pieces), rem = i - which * nt * pieces;
+      const int tt = rem / pieces, c4 = rem - tt * pieces;
+      const float* src = xbc + (size_t)(first + t0 + tt) * ld + inner + (which ? G + g : g) * N + 4 * c4;
+      gb_cp_async_16((which ? C : B) + tt * NR + 4 * c4, src);
+    }
+    for (int i = threadIdx.x; i < nt * xpieces; i += blockDim.x) {
+      const int tt = i / xpieces, c4 = i - tt * xpieces;
+      gb_cp_async_16(X + tt * COLS + 4 * c4, xbc + (size_t)(first + t0 + tt) * ld + h * P + p0 + 4 * c4);
+    }
+    if ((int)threadIdx.x < nt)
+      gb_cp_async_4(sRaw + b * SCOL_TOKENS + threadIdx.x, dt_raw + (size_t)(first + t0 + threadIdx.x) * ld_dt + h);
+    scol_commit();
+  };
+
+  if (len > 0) stage(0, 0);
+  int b = 0;
+  for (int t0 = 0; t0 < len; t0 += SCOL_TOKENS, b ^= 1) {
+    const int nt = min(SCOL_TOKENS, len - t0);
+    if (t0 + SCOL_TOKENS < len) {
+      stage(t0 + SCOL_TOKENS, b ^ 1);
+      scol_wait<1>();                                      // this chunk has landed, the next is on its way
+    } else {
+      scol_wait<0>();
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nt) {
+      const float dt = hy_softplus(sRaw[b * SCOL_TOKENS + threadIdx.x] + bias);
+      sDt[threadIdx.x] = dt;
+      sDecay[threadIdx.x] = expf(neg_a * dt);
+    }
+    __syncthreads();
+    const float* B = scol + b * PER;
+    const float* C = B + SCOL_TOKENS * NR;
+    const float* X = C + SCOL_TOKENS * NR;
+    for (int tt = 0; tt < nt; ++tt) {
+      const float decay = sDecay[tt], xv = active ? X[tt * COLS + col] : 0.f, dx = sDt[tt] * xv;
+      float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;        // four chains; added in a fixed order
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 b4 = *reinterpret_cast<const float4*>(B + tt * NR + 4 * i);
+        const float4 c4 = *reinterpret_cast<const float4*>(C + tt * NR + 4 * i);
+        s[4 * i] = fmaf(decay, s[4 * i], b4.x * dx);
+        y0 = fmaf(s[4 * i], c4.x, y0);
+        s[4 * i + 1] = fmaf(decay, s[4 * i + 1], b4.y * dx);
+        y1 = fmaf(s[4 * i + 1], c4.y, y1);
+        s[4 * i + 2] = fmaf(decay, s[4 * i + 2], b4.z * dx);
+        y2 = fmaf(s[4 * i + 2], c4.z, y2);
+        s[4 * i + 3] = fmaf(decay, s[4 * i + 3], b4.w * dx);
+        y3 = fmaf(s[4 * i + 3], c4.w, y3);
+      }
+      const float ys = (y0 + y1) + (y2 + y3);
+      if (active) y[(size_t)(first + t0 + tt) * ldy + h * P + p] = ys + dsk * xv;
+    }
+    __syncthreads();                                       // before the copies of the chunk after next land here
+  }
+  if (active) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int n = 4 * i + e;
+        if (n < N) S[(size_t)n * P] = s[n];
+      }
+  }
+}
+
+// MANY: more blocks than stay on the chip at two an SM.  The compiler then takes 148 registers and three blocks an SM hide a
+// request's trips to memory; kept from seeing that a thread's two columns lie side by side it takes 180, reads further ahead, and
+// a long portion's chain of tokens is shorter (128 state values; the same arithmetic).  Measured, us of the first and the second:
+// 64 heads, 64 requests of one token 82 and 105, 8 of 256 tokens 184 and 215, portions of 1801 and 333 tokens 475 and 418;
+// 128 heads, one portion of 512 tokens 156 and 123.
+template <int SPLIT, bool MANY>
 __global__ void __launch_bounds__(128)
 ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long long ld_dt, const float* __restrict__ dt_bias,
                      const float* __restrict__ a_log, const float* __restrict__ dskip, float* state, long long slot_stride,
@@ -300,15 +417,16 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
                      int G) {
   constexpr int NR = SCOL_NV * SPLIT, NQ = SCOL_NV / 4;
   extern __shared__ __align__(16) float scol[];
-  const int COLS = SCOL_CP * (int)blockDim.x / SPLIT, half = COLS / SCOL_CP;
+  const int COLS = SCOL_CP * (int)blockDim.x / SPLIT;
   const int PER = SCOL_TOKENS * (2 * NR + COLS);           // one buffer: B [T][NR] | C [T][NR] | x [T][COLS]
   float* sRaw = scol + 2 * PER;                            // [2][T] dt before the bias
   float2* sDt = reinterpret_cast<float2*>(sRaw + 2 * SCOL_TOKENS);         // [T] (step size, decay)
   pdl_trigger();
-  // columns col and col + half, the column's share q.  (Neighbouring lanes have neighbouring columns and the SAME share: a
-  // quarter of a warp then reads one or two pieces of B or C, which cost shared memory one pass and not four.)
+  // columns col and col + 1 (the lanes of a share read and write whole sectors of the state, two values at a time), their share q.
+  // (Neighbouring lanes have neighbouring columns and the SAME share: a quarter of a warp then reads one or two pieces of B or
+  // C, which cost shared memory one pass and not four.)
   constexpr int CPW = 32 / SPLIT;
-  const int lane = threadIdx.x & 31, col = (threadIdx.x >> 5) * CPW + lane % CPW, q = lane / CPW;
+  const int lane = threadIdx.x & 31, col = SCOL_CP * ((threadIdx.x >> 5) * CPW + lane % CPW), q = lane / CPW;
   const int pb = (P + COLS - 1) / COLS, hp = blockIdx.x % (H * pb), r = blockIdx.x / (H * pb), h = hp % H, p0 = hp / H * COLS;
   const int g = h / (H / G);
   const int inner = H * P;
@@ -316,9 +434,11 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
   const int first = q_start[r], len = q_len[r];
   // (this kernel keeps a head's state as [state][head_dim], so that neighbouring columns lie side by side)
   float* S = state + (size_t)slot_ids[r] * slot_stride + (size_t)h * P * N;
-  bool active[SCOL_CP];
-#pragma unroll
-  for (int c = 0; c < SCOL_CP; ++c) active[c] = p0 + col + c * half < P;
+  const bool active = p0 + col < P;                        // (P is even)
+  S += active ? p0 + col : 0;
+  const bool pairs = ((uintptr_t)S & 7) == 0;
+  int one = 1;
+  if constexpr (!MANY) gb_pin(one);                        // (not known to the compiler, see above)
   // (the padding N .. NR of B and C and the columns beyond P stay zero)
   if (N < NR || p0 + COLS > P)
     for (int i = threadIdx.x; i < 2 * PER; i += blockDim.x) scol[i] = 0.f;
@@ -326,12 +446,22 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
   // this thread's state values: n = 4 (q + SPLIT i) + e, i < NQ, e < 4, in pairs (N is a multiple of 4)
   scol_f2 s[SCOL_CP][2 * NQ];
 #pragma unroll
-  for (int c = 0; c < SCOL_CP; ++c)
-#pragma unroll
-    for (int i = 0; i < 2 * NQ; ++i) {
-      const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1), at = p0 + col + c * half;
-      s[c][i] = scol_pack(active[c] && n < N ? S[(size_t)n * P + at] : 0.f, active[c] && n < N ? S[(size_t)(n + 1) * P + at] : 0.f);
+  for (int i = 0; i < 2 * NQ; ++i) {
+    const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1);
+    const float* at = S + (size_t)n * P;
+    float2 lo = make_float2(0.f, 0.f), hi = lo;
+    if (active && n < N) {
+      if (pairs) {
+        lo = *reinterpret_cast<const float2*>(at);
+        hi = *reinterpret_cast<const float2*>(at + P);
+      } else {
+        lo = make_float2(at[0], at[1]);
+        hi = make_float2(at[P], at[P + 1]);
+      }
     }
+    s[0][i] = scol_pack(lo.x, hi.x);
+    s[1][i] = scol_pack(lo.y, hi.y);
+  }
   __syncthreads();
 
   const int pieces = N >> 2, xpieces = min(COLS, P - p0) >> 2;
@@ -387,7 +517,7 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
       }
       in.dt = sDt[tt];
 #pragma unroll
-      for (int c = 0; c < SCOL_CP; ++c) in.x[c] = X[tt * COLS + c * half];
+      for (int c = 0; c < SCOL_CP; ++c) in.x[c] = X[tt * COLS + c * one];
     };
     // a token's step: this thread's share of its read-outs
     auto token = [&](const Inputs& in, float (&ys)[SCOL_CP]) {
@@ -431,8 +561,7 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
             ys[u][c] = keep + __shfl_xor_sync(0xffffffffu, give, o * CPW);
           }
         }
-        if (active[c])
-          y[(size_t)(first + t0 + tt + q) * ldy + h * P + p0 + col + c * half] = ys[0][c] + dsk * X[(tt + q) * COLS + c * half];
+        if (active) y[(size_t)(first + t0 + tt + q) * ldy + h * P + p0 + col + c] = ys[0][c] + dsk * X[(tt + q) * COLS + c];
       }
     }
     for (; tt < nt; ++tt) {
@@ -443,22 +572,24 @@ ssm_scan_cols_kernel(const float* xbc, long long ld, const float* dt_raw, long l
       for (int c = 0; c < SCOL_CP; ++c) {
 #pragma unroll
         for (int o = 1; o < SPLIT; o <<= 1) ys[c] += __shfl_xor_sync(0xffffffffu, ys[c], o * CPW);
-        if (active[c] && q == 0)
-          y[(size_t)(first + t0 + tt) * ldy + h * P + p0 + col + c * half] = ys[c] + dsk * X[tt * COLS + c * half];
+        if (active && q == 0) y[(size_t)(first + t0 + tt) * ldy + h * P + p0 + col + c] = ys[c] + dsk * X[tt * COLS + c];
       }
     }
     __syncthreads();                                       // before the copies of the chunk after next land here
   }
 #pragma unroll
-  for (int c = 0; c < SCOL_CP; ++c)
-#pragma unroll
-    for (int i = 0; i < 2 * NQ; ++i) {
-      const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1), at = p0 + col + c * half;
-      if (!active[c] || n >= N) continue;
-      const float2 v = scol_unpack(s[c][i]);
-      S[(size_t)n * P + at] = v.x;
-      S[(size_t)(n + 1) * P + at] = v.y;
+  for (int i = 0; i < 2 * NQ; ++i) {
+    const int n = 4 * (q + SPLIT * (i >> 1)) + 2 * (i & 1);
+    if (!active || n >= N) continue;
+    float* at = S + (size_t)n * P;
+    const float2 a = scol_unpack(s[0][i]), b = scol_unpack(s[1][i]);
+    if (pairs) {
+      *reinterpret_cast<float2*>(at) = make_float2(a.x, b.x);
+      *reinterpret_cast<float2*>(at + P) = make_float2(a.y, b.y);
+    } else {
+      at[0] = a.x; at[1] = b.x; at[P] = a.y; at[P + 1] = b.y;
     }
+  }
 }
 
 }  // namespace
@@ -515,20 +646,32 @@ GB_OP(gb_op_ssm_scan) {
   if (N > 256) GB_FAIL(GB_ERR_ARG, "ssm_scan: state size %d (at most 256)", N);
   // states of up to 128 values whose rows can be copied in 16-byte pieces: state in registers, 16 values of two columns a thread
   if (N <= 128 && N % 4 == 0 && P % 4 == 0 && a[1] % 4 == 0 && (a[0] & 15) == 0) {
-    const int split = N <= 32 ? 2 : (N <= 64 ? 4 : 8);
-    // four warps a block (they share the copies of B and C), two where that leaves SMs without a block
-    const int threads = (long long)R * H * gb_div_up(P, SCOL_CP * 128 / split) >= 148 ? 128 : 64;
+    if (N <= SNAR_N) {
+      const size_t smem = sizeof(float) * (2 * (size_t)SCOL_TOKENS * (2 * SNAR_N + SNAR_THREADS) + 4 * SCOL_TOKENS);
+      gb_launch(ssm_scan_narrow_kernel, dim3(R, H, gb_div_up(P, SNAR_THREADS)), dim3(SNAR_THREADS), smem,
+                ctx->stream, op_ptr<const float>(a[0]), a[1], op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]),
+                op_ptr<const float>(a[5]), op_ptr<const float>(a[6]), op_ptr<float>(a[7]), a[8], op_ptr<const int>(a[9]),
+                op_ptr<const int>(a[10]), op_ptr<const int>(a[11]), op_ptr<float>(a[12]), a[13], H, P, N, G);
+      GB_CHECK_LAUNCH("ssm_scan (a column a thread)");
+      return 1;
+    }
+    const int split = N <= 64 ? 4 : 8;
+    // four warps a block (they share the copies of B and C), two where that leaves SMs without a block, no more than have columns
+    int threads = (long long)R * H * gb_div_up(P, SCOL_CP * 128 / split) >= 148 ? 128 : 64;
+    while (threads > 32 && SCOL_CP * threads / split > P) threads /= 2;
     const int cols = SCOL_CP * threads / split;
     const size_t smem_cols = sizeof(float) * (2 * (size_t)SCOL_TOKENS * (2 * SCOL_NV * split + cols) + 4 * SCOL_TOKENS);
     // (a request's blocks follow one another, so that a long portion's are spread over all SMs: with the requests as the
     // fastest dimension every other SM got all of a long portion's blocks and the rest those of a short one)
     const dim3 grid_cols((unsigned)((long long)R * H * gb_div_up(P, cols)));
-#define SCOL_LAUNCH(SP)                                                                                               \
-    gb_launch(ssm_scan_cols_kernel<SP>, grid_cols, dim3(threads), smem_cols, ctx->stream, op_ptr<const float>(a[0]), \
+#define SCOL_LAUNCH(SP, MANY)                                                                                               \
+    gb_launch(ssm_scan_cols_kernel<SP, MANY>, grid_cols, dim3(threads), smem_cols, ctx->stream, op_ptr<const float>(a[0]), \
               a[1], op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<const float>(a[5]),              \
               op_ptr<const float>(a[6]), op_ptr<float>(a[7]), a[8], op_ptr<const int>(a[9]), op_ptr<const int>(a[10]),   \
               op_ptr<const int>(a[11]), op_ptr<float>(a[12]), a[13], H, P, N, G)
-    if (split == 2) SCOL_LAUNCH(2); else if (split == 4) SCOL_LAUNCH(4); else SCOL_LAUNCH(8);
+    if (split == 4) SCOL_LAUNCH(4, false);
+    else if (grid_cols.x > 4 * 148) SCOL_LAUNCH(8, true);
+    else SCOL_LAUNCH(8, false);
 #undef SCOL_LAUNCH
     GB_CHECK_LAUNCH("ssm_scan (columns)");
     return 1;

@@ -421,6 +421,36 @@ def test_state_space_scan_at_the_edges_of_its_groups_of_tokens(H, P, N, G):
         assert torch.equal(state[0].cpu(), S0[0]) and torch.equal(state[R + 1].cpu(), S0[R + 1])
 
 
+@pytest.mark.parametrize("H,P,N,R", [(3, 36, 32, 2), (3, 36, 36, 2), (2, 64, 64, 2), (16, 64, 128, 2), (64, 64, 128, 6), (8, 16, 128, 3)])
+def test_state_space_scan_has_the_same_bits_however_states_lie_and_portions_are_cut(H, P, N, R):
+    """States on 4-byte boundaries beside 8-byte ones; portions whole, cut in two and token by token, alone and together (few
+    blocks and many: the two forms of the kernel for 128 values)."""
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(N)
+    G, n = 1, 19
+    ld = H * P + 2 * G * N
+    xbc, dt = torch.randn(R * n, ld, device=DEV), torch.rand(R * n, H, device=DEV)
+    bias, alog, D, S0 = torch.rand(H, device=DEV), torch.rand(H, device=DEV), torch.randn(H, device=DEV), torch.randn(R, H * N * P, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def run(cuts, together, pad):
+        store = torch.zeros(R * (H * N * P + pad) + pad, device=DEV)
+        state = store[pad:].as_strided((R, H * N * P), (H * N * P + pad, 1))
+        state.copy_(S0)
+        y = torch.full((R * n, H * P), float("nan"), device=DEV)
+        for a, b in zip(cuts, cuts[1:]):
+            for who in ([list(range(R))] if together else [[r] for r in range(R)]):
+                ids, at, ln = i32(who), i32([r * n + a for r in who]), i32([b - a] * len(who))
+                hybrid.call("ssm_scan", [xbc.data_ptr(), ld, dt.data_ptr(), H, bias.data_ptr(), alog.data_ptr(), D.data_ptr(), state.data_ptr(),
+                                         H * N * P + pad, ids.data_ptr(), at.data_ptr(), ln.data_ptr(), y.data_ptr(), H * P, len(who), H, P, N, G])
+        return torch.cat([y.flatten(), state.flatten()])
+
+    want = run([0, n], True, 0)
+    assert not want.isnan().any()
+    for cuts, together, pad in (([0, n], True, 1), ([0, n], False, 0), ([0, 7, n], True, 3), (list(range(n + 1)), True, 0), (list(range(n + 1)), False, 1)):
+        assert torch.equal(run(cuts, together, pad), want), (cuts, together, pad)
+
+
 @pytest.mark.parametrize("weights,result", [("float32", "float32"), ("bfloat16", "float32"), ("bfloat16", "bfloat16")])
 @pytest.mark.parametrize("H,O,I", [(1, 1, 8), (3, 5, 24), (16, 128, 512), (2, 17, 1024), (2, 18, 1032), (4, 512, 128), (2, 9, 20)])
 def test_head_products_of_a_few_rows(H, O, I, weights, result):
