@@ -75,7 +75,7 @@ __device__ __forceinline__ void store_out(void* out, int out_dtype, int accumula
 // thread walks one segment for CPT columns and MT of the RG x MT rows, so a weight of N rows is spread
 // over N / (8 CG CPT) blocks and a chain of additions is K / 8 long.  Rows of weight and activations pass
 // through a ring of ST stages of 32 k per segment, copied 16 bytes (8 for bfloat16) a thread; the
-// weight's first stages are on their way before the kernel in front has finished.  Rows are padded
+// weight's first stages are on their way before the kernel in front has finished where no such kernel writes it (`ahead`).  Rows are padded
 // to 36 elements, which leaves the 16-byte reads of eight columns without bank conflicts.
 // Measured (weights not in L2, us; one accumulator over all of K, no ring before -> now): 2 rows
 // 1536 x 4608 51 -> 9, 1536 x 1536 25 -> 3.8, 1536 x 13824 119 -> 19 (4.4 TB/s), 6912 x 1536 94 -> 14,
@@ -95,7 +95,7 @@ template <typename TA, typename TW, int RG, int CG, int MT, int CPT, int ST>
 __global__ void __launch_bounds__(64 * RG * CG)
 gemm_simt_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
                       const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
-                      int accumulate, int M, int N, int K, int L) {
+                      int accumulate, int M, int N, int K, int L, int ahead) {
   using Ring = RowsRing<TA, TW, RG, CG, MT, CPT, ST>;
   constexpr int NB = 8 * CG * CPT, MR = RG * MT, T = 64 * RG * CG;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -131,10 +131,11 @@ gemm_simt_rows_kernel(const TA* A, long long lda, const TW* __restrict__ W, long
       copy4(dst + s * Ring::A_SEG + m * RPAD, A + (size_t)m * lda + gk, m < M && gk < K);
     }
   };
+  if (!ahead) pdl_wait();
 #pragma unroll
   for (int i = 0; i < ST - 1; ++i)
     if (i < steps) copy_w(i);
-  pdl_wait();
+  if (ahead) pdl_wait();
 #pragma unroll
   for (int i = 0; i < ST - 1; ++i) {
     if (i < steps) copy_a(i);
@@ -217,7 +218,7 @@ template <typename TA, typename TW>
 __global__ void __launch_bounds__(BM * BNT / 64, 8)
 gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long ldw,
                       const float* __restrict__ bias, void* __restrict__ out, long long ldo, int out_dtype,
-                      int accumulate, int M, int N, int K, int L, int segs, int whole) {
+                      int accumulate, int M, int N, int K, int L, int segs, int whole, int ahead) {
   constexpr int T = BM * BNT / 64, TX = BNT / 8, TY = BM / 8, RT = T * 4 / TK;     // RT rows of a tile are copied at once
   static_assert(BM % RT == 0 && BNT % RT == 0, "");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -246,10 +247,11 @@ gemm_simt_tile_kernel(const TA* A, long long lda, const TW* __restrict__ W, long
 #pragma unroll
     for (int i = 0; i < BM / RT; ++i, src += RT * lda) copy4(dst + RT * i * TPAD, src, RT * i < rows);
   };
+  if (!ahead) pdl_wait();
 #pragma unroll
   for (int i = 0; i < TST - 1; ++i)
     if (i < steps) copy_w(i);
-  pdl_wait();
+  if (ahead) pdl_wait();
 #pragma unroll
   for (int i = 0; i < TST - 1; ++i) {
     if (i < steps) copy_a(i);
@@ -429,18 +431,18 @@ gemm_simt_kernel(const TA* A, long long lda, const TW* __restrict__ W, long long
 
 template <typename TA, typename TW, int RG, int CG, int MT, int CPT, int ST>
 cudaError_t launch_rows(const TA* A, long long lda, const TW* W, long long ldw, const float* bias, void* out, long long ldo,
-                        int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+                        int out_dtype, int accumulate, int ahead, int M, int N, int K, cudaStream_t stream) {
   auto kernel = gemm_simt_rows_kernel<TA, TW, RG, CG, MT, CPT, ST>;
   constexpr int smem = RowsRing<TA, TW, RG, CG, MT, CPT, ST>::BYTES;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return gb_launch(kernel, dim3(gb_div_up(N, 8 * CG * CPT)), dim3(64 * RG * CG), smem, stream, A, lda, W, ldw, bias, out, ldo, out_dtype,
-                   accumulate, M, N, K, simt_segment(K));
+                   accumulate, M, N, K, simt_segment(K), ahead);
 }
 
 template <typename TA, typename TW>
 cudaError_t launch_tile(const TA* A, long long lda, const TW* W, long long ldw, const float* bias, void* out, long long ldo,
-                        int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+                        int out_dtype, int accumulate, int ahead, int M, int N, int K, cudaStream_t stream) {
   auto kernel = gemm_simt_tile_kernel<TA, TW>;
   using Smem = TileSmem<TA, TW>;
   static_assert(Smem::BYTES_WHOLE <= 48 * 1024, "no more shared memory than every launch may have");
@@ -463,18 +465,18 @@ cudaError_t launch_tile(const TA* A, long long lda, const TW* W, long long ldw, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, L, segs, whole);
+  return cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, L, segs, whole, ahead);
 }
 
 template <typename TA, typename TW>
 cudaError_t launch(const void* a, long long lda, const void* w, long long ldw, const float* bias, void* out, long long ldo,
-                   int out_dtype, int accumulate, int M, int N, int K, cudaStream_t stream) {
+                   int out_dtype, int accumulate, int ahead, int M, int N, int K, cudaStream_t stream) {
   const TA* A = (const TA*)a;
   const TW* W = (const TW*)w;
   // (K up to 2^30: the last segment's end is worked out in 32 bits)
   const bool rows4 = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A % (4 * sizeof(TA))) == 0 &&
                      ((uintptr_t)W % (4 * sizeof(TW))) == 0 && K <= (1 << 30);
-#define GB_ARGS A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream
+#define GB_ARGS A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, ahead, M, N, K, stream
   if (rows4 && M <= 16) {
     // Every block reads the same activations, all of them at about the same k, so those few lines of L2
     // bound the stream: 32 columns a block where the weight has enough rows for the chip (two rows,
@@ -503,11 +505,12 @@ cudaError_t launch(const void* a, long long lda, const void* w, long long ldw, c
 }  // namespace
 
 // A: [M, K] with row stride lda; W: [N, K] with row stride ldw; out: [M, N]
-// with row stride ldo (strides in elements).  accumulate != 0 adds into a
-// 32-bit output.
+// with row stride ldo (strides in elements).  `mode` bits 0 to 29, if any is set: adds into a 32-bit output; bit 30: W and the
+// bias are a model's, which no kernel in front on the stream writes, so that W is asked for before those kernels have finished.
 GB_API int gb_linear_simt(const void* A, int a_dtype, long long lda, const void* W, int w_dtype, long long ldw,
-                          const float* bias, void* out, int out_dtype, long long ldo, int accumulate, int M, int N,
-                          int K, cudaStream_t stream) {
+                          const float* bias, void* out, int out_dtype, long long ldo, int mode, int M, int N, int K,
+                          cudaStream_t stream) {
+  const int accumulate = (mode & ~(1 << 30)) != 0, ahead = (mode >> 30) & 1;
   if (M <= 0 || N <= 0) return GB_OK;
   if (K <= 0) GB_FAIL(GB_ERR_ARG, "gb_linear_simt: K = %d", K);
   if (accumulate && out_dtype != GB_F32)
@@ -517,13 +520,13 @@ GB_API int gb_linear_simt(const void* A, int a_dtype, long long lda, const void*
     GB_FAIL(GB_ERR_ARG, "gb_linear_simt: M = %d or N = %d is too large", M, N);
   cudaError_t e;
   if (a_dtype == GB_F32 && w_dtype == GB_F32)
-    e = launch<float, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<float, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, ahead, M, N, K, stream);
   else if (a_dtype == GB_BF16 && w_dtype == GB_BF16)
-    e = launch<bf16, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<bf16, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, ahead, M, N, K, stream);
   else if (a_dtype == GB_BF16 && w_dtype == GB_F32)
-    e = launch<bf16, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<bf16, float>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, ahead, M, N, K, stream);
   else if (a_dtype == GB_F32 && w_dtype == GB_BF16)
-    e = launch<float, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, M, N, K, stream);
+    e = launch<float, bf16>(A, lda, W, ldw, bias, out, ldo, out_dtype, accumulate, ahead, M, N, K, stream);
   else
     GB_FAIL(GB_ERR_ARG, "gb_linear_simt: operand dtypes %d, %d", a_dtype, w_dtype);
   if (e != cudaSuccess) GB_FAIL(GB_ERR_CUDA, "gb_linear_simt: %s", cudaGetErrorString(e));

@@ -269,7 +269,7 @@ int run_op(Walk& w, const PlanOp& o, bool force = false) {
       } else {
         PLAN_CALL(w, F_LINEAR_SIMT, ((LinearSimtFn)g_fn[F_LINEAR_SIMT])(
             ptr<const void>(w, a[0]), (int)a[12], a[1], ptr<const void>(w, a[2]), (int)a[13], a[3], bias,
-            ptr<void>(w, a[5]), (int)a[14], a[6], a[11] == 2 ? 1 : 0, M, (int)a[8], (int)a[9], w.stream));
+            ptr<void>(w, a[5]), (int)a[14], a[6], (a[11] == 2 ? 1 : 0) | 1 << 30 /* a model's weight */, M, (int)a[8], (int)a[9], w.stream));
         if (o.flags & LF_RESIDUAL) w.pend_splits = 0; else w.part_splits = 0;
       }
       return 0;

@@ -1052,6 +1052,23 @@ def test_linear_simt_at_the_edges_of_segments_and_tiles(k, pair):
                 (k / 16 + 33) * 2.0 ** -24 * (size[:33] + res.double().abs())).all()
 
 
+@pytest.mark.parametrize("rows", [1, 2, 12, 40])
+def test_linear_simt_takes_a_weight_that_the_kernel_in_front_writes(rows):
+    """The product waits for the kernel in front of it before it reads the weight (only a plan's products, whose weights no
+    kernel writes, ask for it earlier)."""
+    from gibbs_b200 import ops
+    torch.manual_seed(rows)
+    sources = [torch.randn(2048, 2048, device=DEV).to(torch.bfloat16) for _ in range(4)]
+    a, w = torch.randn(rows, 2048, device=DEV), torch.zeros(2048, 2048, device=DEV)
+    outs = [torch.empty(rows, 2048, device=DEV) for _ in range(12)]
+    for i, out in enumerate(outs):
+        ops.cast(sources[i % 4], w)
+        ops.linear_simt(a, w, None, out)
+    for i, out in enumerate(outs):
+        want = a.double() @ sources[i % 4].double().T
+        assert float((out.double() - want).norm() / want.norm()) < 1e-6, i
+
+
 @pytest.mark.parametrize("hd,group", [(4, 1), (12, 3), (32, 5), (36, 4), (64, 3), (100, 2), (128, 1), (192, 8), (256, 9)])
 def test_float32_attention_at_the_edges_of_tiles_and_warps(hd, group):
     """Contexts at the edges of key tiles and of a round of all warps' tiles, windows and soft caps.  A score is off
