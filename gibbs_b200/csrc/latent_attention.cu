@@ -545,22 +545,22 @@ latent_attention_merge_rows_kernel(const float* ws, int splits, const float* gat
   const float g = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + h]) : 1.f;
   const float inv = g / L;
   float* dst = out + (size_t)t * ldo + (size_t)h * r;
-  for (int d0 = 0; d0 < r; d0 += 256) {                    // eight columns a lane at a time
-    float a[8];
+  for (int d0 = 0; d0 < r; d0 += 128) {                    // four columns a lane at a time
+    float a[4];
 #pragma unroll
-    for (int v = 0; v < 8; ++v) a[v] = 0.f;
+    for (int v = 0; v < 4; ++v) a[v] = 0.f;
     for (int s = 0; s < splits; ++s) {
       const float es = __shfl_sync(0xffffffffu, e, s);
       if (es == 0.f) continue;                             // (the whole warp together)
       const float* ws_s = w + s * ld + 2;
-      float x[8];
+      float x[4];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) x[v] = d0 + lane + 32 * v < r ? ldcg_now(ws_s + d0 + lane + 32 * v) : 0.f;
+      for (int v = 0; v < 4; ++v) x[v] = d0 + lane + 32 * v < r ? ldcg_now(ws_s + d0 + lane + 32 * v) : 0.f;
 #pragma unroll
-      for (int v = 0; v < 8; ++v) a[v] = fmaf(es, x[v], a[v]);
+      for (int v = 0; v < 4; ++v) a[v] = fmaf(es, x[v], a[v]);
     }
 #pragma unroll
-    for (int v = 0; v < 8; ++v)
+    for (int v = 0; v < 4; ++v)
       if (d0 + lane + 32 * v < r) dst[d0 + lane + 32 * v] = a[v] * inv;
   }
 }
