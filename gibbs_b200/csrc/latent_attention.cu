@@ -647,6 +647,18 @@ static int split_chunks(int n, int H, int window, int max_ctx, int* chunk_out) {
   *chunk_out = chunk;
   return splits;
 }
+// Whether that kernel pays where the generic one could run: its CTA prepares 32 rows however few a token brings, and has an SM to
+// itself.  Measured (us, generic and whole weights on tensor cores): contexts of 2 and 7 keys 3.3 to 5.7 and 4.9 to 10.8; of 15, up to
+// 288 entries, 5.1 to 7.0 and 5.3 to 7.9, 256 tokens of 512 + 64 17 and 22; single tokens of up to 8 heads and 160 entries, 16
+// tokens at 1024 keys 16 to 19 and 17 to 21, 64 at 256 12 to 18 and 18 to 23, at 64 14 and 8 to 9, 128 at 1024 70 to 95 and 77 to 97,
+// 64 with a window of 128 11 to 13 and 14 to 15 (16 heads of 160: 16 and 18); 8 heads of 288 entries, 64 tokens with a window of 256 23 and 27, at 1024 keys without one 70 and 73, 32 tokens 40 and 38.
+static bool split_pays(int n, int R, int H, int dk, int window, int max_ctx) {
+  const int longest = max_ctx > 0 ? max_ctx : 1, span = window > 0 && window < longest ? window : longest;
+  if (span <= 8 || (span <= 16 && (dk <= 288 || n >= 192))) return false;
+  const bool near = window > 0 && window <= 256;
+  return !(n == R && n >= 16 && (dk <= 160 || (dk <= 288 && near)) && (H <= 8 || (dk <= 160 && window > 0 && window <= 128)) &&
+           (long long)n * span >= (near ? 8192 : 16384));
+}
 // Rows of (latent size + 2) floats a launch's partial results may need, whatever its sizes.
 // (also: two partial results a row for a prompt of up to 2,048 tokens and 16 heads on the tensor-core kernel)
 GB_API int gb_latent_attention_workspace_rows() { return 65536 > LA_HB * 2 * (592 + 592) ? 65536 : LA_HB * 2 * (592 + 592); }
@@ -760,7 +772,8 @@ GB_OP(gb_op_latent_attention) {
   // Measured at 16 heads, 512 + 64 entries, window 1024, portions of 1801 and 333 tokens: 0.9 ms against 4.5 on the kernel
   // below; one token each: 14 us against 38.
   if (a[22] && gb_latent_attention_split_takes(n, (int)a[21], H, r, dr, a[2] == GB_BF16, op_ptr<const void>(a[1]),
-                                               op_ptr<const void>(a[0]), op_ptr<const void>(a[11]), a[12])) {
+                                               op_ptr<const void>(a[0]), op_ptr<const void>(a[11]), a[12]) &&
+      split_pays(n, (int)a[21], H, r + dr, (int)a[17], (int)a[18])) {
     splits = split_chunks(n, H, (int)a[17], (int)a[18], &chunk);
     if (ws == nullptr || (long long)n * H * splits > gb_latent_attention_workspace_rows()) splits = 1;
     const cudaError_t e = gb_latent_attention_split_launch(

@@ -451,6 +451,44 @@ def test_state_space_scan_has_the_same_bits_however_states_lie_and_portions_are_
         assert torch.equal(run(cuts, together, pad), want), (cuts, together, pad)
 
 
+@pytest.mark.parametrize("H,r,dr,spans,window,longest,generic", [
+    (16, 128, 32, [(0, 7)], 0, 8, True), (16, 128, 32, [(0, 7)], 0, 16, True), (16, 128, 32, [(0, 7)], 0, 17, False),
+    (16, 512, 64, [(0, 7)], 0, 8, True), (16, 512, 64, [(0, 7)], 0, 9, False), (16, 512, 0, [(300, 2)] * 2, 16, 320, False),
+    (16, 256, 32, [(300, 2)] * 2, 16, 320, True), (16, 256, 32, [(300, 2)] * 2, 17, 320, False),
+    (8, 128, 32, [(300, 1)] * 16, 0, 1024, True), (8, 128, 32, [(300, 1)] * 16, 0, 1023, False), (8, 128, 32, [(300, 1)] * 15, 0, 1024, False),
+    (9, 128, 32, [(300, 1)] * 16, 0, 1024, False), (8, 136, 32, [(300, 1)] * 16, 0, 1024, False), (8, 136, 32, [(300, 1)] * 64, 256, 1024, True),
+    (8, 136, 32, [(300, 1)] * 64, 264, 1024, False), (16, 128, 32, [(300, 1)] * 64, 128, 1024, True), (16, 128, 32, [(300, 1)] * 63, 128, 1024, False),
+    (16, 128, 32, [(300, 1)] * 64, 129, 1024, False), (2, 64, 0, [(300, 1)] * 15 + [(300, 2)], 0, 1024, False)])
+def test_latent_attention_takes_the_kernel_that_pays(H, r, dr, spans, window, longest, generic):
+    """Both sides of every line of the rule: the generic kernel's bits or not, and 64 bits either way."""
+    call = LatentCalls(H, r, dr)
+    torch.manual_seed(longest)
+    n = sum(k for _, k in spans)
+    q, gate, sink = (torch.randn(*s, device=DEV) for s in ((n, H, r + dr), (n, H), (H,)))
+    got, pos = call(q, gate, sink, spans, window, longest), [p + j for p, k in spans for j in range(k)]
+    assert torch.equal(got, _generic_latent(call, q, gate, sink, spans, window, longest)) == generic
+    rows = call.pages[call.table.long()].reshape(-1, r + dr).double()
+    for t in (0, n - 1):
+        c = rows[max(0, pos[t] - window + 1) if window else 0:pos[t] + 1]
+        sc = torch.cat([q[t].double() @ c.T * (r + dr) ** -0.5, sink.double()[:, None]], 1)
+        want = (torch.softmax(sc, 1)[:, :-1] @ c[:, :r]) * torch.sigmoid(gate[t].double())[:, None]
+        assert rel_rows(got[t].view(H, r).cpu(), want.cpu()).max() < 2e-6
+
+
+def _generic_latent(call, q, gate, sink, spans, window, longest):
+    """The same call on the generic kernel (no row starts per request)."""
+    from gibbs_b200.ops import hybrid
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    R, n = len(spans), sum(k for _, k in spans)
+    req, pos = i32([i for i, (p, k) in enumerate(spans) for _ in range(k)]), i32([p + j for p, k in spans for j in range(k)])
+    out, bt = torch.full((n, call.H * call.r), float("nan"), device=DEV), call.table.expand(R, -1).contiguous()
+    hybrid.call("latent_attention", [q.data_ptr(), call.pages.data_ptr(), 1, bt.data_ptr(), call.blocks, call.ps, call.blocks,
+                                     req.data_ptr(), pos.data_ptr(), gate.data_ptr(), call.H, out.data_ptr(), call.H * call.r, n,
+                                     call.H, call.r, call.dr, window, longest, call.ws.data_ptr(), sink.data_ptr(), 0, 0],
+                [(call.r + call.dr) ** -0.5])
+    return out
+
+
 @pytest.mark.parametrize("weights,result", [("float32", "float32"), ("bfloat16", "float32"), ("bfloat16", "bfloat16")])
 @pytest.mark.parametrize("H,O,I", [(1, 1, 8), (3, 5, 24), (16, 128, 512), (2, 17, 1024), (2, 18, 1032), (4, 512, 128), (2, 9, 20)])
 def test_head_products_of_a_few_rows(H, O, I, weights, result):
