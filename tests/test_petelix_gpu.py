@@ -554,6 +554,33 @@ def test_a_chunk_whose_factor_is_zero_still_counts_where_its_sum_is_no_number():
         assert bad[:, 7].all() and int(bad.sum()) == H
 
 
+@pytest.mark.parametrize("splits,vdim", [(2, 8), (3, 33), (4, 128), (6, 200)])
+@pytest.mark.parametrize("sink", [0, 1])
+def test_merge_by_a_block_and_by_a_warp_a_row_has_the_same_bits(splits, vdim, sink):
+    """Steps on both sides of the number of rows (128 a chunk) from which a warp takes a row; contexts that leave chunks empty."""
+    from gibbs_b200.ops import hybrid, library
+    torch.manual_seed(vdim)
+    H, G, dim, ps, longest = 16, 2, 16, 16, 256 * splits
+    n, blocks = 8 * splits, longest // 16
+    q, gate = torch.randn(n, H * dim, device=DEV), torch.randn(n, H * vdim, device=DEV)
+    kp, vp = torch.randn(blocks, G, ps, dim, device=DEV), torch.randn(blocks, G, ps, vdim, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    lib = library("hybrid")
+    import ctypes
+    chunk, got = ctypes.c_int(0), {}
+    ws = torch.empty(lib.gb_sink_attention_workspace_rows(), vdim + 2, device=DEV)
+    for k in (n - 1, n):                                     # n * H = 128 * splits is the first launch by warps
+        assert lib.gb_sink_attention_chunks(k, H, G, 0, longest, ctypes.byref(chunk)) == splits
+        table, req, pos = i32([list(range(blocks))] * k), i32(list(range(k))), i32([(97 * i) % longest for i in range(k)])
+        out = torch.full((k, H * vdim), float("nan"), device=DEV)
+        launched = hybrid.call("sink_attention", [q.data_ptr(), kp.data_ptr(), vp.data_ptr(), table.data_ptr(), blocks, ps, blocks, req.data_ptr(), pos.data_ptr(),
+                                                  gate.data_ptr(), H * vdim, out.data_ptr(), H * vdim, k, H, G, dim, vdim, 0, longest, ws.data_ptr()],
+                               [dim ** -0.5, 0.0, 0.0], flags=sink)
+        assert launched == 2
+        got[k] = out
+    assert not got[n].isnan().any() and torch.equal(got[n - 1], got[n][:n - 1])
+
+
 @pytest.mark.parametrize("H,G,dim,vdim,maps", [(1, 1, 16, 8, 1), (4, 2, 40, 24, 1), (32, 8, 64, 64, 1), (9, 3, 64, 96, 2), (70, 7, 32, 32, 1), (8, 8, 300, 64, 1)])
 @pytest.mark.parametrize("flags", [0, 1, 8, 8 | 16, 32])
 def test_queries_and_keys_have_the_same_bits_in_a_step_of_few_tokens_and_of_many(H, G, dim, vdim, maps, flags):
