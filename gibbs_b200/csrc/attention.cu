@@ -478,11 +478,11 @@ paged_attention_f32_kernel(const float* q, long long ldq, const float* k_pages, 
   float* ks = sm + HEADS * hd + warp * warp_floats;                       // [AF_KT][hd + 4]: this warp's
   float* vs = ks + AF_KT * (hd + 4);                                         // [AF_KT][hd]
   float* ps = vs + AF_KT * hd;                                               // [AF_KT][HEADS]
+  const int pieces = hd >> 2;
+  pdl_wait();                                          // (positions and tables may be the work of the kernel in front)
   const int pos = tok_pos[t];
   const int* bt = block_table + (size_t)tok_req[t] * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-  const int pieces = hd >> 2;
-  pdl_wait();
   for (int i = threadIdx.x; i < HEADS * hd; i += blockDim.x) {
     const int g = i / hd;
     qs[i] = g < live_heads ? q[(size_t)t * ldq + (size_t)(h0 + g) * hd + (i - g * hd)] : 0.f;

@@ -206,7 +206,8 @@ def add_pending(x: torch.Tensor, ws: torch.Tensor, bias: Optional[torch.Tensor])
 
 def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
                 accumulate: bool = False) -> torch.Tensor:
-    """out (+)= a @ w.T (+ bias) with 32-bit FMA on the CUDA cores."""
+    """out (+)= a @ w.T (+ bias) with 32-bit FMA on the CUDA cores.  All operands, the weight among them, may be what
+    the kernel in front on the stream writes."""
     _need_cuda(a, w, bias, out)
     lib = library("core")
     m, k = a.shape

@@ -1137,6 +1137,27 @@ def test_float32_attention_is_as_exact_as_the_general_kernel(hd, group):
     assert off[0] <= off[1], (off[0] / off[1]) ** 0.5
 
 
+def test_float32_attention_takes_positions_that_the_kernel_in_front_writes():
+    """A caller that counts its positions up on the device, directly in front of each call."""
+    from gibbs_b200 import ops
+    torch.manual_seed(5)
+    kvh, group, hd, ps, n = 2, 3, 64, 16, 40
+    kp, vp = torch.randn(n * 4, kvh, ps, hd, device=DEV), torch.randn(n * 4, kvh, ps, hd, device=DEV)
+    bt, req = torch.arange(n * 4, dtype=torch.int32, device=DEV).view(n, 4), torch.arange(n, dtype=torch.int32, device=DEV)
+    pos, status = torch.zeros(n, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    q, filler = torch.randn(n, kvh * group * hd, device=DEV), torch.zeros(1 << 22, device=DEV)
+    outs = [torch.empty_like(q) for _ in range(24)]
+    for out in outs:
+        filler.add_(1.0)
+        pos.add_(2)
+        ops.paged_attention(q, kvh * group, kvh, hd, kp, vp, bt, req, pos, hd ** -0.5, 0, out, status)
+    for i, out in enumerate(outs):
+        last, want = torch.full((n,), 2 * (i + 1), dtype=torch.int32, device=DEV), torch.empty_like(q)
+        torch.cuda.synchronize()
+        ops.paged_attention(q, kvh * group, kvh, hd, kp, vp, bt, req, last, hd ** -0.5, 0, want, status)
+        assert torch.equal(out, want), i
+
+
 @pytest.mark.parametrize("vocab,k", [(1000, 5), (65536, 20), (50257, 1), (7, 32)])
 def test_logprob_info_matches_the_plain_rule(vocab, k):
     """Probability of the chosen token, entropy and the k most probable tokens of every row,
