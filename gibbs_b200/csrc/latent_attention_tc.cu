@@ -330,8 +330,9 @@ template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStrea
 //  columns.  Key tiles lie at multiples of 32, so a row's sums are grouped by its position alone, whatever the rows
 //  beside it.  With `splits`, blockIdx.y takes a chunk of keys, a multiple of `chunk` from position 0, and leaves (maximum,
 //  sum, weighted sum) per row for the merge kernel.
-//  Bound by the shared-memory reads of the tensor operands (about 2,700 cycles a tile of 32 x 32 at 512 + 64 entries
-//  against 1,600 of mma.sync).
+//  Bound by waiting: a step of 32 rows x 32 keys takes about 10,000 cycles at 512 + 64 entries, where its operand reads
+//  from shared memory need 2,700 and its mma.sync 1,600; one CTA an SM meets three barriers a key tile, and scores, softmax
+//  and weighted sum follow one another.
 constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLD = 36, LTX_PLD = 40;
 
 struct LtxParams {
