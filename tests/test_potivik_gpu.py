@@ -137,11 +137,11 @@ def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H
     rows = library("hybrid").gb_latent_attention_workspace_rows()
     ws = torch.full((rows, r + 2), float("nan"), device=DEV)
     for what, spans in lens_of.items():
-        if window == 0 and what != "single":
-            continue                                        # (such steps run on the kernel without windows)
         tok_req = [i for i, (p, k) in enumerate(spans) for _ in range(k)]
         tok_pos = [p + j for p, k in spans for j in range(k)]
         n = len(tok_req)
+        if window == 0 and n >= 8 * R and n * H >= 256:
+            continue                                        # (such steps run on the kernel without windows)
         starts = [sum(k for _, k in spans[:i]) for i in range(R)]
         q, gate = torch.randn(n, H, Dk), torch.randn(n, H)
         dev = {k: v.to(DEV).contiguous() for k, v in dict(q=q, pages=pages, gate=gate, sink=sink).items()}
@@ -168,10 +168,10 @@ def test_latent_attention_with_whole_weights_is_as_exact_as_the_generic_kernel(H
             assert ((got[True][t] - want).abs() <= tol).all(), (what, t)
             for tc in off:
                 off[tc] += float((got[tc][t] - want).pow(2).sum())
-        # (two kernels did run; one key of few entries gives both the same sums, and both end by the merge's arithmetic)
+        # (two kernels did run; a window of one key runs on the generic kernel)
         assert window == 1 or not torch.equal(got[True], got[False])
-        if what == "portions":                              # (rows enough for the two errors to be compared: measured 0.4 to 1.1)
-            assert off[True] <= 1.25 ** 2 * off[False], (off[True] / off[False]) ** 0.5
+        if what != "single":                                # (rows enough for the two errors to be compared: measured 0.55 to 1)
+            assert off[True] <= off[False], (off[True] / off[False]) ** 0.5
 
 
 @pytest.mark.parametrize("H,r,dr", [(1, 32, 0), (2, 64, 0), (4, 64, 16), (16, 128, 0), (16, 128, 32), (8, 256, 32), (16, 512, 0), (16, 512, 64)])
