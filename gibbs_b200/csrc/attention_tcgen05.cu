@@ -19,6 +19,10 @@
 // 64, and at head_dim 128 with 64-key tiles): while one is in its softmax the other's products
 // run.  The softmax warps meet at no barrier: each waits for the products itself.
 //
+// A launch of few tiles (a portion of a few hundred tokens over a long context) would take as long as one CTA needs for all
+// of a row tile's keys: there a cluster of up to four CTAs shares them.  Each leaves its unnormalised O, maximum and sum in its
+// own shared memory, and each adds up a share of the columns of all of them through distributed shared memory.
+//
 // V lies in shared memory as [key][head_dim]: for O = P V it is the B operand with its N index
 // contiguous ("MN-major"), which tcgen05 reads directly; nothing is transposed.
 //
@@ -40,6 +44,8 @@ using namespace sm100;
 constexpr int ROWS = 128;            // rows of a CTA's tile: tokens x heads of the group
 constexpr int RING = 3;              // buffers of one K or V tile each
 constexpr int STATUS_ATTN_TIMEOUT = 24;
+constexpr int MAX_PARTS = 4;         // most CTAs a row tile's keys are shared among
+constexpr int MIN_PART_TILES = 3;    // key tiles a share has at least (the exchange costs about one)
 
 struct Params {
   const int* block_table; int bt_stride; int page_size; int n_pages;
@@ -56,6 +62,7 @@ template <int HD, int KEYS> struct Cfg {
   static constexpr int Q_BYTES = ROWS * HD * 2;
   static constexpr int KV_BYTES = KEYS * HD * 2;
   static constexpr int P_BYTES = ROWS * KEYS * 2;
+  static_assert(Q_BYTES + P_BYTES + RING * KV_BYTES >= ROWS * HD * 4 + ROWS * 8, "a share of O and its (m, l) fit over the operands");
   static constexpr int SMEM_BYTES = Q_BYTES + P_BYTES + RING * KV_BYTES + 1024;
   static constexpr int TMEM_COLS = KEYS + HD <= 128 ? 128 : 256;   // S: KEYS columns, O: HD columns
   // CTAs per SM: by tensor memory (512 columns), shared memory and registers (64 K for 192 threads each).
@@ -101,6 +108,24 @@ __device__ __forceinline__ float exp_row(const float (&v)[KEYS], float scale, fl
   upk2(add2(ls2[0], ls2[1]), a0, a1);
   upk2(add2(ls2[2], ls2[3]), b0, b1);
   return (a0 + a1) + (b0 + b1);
+}
+
+// A value at the same shared-memory place of CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(const float2* p, int rank) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(const float4* p, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
 }
 
 template <int HD, int KEYS>
@@ -163,7 +188,16 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int pos0 = spos + first_tok;                           // its position
   const int hi_all = pos0 + n_tok;                             // keys < hi_all may be visible
   const int lo_all = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
-  const int t_lo = lo_all / KEYS, t_hi = (hi_all + KEYS - 1) / KEYS;
+  int t_lo = lo_all / KEYS, t_hi = (hi_all + KEYS - 1) / KEYS;
+  // The key tiles in `parts` contiguous shares, one for each of the first CTAs of the cluster; the others have nothing to do
+  // (a thread that has left counts as arrived at the cluster's barriers).
+  const int parts = max(1, min((int)gridDim.z, (t_hi - t_lo) / MIN_PART_TILES)), part = (int)blockIdx.z;
+  if (part >= parts) return;
+  {
+    const int whole = t_hi - t_lo, from = t_lo;
+    t_lo = from + whole * part / parts;
+    t_hi = from + whole * (part + 1) / parts;
+  }
   const int n_tiles = t_hi - t_lo;
 
   if (warp == 1) {
@@ -182,7 +216,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   };
   int first_page = 0, page_cur = OUTSIDE;
   if (warp == 0) {
-    first_page = bt[lo_all / p.page_size];
+    first_page = bt[max(lo_all, t_lo * KEYS) / p.page_size];
     page_cur = t_lo < t_hi ? lookup(t_lo) : OUTSIDE;
     gb_pin(first_page);                                        // (stay in front of the waits below, see gb_pin)
     gb_pin(page_cur);
@@ -417,7 +451,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       }
     }
     tc_fence_after();
-    if (alive) {
+    if (parts > 1) {
+      // This share's O (not divided by its sum), maximum and sum, for the cluster: [HD / 4][128 rows] pieces of four columns
+      // over the operands' buffers, which nothing reads any more, then the rows' (m, l).
+      float4* po = reinterpret_cast<float4*>(base);
+      float2* pm = reinterpret_cast<float2*>(base + HD * ROWS * 4);
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD; c0 += 32) {
+        float o[32];
+        tmem_ld_32(tmem_o + lane_off + (uint32_t)c0, o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          po[(size_t)(c0 / 4 + i) * ROWS + row] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      }
+      pm[row] = make_float2(m_used, l_run);
+    } else if (alive) {
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       bf16* dst = p.out + (size_t)(row0 + tl) * p.ldo + (size_t)(kvh * group + g) * HD;
 #pragma unroll 1
@@ -443,6 +491,60 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
       }
     }
+  }
+  if (parts > 1) {
+    cluster_sync_all();                                        // every share lies in its CTA's shared memory
+    if (warp >= 2) {
+      // O = sum_z 2^(m_z - M) O_z / sum_z 2^(m_z - M) l_z, in the keys' order
+      const int row = 32 * (warp & 3) + lane;
+      const int tl = row / group, g = row - tl * group;
+      float wgt[MAX_PARTS], top = -INFINITY, sum = 0.f;
+      float2 ml[MAX_PARTS];
+#pragma unroll
+      for (int z = 0; z < MAX_PARTS; ++z) {
+        ml[z] = make_float2(-INFINITY, 0.f);
+        if (z < parts) ml[z] = ld_cluster_f2(reinterpret_cast<const float2*>(base + HD * ROWS * 4) + row, z);
+        top = fmaxf(top, ml[z].x);
+      }
+#pragma unroll
+      for (int z = 0; z < MAX_PARTS; ++z) {
+        wgt[z] = ml[z].x == -INFINITY ? 0.f : exp2f(ml[z].x - top);
+        sum += wgt[z] * ml[z].y;
+      }
+      const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+      bf16* dst = p.out + (size_t)(row0 + tl) * p.ldo + (size_t)(kvh * group + g) * HD;
+      // (HD / 8 pieces of eight columns; a CTA takes an even share of them)
+      const int piece_end = HD / 8 * (part + 1) / parts;
+      for (int piece = HD / 8 * part / parts; piece < piece_end; ++piece) {
+        float4 v[MAX_PARTS][2];
+#pragma unroll
+        for (int z = 0; z < MAX_PARTS; ++z)
+          if (z < parts) {
+            v[z][0] = ld_cluster_f4(reinterpret_cast<const float4*>(base) + (size_t)(2 * piece) * ROWS + row, z);
+            v[z][1] = ld_cluster_f4(reinterpret_cast<const float4*>(base) + (size_t)(2 * piece + 1) * ROWS + row, z);
+          }
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int z = 0; z < MAX_PARTS; ++z)
+          if (z < parts && wgt[z] != 0.f) {                    // (a share of which a row sees nothing is not added, whatever it holds)
+            a[0] = fmaf(wgt[z], v[z][0].x, a[0]); a[1] = fmaf(wgt[z], v[z][0].y, a[1]);
+            a[2] = fmaf(wgt[z], v[z][0].z, a[2]); a[3] = fmaf(wgt[z], v[z][0].w, a[3]);
+            a[4] = fmaf(wgt[z], v[z][1].x, a[4]); a[5] = fmaf(wgt[z], v[z][1].y, a[5]);
+            a[6] = fmaf(wgt[z], v[z][1].z, a[6]); a[7] = fmaf(wgt[z], v[z][1].w, a[7]);
+          }
+        if (tl < n_tok) {
+          uint32_t pk[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            __nv_bfloat162 b2 = __floats2bfloat162_rn(a[2 * e] * inv, a[2 * e + 1] * inv);
+            pk[e] = *reinterpret_cast<uint32_t*>(&b2);
+          }
+          *reinterpret_cast<uint4*>(dst + 8 * piece) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();                                        // nobody leaves while another CTA reads its share
   }
   tc_fence_before();
   __syncthreads();
@@ -509,6 +611,16 @@ bool pages_map(CUtensorMap* out, const void* pages, long long rows, int hd, int 
   return true;
 }
 
+// CTAs that share a row tile's keys: as many as stay on the chip at two an SM.  GIBBS_B200_ATTN_PARTS=1..4 overrides.
+int key_parts(long long ctas) {
+  static const int forced = [] {
+    const char* e = getenv("GIBBS_B200_ATTN_PARTS");
+    return e ? atoi(e) : 0;
+  }();
+  if (forced >= 1 && forced <= MAX_PARTS) return forced;
+  return ctas <= 74 ? 4 : (ctas <= 296 ? 2 : 1);
+}
+
 template <int HD, int KEYS>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, int n_tiles,
            cudaStream_t stream) {
@@ -518,8 +630,27 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
                                  Cfg<HD, KEYS>::SMEM_BYTES));
     attr_set = true;
   }
-  gb_launch(attention_tcgen05_kernel<HD, KEYS>, dim3(p.kv_heads, n_tiles), dim3(192), Cfg<HD, KEYS>::SMEM_BYTES, stream,
-            mq, mk, mv, p);
+  const int parts = key_parts((long long)n_tiles * p.kv_heads);
+  if (parts == 1) {
+    gb_launch(attention_tcgen05_kernel<HD, KEYS>, dim3(p.kv_heads, n_tiles), dim3(192), Cfg<HD, KEYS>::SMEM_BYTES, stream,
+              mq, mk, mv, p);
+    return GB_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.kv_heads, n_tiles, parts);
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = Cfg<HD, KEYS>::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = parts;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
+  GB_CUDA(cudaLaunchKernelEx(&cfg, attention_tcgen05_kernel<HD, KEYS>, mq, mk, mv, p));
   return GB_OK;
 }
 

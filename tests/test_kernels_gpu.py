@@ -596,6 +596,43 @@ def test_attention_tensor_cores(heads, kvh, hd, ps, window, before, q_lens):
         assert ops.launch_count() - before_launches == 2        # split keys + merge
 
 
+# long contexts in launches of few tiles: a row tile's keys are shared by 2 or 4 CTAs of a cluster; unequal shares, windows, single
+# tokens beside a portion, shares whose every key some rows do not see
+@pytest.mark.parametrize("heads,kvh,hd,ps,window,before,lens", [
+    (24, 8, 64, 16, 0, [1500, 700, 3000, 90], [400, 1, 1, 1]), (4, 4, 64, 128, 0, [1100], [10]), (2, 1, 64, 16, 0, [0], [1000]),
+    (12, 2, 128, 32, 900, [1200, 0], [150, 43]), (16, 2, 128, 16, 0, [4000], [20]), (32, 8, 64, 16, 0, [0], [1500]),
+    (8, 2, 64, 8, 500, [2000], [130]),
+])
+def test_attention_of_portions_over_long_contexts(heads, kvh, hd, ps, window, before, lens):
+    from gibbs_b200 import ops
+    torch.manual_seed(heads + hd)
+    n, group, total = sum(lens), heads // kvh, sum(before) + sum(lens)
+    n_pages = total // ps + len(lens) + 8
+    bt, tok_req, tok_pos = _layout(before, lens, ps, n_pages, seed=hd)
+    q, kp, vp = (torch.randn(*shape, device=DEV).bfloat16() for shape in ((n, heads * hd), (n_pages, kvh, ps, hd), (n_pages, kvh, ps, hd)))
+    out = torch.empty(n, heads * hd, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    tables = t(bt)
+    ops.paged_attention(q, heads, kvh, hd, kp, vp, tables, t(tok_req), t(tok_pos), hd ** -0.5, window, out, status, hints=_Hints(before, lens))
+    row = 0
+    for r, (a, b) in enumerate(zip(before, lens)):
+        idx = torch.arange(a + b, device=DEV)
+        pages = tables[r].long()[idx // ps]
+        k, v = (x[pages, :, idx % ps].double().repeat_interleave(group, 1) for x in (kp, vp))
+        at = torch.arange(a, a + b, device=DEV)
+        seen = idx[None] <= at[:, None]
+        if window:
+            seen &= idx[None] > at[:, None] - window
+        s = torch.einsum("thd,khd->thk", q[row:row + b].double().reshape(b, heads, hd), k) * hd ** -0.5
+        w = torch.softmax(s.masked_fill(~seen[:, None], -math.inf), 2)
+        want, size = torch.einsum("thk,khd->thd", w, v), torch.einsum("thk,khd->thd", w, v.abs())
+        err = (out[row:row + b].double().reshape(b, heads, hd) - want).abs()
+        assert (err <= 2.0 ** -8 * (size + want.abs()) + 1e-6).all(), r          # weights and outputs of 8 bits
+        row += b
+    assert int(status.item()) == 0
+
+
 def test_attention_tensor_cores_far_key_and_tile_edges():
     """A dominant key at the edges of the 64-key tiles and of the splits."""
     from gibbs_b200 import ops
