@@ -18,6 +18,8 @@
 
 namespace {
 
+constexpr int CONV_RUN_THREADS = 64;
+
 constexpr int MAX_TAPS = 16;
 
 template <typename T>
@@ -110,24 +112,42 @@ __global__ void short_conv_out_vec8_kernel(const bf16* bcx, long long ld, const 
   *reinterpret_cast<uint4*>(out + (size_t)t * hidden + c) = o;
 }
 
-// The same for narrow filters (K <= 4), eight consecutive tokens per thread: the products B*x a
-// filter position needs are kept in registers while the window slides along the tokens, so every
-// row of [B | C | x] is read once instead of K times and the taps once per thread.  Where the run
-// crosses into another request the window restarts from that request's state.  The terms are
-// added in the order of the kernels above (oldest tap first), so the results are the same bits.
-template <int K>
-__global__ void short_conv_out_run_kernel(const bf16* bcx, long long ld, const float* __restrict__ taps,
-                                          const float* __restrict__ bias, const float* state,
-                                          long long slot_stride, const int* slot_ids,
-                                          const int* tok_req, const int* q_start,
-                                          bf16* __restrict__ out, int n_tokens, int hidden) {
-  constexpr int RUN = 8;
+// The same for narrow filters (K <= 4), RUN consecutive tokens of one portion per thread, and the state update with it: the
+// products B*x a filter position needs are kept in registers while the window slides along the tokens, so every
+// row of [B | C | x] is read once (and K - 1 rows of the run in front) and the taps once per thread.  Runs start with
+// their portion, so with K - 1 <= RUN only the first run's thread reads the request's state: it leaves the new one
+// there too (a kernel of its own for that cost 2.4 us of every launch).  The terms are added in the order of the kernels
+// above (oldest tap first), so the results are the same bits.
+template <int K, int RUN>
+__global__ void __launch_bounds__(CONV_RUN_THREADS)
+short_conv_run_kernel(const bf16* bcx, long long ld, const float* __restrict__ taps, const float* __restrict__ bias,
+                      float* state, long long slot_stride, const int* slot_ids, const int* q_start, const int* q_len,
+                      bf16* __restrict__ out, int n_requests, int hidden) {
+  static_assert(K - 1 <= RUN, "only a portion's first run may reach back to the state");
   pdl_trigger();
-  const int groups = hidden >> 3;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n_runs = ((long long)n_tokens + RUN - 1) / RUN;
-  if (gid >= n_runs * groups) return;
-  const int run = (int)(gid / groups), c = (int)(gid - (long long)run * groups) << 3;
+  const int lane = threadIdx.x & 31;
+  // which request's which run: a request has ceil(tokens / RUN) of them, one after the other
+  int req = -1, run = 0, len = 0, before = 0;
+  for (int r0 = 0; r0 < n_requests && req < 0; r0 += 32) {
+    const int mine = r0 + lane, n = mine < n_requests ? q_len[mine] : 0;
+    const int runs = n > 0 ? (n + RUN - 1) / RUN : 0;
+    int upto = runs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.x);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      req = r0 + src;
+      len = __shfl_sync(0xffffffffu, n, src);
+      run = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - runs, src);
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  const int c = (blockIdx.y * CONV_RUN_THREADS + threadIdx.x) << 3;
+  if (req < 0 || c >= hidden) return;
   auto unpack = [](uint4 u, float* f) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
@@ -137,6 +157,9 @@ __global__ void short_conv_out_run_kernel(const bf16* bcx, long long ld, const f
       f[2 * e + 1] = v.y;
     }
   };
+  // Taps, bias and the step's metadata do not come from the product in front: they are read before the wait for it.  Behind
+  // the wait all rows of the run, and the K-1 older positions of its first token, are requested before the first is used
+  // (a thread that fetched them one by one would spend as many memory latencies one after the other).
   float tap[K][8], bs[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
@@ -144,107 +167,92 @@ __global__ void short_conv_out_run_kernel(const bf16* bcx, long long ld, const f
     for (int j = 0; j < K; ++j) tap[j][e] = taps[(size_t)(c + e) * K + j];
     bs[e] = bias ? bias[c + e] : 0.f;
   }
-  float win[K][8];                                           // win[j]: the product that meets tap j for the current token
-  const int t0 = run * RUN, t1 = min(t0 + RUN, n_tokens);
-  // Taps, bias and the step's metadata (which request a token belongs to, where the request starts
-  // in the batch, its state slot) do not come from the product in front: they are read before the
-  // wait for it.  Behind the wait all rows of the run, and the K-1 older positions of its first
-  // token, are requested before the first is used (a thread that fetched them one by one would spend
-  // as many memory latencies one after the other).
-  int rreq[RUN];
-#pragma unroll
-  for (int u = 0; u < RUN; ++u) rreq[u] = tok_req[t0 + u < t1 ? t0 + u : t1 - 1];
-  int cur_req = rreq[0], first = q_start[cur_req];
-  const float* st0 = state + (size_t)slot_ids[cur_req] * slot_stride;
+  int first = q_start[req];
+  float* st = state + (size_t)slot_ids[req] * slot_stride + c;
   gb_pin(first);
-  gb_pin(st0);
-#pragma unroll
-  for (int u = 0; u < RUN; ++u) gb_pin(rreq[u]);
+  gb_pin(st);
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
 #pragma unroll
     for (int j = 0; j < K; ++j) gb_pin(tap[j][e]);
     gb_pin(bs[e]);
   }
+  const int i0 = run * RUN, n = min(RUN, len - i0);          // the run's first token of the portion, its tokens
+  const bf16* rows = bcx + (size_t)first * ld + c;           // the portion's rows
   pdl_wait();
-  uint4 rb[RUN], rx[RUN], rg[RUN];
+  uint4 rb[RUN], rx[RUN], rg[RUN], ob[K - 1], ox[K - 1], eb[K - 1], ex[K - 1];
 #pragma unroll
   for (int u = 0; u < RUN; ++u) {
-    const int t = t0 + u < t1 ? t0 + u : t1 - 1;
-    const bf16* row = bcx + (size_t)t * ld;
-    rb[u] = __ldcg(reinterpret_cast<const uint4*>(row + c));
-    rx[u] = __ldcg(reinterpret_cast<const uint4*>(row + 2 * hidden + c));
-    rg[u] = __ldcg(reinterpret_cast<const uint4*>(row + hidden + c));
+    const bf16* row = rows + (size_t)(i0 + (u < n ? u : n - 1)) * ld;
+    rb[u] = __ldcg(reinterpret_cast<const uint4*>(row));
+    rx[u] = __ldcg(reinterpret_cast<const uint4*>(row + 2 * hidden));
+    rg[u] = __ldcg(reinterpret_cast<const uint4*>(row + hidden));
   }
-  {
-    // the K-1 older positions of the run's first token: earlier tokens of its request in the batch, or its state
-    const int i0 = t0 - first;
-    uint4 ob[K - 1], ox[K - 1];
 #pragma unroll
-    for (int j = 0; j < K - 1; ++j) {
-      const int src = i0 - (K - 1 - j);
-      if (src >= 0) {
-        const bf16* prow = bcx + (size_t)(first + src) * ld;
-        ob[j] = __ldcg(reinterpret_cast<const uint4*>(prow + c));
-        ox[j] = __ldcg(reinterpret_cast<const uint4*>(prow + 2 * hidden + c));
-      } else {
-        const uint4* sp = reinterpret_cast<const uint4*>(st0 + (size_t)(K - 1 + src) * hidden + c);
-        ob[j] = __ldcg(sp);
-        ox[j] = __ldcg(sp + 1);
-      }
+  for (int j = 0; j < K - 1; ++j) {
+    if (run > 0) {
+      const bf16* row = rows + (size_t)(i0 - (K - 1 - j)) * ld;
+      ob[j] = __ldcg(reinterpret_cast<const uint4*>(row));
+      ox[j] = __ldcg(reinterpret_cast<const uint4*>(row + 2 * hidden));
+    } else {
+      const uint4* sp = reinterpret_cast<const uint4*>(st + (size_t)j * hidden);
+      ob[j] = __ldcg(sp);
+      ox[j] = __ldcg(sp + 1);
+      // the new state: the last K-1 products (a portion of fewer tokens keeps old ones in front of its own)
+      const bf16* row = rows + (size_t)max(len - (K - 1) + j, 0) * ld;
+      eb[j] = __ldcg(reinterpret_cast<const uint4*>(row));
+      ex[j] = __ldcg(reinterpret_cast<const uint4*>(row + 2 * hidden));
     }
+  }
+  float win[K][8];                                           // win[j]: the product that meets tap j for the current token
+#pragma unroll
+  for (int j = 0; j < K - 1; ++j) {
+    if (run > 0) {
+      float pb[8], px[8];
+      unpack(ob[j], pb);
+      unpack(ox[j], px);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) win[j][e] = pb[e] * px[e];
+    } else {
+      win[j][0] = __uint_as_float(ob[j].x); win[j][1] = __uint_as_float(ob[j].y);
+      win[j][2] = __uint_as_float(ob[j].z); win[j][3] = __uint_as_float(ob[j].w);
+      win[j][4] = __uint_as_float(ox[j].x); win[j][5] = __uint_as_float(ox[j].y);
+      win[j][6] = __uint_as_float(ox[j].z); win[j][7] = __uint_as_float(ox[j].w);
+    }
+  }
+  if (run == 0) {
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) {
-      if (i0 - (K - 1 - j) >= 0) {
+      float v[8];
+      if (len + j >= K - 1) {
         float pb[8], px[8];
-        unpack(ob[j], pb);
-        unpack(ox[j], px);
+        unpack(eb[j], pb);
+        unpack(ex[j], px);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) win[j][e] = pb[e] * px[e];
+        for (int e = 0; e < 8; ++e) v[e] = pb[e] * px[e];
       } else {
-        win[j][0] = __uint_as_float(ob[j].x); win[j][1] = __uint_as_float(ob[j].y);
-        win[j][2] = __uint_as_float(ob[j].z); win[j][3] = __uint_as_float(ob[j].w);
-        win[j][4] = __uint_as_float(ox[j].x); win[j][5] = __uint_as_float(ox[j].y);
-        win[j][6] = __uint_as_float(ox[j].z); win[j][7] = __uint_as_float(ox[j].w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+#pragma unroll
+        for (int w = 1; w < K - 1; ++w)
+          if (w == len + j) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = win[w][e];
+          }
       }
+      float4* dst = reinterpret_cast<float4*>(st + (size_t)j * hidden);
+      dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+      dst[1] = make_float4(v[4], v[5], v[6], v[7]);
     }
   }
+  bf16* dst = out + (size_t)(first + i0) * hidden + c;
 #pragma unroll
   for (int u = 0; u < RUN; ++u) {
-    const int t = t0 + u;
-    if (t >= t1) break;
-    const int r = rreq[u];
-    const bool restart = r != cur_req;                       // (never the run's first token: it is prepared above)
-    if (restart) {
-      cur_req = r;
-      first = q_start[r];
-    }
-    const int i = t - first;
+    if (u >= n) break;
     float b[8], x[8], g[8];
     unpack(rb[u], b);
     unpack(rx[u], x);
     unpack(rg[u], g);
-    if (restart) {
-      // the K-1 older positions: earlier tokens of this request in the batch, or its state
-      const float* st = state + (size_t)slot_ids[r] * slot_stride;
-#pragma unroll
-      for (int j = 0; j < K - 1; ++j) {
-        const int src = i - (K - 1 - j);
-        if (src >= 0) {
-          const bf16* prow = bcx + (size_t)(first + src) * ld;
-          float pb[8], px[8];
-          unpack(*reinterpret_cast<const uint4*>(prow + c), pb);
-          unpack(*reinterpret_cast<const uint4*>(prow + 2 * hidden + c), px);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) win[j][e] = pb[e] * px[e];
-        } else {
-          const float4* sp = reinterpret_cast<const float4*>(st + (size_t)(K - 1 + src) * hidden + c);
-          const float4 s0 = sp[0], s1 = sp[1];
-          win[j][0] = s0.x; win[j][1] = s0.y; win[j][2] = s0.z; win[j][3] = s0.w;
-          win[j][4] = s1.x; win[j][5] = s1.y; win[j][6] = s1.z; win[j][7] = s1.w;
-        }
-      }
-    }
 #pragma unroll
     for (int e = 0; e < 8; ++e) win[K - 1][e] = b[e] * x[e];
     uint4 o;
@@ -259,7 +267,7 @@ __global__ void short_conv_out_run_kernel(const bf16* bcx, long long ld, const f
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(g[2 * e] * acc[2 * e], g[2 * e + 1] * acc[2 * e + 1]);
-    *reinterpret_cast<uint4*>(out + (size_t)t * hidden + c) = o;
+    *reinterpret_cast<uint4*>(dst + (size_t)u * hidden) = o;
     // slide: the next token's tap j meets what tap j+1 met now
 #pragma unroll
     for (int j = 0; j < K - 1; ++j)
@@ -469,17 +477,17 @@ GB_API int gb_short_conv(const void* bcx, int dtype, long long ld, const float* 
     const bool vec = hidden % 8 == 0 && ld % 8 == 0 && slot_stride % 4 == 0 && ((uintptr_t)bcx & 15) == 0 &&
                      ((uintptr_t)out & 15) == 0 && ((uintptr_t)state & 15) == 0;
     if (vec && K <= 4) {
-      const long long work = (((long long)n_tokens + 7) / 8) * (hidden / 8);
-      const dim3 grid(gb_div_up(work, 128)), block(128);
-      if (K == 2)
-        gb_launch(short_conv_out_run_kernel<2>, grid, block, 0, stream, (const bf16*)bcx, ld, taps, bias,
-                  (const float*)state, slot_stride, slot_ids, tok_req, q_start, (bf16*)out, n_tokens, hidden);
-      else if (K == 3)
-        gb_launch(short_conv_out_run_kernel<3>, grid, block, 0, stream, (const bf16*)bcx, ld, taps, bias,
-                  (const float*)state, slot_stride, slot_ids, tok_req, q_start, (bf16*)out, n_tokens, hidden);
-      else
-        gb_launch(short_conv_out_run_kernel<4>, grid, block, 0, stream, (const bf16*)bcx, ld, taps, bias,
-                  (const float*)state, slot_stride, slot_ids, tok_req, q_start, (bf16*)out, n_tokens, hidden);
+      // (short runs while there are too few threads to fill the chip: four tokens a thread below 2,048)
+      const bool few = n_tokens < 2048;
+      // (a portion's last run may be partly filled: at most one per request beside the whole ones)
+      const dim3 grid(n_tokens / (few ? 4 : 8) + n_requests, gb_div_up(hidden / 8, CONV_RUN_THREADS)), block(CONV_RUN_THREADS);
+      auto kernel = K == 2 ? (few ? short_conv_run_kernel<2, 4> : short_conv_run_kernel<2, 8>)
+                    : K == 3 ? (few ? short_conv_run_kernel<3, 4> : short_conv_run_kernel<3, 8>)
+                             : (few ? short_conv_run_kernel<4, 4> : short_conv_run_kernel<4, 8>);
+      gb_launch(kernel, grid, block, 0, stream, (const bf16*)bcx, ld, taps, bias, state, slot_stride, slot_ids, q_start, q_len,
+                (bf16*)out, n_requests, hidden);
+      GB_CHECK_LAUNCH("gb_short_conv (runs)");
+      return 1;
     } else if (vec)
       gb_launch(short_conv_out_vec8_kernel, dim3(gb_div_up(total / 8, threads)), dim3(threads), 0, stream,
                 (const bf16*)bcx, ld, taps, bias, (const float*)state, slot_stride, slot_ids, tok_req, q_start,

@@ -195,6 +195,33 @@ def test_short_conv_ragged_batch(dtype, hidden, k, use_bias):
     assert torch.equal(got_state[untouched], state[untouched]) and torch.equal(got_state[:, 0], state[:, 0])
 
 
+# runs of four and of eight tokens and their remainders, portions shorter than the state, more requests than a warp has lanes
+@pytest.mark.parametrize("hidden,k,lens", [(1536, 3, [1, 2, 3, 4, 5, 8, 9, 31, 512]), (64, 4, [1, 2, 3, 4, 5, 6, 7] * 6),
+                                           (96, 2, [1, 2, 1, 5, 2100]), (2048, 4, [2, 700, 1400, 3])])
+def test_short_conv_of_portions_and_the_state_they_leave(hidden, k, lens):
+    from gibbs_b200 import ops
+    torch.manual_seed(hidden + k)
+    n, R = sum(lens), len(lens)
+    bcx = torch.randn(n, 3 * hidden, device=DEV).bfloat16()
+    taps, bias, state = torch.randn(hidden, k), torch.randn(hidden), torch.randn(R + 2, k - 1, hidden)
+    ids = torch.randperm(R + 2)[:R].tolist()
+    st, first = state.to(DEV), np.cumsum([0] + lens[:-1]).tolist()
+    out = torch.empty(n, hidden, dtype=torch.bfloat16, device=DEV)
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    ops.short_conv(bcx, taps.to(DEV), bias.to(DEV), st, t(ids), t([r for r, m in enumerate(lens) for _ in range(m)]), t(first), t(lens), out)
+    b, c, x = (v.float().cpu() for v in bcx.split(hidden, 1))
+    prod, want_state, got, w = b * x, state.clone(), out.double().cpu(), taps.double()
+    for r, m in enumerate(lens):
+        rows = slice(first[r], first[r] + m)
+        seq = torch.cat([state[ids[r]], prod[rows]])
+        want = c[rows].double() * (sum(w[:, j] * seq[j:j + m].double() for j in range(k)) + bias.double())
+        size = c[rows].double().abs() * (sum((w[:, j] * seq[j:j + m].double()).abs() for j in range(k)) + bias.double().abs())
+        # (half a place of bfloat16, and k + 2 roundings of 32-bit sums)
+        assert ((got[rows] - want).abs() <= 2.0 ** -9 * (1 + 2.0 ** -7) * want.abs() + (k + 2) * 2.0 ** -23 * size).all(), r
+        want_state[ids[r]] = seq[m:]
+    assert torch.equal(st.cpu(), want_state)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("hidden,k,use_bias", [(96, 4, True), (200, 2, False), (2048, 3, False)])
 def test_short_conv_one_token_per_request(dtype, hidden, k, use_bias):
