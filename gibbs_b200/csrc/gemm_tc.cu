@@ -536,12 +536,25 @@ struct PairCfg {
 #define GB_PAIR_STAGES 6
 #endif
   static constexpr int STAGES = GB_PAIR_STAGES;
-  static constexpr int STAGING_BYTES = 32 * 1024;        // 64 token rows in 32-bit, or 128 in bfloat16
+  // Two groups of four epilogue warps, each takes every other piece of a tile: with one group a tile's epilogue is a chain of
+  // tensor-memory loads, shared memory and stores on one warp a scheduler, and the last tile's is waited for.
+  static constexpr int GROUPS = 2;
+  static constexpr int THREADS = 64 + GROUPS * 128;
+  static constexpr int STAGING_BYTES = 16 * 1024;        // of a group: 32 token rows in 32-bit, or 64 in bfloat16
   static constexpr int TMEM_COLS = 512;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + GROUPS * STAGING_BYTES + 1024;
 };
 
-__global__ void __launch_bounds__(192)
+// Barrier of one group of epilogue warps; true for all of its threads when any of them brought true.
+__device__ __forceinline__ bool group_any(int group, bool v) {
+  int r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.or.pred q, %1, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+               : "=r"(r) : "r"(1 + group), "r"((int)v) : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
+__global__ void __launch_bounds__(PairCfg::THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                     const GemmParams p) {
   using C = PairCfg;
@@ -554,7 +567,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   pdl_trigger();
 
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* staging = tiles + (size_t)C::STAGES * C::STAGE_BYTES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                // 0: leader
   const int M = p.M, N = p.N, nkb = p.total_kb;
@@ -585,7 +597,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full_bar[a], 1);  // one multicast commit
-      mbar_init(&tmem_empty_bar[a], 2); // the epilogues of both CTAs (only the leader's copy is used)
+      mbar_init(&tmem_empty_bar[a], 2 * C::GROUPS); // the epilogue groups of both CTAs (only the leader's copy is used)
     }
     abort_flag = 0;
     fence_barrier_init();
@@ -699,8 +711,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     __syncwarp();
   } else {
-    const int et = threadIdx.x - 64;
+    const int eg = (warp - 2) >> 2, et = threadIdx.x - 64 - 128 * eg;      // group, thread of the group
     const int q = warp & 3, row = 32 * q + lane;
+    uint8_t* staging = tiles + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)eg * C::STAGING_BYTES;
     pdl_wait();
     int tile_i = 0;
     for (int t = pair; t < n_tiles; t += n_pairs, ++tile_i) {
@@ -717,22 +730,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) atomicExch(p.status, STATUS_TIMEOUT + 11);
       }
       tc_fence_after();
-      epilogue_barrier();
-      if (abort_flag) break;
+      if (group_any(eg, abort_flag != 0)) break;
       const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * ACC_COLS);
       const int cols = max(0, min(BNP, M - m0));
       const bool fast = p.vec_store && n0 + BM <= N;
       const float b = (p.bias && n < N) ? p.bias[n] : 0.f;
       const bool f32out = p.mode == OUT_F32 || p.mode == OUT_F32_ACC;
-      const int RC = (f32out || p.mode == OUT_SWIGLU) ? 64 : 128;   // token rows staged at a time
-      for (int h0 = 0; h0 < BNP; h0 += RC) {
+      const int RC = (f32out || p.mode == OUT_SWIGLU) ? 32 : 64;    // token rows of a piece
+      for (int h0 = eg * RC; h0 < BNP; h0 += C::GROUPS * RC) {
         const int hc = max(0, min(RC, cols - h0));
-        const bool last = h0 + RC >= BNP;
+        const bool last = h0 + C::GROUPS * RC >= BNP;              // this group's last piece of the tile (BNP >= 128: each has one)
         if (hc > 0 && fast && p.mode == OUT_SWIGLU) {
-          // g (accumulator rows 0-63) and u (rows 64-127) of 64 token rows go to shared memory
-          // in 32-bit; then all 128 threads share the 64 x 64 activations, two features each.
-          float* gs = reinterpret_cast<float*>(staging);          // [64][64]
-          float* us = gs + 64 * 64;                               // [64][64]
+          // g (accumulator rows 0-63) and u (rows 64-127) of 32 token rows go to shared memory
+          // in 32-bit; then the group's 128 threads share the 32 x 64 activations.
+          float* gs = reinterpret_cast<float*>(staging);          // [32][64]
+          float* us = gs + 32 * 64;                               // [32][64]
           float* mine = row < 64 ? gs + row : us + (row - 64);
 #pragma unroll 1
           for (int c0 = 0; c0 < hc; c0 += 32) {
@@ -743,7 +755,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               if (c0 + j < hc) mine[(c0 + j) * 64] = v[j] + b;
           }
           tc_fence_before();
-          epilogue_barrier();
+          group_barrier(eg);
           if (last && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
           bf16* dst = (bf16*)p.out + (size_t)(m0 + h0) * p.ldo + (n0 >> 1);
           // The epilogue warps are what this product waits for (they issue several times the
@@ -764,7 +776,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             packed.y = *reinterpret_cast<uint32_t*>(&hi);
             *reinterpret_cast<uint2*>(dst + (size_t)mm * p.ldo + f) = packed;
           }
-          epilogue_barrier();
+          group_barrier(eg);
         } else if (hc > 0 && fast && p.mode == OUT_BF16) {
           bf16* ob = reinterpret_cast<bf16*>(staging);
 #pragma unroll 1
@@ -776,7 +788,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
               if (c0 + j < hc) ob[(c0 + j) * BM + row] = __float2bfloat16_rn(apply_act(p.act, v[j] + b));
           }
           tc_fence_before();
-          epilogue_barrier();
+          group_barrier(eg);
           if (last && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
           bf16* dst = (bf16*)p.out + (size_t)(m0 + h0) * p.ldo + n0;
           for (int idx = et; idx < hc * 16; idx += 128) {
@@ -784,7 +796,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             *reinterpret_cast<uint4*>(dst + (size_t)mm * p.ldo + piece * 8) =
                 *reinterpret_cast<const uint4*>(ob + mm * BM + piece * 8);
           }
-          epilogue_barrier();
+          group_barrier(eg);
         } else if (hc > 0 && fast && p.mode == OUT_F32) {
           // A plain 32-bit store needs no staging: a lane is a weight row, so one store of a warp
           // is 128 contiguous bytes of one token's row, a whole line.
@@ -795,7 +807,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             tmem_ld_32(acc + (uint32_t)(h0 + c0), v);
             if (last && c0 + 32 >= hc) {
               tc_fence_before();
-              epilogue_barrier();
+              group_barrier(eg);
               if (et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
             }
 #pragma unroll
@@ -815,7 +827,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           }
           PPHASE(6);
           tc_fence_before();
-          epilogue_barrier();
+          group_barrier(eg);
           PPHASE(0);
           if (last && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
           float* dst = (float*)p.out + (size_t)(m0 + h0) * p.ldo + n0;
@@ -843,7 +855,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
           }
           PPHASE(7);
-          epilogue_barrier();
+          group_barrier(eg);
           PPHASE(0);
         } else {
           // nothing to store from this chunk, a ragged edge or an unaligned output: element by element
@@ -858,7 +870,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 for (int j = 0; j < 16; ++j) ub[(c0 + j) * 64 + (row - 64)] = v[j] + b;
               }
             }
-            epilogue_barrier();
+            group_barrier(eg);
             if (row < 64 && n + 64 < N) {
 #pragma unroll 1
               for (int c0 = 0; c0 < hc; c0 += 16) {
@@ -884,7 +896,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
           }
           tc_fence_before();
-          epilogue_barrier();
+          group_barrier(eg);
           if (last && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
         }
       }
@@ -1117,7 +1129,7 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& 
   const int pairs = (int)(tiles < n_sm / 2 ? tiles : n_sm / 2);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(192);
+  cfg.blockDim = dim3(PairCfg::THREADS);
   cfg.dynamicSmemBytes = PairCfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
