@@ -17,6 +17,8 @@
 //   GLU     act[row, f] = g' sigmoid(alpha g') (u' + up_add), g' = min(g, limit), u' = clamp(u, +-limit),
 //           for weights whose rows alternate in blocks of 64 between gate and up of the same 64 features
 //           (lanes 0-63 of a tile hold g, lanes 64-127 u).
+#include <stdlib.h>
+
 #include <mutex>
 #include <unordered_map>
 
@@ -219,6 +221,262 @@ moe_experts_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// ---------------------------------------------------------------- CTA pairs (many rows an expert)
+// Two CTAs of a cluster compute 256 weight rows x up to 256 token rows with tcgen05.mma.cta_group::2, as the dense
+// product's pair kernel does (gemm_tc.cu): each stages 128 weight rows and half of the token rows a k-block, the leader
+// issues for both, six stages, the accumulator twice in tensor memory so that a tile's epilogue (two groups of four warps,
+// every other 32 token rows each) runs beside the next tile's products.  Persistent: the pairs walk the (expert, 256 weight
+// rows, token tile) tiles, the token tiles of the same weights next to each other.
+// An expert's rows are cut evenly into ceil(rows / 256) tiles of a multiple of 32 rows: the width is the instruction's N and
+// known on the device only, so the token rows arrive in boxes of 16 (whole 8-row groups of the 128-byte swizzle).
+// Bound by what the tiles read from L2: one CTA of 128 x 128 reads 32 KB a k-block for 128 x 128 multiply-adds; here it is
+// 32 KB for 128 x 256, and experts of 257 rows take two tiles of 160 and not three of 128.
+constexpr int PAIR_STAGES = 6, PAIR_GROUPS = 2, PAIR_THREADS = 64 + PAIR_GROUPS * 128, PAIR_ROWS = 256, PAIR_BOX = 16;
+constexpr int PAIR_STAGE_BYTES = W_TILE_BYTES + PAIR_ROWS / 2 * BK * 2;
+constexpr int PAIR_STAGING_BYTES = 16 * 1024;                      // of a group: 32 token rows of 64 (g, u) in 32-bit
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_GROUPS * PAIR_STAGING_BYTES + 1024;
+// Rows an expert on average from which the pairs take a launch.  GIBBS_B200_MOE_PAIR_ROWS moves the line (for comparison runs).
+constexpr int PAIR_MIN_ROWS = 64;
+constexpr int PAIR_MAX_EXPERTS = 128;                              // (by what shared memory is left)
+
+// Barrier of one group of epilogue warps; true for all of its threads when any of them brought true.
+__device__ __forceinline__ bool group_any(int group, bool v) {
+  int r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.or.pred q, %1, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+               : "=r"(r) : "r"(1 + group), "r"((int)v) : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
+__global__ void __launch_bounds__(PAIR_THREADS)
+moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                           const GroupedParams p) {
+  pdl_trigger();
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full_bar[PAIR_STAGES], empty_bar[PAIR_STAGES], tmem_full_bar[2], tmem_empty_bar[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int abort_flag;
+  __shared__ int row_at[PAIR_MAX_EXPERTS + 1], tile_at[PAIR_MAX_EXPERTS + 1];    // first row, first token tile of every expert
+  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();                          // 0: leader
+  const int nkb = p.total_kb, E = p.E;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);                                   // the leader's producer arrives; both CTAs' loads add bytes
+      mbar_init(&empty_bar[s], 1);                                  // one multicast commit
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tmem_full_bar[a], 1);                              // one multicast commit
+      mbar_init(&tmem_empty_bar[a], 2 * PAIR_GROUPS);               // the epilogue groups of both CTAs (the leader's copy is used)
+    }
+    abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&tmem_slot, 512);
+    tmem_relinquish_pair();
+  }
+  pdl_wait();                                                       // the offsets and the rows come from the kernels before
+  if (warp == 2) {
+    int before = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, lo = e < E ? p.offsets[e] : 0, hi = e < E ? p.offsets[e + 1] : 0;
+      const int mine = (hi - lo + PAIR_ROWS - 1) / PAIR_ROWS;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (e < E) {
+        row_at[e] = lo;
+        tile_at[e] = before + upto - mine;
+        if (e + 1 == E) {
+          row_at[E] = hi;
+          tile_at[E] = before + upto;
+        }
+      }
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                               // both CTAs' barriers are initialised before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  const int weight_tiles = (p.rows_per_expert + 2 * BM - 1) / (2 * BM);
+  const int n_tiles = tile_at[E] * weight_tiles;
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+
+  struct Tile { int e, wt, r0, width, rows; };                      // expert, weight tile, first token row, N, rows that are the expert's
+  auto tile_of = [&](int t) {
+    // the expert whose tiles hold t: the last one with tile_at[e] * weight_tiles <= t
+    int lo = 0, hi = E;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (tile_at[mid] * weight_tiles <= t) lo = mid; else hi = mid;
+    }
+    const int mine = tile_at[lo + 1] - tile_at[lo], rows = row_at[lo + 1] - row_at[lo];
+    const int rem = t - tile_at[lo] * weight_tiles;
+    Tile r;
+    r.e = lo;
+    r.wt = rem / mine;
+    const int rt = rem - r.wt * mine;
+    r.width = ((rows + mine - 1) / mine + 31) & ~31;
+    r.r0 = row_at[lo] + rt * r.width;
+    r.rows = max(0, min(r.width, row_at[lo + 1] - r.r0));
+    return r;
+  };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int it = 0;
+      for (int t = pair; t < n_tiles && !abort_flag; t += n_pairs) {
+        const Tile tl = tile_of(t);
+        const int n0 = tl.e * p.rows_per_expert + tl.wt * 2 * BM + (int)rank * BM;     // this CTA's rows of the stacked weights
+        const int half = tl.width / 2, m0 = tl.r0 + (int)rank * half;                  // this CTA's half of the token rows
+        for (int i = 0; i < nkb; ++i, ++it) {
+          const int s = it % PAIR_STAGES;
+          const uint32_t ph = (it / PAIR_STAGES) & 1;
+          if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
+            abort_flag = 1;
+            atomicExch(p.status, STATUS_TIMEOUT);
+            break;
+          }
+          if (abort_flag) break;
+          uint8_t* st = tiles + (size_t)s * PAIR_STAGE_BYTES;
+          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * (W_TILE_BYTES + half * BK * 2));
+          tma_load_2d_pair(st, &tmap_w, i * BK, n0, &full_bar[s]);
+          for (int b = 0; b < half; b += PAIR_BOX)
+            tma_load_2d_pair(st + W_TILE_BYTES + b * BK * 2, &tmap_x, i * BK, m0 + b, &full_bar[s]);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && elect_one()) {
+      int it = 0, tile_i = 0;
+      for (int t = pair; t < n_tiles && !abort_flag; t += n_pairs, ++tile_i) {
+        const uint32_t idesc = idesc_bf16_f32(2 * BM, tile_of(t).width);
+        const int a = tile_i & 1;
+        if (!mbar_wait(&tmem_empty_bar[a], ((tile_i >> 1) & 1) ^ 1)) {
+          abort_flag = 1;
+          atomicExch(p.status, STATUS_TIMEOUT + 1);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t acc = tmem_base + (uint32_t)(a * PAIR_ROWS);
+        for (int i = 0; i < nkb; ++i, ++it) {
+          const int s = it % PAIR_STAGES;
+          const uint32_t ph = (it / PAIR_STAGES) & 1;
+          if (!mbar_wait(&full_bar[s], ph)) {
+            abort_flag = 1;
+            atomicExch(p.status, STATUS_TIMEOUT + 2);
+            break;
+          }
+          if (abort_flag) break;
+          tc_fence_after();
+          uint8_t* st = tiles + (size_t)s * PAIR_STAGE_BYTES;
+          const uint64_t da = smem_desc_sw128(st);
+          const uint64_t db = smem_desc_sw128(st + W_TILE_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (uint32_t)((i | k) != 0));
+          umma_commit_pair(&empty_bar[s]);
+        }
+        umma_commit_pair(&tmem_full_bar[a]);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue ----
+    const int eg = (warp - 2) >> 2, et = threadIdx.x - 64 - 128 * eg;          // group, thread of the group
+    const int q = warp & 3, row = 32 * q + lane;                               // lane of the accumulator = weight row of this CTA's 128
+    uint8_t* staging = tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + (size_t)eg * PAIR_STAGING_BYTES;
+    int tile_i = 0;
+    for (int t = pair; t < n_tiles; t += n_pairs, ++tile_i) {
+      const Tile tl = tile_of(t);
+      const int a = tile_i & 1;
+      const bool ok = mbar_wait(&tmem_full_bar[a], (tile_i >> 1) & 1);
+      if (!ok) {
+        abort_flag = 1;
+        if (lane == 0) atomicExch(p.status, STATUS_TIMEOUT + 3);
+      }
+      tc_fence_after();
+      if (group_any(eg, abort_flag != 0)) break;
+      const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * PAIR_ROWS);
+      const int w0 = tl.wt * 2 * BM + (int)rank * BM;                          // first weight row of this CTA within the expert
+      bool arrived = false;
+      for (int h0 = eg * 32; h0 < tl.width; h0 += 32 * PAIR_GROUPS) {
+        const int hc = max(0, min(32, tl.rows - h0));
+        float v[32];
+        tmem_ld_32(acc + (uint32_t)h0, v);
+        if (h0 + 32 * PAIR_GROUPS >= tl.width) {                               // this group's last piece: the accumulator is read
+          tc_fence_before();
+          group_barrier(eg);
+          if (et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
+          arrived = true;
+        }
+        if (p.mode == 0) {
+          // g (rows 0-63) and u (rows 64-127) meet in shared memory; all threads share the 32 x 64 activations, four a step
+          float* gs = reinterpret_cast<float*>(staging);                       // [32][64]
+          float* us = gs + 32 * 64;                                            // [32][64]
+          float* mine = row < 64 ? gs + row : us + (row - 64);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) mine[j * 64] = v[j];
+          group_barrier(eg);
+          if ((w0 >> 1) < p.n_valid) {                                         // (n_valid is a multiple of 64)
+            bf16* dst = (bf16*)p.out + (size_t)(tl.r0 + h0) * p.ldo + (w0 >> 1);
+            for (int idx = et; idx < hc * 16; idx += 128) {
+              const int mm = idx >> 4, f = (idx & 15) * 4;
+              const float4 g4 = *reinterpret_cast<const float4*>(gs + mm * 64 + f);
+              const float4 u4 = *reinterpret_cast<const float4*>(us + mm * 64 + f);
+              __nv_bfloat162 x, y;
+              x.x = __float2bfloat16_rn(hy_clamped_glu(g4.x, u4.x, p.alpha, p.limit, p.up_add));
+              x.y = __float2bfloat16_rn(hy_clamped_glu(g4.y, u4.y, p.alpha, p.limit, p.up_add));
+              y.x = __float2bfloat16_rn(hy_clamped_glu(g4.z, u4.z, p.alpha, p.limit, p.up_add));
+              y.y = __float2bfloat16_rn(hy_clamped_glu(g4.w, u4.w, p.alpha, p.limit, p.up_add));
+              uint2 packed;
+              packed.x = *reinterpret_cast<uint32_t*>(&x);
+              packed.y = *reinterpret_cast<uint32_t*>(&y);
+              *reinterpret_cast<uint2*>(dst + (size_t)mm * p.ldo + f) = packed;
+            }
+          }
+          group_barrier(eg);                                                   // (the pieces are rewritten by the next 32 rows)
+        } else if (w0 + row < p.n_valid) {
+          const int n = w0 + row;
+          if (p.mode == 1) {
+            float* dst = (float*)p.out + (size_t)(tl.r0 + h0) * p.ldo + n;     // a warp's store: 128 bytes of one token's row
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < hc) dst[(size_t)j * p.ldo] = v[j];
+          } else {
+            bf16* dst = (bf16*)p.out + (size_t)(tl.r0 + h0) * p.ldo + n;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < hc) dst[(size_t)j * p.ldo] = __float2bfloat16_rn(hy_act(v[j], p.fn));
+          }
+        }
+      }
+      if (!arrived && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);         // (a tile of 32 rows has none for the second group)
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (abort_flag && threadIdx.x == 0) {
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  }
+  __syncthreads();
+  cluster_sync_all();                                               // nobody leaves while its partner may still use its memory
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
 // ---------------------------------------------------------------- host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -276,6 +534,31 @@ int launch(const CUtensorMap& tw, const CUtensorMap& tx, const GroupedParams& p,
   return 1;
 }
 
+int launch_pairs(const CUtensorMap& tw, const CUtensorMap& tx, const GroupedParams& p, long long most_tiles, cudaStream_t stream) {
+  static bool raised = false;
+  if (!raised) {
+    GB_CUDA(cudaFuncSetAttribute(moe_experts_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
+    raised = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (unsigned)(most_tiles < 74 ? most_tiles : 74));
+  cfg.blockDim = dim3(PAIR_THREADS);
+  cfg.dynamicSmemBytes = PAIR_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
+  GB_CUDA(cudaLaunchKernelEx(&cfg, moe_experts_tc_pair_kernel, tw, tx, p));
+  GB_CHECK_LAUNCH("moe_experts_tc (pairs)");
+  return 1;
+}
+
 }  // namespace
 
 // Whether gb_op_moe_experts_tc takes these sizes (mode 0: GLU, the weights' gate and up rows alternating
@@ -311,7 +594,10 @@ GB_OP(gb_op_moe_experts_tc) {
   // few rows an expert (decoding): narrow token tiles
   // (and wide ones where an expert has many: a tile's weights are read from L2 once for twice the tokens)
   const int BN = pairs <= 16 * E ? 16 : pairs < 192 * E ? 64 : 128;
-  if (!make_tmap(&tx, op_ptr<const void>(a[0]), a[2], K, a[1], BN))
+  static const int pair_rows = [] { const char* e = getenv("GIBBS_B200_MOE_PAIR_ROWS"); return e ? atoi(e) : PAIR_MIN_ROWS; }();
+  const bool on_pairs = (long long)pairs >= (long long)pair_rows * E && E <= PAIR_MAX_EXPERTS &&
+                        (mode != 0 || (a[8] % 4 == 0 && (a[7] & 7) == 0));
+  if (!make_tmap(&tx, op_ptr<const void>(a[0]), a[2], K, a[1], on_pairs ? PAIR_BOX : BN))
     GB_FAIL(GB_ERR_CUDA, "moe_experts_tc: cuTensorMapEncodeTiled failed (rows)");
   GroupedParams p;
   p.offsets = op_ptr<const int>(a[5]);
@@ -321,6 +607,8 @@ GB_OP(gb_op_moe_experts_tc) {
   p.total_kb = gb_div_up(K, BK);
   p.alpha = (float)f[0]; p.limit = (float)f[1]; p.up_add = (float)f[2];
   p.status = ctx->status;
+  if (on_pairs)                                                     // (rows / 256 + E: at most this many token tiles over all experts)
+    return launch_pairs(tw, tx, p, (long long)gb_div_up(rows_per_expert, 2 * BM) * (pairs / PAIR_ROWS + E), ctx->stream);
   const int weight_tiles = gb_div_up(rows_per_expert, BM);
   const int row_tiles = gb_div_up(pairs, BN) + E;          // at most this many over all experts
   return BN == 16   ? launch<16>(tw, tx, p, weight_tiles, row_tiles, ctx->stream)

@@ -469,6 +469,47 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     assert len(generated) == 5 and generated[0] == top["ids"][0]
 
 
+# experts of many rows on CTA pairs (edges of 32 and 256 rows, empty experts, weight rows that are no whole tiles, as many experts as
+# the kernel takes) and of few
+@pytest.mark.parametrize("E,K,out,mode,counts", [
+    (4, 64, 64, 0, [256, 257, 0, 33]), (3, 136, 448, 0, [1, 512, 700]), (5, 512, 256, 0, [129, 128, 127, 300, 31]),
+    (4, 64, 130, 1, [256, 257, 0, 33]), (3, 136, 448, 1, [1, 512, 700]), (2, 1024, 2048, 1, [300, 96]),
+    (3, 200, 320, 2, [64, 300, 200]), (1, 64, 64, 1, [2500]), (128, 64, 64, 0, [64] * 127 + [200]),
+    (5, 512, 256, 0, [1, 0, 3, 16, 17]), (40, 512, 256, 1, [0] * 38 + [2, 1]), (3, 136, 448, 0, [60, 0, 64]),
+])
+def test_routed_experts_products_of_many_rows_and_of_few(E, K, out, mode, counts):
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(K + out)
+    rows, per = sum(counts), (2 * out if mode == 0 else out)
+    room = rows + 5
+    x = torch.randn(room, K, device="cuda").bfloat16()
+    x[rows:] = float("nan")                                    # rows behind the last expert's
+    w = (torch.randn(E, per, K, device="cuda") / K ** 0.5).bfloat16()
+    off = torch.tensor([sum(counts[:e]) for e in range(E + 1)], dtype=torch.int32, device="cuda")
+    y = torch.full((room, out + 8), 7.0, device="cuda", dtype=torch.float32 if mode == 1 else torch.bfloat16)
+    hybrid.call("moe_experts_tc", [x.data_ptr(), K, room, w.data_ptr(), 0, off.data_ptr(), E, y.data_ptr(), y.stride(0), rows, out, K, mode, 1, 4],
+                [1.702, 7.0, 1.0] if mode == 0 else [0.0, 0.0, 0.0])
+    assert (y[:, out:] == 7.0).all() and (y[rows:] == 7.0).all()
+    at = 0
+    for e, c in enumerate(counts):
+        z, size = x[at:at + c].double() @ w[e].double().T, x[at:at + c].double().abs() @ w[e].double().abs().T
+        ulp = K * 2.0 ** -24                                   # (of every term of a sum that is truncated K times at most)
+        if mode == 0:
+            z, size = z.reshape(c, -1, 2, 64), size.reshape(c, -1, 2, 64)
+            g, u = z[:, :, 0].reshape(c, -1).clamp(max=7.0), z[:, :, 1].reshape(c, -1).clamp(-7.0, 7.0)
+            want = g * torch.sigmoid(1.702 * g) * (u + 1.0)
+            # (the unit grows by at most 8 x 1.1 times what g does, and by 7 times what u does)
+            tol = 9 * ulp * size.sum(2).reshape(c, -1) + 2.0 ** -8 * want.abs()
+        elif mode == 2:
+            want = z.clamp(min=0.0) ** 2
+            tol = 2 * z.abs() * ulp * size + (ulp * size) ** 2 + 2.0 ** -8 * want
+        else:
+            want, tol = z, ulp * size
+        err = (y[at:at + c, :out].double() - want).abs()
+        assert (err <= tol + 1e-9).all(), (e, (err - tol).max().item())
+        at += c
+
+
 @pytest.mark.parametrize("cfg,layer", [(CFG_D, 0), (CFG_D, 2), (CFG_D, 3), (CFG_D, 4)])
 def test_tensor_core_attention_against_the_generic_kernel(cfg, layer, monkeypatch):
     """In bfloat16 the two kernels read the same pages; they differ by the rounding of the queries and of
