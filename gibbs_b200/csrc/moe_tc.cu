@@ -31,7 +31,7 @@ using namespace sm100;
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 // (stages: as many as leave room for two blocks an SM)
-template <int BN> constexpr int stages_of() { return BN <= 64 ? 4 : 3; }
+template <int BN> constexpr int stages_of() { return BN <= 16 ? 6 : BN <= 64 ? 4 : 3; }
 constexpr int W_TILE_BYTES = BM * BK * 2;
 constexpr int STATUS_TIMEOUT = 24;
 
@@ -60,24 +60,8 @@ moe_experts_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
-  pdl_wait();                                   // the offsets and the rows come from the kernels before
-
-  // this CTA's expert and rows (the same walk in every thread; E is small)
-  int e = 0, r0 = 0, r1 = 0;
-  {
-    int tile = blockIdx.y;
-    bool found = false;
-    for (e = 0; e < p.E; ++e) {
-      const int lo = p.offsets[e], hi = p.offsets[e + 1];
-      const int tiles = (hi - lo + BN - 1) / BN;
-      if (tile < tiles) { r0 = lo + BN * tile; r1 = hi; found = true; break; }
-      tile -= tiles;
-    }
-    if (!found) return;                         // (before any barrier or tensor-memory allocation)
-  }
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = e * p.rows_per_expert + blockIdx.x * BM;     // row of the stacked weights
   const int nkb = p.total_kb;
 
   if (threadIdx.x == 0) {
@@ -93,6 +77,30 @@ moe_experts_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
   }
+  pdl_wait();                                   // the offsets and the rows come from the kernels before
+
+  // this CTA's expert and rows: every warp asks for the ranges of 32 experts at a time (one by one they were a chain of loads)
+  int e = -1, r0 = 0, r1 = 0;
+  for (int e0 = 0, before = 0; e0 < p.E && e < 0; e0 += 32) {
+    const int mine = e0 + lane, lo = mine < p.E ? p.offsets[mine] : 0, hi = mine < p.E ? p.offsets[mine + 1] : 0;
+    const int n_tiles = (hi - lo + BN - 1) / BN;
+    int upto = n_tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.y);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      e = e0 + src;
+      r0 = __shfl_sync(0xffffffffu, lo, src) + BN * ((int)blockIdx.y - before - __shfl_sync(0xffffffffu, upto - n_tiles, src));
+      r1 = __shfl_sync(0xffffffffu, hi, src);
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  if (e < 0) return;                            // (before any tensor-memory allocation)
+  const int n0 = e * p.rows_per_expert + blockIdx.x * BM;     // row of the stacked weights
   if (warp == 1) {
     tmem_alloc(&tmem_slot, TMEM_COLS);
     tmem_relinquish();
