@@ -32,7 +32,7 @@ LIBRARIES = {
     # layer norms, clamped gated units, latent, gated and sigmoid attention, state-space, delta-rule and linear recurrences, residual
     # streams, routed experts: every entry
     # point has the signature of a step-plan operation (hybrid.cuh)
-    "hybrid": ["errors.cu", "norms.cu", "latent_attention.cu", "latent_attention_tc.cu", "gated_attention.cu", "gated_attention_tc.cu",
+    "hybrid": ["errors.cu", "norms.cu", "latent_attention.cu", "latent_attention_tc.cu", "gated_attention.cu", "gated_attention_tc.cu", "gated_attention_tcgen05.cu",
                "sigmoid_attention_tc.cu", "ssm.cu", "selective_scan.cu", "delta_rule.cu", "delta_chunks.cu", "linear_scan.cu", "streams.cu", "moe.cu",
                "moe_tc.cu"],
 }

@@ -469,6 +469,75 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     assert len(generated) == 5 and generated[0] == top["ids"][0]
 
 
+# launches of more than 296 tiles of 64 rows: windows within a key tile and across tiles, groups that do not divide 128, pages of 8 to
+# 64, a single token beside portions, two maps, the edges of 64 keys, no softmax
+@pytest.mark.parametrize("heads,kvh,maps,vdim,ps,window,cap,sink,gate,sig,starts,lens", [
+    (16, 4, 1, 64, 16, 0, 30.0, True, True, False, [0, 63], [1000, 230]),
+    (32, 8, 1, 64, 16, 100, 30.0, True, False, False, [0, 1000, 64], [433, 1, 260]),
+    (24, 8, 1, 128, 8, 64, 0.0, False, False, False, [127, 65], [800, 7]),
+    (20, 4, 2, 128, 64, 1, 0.0, True, False, False, [0, 5], [300, 300]),
+    (16, 4, 2, 128, 32, 193, 0.0, False, False, False, [1000], [677]),
+    (16, 4, 1, 64, 16, 0, 0.0, False, False, True, [3, 0], [640, 700]),
+    (8, 8, 1, 64, 16, 40, 5.0, False, True, True, [0], [2500]),
+])
+def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens):
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(heads * 1000 + window)
+    dk, n, group = 64, sum(lens), heads // kvh
+    need = [(a + b + ps - 1) // ps for a, b in zip(starts, lens)]
+    n_pages, first = sum(need) + 3, [sum(lens[:r]) for r in range(len(lens))]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    perm = torch.randperm(n_pages).tolist()
+    bt = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    for r, k in enumerate(need):
+        bt[r, :k] = torch.tensor(perm[sum(need[:r]):sum(need[:r]) + k])
+    q = torch.randn(n, heads * maps * dk, device="cuda").bfloat16()
+    kp, vp = torch.randn(n_pages, kvh, ps, maps * dk, device="cuda").bfloat16(), torch.randn(n_pages, kvh, ps, vdim, device="cuda").bfloat16()
+    # what no row sees is not finite: the rest of every last page, and what lies in front of a window
+    for r, (a, b) in enumerate(zip(starts, lens)):
+        at = torch.arange(need[r] * ps)
+        at = at[(at >= a + b) | (at <= (a - window if window else -1))]
+        vp[bt[r][at // ps].long().cuda(), :, (at % ps).cuda()] = float("nan")
+        kp[bt[r][at // ps].long().cuda(), :, (at % ps).cuda()] = float("inf")
+    logits = torch.randn(n, heads * vdim, device="cuda") if gate else None
+    score, scale, factor = torch.randn(heads, device="cuda"), 0.3, 1.5
+    out = torch.full((n, heads * maps * vdim + 8), 7.0, device="cuda")
+    tables, tok_req, starts_, pos = (bt.cuda(), i32([r for r, b in enumerate(lens) for _ in range(b)]), i32(first),
+                                     i32([a + i for a, b in zip(starts, lens) for i in range(b)]))
+    hybrid.call("sigmoid_attention_tc" if sig else "sink_attention_tc",
+                [q.data_ptr(), kp.data_ptr(), vp.data_ptr(), tables.data_ptr(), bt.shape[1], ps, n_pages, tok_req.data_ptr(), pos.data_ptr(),
+                 logits.data_ptr() if gate else 0, logits.stride(0) if gate else 0, out.data_ptr(), out.stride(0), n, heads, kvh, dk, vdim, window,
+                 max(a + b for a, b in zip(starts, lens)), 0, len(lens), starts_.data_ptr(), score.data_ptr() if sink or sig else 0],
+                [scale, cap, factor if sig else 0.0], flags=(1 if sink else 0) | 2 | maps << 8)
+    assert (out[:, heads * maps * vdim:] == 7.0).all()
+    got = out[:, :heads * maps * vdim].reshape(n, heads, maps, vdim).double()
+    for r, (a, b) in enumerate(zip(starts, lens)):
+        rows, idx, at = slice(first[r], first[r] + b), torch.arange(a + b, device="cuda"), torch.arange(a, a + b, device="cuda")
+        pages = tables[r].long()[idx // ps]
+        seen = idx[None] <= at[:, None]
+        if window:
+            seen &= idx[None] > at[:, None] - window
+        k = kp[pages, :, idx % ps].double().reshape(a + b, kvh, maps, dk).repeat_interleave(group, 1)
+        v = vp[pages, :, idx % ps].double().repeat_interleave(group, 1)
+        v = torch.where(seen.any(0)[:, None, None], v, torch.zeros_like(v))
+        s = torch.einsum("thmd,khmd->thmk", q[rows].double().reshape(b, heads, maps, dk), k) * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if sig:
+            w = torch.sigmoid(s + score.double()[None, :, None, None]).masked_fill(~seen[:, None, None], 0.0) * factor
+        else:
+            s = s.masked_fill(~seen[:, None, None], -math.inf)
+            z = score.double()[None, :, None, None].expand(b, heads, maps, 1)
+            w = torch.softmax(torch.cat([s, z], 3), 3)[..., :-1] if sink else torch.softmax(s, 3)
+        want, size = torch.einsum("thmk,khd->thmd", w, v), torch.einsum("thmk,khd->thmd", w, v.abs())
+        if gate:
+            o = torch.sigmoid(logits[rows].double()).reshape(b, heads, 1, vdim)
+            want, size = want * o, size * o
+        # weights of 16 bits (2^-17), scores of up to 30 formed and rounded in 32-bit a few times (2^-16 of a weight at most), sums
+        # that the tensor core truncates (160 terms of 2^-24)
+        assert ((got[rows] - want).abs() <= 2.0 ** -14.5 * size + 1e-6).all(), r
+
+
 # experts of many rows on CTA pairs (edges of 32 and 256 rows, empty experts, weight rows that are no whole tiles, as many experts as
 # the kernel takes) and of few
 @pytest.mark.parametrize("E,K,out,mode,counts", [
