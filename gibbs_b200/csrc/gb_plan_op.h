@@ -15,8 +15,7 @@
 // Before the call the 32-bit residual stream is whole (sums that a product had left to be added
 // are added), unless the record's flags have GB_OP_TAKES_PENDING: then the function gets those sums
 // (ctx->pend ...) and must itself leave the stream whole: x[m, :] += pend[0][m, :] + pend[1][m, :] + ...
-// (+ pend_bias), in this order, for every row of the step.  Steps of fewer than GB_OP_PENDING_MIN_ROWS tokens are
-// made whole before the call whatever the flags.
+// (+ pend_bias), in this order, for every row of the step.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -41,7 +40,6 @@ struct GbPlanCtx {
 
 #define GB_OP_TAKES_PENDING (1 << 30)
 #define GB_OP_TAKES_PARTIALS (1 << 29)
-#define GB_OP_PENDING_MIN_ROWS 64
 
 typedef int (*GbPlanOpFn)(const GbPlanCtx* ctx, const long long* a, const double* f, int flags);
 

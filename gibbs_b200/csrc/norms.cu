@@ -177,6 +177,68 @@ row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ ga
   }
 }
 
+// The same for few rows (a decode step): a block a row, a piece of four values a thread (dim <= 2048, a multiple of 4), the
+// partial sums of all splits in one trip, the gain read before the wait.  The sums are added in the order of the kernel above
+// (a lane's pieces, then the lanes), so the bits are the same.
+template <typename TO>
+__global__ void __launch_bounds__(512)
+row_norm_block_kernel(const float* x, long long ldx, const float* __restrict__ gain, TO* out, const int* rows, int n_rows, int dim,
+                      int kind, float eps, const float* pend, int pend_splits, const float* __restrict__ pend_bias) {
+  extern __shared__ __align__(16) float parts[];          // [splits][dim], then two rows of a number a thread
+  pdl_trigger();
+  const int r = blockIdx.x, lane = threadIdx.x & 31, d = 4 * threadIdx.x;
+  const bool in = d < dim;
+  long long src = rows ? rows[r] : r;
+  gb_pin(src);
+  float* row = const_cast<float*>(x) + (size_t)src * ldx + d;
+  float4 g = in ? *reinterpret_cast<const float4*>(gain + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 b = in && pend_bias ? *reinterpret_cast<const float4*>(pend_bias + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  gb_pin(row);
+  gb_pin(g);
+  gb_pin(b);
+  float* sums = parts + (size_t)pend_splits * dim;
+  pdl_wait();
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (in) {
+    const float* from = pend + (size_t)src * dim + d;
+    for (int u = 0; u < pend_splits; ++u) gb_cp_async_16(parts + (size_t)u * dim + d, from + (size_t)u * n_rows * dim);
+    v = ldcg_now(reinterpret_cast<const float4*>(row));
+    if (pend_splits > 0) {
+      gb_cp_async_wait_all();
+      for (int u = 0; u < pend_splits; ++u) {
+        const float4 q = *reinterpret_cast<const float4*>(parts + (size_t)u * dim + d);
+        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+      }
+      if (pend_bias) { v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+      *reinterpret_cast<float4*>(row) = v;
+    }
+  }
+  // a row's sum: every lane its pieces in ascending order, then the lanes
+  auto row_sum = [&](float mine, float* at) {
+    at[threadIdx.x] = mine;
+    __syncthreads();
+    float s = 0.f;
+    for (int i = lane; i < (int)blockDim.x; i += 32) s += at[i];
+    return warp_sum(s);
+  };
+  const float mean = kind == NORM_LAYER ? row_sum((v.x + v.y) + (v.z + v.w), sums) / (float)dim : 0.f;
+  const float a0 = v.x - mean, a1 = v.y - mean, a2 = v.z - mean, a3 = v.w - mean;
+  const float ss = row_sum(in ? (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3) : 0.f, sums + blockDim.x);
+  const float rstd = 1.0f / sqrtf(ss / (float)dim + eps);
+  if (!in) return;
+  TO* o = out + (size_t)r * dim + d;
+  const float r0 = a0 * rstd * g.x, r1 = a1 * rstd * g.y, r2 = a2 * rstd * g.z, r3 = a3 * rstd * g.w;
+  if constexpr (sizeof(TO) == 2) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(r0, r1), hi = __floats2bfloat162_rn(r2, r3);
+    uint2 w;
+    w.x = *reinterpret_cast<unsigned*>(&lo);
+    w.y = *reinterpret_cast<unsigned*>(&hi);
+    *reinterpret_cast<uint2*>(o) = w;
+  } else {
+    *reinterpret_cast<float4*>(o) = make_float4(r0, r1, r2, r3);
+  }
+}
+
 // AHEAD: the gains are on hand before the kernel in front has finished (pinned, see gb_pin): read behind the sums, each was a
 // trip to L2 of its own (2 rows of 2048 in a decode step: 6.3 us; 2.8 so).  They cost registers, so blocks an SM, which a launch
 // of many rows needs more.
@@ -621,6 +683,7 @@ __global__ void normed_sum_any_kernel(float* x, long long ldx, const float* y1, 
   if (then.gain != nullptr) hy_then_norm_row(o, dim, then, row, scratch);
 }
 
+constexpr int NORM_FEW_ROWS = 64;
 inline int norm_threads(int dim) { return dim <= 256 ? 64 : dim <= 1024 ? 128 : 256; }
 
 }  // namespace
@@ -652,6 +715,26 @@ GB_OP(gb_op_row_norm) {
       pend = nullptr;
       launched = 1;
     }
+  }
+  const size_t block_smem = sizeof(float) * ((size_t)(pend != nullptr ? ctx->pend_splits : 0) * dim + 2 * 512);
+  if (by_warps && n < NORM_FEW_ROWS && block_smem <= 160 * 1024) {
+    // (whole warps; a thread without a piece adds zeros)
+    const dim3 block(32 * gb_div_up(dim, 128));
+#define BLOCK_NORM(TO)                                                                                                     \
+    do {                                                                                                                  \
+      static bool raised = false;                                                                                         \
+      if (!raised) {                                                                                                      \
+        GB_CUDA(cudaFuncSetAttribute(row_norm_block_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); \
+        raised = true;                                                                                                    \
+      }                                                                                                                   \
+      gb_launch(row_norm_block_kernel<TO>, dim3(n), block, block_smem, ctx->stream, op_ptr<const float>(a[0]), a[1],      \
+                op_ptr<const float>(a[2]), op_ptr<TO>(a[3]), op_ptr<const int>(a[5]), n, dim, kind, (float)f[0], pend,    \
+                pend != nullptr ? ctx->pend_splits : 0, pend != nullptr ? ctx->pend_bias : nullptr);                      \
+    } while (0)
+    if (a[4] == GB_BF16) BLOCK_NORM(bf16); else BLOCK_NORM(float);
+#undef BLOCK_NORM
+    GB_CHECK_LAUNCH("row_norm (a block a row)");
+    return launched + 1;
   }
   if (by_warps) {
     const dim3 wgrid(gb_div_up(n, 4)), wblock(128);

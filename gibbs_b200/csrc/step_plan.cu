@@ -392,8 +392,8 @@ int run_registered(Walk& w, const PlanOp& o) {
   }
   // such an operation sees the stream whole: what a product left to be added is added first, and
   // what this file remembers about the stream no longer holds afterwards
-  // (it adds them itself; the few rows of a small step, each with many partial sums, are added faster here)
-  const bool takes = (o.flags & GB_OP_TAKES_PENDING) != 0 && w.pend_splits > 0 && w.sym[S_N] >= GB_OP_PENDING_MIN_ROWS;
+  // (or it adds them itself)
+  const bool takes = (o.flags & GB_OP_TAKES_PENDING) != 0 && w.pend_splits > 0;
   if (w.pend_splits > 0 && !takes) {
     const int N = (int)w.sym[S_N];
     PLAN_CALL(w, F_ADD_PENDING, ((AddPendingFn)g_fn[F_ADD_PENDING])(

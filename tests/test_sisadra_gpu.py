@@ -609,3 +609,46 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     out = capsys.readouterr().out
     generated = [int(t) for t in out.split("Output:\n")[1].splitlines()[0].split(",")]
     assert len(generated) == 5 and generated[0] == top["ids"][0]
+
+
+@pytest.mark.parametrize("dim,kind,dtype,splits,bias", [(2048, 0, 1, 9, False), (2048, 1, 0, 16, True), (2044, 0, 1, 2, True), (1024, 0, 0, 0, False),
+                                                        (132, 1, 1, 3, False), (128, 0, 1, 1, True), (4, 0, 0, 2, False)])
+def test_row_norm_of_few_rows_and_of_many_has_the_same_bits(dim, kind, dtype, splits, bias):
+    """The kernel with a block a row (below 64 rows) and the one with a warp a row, with sums of a product left to be added."""
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(dim + splits)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 65
+    x0, gain, add = torch.randn(many, dim, device=dev), torch.randn(dim, device=dev), torch.randn(dim, device=dev)
+    pend = torch.randn(max(splits, 1), many, dim, device=dev)
+
+    def run(n, rows=None):
+        x, parts = x0[:n].clone(), pend[:, :n].contiguous()
+        out = torch.full((n if rows is None else len(rows), dim), 7.0, device=dev, dtype=torch.bfloat16 if dtype else torch.float32)
+        sym = (ctypes.c_longlong * 32)(n)
+        stream = _stream()
+        pending = rows is None and splits > 0
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), ctypes.cast(sym, ctypes.c_void_p),
+                          32, x.data_ptr(), dim, parts.data_ptr() if pending else None, splits if pending else 0, add.data_ptr() if pending and bias else None,
+                          None, 0, None)
+        a = (ctypes.c_longlong * 24)(x.data_ptr(), dim, gain.data_ptr(), out.data_ptr(), dtype, 0 if rows is None else rows.data_ptr(), len(out), dim, kind)
+        rc = hybrid._function("row_norm")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(1e-6), ctypes.c_int(hybrid.TAKES_PENDING))
+        assert rc == 1
+        torch.cuda.synchronize()
+        return x, out
+
+    whole_x, whole = run(many)
+    want = x0.double()
+    for u in range(splits):
+        want = want + pend[u].double()
+    want = want + add.double() if splits and bias else want
+    # (a rounding of 2^-24 of what is in hand for every split and the bias)
+    size = x0.abs() + pend[:splits].abs().sum(0) + add.abs()
+    assert ((whole_x.double() - want).abs() <= (splits + 1) * 2.0 ** -24 * size.double()).all()
+    for n in (1, 2, 63):
+        x, out = run(n)
+        assert torch.equal(x, whole_x[:n]) and torch.equal(out, whole[:n]), n
+    if not splits:
+        rows = torch.tensor([64, 0, 7], dtype=torch.int32, device=dev)
+        assert torch.equal(run(many, rows)[1], whole[rows.long()])
