@@ -250,9 +250,21 @@ moe_dispatch_kernel(RouteParams p, int* idx, float* weight, int* offsets, int* r
   __shared__ int s_idx[DISPATCH_PAIRS], s_row[DISPATCH_PAIRS];
   __shared__ float s_w[DISPATCH_PAIRS];
   pdl_trigger();
-  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = DISPATCH_THREADS / 32;
   const int pairs = p.n * p.top;
+  const int pieces = width * (int)sizeof(T) / 16;
+  pdl_wait();
+  // this block's first row does not depend on the choice: it is asked for beside the logits
+  constexpr int ROW = 2;
+  const bool ahead = vec && !weight_rows && pieces <= ROW * DISPATCH_THREADS;
+  uint4 first_row[ROW];
+#pragma unroll
+  for (int i = 0; i < ROW; ++i) {
+    const int at = threadIdx.x + i * DISPATCH_THREADS;
+    first_row[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (ahead && (int)blockIdx.x < pairs && at < pieces)
+      first_row[i] = __ldcg(reinterpret_cast<const uint4*>(h + (size_t)(blockIdx.x / p.top) * ldh) + at);
+  }
   float* s = dispatch_sm + (size_t)warp * (2 * p.n_out + p.groups);
   for (int t = warp; t < p.n; t += warps) route_token(p, t, s, s + p.n_out, s + 2 * p.n_out, lane, s_idx + t * p.top, s_w + t * p.top);
   int* start = reinterpret_cast<int*>(dispatch_sm + (size_t)warps * (2 * p.n_out + p.groups));
@@ -285,8 +297,14 @@ moe_dispatch_kernel(RouteParams p, int* idx, float* weight, int* offsets, int* r
     const float w = weight_rows ? s_w[q] : 1.f;
     const T* src = h + (size_t)(q / p.top) * ldh;
     T* dst = rows + (size_t)s_row[q] * ldr;
+    if (ahead && q == (int)blockIdx.x) {
+#pragma unroll
+      for (int i = 0; i < ROW; ++i)
+        if ((int)threadIdx.x + i * DISPATCH_THREADS < pieces) reinterpret_cast<uint4*>(dst)[threadIdx.x + i * DISPATCH_THREADS] = first_row[i];
+      continue;
+    }
     if (vec && !weight_rows) {
-      copy_row16(src, dst, width * (int)sizeof(T) / 16);
+      copy_row16(src, dst, pieces);
       continue;
     }
     for (int d = threadIdx.x; d < width; d += DISPATCH_THREADS) dst[d] = from_f32<T>(w * to_f32(src[d]));
@@ -434,6 +452,32 @@ __global__ void moe_combine_kernel(const float* out, long long ldo, const int* p
     if (shared) v += g * shared[(size_t)t * lds + d];
     y[(size_t)t * ldy + d] = v;
   }
+}
+
+// The same arithmetic per value for rows of 16-byte pieces: the rows of four choices on their way together, a piece a thread.
+__global__ void moe_combine4_kernel(const float* out, long long ldo, const int* pair_row, const float* shared_gate,
+                                    const float* shared, long long lds, float* y, long long ldy, int width, int top) {
+  pdl_trigger();
+  const int t = blockIdx.x, d = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  pdl_wait();
+  if (d >= width) return;
+  const float g = shared_gate ? shared_gate[t] : 0.f;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 sh = shared ? ldcg_now(reinterpret_cast<const float4*>(shared + (size_t)t * lds + d)) : zero;
+  float4 v = zero;
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float4 x[4];
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = pair_row[(size_t)t * top + min(k0 + u, top - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = ldcg_now(reinterpret_cast<const float4*>(out + (size_t)row[u] * ldo + d));
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k0 + u < top) { v.x += x[u].x; v.y += x[u].y; v.z += x[u].z; v.w += x[u].w; }
+  }
+  if (shared) { v.x += g * sh.x; v.y += g * sh.y; v.z += g * sh.z; v.w += g * sh.w; }
+  *reinterpret_cast<float4*>(y + (size_t)t * ldy + d) = v;
 }
 
 // rows of any length; `then`: the norm in front of the next sublayer, of the new row
@@ -720,6 +764,14 @@ GB_OP(gb_op_moe_experts) {
 GB_OP(gb_op_moe_combine) {
   const int n = (int)a[8], width = (int)a[9];
   if (n <= 0) return 0;
+  if (((a[0] | a[4] | a[6] | 4 * (a[1] | a[5] | a[7] | width)) & 15) == 0) {
+    const int threads = width <= 1024 ? 64 : 128;
+    gb_launch(moe_combine4_kernel, dim3(n, gb_div_up(width, 4 * threads)), dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
+              op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), a[5], op_ptr<float>(a[6]), a[7],
+              width, (int)a[10]);
+    GB_CHECK_LAUNCH("moe_combine (pieces)");
+    return 1;
+  }
   gb_launch(moe_combine_kernel, dim3(n), dim3(width <= 256 ? 64 : 256), 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
             op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), a[5], op_ptr<float>(a[6]), a[7],
             width, (int)a[10]);
