@@ -35,43 +35,119 @@ __global__ void latent_prep_kernel(const float* fused, long long ld, int dkv_col
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int pos = tok_pos[t];
   const int half = rot_dims >> 1;
+  // The angles, the page and the gains are known before the kernel in front has finished (pinned, see gb_pin); behind the wait
+  // all of a row's values are asked for before the first is used.
+  constexpr int ROT = 2, LAT = 16, HEADS = 3;              // rotated pairs and latent entries a lane holds; heads a warp takes at a time
+  const bool rot_here = half <= 32 * ROT, lat_here = r <= 32 * LAT;
+  float c[ROT], s[ROT], g[LAT];
+#pragma unroll
+  for (int i = 0; i < ROT; ++i) {
+    const int j = lane + 32 * i;
+    const float ang = rot_here && j < half ? (float)pos * inv_freq[j] : 0.f;
+    c[i] = cosf(ang);
+    s[i] = sinf(ang);
+    gb_pin(c[i]);
+    gb_pin(s[i]);
+  }
+  int page = 0;
+  if (warp == 0) {
+    page = block_table[(size_t)tok_req[t] * bt_stride + pos / page_size];
+#pragma unroll
+    for (int i = 0; i < LAT; ++i) {
+      g[i] = lat_here && lane + 32 * i < r ? gain[lane + 32 * i] : 0.f;
+      gb_pin(g[i]);
+    }
+  }
+  gb_pin(page);
   pdl_wait();
   const float* row = fused + (size_t)t * ld;
   if (warp == 0) {
-    const int page = block_table[(size_t)tok_req[t] * bt_stride + pos / page_size];
     if (page < 0 || page >= n_pages) {
       if (lane == 0) atomicExch(status, STATUS_BAD_PAGE_WRITE);
     } else {
       TC* dst = pages + ((size_t)page * page_size + pos % page_size) * (r + dr);
       const float* lat = row + dkv_col;
-      float ss = 0.f;
-      for (int d = lane; d < r; d += 32) ss += lat[d] * lat[d];
-      const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)r + eps);
-      for (int d = lane; d < r; d += 32) dst[d] = from_f32<TC>(lat[d] * rstd * gain[d]);
       const float* kr = lat + r;
-      for (int j = lane; j < half; j += 32) {
-        const float ang = (float)pos * inv_freq[j];
-        const float c = cosf(ang), s = sinf(ang);
-        const float u = kr[2 * j], v = kr[2 * j + 1];
-        dst[r + 2 * j] = from_f32<TC>(u * c - v * s);
-        dst[r + 2 * j + 1] = from_f32<TC>(v * c + u * s);
+      float u[ROT], v[ROT];
+#pragma unroll
+      for (int i = 0; i < ROT; ++i) {
+        const int j = lane + 32 * i;
+        u[i] = rot_here && j < half ? ldcg_now(kr + 2 * j) : 0.f;
+        v[i] = rot_here && j < half ? ldcg_now(kr + 2 * j + 1) : 0.f;
       }
+      float ss = 0.f;
+      if (lat_here) {
+        float x[LAT];
+#pragma unroll
+        for (int i = 0; i < LAT; ++i) x[i] = lane + 32 * i < r ? ldcg_now(lat + lane + 32 * i) : 0.f;
+#pragma unroll
+        for (int i = 0; i < LAT; ++i)
+          if (lane + 32 * i < r) ss += x[i] * x[i];
+        const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)r + eps);
+#pragma unroll
+        for (int i = 0; i < LAT; ++i)
+          if (lane + 32 * i < r) dst[lane + 32 * i] = from_f32<TC>(x[i] * rstd * g[i]);
+      } else {
+        for (int d = lane; d < r; d += 32) ss += lat[d] * lat[d];
+        const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)r + eps);
+        for (int d = lane; d < r; d += 32) dst[d] = from_f32<TC>(lat[d] * rstd * gain[d]);
+      }
+#pragma unroll
+      for (int i = 0; i < ROT; ++i) {
+        const int j = lane + 32 * i;
+        if (rot_here && j < half) {
+          dst[r + 2 * j] = from_f32<TC>(u[i] * c[i] - v[i] * s[i]);
+          dst[r + 2 * j + 1] = from_f32<TC>(v[i] * c[i] + u[i] * s[i]);
+        }
+      }
+      if (!rot_here)
+        for (int j = lane; j < half; j += 32) {
+          const float ang = (float)pos * inv_freq[j], cj = cosf(ang), sj = sinf(ang);
+          const float uj = kr[2 * j], vj = kr[2 * j + 1];
+          dst[r + 2 * j] = from_f32<TC>(uj * cj - vj * sj);
+          dst[r + 2 * j + 1] = from_f32<TC>(vj * cj + uj * sj);
+        }
       for (int d = 2 * half + lane; d < dr; d += 32) dst[r + d] = from_f32<TC>(kr[d]);
     }
   }
   const int w0 = warps > 1 ? 1 : 0, step = warps > 1 ? warps - 1 : 1;
   if (warps > 1 && warp == 0) return;
-  for (int h = warp - w0; h < H; h += step) {
-    const float* q = queries + (size_t)t * ldq + (size_t)h * (dn + dr) + dn;
-    float* o = qp + ((size_t)t * H + h) * (r + dr) + r;
-    for (int j = lane; j < half; j += 32) {
-      const float ang = (float)pos * inv_freq[j];
-      const float c = cosf(ang), s = sinf(ang);
-      const float u = q[2 * j], v = q[2 * j + 1];
-      o[2 * j] = u * c - v * s;
-      o[2 * j + 1] = v * c + u * s;
+  const float* q0 = queries + (size_t)t * ldq + dn;        // a head's rotated part lies dn behind its first entry
+  float* o0 = qp + (size_t)t * H * (r + dr) + r;
+  for (int h0 = warp - w0; h0 < H; h0 += HEADS * step) {
+    float u[HEADS][ROT], v[HEADS][ROT];
+#pragma unroll
+    for (int k = 0; k < HEADS; ++k)
+#pragma unroll
+      for (int i = 0; i < ROT; ++i) {
+        const int h = h0 + k * step, j = lane + 32 * i;
+        const bool in = rot_here && h < H && j < half;
+        u[k][i] = in ? ldcg_now(q0 + (size_t)h * (dn + dr) + 2 * j) : 0.f;
+        v[k][i] = in ? ldcg_now(q0 + (size_t)h * (dn + dr) + 2 * j + 1) : 0.f;
+      }
+#pragma unroll
+    for (int k = 0; k < HEADS; ++k) {
+      const int h = h0 + k * step;
+      if (h >= H) break;
+      const float* q = q0 + (size_t)h * (dn + dr);
+      float* o = o0 + (size_t)h * (r + dr);
+#pragma unroll
+      for (int i = 0; i < ROT; ++i) {
+        const int j = lane + 32 * i;
+        if (rot_here && j < half) {
+          o[2 * j] = u[k][i] * c[i] - v[k][i] * s[i];
+          o[2 * j + 1] = v[k][i] * c[i] + u[k][i] * s[i];
+        }
+      }
+      if (!rot_here)
+        for (int j = lane; j < half; j += 32) {
+          const float ang = (float)pos * inv_freq[j], cj = cosf(ang), sj = sinf(ang);
+          const float uj = q[2 * j], vj = q[2 * j + 1];
+          o[2 * j] = uj * cj - vj * sj;
+          o[2 * j + 1] = vj * cj + uj * sj;
+        }
+      for (int d = 2 * half + lane; d < dr; d += 32) o[d] = q[d];
     }
-    for (int d = 2 * half + lane; d < dr; d += 32) o[d] = q[d];
   }
 }
 

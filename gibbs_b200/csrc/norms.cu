@@ -466,24 +466,56 @@ __global__ void gelu_mul_rows_kernel(float* g, long long ld, const TT* __restric
 }
 
 // one block per (row, group)
+constexpr int GROUP_CACHE = 8;
+
 template <typename TO>
 __global__ void gated_group_norm_kernel(const float* y, long long ldy, const float* z, long long ldz,
                                         const float* __restrict__ gain, TO* out, long long ldo, int inner, int groups,
                                         float eps) {
   __shared__ float scratch[32];
   pdl_trigger();
-  pdl_wait();
   const int t = blockIdx.x, g = blockIdx.y;
   const int width = inner / groups, c0 = g * width;
   const float* yr = y + (size_t)t * ldy + c0;
   const float* zr = z + (size_t)t * ldz + c0;
+  TO* o = out + (size_t)t * ldo + c0;
+  if (width <= GROUP_CACHE * (int)blockDim.x) {
+    // the group in registers; its gains are on hand before the kernel in front has finished (pinned, see gb_pin)
+    float v[GROUP_CACHE], a[GROUP_CACHE], b[GROUP_CACHE];
+#pragma unroll
+    for (int i = 0; i < GROUP_CACHE; ++i) {
+      const int d = threadIdx.x + i * blockDim.x;
+      v[i] = d < width ? gain[c0 + d] : 0.f;
+      gb_pin(v[i]);
+    }
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < GROUP_CACHE; ++i) {
+      const int d = threadIdx.x + i * blockDim.x;
+      a[i] = d < width ? ldcg_now(yr + d) : 0.f;
+      b[i] = d < width ? ldcg_now(zr + d) : 0.f;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < GROUP_CACHE; ++i) {
+      a[i] *= hy_silu(b[i]);
+      ss += a[i] * a[i];
+    }
+    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < GROUP_CACHE; ++i) {
+      const int d = threadIdx.x + i * blockDim.x;
+      if (d < width) o[d] = from_f32<TO>(a[i] * rstd * v[i]);
+    }
+    return;
+  }
+  pdl_wait();
   float ss = 0.f;
   for (int d = threadIdx.x; d < width; d += blockDim.x) {
     const float v = yr[d] * hy_silu(zr[d]);
     ss += v * v;
   }
   const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
-  TO* o = out + (size_t)t * ldo + c0;
   for (int d = threadIdx.x; d < width; d += blockDim.x)
     o[d] = from_f32<TO>(yr[d] * hy_silu(zr[d]) * rstd * gain[c0 + d]);
 }
@@ -539,20 +571,32 @@ __global__ void head_norm_kernel(const float* x, long long ldx, long long xh, co
                                  const float* den, const float* floor_, int gain_whole, int gate_silu) {
   // (with `den`, lambda is what is added to the divisor)
   pdl_trigger();
-  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long idx = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (idx >= (long long)n * H) return;
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
   const size_t at = (size_t)t * ldx + (size_t)h * xh;
-  float v[HN_VR];
+  // the gains before the wait (pinned, see gb_pin), the gate's logits with the row
+  float v[HN_VR], g[HN_VR], z[HN_VR];
+#pragma unroll
+  for (int i = 0; i < HN_VR; ++i) {
+    const int d = lane + 32 * i;
+    g[i] = gain && d < vdim ? gain[gain_whole ? h * vdim + d : d] : 1.f;
+    gb_pin(g[i]);
+  }
+  pdl_wait();
   float ss = 0.f;
   const float div = den ? fmaxf(fabsf(den[idx]), floor_[idx]) + lambda : 1.f;
 #pragma unroll
   for (int i = 0; i < HN_VR; ++i) {
     const int d = lane + 32 * i;
-    v[i] = 0.f;
-    if (d < vdim) v[i] = x2 ? x[at + d] - lambda * x2[at + d] : den ? x[at + d] / div : x[at + d];
+    v[i] = d < vdim ? ldcg_now(x + at + d) : 0.f;
+    z[i] = gate && d < vdim ? ldcg_now(gate + (size_t)t * ld_gate + (size_t)h * vdim + d) : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < HN_VR; ++i) {
+    const int d = lane + 32 * i;
+    if (d < vdim) v[i] = x2 ? v[i] - lambda * x2[at + d] : den ? v[i] / div : v[i];
     ss += v[i] * v[i];
   }
   const float rstd = factor / sqrtf(warp_sum(ss) / (float)vdim + eps);
@@ -561,11 +605,8 @@ __global__ void head_norm_kernel(const float* x, long long ldx, long long xh, co
     const int d = lane + 32 * i;
     if (d >= vdim) continue;
     float o = v[i] * rstd;
-    if (gain) o *= gain[gain_whole ? h * vdim + d : d];
-    if (gate) {
-      const float z = gate[(size_t)t * ld_gate + (size_t)h * vdim + d];
-      o *= gate_silu ? hy_silu(z) : hy_sigmoid(z);
-    }
+    if (gain) o *= g[i];
+    if (gate) o *= gate_silu ? hy_silu(z[i]) : hy_sigmoid(z[i]);
     out[(size_t)t * ldo + (size_t)h * vdim + d] = from_f32<TO>(o);
   }
 }
