@@ -322,18 +322,18 @@ template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStrea
 // kernel's, 12 sizes from 1 head of 32 entries to 64 of 512 + 64, steps of 1 to 300 tokens: 0.77 in the mean, 1.07 at most
 // (two rows of one head; with the terms in one chain and scores in base 2 it was 0.93, and up to 1.54 for small latents).
 //
-//  CTA: 32 consecutive (token, head) rows of one request, whatever the number of heads; 8 warps = 2 groups of 16 rows x
-//  4 slices.  Key tiles of 32 rows by cp.async into two buffers.  For S a slice is a quarter of the row's entries: a
-//  warp takes 16 rows x 32 keys over its quarter (the queries' three terms would otherwise be read from shared memory
-//  by every warp: 3 x 37 KB a tile), the four partial scores are added in shared memory, eight threads a row keep the
-//  maximum and the sum in 32-bit and leave the weights' three terms there.  For O a slice is a quarter of the latent's
+//  CTA: 32 consecutive (token, head) rows of one request, whatever the number of heads; 16 warps = 2 groups of 16 rows x
+//  8 slices.  Key tiles of 32 rows by cp.async into two buffers.  For S a slice is an eighth of the row's entries: a
+//  warp takes 16 rows x 32 keys over its eighth (the queries' three terms would otherwise be read from shared memory
+//  by every warp: 3 x 37 KB a tile), the eight partial scores are added in shared memory, sixteen threads a row keep the
+//  maximum and the sum in 32-bit and leave the weights' three terms there.  For O a slice is an eighth of the latent's
 //  columns.  Key tiles lie at multiples of 32, so a row's sums are grouped by its position alone, whatever the rows
 //  beside it.  With `splits`, blockIdx.y takes a chunk of keys, a multiple of `chunk` from position 0, and leaves (maximum,
 //  sum, weighted sum) per row for the merge kernel.
 //  Bound by waiting: a step of 32 rows x 32 keys takes about 10,000 cycles at 512 + 64 entries, where its operand reads
 //  from shared memory need 2,700 and its mma.sync 1,600; one CTA an SM meets three barriers a key tile, and scores, softmax
 //  and weighted sum follow one another.
-constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLD = 36, LTX_PLD = 40;
+constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLICES = 8, LTX_WARPS = 2 * LTX_SLICES, LTX_SLD = 32, LTX_PLD = 40;
 
 struct LtxParams {
   const float* qp;          // [tokens * heads][dk]
@@ -355,7 +355,7 @@ struct LtxParams {
 };
 
 size_t ltx_smem(int stride) {
-  return sizeof(bf16) * (3 * LTX_ROWS + 2 * LTX_KEYS) * (size_t)stride + sizeof(float) * 4 * LTX_ROWS * LTX_SLD +
+  return sizeof(bf16) * (3 * LTX_ROWS + 2 * LTX_KEYS) * (size_t)stride + sizeof(float) * LTX_SLICES * LTX_ROWS * LTX_SLD +
          sizeof(bf16) * 3 * LTX_ROWS * LTX_PLD + sizeof(float) * 3 * LTX_ROWS + 2 * sizeof(int);
 }
 
@@ -382,19 +382,21 @@ __device__ __noinline__ float ltx_score(const bf16* Qs, const bf16* C, int row, 
 }
 
 template <int OC>                                          // columns of the latent a warp takes
-__global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const LtxParams p) {
+__global__ void __launch_bounds__(32 * LTX_WARPS, 1) latent_attention_split_kernel(const LtxParams p) {
   extern __shared__ __align__(16) unsigned char ltc_smem[];
   const int STRIDE = p.stride, dk = p.dk, H = p.H, r = p.r;
   bf16* Qs = reinterpret_cast<bf16*>(ltc_smem);            // [3][32][STRIDE]
   bf16* Cs = Qs + 3 * LTX_ROWS * STRIDE;                   // [2][32][STRIDE]
-  float* Sp = reinterpret_cast<float*>(Cs + 2 * LTX_KEYS * STRIDE);      // [4][32][LTX_SLD]
-  bf16* Pt = reinterpret_cast<bf16*>(Sp + 4 * LTX_ROWS * LTX_SLD);       // [3][32][LTX_PLD]
+  float* Sp = reinterpret_cast<float*>(Cs + 2 * LTX_KEYS * STRIDE);      // [8][32][LTX_SLD]
+  bf16* Pt = reinterpret_cast<bf16*>(Sp + LTX_SLICES * LTX_ROWS * LTX_SLD);       // [3][32][LTX_PLD]
   float* corr = reinterpret_cast<float*>(Pt + 3 * LTX_ROWS * LTX_PLD);   // [3][32]
   volatile int* odd = reinterpret_cast<int*>(corr + 3 * LTX_ROWS);       // [2]: whether a tile holds what is not finite
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = warp & 1, wk = warp >> 1, g = lane >> 2, t4 = lane & 3;
-  // which request's which tile: requests have ceil(rows / 32) tiles each, one after the other
+  // which request's which tile: requests have ceil(rows / 32) tiles each, one after the other; taken from the last to the first
+  // (a prompt's last tiles see the most keys: they start first)
+  const int order = (int)(gridDim.x - 1 - blockIdx.x);
   int req = -1, tile = 0, first = 0, len = 0, before = 0;
   for (int r0 = 0; r0 < p.R && req < 0; r0 += 32) {
     const int mine = r0 + lane;
@@ -406,13 +408,13 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
       const int v = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += v;
     }
-    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.x);
+    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > order);
     if (hit) {
       const int src = __ffs(hit) - 1;
       req = r0 + src;
       first = __shfl_sync(0xffffffffu, b, src);
       len = __shfl_sync(0xffffffffu, e - b, src);
-      tile = (int)blockIdx.x - before - __shfl_sync(0xffffffffu, upto - tiles, src);
+      tile = order - before - __shfl_sync(0xffffffffu, upto - tiles, src);
     }
     before += __shfl_sync(0xffffffffu, upto, 31);
   }
@@ -439,15 +441,15 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
   }
   // zeros where nothing is copied: columns dk .. stride
   const int pad = (STRIDE - dk) >> 3;
-  for (int i = tid; i < (3 * LTX_ROWS + 2 * LTX_KEYS) * pad; i += 256)
+  for (int i = tid; i < (3 * LTX_ROWS + 2 * LTX_KEYS) * pad; i += 32 * LTX_WARPS)
     *reinterpret_cast<uint4*>(Qs + (size_t)(i / pad) * STRIDE + dk + 8 * (i % pad)) = make_uint4(0u, 0u, 0u, 0u);
 
   const int pieces = dk >> 3;                              // 16-byte pieces of a cached row
   auto stage = [&](int k0, int b) {
     bf16* dst = Cs + (size_t)b * LTX_KEYS * STRIDE;
 #pragma unroll
-    for (int u = 0; u < LTX_KEYS / 8; ++u) {
-      const int j = warp + 8 * u, key = min(max(k0 + j, base), k_end);    // (rows in front of the first key and behind the last are masked)
+    for (int u = 0; u < LTX_KEYS / LTX_WARPS; ++u) {
+      const int j = warp + LTX_WARPS * u, key = min(max(k0 + j, base), k_end);    // (rows in front of the first key and behind the last are masked)
       const int page = table[key / p.page_size];
       const bool bad = page < 0 || page >= p.n_pages;
       if (bad && lane == 0) atomicExch(p.status, LTC_BAD_PAGE_READ);
@@ -467,11 +469,11 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     constexpr int QL = 5;                                  // quads a lane takes of a row: 32 * 5 >= 576 / 4
     const int quads = dk >> 2;
 #pragma unroll
-    for (int rr = 0; rr < LTX_ROWS / 8; rr += 2) {
+    for (int rr = 0; rr < LTX_ROWS / LTX_WARPS; rr += 2) {
       float4 v[2][QL];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int row = warp + 8 * (rr + u);
+        const int row = warp + LTX_WARPS * (rr + u);
 #pragma unroll
         for (int i = 0; i < QL; ++i)
           v[u][i] = row < rows_live && lane + 32 * i < quads
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int row = warp + 8 * (rr + u);
+        const int row = warp + LTX_WARPS * (rr + u);
 #pragma unroll
         for (int i = 0; i < QL; ++i) {
           if (lane + 32 * i >= quads) break;
@@ -498,15 +500,15 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     }
   }
   if (tid < 2) odd[tid] = 0;
-  // the softmax's view: eight threads a row, four keys each
-  const int srow = tid >> 3, scol = (tid & 7) * 4;
+  // the softmax's view: sixteen threads a row, two keys each
+  const int srow = tid >> 4, scol = (tid & 15) * 2;
   const int spos = pos_req + (row0 + srow) / H, slo = p.window > 0 ? spos - p.window + 1 : 0;
   float m = -INFINITY, l = 0.f;
   float o[OC / 8][4];
 #pragma unroll
   for (int j = 0; j < OC / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-  const int ksteps = (dk + 15) >> 4, per = (ksteps + 3) >> 2;
-  const int ks_begin = wk * per, ks_end = min(ksteps, ks_begin + per);
+  const int ksteps = (dk + 15) >> 4;
+  const int ks_begin = ksteps * wk / LTX_SLICES, ks_end = ksteps * (wk + 1) / LTX_SLICES;
   const int npairs = min(OC / 16, max(0, (r - wk * OC + 15) >> 4));       // pairs of 8 output columns that hold anything
   const bool warp_live = wr * 16 < rows_live;
 
@@ -525,88 +527,84 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
       }
       const bf16* qa = Qs + (wr * 16 + (lane & 15)) * STRIDE + (lane >> 4) * 8;
       const bf16* cb = C + ((lane & 7) + (lane >> 4) * 8) * STRIDE + ((lane >> 3) & 1) * 8;
-#pragma unroll 3
+#pragma unroll 1
       for (int ks = ks_begin; ks < ks_end; ++ks) {
         unsigned bb[2][4], a[3][4];
         ltc_ldmatrix(bb[0], cb + ks * 16);
         ltc_ldmatrix(bb[1], cb + 16 * STRIDE + ks * 16);
 #pragma unroll
         for (int t = 0; t < 3; ++t) ltc_ldmatrix(a[t], qa + (size_t)t * LTX_ROWS * STRIDE + ks * 16);
-        float low[4][4], top[4][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          low[j][0] = low[j][1] = low[j][2] = low[j][3] = 0.f;
-          top[j][0] = top[j][1] = top[j][2] = top[j][3] = 0.f;
-        }
+        for (int np = 0; np < 2; ++np) {
+          float low[2][4], top[2][4];
 #pragma unroll
-        for (int t = 2; t >= 0; --t) {
-#pragma unroll
-          for (int np = 0; np < 2; ++np) {
-            ltc_mma(t == 0 ? top[2 * np] : low[2 * np], a[t], bb[np][0], bb[np][1]);
-            ltc_mma(t == 0 ? top[2 * np + 1] : low[2 * np + 1], a[t], bb[np][2], bb[np][3]);
+          for (int j = 0; j < 2; ++j) {
+            low[j][0] = low[j][1] = low[j][2] = low[j][3] = 0.f;
+            top[j][0] = top[j][1] = top[j][2] = top[j][3] = 0.f;
           }
-        }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s[j][e] += top[j][e];
-            s_low[j][e] += low[j][e];
+          for (int t = 2; t >= 0; --t) {
+            ltc_mma(t == 0 ? top[0] : low[0], a[t], bb[np][0], bb[np][1]);
+            ltc_mma(t == 0 ? top[1] : low[1], a[t], bb[np][2], bb[np][3]);
           }
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              s[2 * np + j][e] += top[j][e];
+              s_low[2 * np + j][e] += low[j][e];
+            }
+        }
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[j][e] += s_low[j][e];
+      // (a row's pieces of eight keys lie in an order that its number gives, so that a half warp meets no bank twice)
       float* dst = Sp + (wk * LTX_ROWS + wr * 16 + g) * LTX_SLD + 2 * t4;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(s[j][0], s[j][1]);
-        *reinterpret_cast<float2*>(dst + 8 * LTX_SLD + 8 * j) = make_float2(s[j][2], s[j][3]);
+        *reinterpret_cast<float2*>(dst + 8 * (j ^ (g & 3))) = make_float2(s[j][0], s[j][1]);
+        *reinterpret_cast<float2*>(dst + 8 * LTX_SLD + 8 * (j ^ (g & 3))) = make_float2(s[j][2], s[j][3]);
       }
     }
     __syncthreads();
     {
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
+      float s[2] = {0.f, 0.f};
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const float4 v = *reinterpret_cast<const float4*>(Sp + (w * LTX_ROWS + srow) * LTX_SLD + scol);
-        s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+      for (int w = 0; w < LTX_SLICES; ++w) {
+        const float2 v = *reinterpret_cast<const float2*>(Sp + (w * LTX_ROWS + srow) * LTX_SLD + (scol ^ 8 * (srow & 3)));
+        s[0] += v.x;
+        s[1] += v.y;
       }
       float mx = -INFINITY;
-      if (srow < rows_live && !(fabsf(s[0]) + fabsf(s[1]) + fabsf(s[2]) + fabsf(s[3]) < INFINITY)) {
+      if (srow < rows_live && !(fabsf(s[0]) + fabsf(s[1]) < INFINITY)) {
         odd[b] = 1;                                        // (a query or a cached row is not finite, or a sum)
-#pragma unroll 1
-        for (int e = 0; e < 4; ++e) {
-          const float x = ltx_score(Qs, C, srow, scol + e, STRIDE, dk);
-          if (e == 0) s[0] = x; else if (e == 1) s[1] = x; else if (e == 2) s[2] = x; else s[3] = x;
-        }
+        s[0] = ltx_score(Qs, C, srow, scol, STRIDE, dk);
+        s[1] = ltx_score(Qs, C, srow, scol + 1, STRIDE, dk);
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         const int k = k0 + scol + e;
         s[e] = (srow < rows_live && k <= min(spos, k_end) && k >= slo) ? s[e] * p.scale : -INFINITY;
         mx = fmaxf(mx, s[e]);
       }
 #pragma unroll
-      for (int x = 1; x < 8; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+      for (int x = 1; x < 16; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
       const float mn = fmaxf(m, mx), ref = mn == -INFINITY ? 0.f : mn;    // (a row may see no key of this tile)
       const float c = expf(m - ref);
       m = mn;
-      unsigned short t[4][3];
-      float sum = 0.f;
+      unsigned short t[2][3];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2; ++e) {
         s[e] = expf(s[e] - ref);
-        sum += s[e];
         ltx_split(s[e], t[e]);
       }
-      l = l * c + sum;                                     // (this thread's share; the row is added at the end)
+      l = l * c + (s[0] + s[1]);                           // (this thread's share; the row is added at the end)
 #pragma unroll
       for (int i = 0; i < 3; ++i)
-        *reinterpret_cast<uint2*>(Pt + (i * LTX_ROWS + srow) * LTX_PLD + scol) =
-            make_uint2(t[0][i] | (unsigned)t[1][i] << 16, t[2][i] | (unsigned)t[3][i] << 16);
-      if ((tid & 7) == 0) corr[srow] = c;
+        *reinterpret_cast<unsigned*>(Pt + (i * LTX_ROWS + srow) * LTX_PLD + scol) = t[0][i] | (unsigned)t[1][i] << 16;
+      if ((tid & 15) == 0) corr[srow] = c;
     }
     // A weight of 0 does not keep what is not finite out of a product, so a tile that holds any such thing takes only the keys
     // each row sees.
@@ -674,15 +672,15 @@ __global__ void __launch_bounds__(256, 1) latent_attention_split_kernel(const Lt
     }
   }
 #pragma unroll
-  for (int x = 1; x < 8; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+  for (int x = 1; x < 16; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
   const size_t flat0 = (size_t)first * H + row0;           // this tile's first (token, head) row of the step
   if (p.splits > 1) {
-    if ((tid & 7) == 0 && srow < rows_live) {
+    if ((tid & 15) == 0 && srow < rows_live) {
       float* w = p.ws + ((flat0 + srow) * p.splits + blockIdx.y) * (size_t)(r + 2);
       w[0] = m;                                            // (-inf: a chunk without keys)
       w[1] = l;
     }
-  } else if ((tid & 7) == 0 && srow < rows_live) {
+  } else if ((tid & 15) == 0 && srow < rows_live) {
     const size_t flat = flat0 + srow, t = flat / H;
     const int h = (int)(flat - t * H);
     // (by the merge kernel's arithmetic, so that one chunk and several of which one holds keys give the same bits)
@@ -722,7 +720,7 @@ template <int OC> cudaError_t ltx_launch(const LtxParams& p, cudaStream_t stream
   if (e != cudaSuccess) return e;
   // (every request's last tile may be partly filled: at most R tiles beside the whole ones)
   const unsigned tiles = (unsigned)((long long)p.n * p.H / LTX_ROWS + p.R);
-  return gb_launch(latent_attention_split_kernel<OC>, dim3(tiles, p.splits), dim3(256), smem, stream, p);
+  return gb_launch(latent_attention_split_kernel<OC>, dim3(tiles, p.splits), dim3(32 * LTX_WARPS), smem, stream, p);
 }
 
 // out[t, h, :] = x[t, h, :] W[h]^T on tensor cores, for the two per-head products around the attention (W_uk^T on the
@@ -899,8 +897,7 @@ cudaError_t gb_latent_attention_split_launch(const float* qp, const bf16* pages,
   p.dk = r + dr; p.stride = 16 * ((p.dk + 15) / 16) + 8; p.window = window; p.splits = splits; p.chunk = chunk;
   p.gate = gate; p.ld_gate = ld_gate; p.out = out; p.ldo = ldo; p.ws = ws; p.scale = scale;
   p.sink = sink; p.status = status;
-  if (r <= 64) return ltx_launch<16>(p, stream);
-  if (r <= 128) return ltx_launch<32>(p, stream);
-  if (r <= 256) return ltx_launch<64>(p, stream);
-  return ltx_launch<128>(p, stream);
+  if (r <= 128) return ltx_launch<16>(p, stream);
+  if (r <= 256) return ltx_launch<32>(p, stream);
+  return ltx_launch<64>(p, stream);
 }
