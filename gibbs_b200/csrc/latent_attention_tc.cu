@@ -81,6 +81,52 @@ struct LtcParams {
   int* status;
 };
 
+// A thread's part of two finished rows: columns wn * OC + 8 j + 2 t4 and the one behind.
+template <int OC>
+__device__ __forceinline__ void ltc_store(const LtcParams& p, const float (&o)[OC / 8][4], float m_a, float m_b, float l_a, float l_b, int row_a,
+                                          int row_b, int rows_live, int tl_a, int tl_b, int h_a, int h_b, int t_first, int wn, int t4) {
+  const int H = p.H, r = p.r;
+  constexpr float LOG2E = 1.4426950408889634f;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int row = half ? row_b : row_a;
+    if (row >= rows_live) continue;
+    const int tl = half ? tl_b : tl_a, h = half ? h_b : h_a;
+    const float m = half ? m_b : m_a, l = half ? l_b : l_a;
+    const size_t t = (size_t)t_first + tl;
+    if (p.splits > 1) {
+      // this half's partial result: maximum (natural units), sum of weights, weighted sum, for the merge kernel
+      float* w = p.ws + ((t * H + h) * p.splits + blockIdx.z) * (size_t)(r + 2);
+      if (wn == 0 && t4 == 0) {
+        w[0] = m * 0.6931471805599453f;                    // (-inf stays -inf: a half without keys)
+        w[1] = l;
+      }
+#pragma unroll
+      for (int j = 0; j < OC / 8; ++j) {
+        const int col = wn * OC + 8 * j + 2 * t4;
+        if (col < r) {
+          w[2 + col] = o[j][2 * half];
+          w[2 + col + 1] = o[j][2 * half + 1];
+        }
+      }
+      continue;
+    }
+    float f = 1.f / l;
+    if (p.sink) {
+      // a learned score without a key or a value: only the denominator knows it
+      const float s2 = p.sink[h] * LOG2E, top = fmaxf(m, s2), e = exp2f(m - top);
+      f = e / (exp2f(s2 - top) + e * l);
+    }
+    if (p.gate) f *= hy_sigmoid(p.gate[t * p.ld_gate + h]);
+    float* dst = p.out + t * p.ldo + (size_t)h * r + wn * OC + 2 * t4;
+#pragma unroll
+    for (int j = 0; j < OC / 8; ++j) {
+      if (wn * OC + 8 * j < r)
+        *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(o[j][2 * half] * f, o[j][2 * half + 1] * f);
+    }
+  }
+}
+
 template <int RP>
 __global__ void __launch_bounds__(RP > 256 ? 256 : 128, 1) latent_attention_tc_kernel(const LtcParams p) {
   constexpr int NSPLIT = RP > 256 ? 2 : 1, OC = RP / NSPLIT, THREADS = 128 * NSPLIT;
@@ -258,45 +304,235 @@ __global__ void __launch_bounds__(RP > 256 ? 256 : 128, 1) latent_attention_tc_k
   l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
   l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
   l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-  constexpr float LOG2E = 1.4426950408889634f;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int row = half ? row_b : row_a;
-    if (row >= rows_live) continue;
-    const int tl = half ? tl_b : tl_a, h = half ? h_b : h_a;
-    const float m = half ? m_b : m_a, l = half ? l_b : l_a;
-    const size_t t = (size_t)t_first + tl;
-    if (p.splits > 1) {
-      // this half's partial result: maximum (natural units), sum of weights, weighted sum, for the merge kernel
-      float* w = p.ws + ((t * H + h) * p.splits + blockIdx.z) * (size_t)(r + 2);
-      if (wn == 0 && t4 == 0) {
-        w[0] = m * 0.6931471805599453f;                    // (-inf stays -inf: a half without keys)
-        w[1] = l;
+  ltc_store<OC>(p, o, m_a, m_b, l_a, l_b, row_a, row_b, rows_live, tl_a, tl_b, h_a, h_b, t_first, wn, t4);
+}
+
+// The same for latents wider than 256 whose rows leave room for the weights in shared memory: 16 warps, four groups of 16 rows x
+// four slices.  For S a slice is 16 of a key tile's 64 keys (every score once, where the kernel above works every score out in
+// both groups of warps), for O a quarter of the latent's columns; maxima and the weights' two terms go through shared memory
+// between the four warps of a row group, which meet at a barrier of their own.
+constexpr int LTW_SLICES = 4, LTW_THREADS = 128 * LTW_SLICES, LTW_OC = 128, LTW_PLD = 72;
+
+size_t ltw_smem(int stride) {
+  return sizeof(bf16) * (3 * LTC_ROWS * (size_t)stride + 2 * LTC_ROWS * LTW_PLD) + sizeof(float) * 2 * LTW_SLICES * LTC_ROWS;
+}
+
+__global__ void __launch_bounds__(LTW_THREADS, 1) latent_attention_tc_wide_kernel(const LtcParams p) {
+  constexpr int OC = LTW_OC;
+  const int STRIDE = p.stride, dk = p.dk;
+  extern __shared__ __align__(16) unsigned char ltc_smem[];
+  bf16* Qs = reinterpret_cast<bf16*>(ltc_smem);            // [64][STRIDE]
+  bf16* Cs = Qs + LTC_ROWS * STRIDE;                       // [2][64][STRIDE]
+  bf16* Ps = Cs + 2 * LTC_KEYS * STRIDE;                   // [2 terms][64][LTW_PLD]
+  float* top = reinterpret_cast<float*>(Ps + 2 * LTC_ROWS * LTW_PLD);    // [slice][64] maxima over a tile, then [slice][64] sums
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wm = warp & 3, wn = warp >> 2;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int req = blockIdx.y;
+  const int first = p.q_start[req], len = (req + 1 < p.R ? p.q_start[req + 1] : p.n) - first;
+  const int tok0 = (int)(gridDim.x - 1 - blockIdx.x) * p.tpt;
+  if (tok0 >= len) return;
+  const int ntok = min(p.tpt, len - tok0), H = p.H, r = p.r;
+  const int rows_live = ntok * H;
+  const int t_first = first + tok0;
+  const int pos0 = p.tok_pos[t_first];
+  const int kmax = pos0 + ntok - 1;
+  const int* table = p.block_table + (size_t)p.tok_req[t_first] * p.bt_stride;
+  // zeros where nothing is copied: rows beyond the live ones, columns dk .. stride
+  for (int i = threadIdx.x; i < 3 * LTC_ROWS * STRIDE / 8; i += LTW_THREADS)
+    reinterpret_cast<uint4*>(ltc_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+
+  const int pieces = dk >> 3;                              // 16-byte pieces of a cached row
+  auto stage = [&](int kt, int b) {
+    bf16* dst = Cs + (size_t)b * LTC_KEYS * STRIDE;
+    for (int j = warp; j < LTC_KEYS; j += LTW_THREADS / 32) {
+      const int key = min(kt * LTC_KEYS + j, kmax);        // (rows behind the last visible key are masked)
+      const int page = table[key / p.page_size];
+      if (page < 0 || page >= p.n_pages) {
+        if (lane == 0) atomicExch(p.status, LTC_BAD_PAGE_READ);
+        continue;                                          // (the row keeps what it had: zeros or an older row)
       }
+      const bf16* src = p.pages + ((size_t)page * p.page_size + key % p.page_size) * dk;
+      for (int c = lane; c < pieces; c += 32) gb_cp_async_16(dst + j * STRIDE + 8 * c, src + 8 * c);
+    }
+    ltc_commit();
+  };
+  const int tiles = kmax / LTC_KEYS + 1;
+  const int half_tiles = (tiles + 1) >> 1;
+  const int kt_begin = p.splits > 1 ? (int)blockIdx.z * half_tiles : 0;
+  const int kt_end = p.splits > 1 ? min(tiles, kt_begin + half_tiles) : tiles;
+  pdl_wait();
+  if (kt_begin < kt_end) stage(kt_begin, 0);
+  {
+    // this tile's queries: rows_live consecutive rows of dk floats, rounded to bfloat16
+    const float* src = p.qp + (size_t)t_first * H * dk;
+    const int quads = dk >> 2;
+    for (int row = warp; row < rows_live; row += LTW_THREADS / 32)
+      for (int c = lane; c < quads; c += 32) {
+        const float4 v = *reinterpret_cast<const float4*>(src + (size_t)row * dk + 4 * c);
+        uint2 w;
+        w.x = ltc_pack(v.x, v.y);
+        w.y = ltc_pack(v.z, v.w);
+        *reinterpret_cast<uint2*>(Qs + row * STRIDE + 4 * c) = w;
+      }
+  }
+  // this thread's two rows: wm * 16 + g and + 8
+  const int row_a = wm * 16 + g, row_b = row_a + 8;
+  const int tl_a = row_a / H, tl_b = row_b / H;
+  const int h_a = row_a - tl_a * H, h_b = row_b - tl_b * H;
+  const int pos_a = pos0 + tl_a, pos_b = pos0 + tl_b;
+  const bool warp_live = wm * 16 < rows_live;              // (the same for the four warps of a row group)
+  auto group_barrier = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + wm) : "memory"); };
+
+  float o[OC / 8][4];
+#pragma unroll
+  for (int j = 0; j < OC / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
+  const int ksteps = (dk + 15) >> 4;                       // k-steps of the first product that hold anything
+  const int npairs = min(OC / 16, max(0, (r - wn * OC + 15) >> 4));   // pairs of 8 output columns likewise
+
+  if (kt_begin >= kt_end) __syncthreads();                 // (the queries and zeros are written; no key tile follows)
+  for (int kt = kt_begin; kt < kt_end; ++kt) {
+    const int b = (kt - kt_begin) & 1;
+    if (kt + 1 < kt_end) {
+      stage(kt + 1, b ^ 1);
+      ltc_wait<1>();
+    } else {
+      ltc_wait<0>();
+    }
+    __syncthreads();
+    if (warp_live) {
+      const bf16* C = Cs + (size_t)b * LTC_KEYS * STRIDE;
+      float s[2][4], s2[2][4];                             // even and odd k-steps: two chains
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        s2[j][0] = s2[j][1] = s2[j][2] = s2[j][3] = 0.f;
+      }
+      const bf16* qa = Qs + (wm * 16 + (lane & 15)) * STRIDE + (lane >> 4) * 8;
+      const bf16* cb = C + (wn * 16 + (lane & 7) + (lane >> 4) * 8) * STRIDE + ((lane >> 3) & 1) * 8;
+#pragma unroll 2
+      for (int ks = 0; ks + 1 < ksteps; ks += 2) {
+        unsigned a[2][4], bb[2][4];
+        ltc_ldmatrix(a[0], qa + ks * 16);
+        ltc_ldmatrix(bb[0], cb + ks * 16);
+        ltc_ldmatrix(a[1], qa + ks * 16 + 16);
+        ltc_ldmatrix(bb[1], cb + ks * 16 + 16);
+        ltc_mma(s[0], a[0], bb[0][0], bb[0][1]);
+        ltc_mma(s[1], a[0], bb[0][2], bb[0][3]);
+        ltc_mma(s2[0], a[1], bb[1][0], bb[1][1]);
+        ltc_mma(s2[1], a[1], bb[1][2], bb[1][3]);
+      }
+      if (ksteps & 1) {
+        unsigned a[4], bb[4];
+        ltc_ldmatrix(a, qa + (ksteps - 1) * 16);
+        ltc_ldmatrix(bb, cb + (ksteps - 1) * 16);
+        ltc_mma(s[0], a, bb[0], bb[1]);
+        ltc_mma(s[1], a, bb[2], bb[3]);
+      }
+      // scores in base 2, the causal mask, the maximum over this slice's keys
+      const int key0 = kt * LTC_KEYS + wn * 16 + 2 * t4;
+      float mx_a = -INFINITY, mx_b = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int k = key0 + 8 * j;
+        s[j][0] = k <= pos_a ? (s[j][0] + s2[j][0]) * p.scale_log2 : -INFINITY;
+        s[j][1] = k + 1 <= pos_a ? (s[j][1] + s2[j][1]) * p.scale_log2 : -INFINITY;
+        s[j][2] = k <= pos_b ? (s[j][2] + s2[j][2]) * p.scale_log2 : -INFINITY;
+        s[j][3] = k + 1 <= pos_b ? (s[j][3] + s2[j][3]) * p.scale_log2 : -INFINITY;
+        mx_a = fmaxf(mx_a, fmaxf(s[j][0], s[j][1]));
+        mx_b = fmaxf(mx_b, fmaxf(s[j][2], s[j][3]));
+      }
+      mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
+      mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
+      mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
+      mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
+      if (t4 == 0) {
+        top[wn * LTC_ROWS + row_a] = mx_a;
+        top[wn * LTC_ROWS + row_b] = mx_b;
+      }
+      group_barrier();
+      float mn_a = m_a, mn_b = m_b;
+#pragma unroll
+      for (int w = 0; w < LTW_SLICES; ++w) {
+        mn_a = fmaxf(mn_a, top[w * LTC_ROWS + row_a]);
+        mn_b = fmaxf(mn_b, top[w * LTC_ROWS + row_b]);
+      }
+      const float ref_a = mn_a == -INFINITY ? 0.f : mn_a, ref_b = mn_b == -INFINITY ? 0.f : mn_b;
+      const float corr_a = exp2f(m_a - ref_a), corr_b = exp2f(m_b - ref_b);
+      m_a = mn_a;
+      m_b = mn_b;
+      float sum_a = 0.f, sum_b = 0.f;
+      unsigned* pw = reinterpret_cast<unsigned*>(Ps + wn * 16 + 2 * t4);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        s[j][0] = exp2f(s[j][0] - ref_a);
+        s[j][1] = exp2f(s[j][1] - ref_a);
+        s[j][2] = exp2f(s[j][2] - ref_b);
+        s[j][3] = exp2f(s[j][3] - ref_b);
+        sum_a += s[j][0] + s[j][1];
+        sum_b += s[j][2] + s[j][3];
+        unsigned hi, lo;
+        ltc_split(s[j][0], s[j][1], hi, lo);
+        pw[(row_a * LTW_PLD + 8 * j) / 2] = hi;
+        pw[((LTC_ROWS + row_a) * LTW_PLD + 8 * j) / 2] = lo;
+        ltc_split(s[j][2], s[j][3], hi, lo);
+        pw[(row_b * LTW_PLD + 8 * j) / 2] = hi;
+        pw[((LTC_ROWS + row_b) * LTW_PLD + 8 * j) / 2] = lo;
+      }
+      l_a = l_a * corr_a + sum_a;                          // (this lane's share of this slice's keys; added up at the end)
+      l_b = l_b * corr_b + sum_b;
 #pragma unroll
       for (int j = 0; j < OC / 8; ++j) {
-        const int col = wn * OC + 8 * j + 2 * t4;
-        if (col < r) {
-          w[2 + col] = o[j][2 * half];
-          w[2 + col + 1] = o[j][2 * half + 1];
+        o[j][0] *= corr_a;
+        o[j][1] *= corr_a;
+        o[j][2] *= corr_b;
+        o[j][3] *= corr_b;
+      }
+      group_barrier();
+      // O += P C, the weights as hi + lo
+      const bf16* ct = C + ((lane & 7) + ((lane >> 3) & 1) * 8) * STRIDE + wn * OC + (lane >> 4) * 8;
+      const bf16* pa = Ps + (wm * 16 + (lane & 15)) * LTW_PLD + (lane >> 4) * 8;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        unsigned hi[4], lo[4];
+        ltc_ldmatrix(hi, pa + kk * 16);
+        ltc_ldmatrix(lo, pa + LTC_ROWS * LTW_PLD + kk * 16);
+#pragma unroll
+        for (int np = 0; np < OC / 16; ++np) {
+          if (np < npairs) {
+            unsigned bb[4];
+            ltc_ldmatrix_t(bb, ct + kk * 16 * STRIDE + np * 16);
+            ltc_mma(o[2 * np], hi, bb[0], bb[1]);
+            ltc_mma(o[2 * np + 1], hi, bb[2], bb[3]);
+            ltc_mma(o[2 * np], lo, bb[0], bb[1]);
+            ltc_mma(o[2 * np + 1], lo, bb[2], bb[3]);
+          }
         }
       }
-      continue;
     }
-    float f = 1.f / l;
-    if (p.sink) {
-      // a learned score without a key or a value: only the denominator knows it
-      const float s2 = p.sink[h] * LOG2E, top = fmaxf(m, s2), e = exp2f(m - top);
-      f = e / (exp2f(s2 - top) + e * l);
-    }
-    if (p.gate) f *= hy_sigmoid(p.gate[t * p.ld_gate + h]);
-    float* dst = p.out + t * p.ldo + (size_t)h * r + wn * OC + 2 * t4;
-#pragma unroll
-    for (int j = 0; j < OC / 8; ++j) {
-      if (wn * OC + 8 * j < r)
-        *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(o[j][2 * half] * f, o[j][2 * half + 1] * f);
-    }
+    __syncthreads();                                       // before the tile after next lands in this buffer
   }
+  if (!warp_live) return;
+  l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
+  l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
+  l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
+  l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
+  float* share = top + LTW_SLICES * LTC_ROWS;
+  if (t4 == 0) {
+    share[wn * LTC_ROWS + row_a] = l_a;
+    share[wn * LTC_ROWS + row_b] = l_b;
+  }
+  group_barrier();
+  l_a = l_b = 0.f;
+#pragma unroll
+  for (int w = 0; w < LTW_SLICES; ++w) {
+    l_a += share[w * LTC_ROWS + row_a];
+    l_b += share[w * LTC_ROWS + row_b];
+  }
+  ltc_store<OC>(p, o, m_a, m_b, l_a, l_b, row_a, row_b, rows_live, tl_a, tl_b, h_a, h_b, t_first, wn, t4);
 }
 
 template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStream_t stream) {
@@ -870,6 +1106,15 @@ int gb_latent_attention_tc_launch(const float* qp, const bf16* pages, const int*
   if (r <= 64) rc = ltc_launch<64>(p, tiles, R, stream);
   else if (r <= 128) rc = ltc_launch<128>(p, tiles, R, stream);
   else if (r <= 256) rc = ltc_launch<256>(p, tiles, R, stream);
+  else if (ltw_smem(p.stride) <= 227 * 1024) {
+    static bool raised = false;                            // (before any stream capture replays the launch)
+    if (!raised) {
+      if (cudaFuncSetAttribute(latent_attention_tc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return -1;
+      raised = true;
+    }
+    gb_launch(latent_attention_tc_wide_kernel, dim3(tiles, R, p.splits), dim3(LTW_THREADS), ltw_smem(p.stride), stream, p);
+    rc = 0;
+  }
   else rc = ltc_launch<512>(p, tiles, R, stream);
   return rc < 0 ? rc : p.splits;
 }
