@@ -499,10 +499,10 @@ int run_attention_tc(const GbPlanCtx* ctx, const long long* a, const double* f, 
   }
   int rc;
   // portions that fill the chip without chunks of keys, where the other kernel takes them
-  if (!narrow && p.splits == 1 && tiles * G * maps > 296 && !p.blocked && p.keep_first == 0) {
+  if (!narrow && p.splits == 1 && tiles * G * maps > 296 && p.keep_first == 0) {
     const GatedTcgen05Launch b = {p.q, p.k_pages, p.v_pages, p.block_table, p.bt_stride, p.page_size, p.n_pages, p.tok_req,
                                   p.tok_pos, p.q_start, p.gate, p.ld_gate, p.out, p.out_f32, p.ldo, n, R, H, G, dim, vdim, maps,
-                                  p.window, p.sink, p.scale, p.softcap, p.sink_scores, SIG, score_bias, factor, p.status};
+                                  p.window, p.blocked, p.sink, p.scale, p.softcap, p.sink_scores, SIG, score_bias, factor, p.status};
     if (gb_gated_tcgen05_takes(b)) return gb_gated_tcgen05_launch(b, ctx->stream);
   }
   const dim3 grid(tiles, G * maps, p.splits);

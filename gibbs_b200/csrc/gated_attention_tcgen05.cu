@@ -1,5 +1,5 @@
 // The attention of gated_attention_tc.cuh for prompt portions on the 5th generation tensor cores: keys of 64 entries, values
-// of 64 or 128, sliding window, soft cap, sink, output gate, maps, and the form with sigmoids in the softmax's place.
+// of 64 or 128, sliding window or blocks, soft cap, sink, output gate, maps, and the form with sigmoids in the softmax's place.
 //
 // A CTA takes one (kv head, map, tile of consecutive tokens of one request); its 128 rows are (token, query head of the
 // group) pairs.  It walks the visible keys in tiles of 64 positions:
@@ -38,7 +38,7 @@ struct GtParams {
   const int* tok_req; const int* tok_pos; const int* q_start;
   const float* gate; long long ld_gate;
   bf16* out; float* out_f32; long long ldo;
-  int N, R, H, G, tpt, maps, window, sink;
+  int N, R, H, G, tpt, maps, window, blocked, sink;
   float scale, softcap;
   const float* sink_scores;
   const float* score_bias; float factor;
@@ -118,7 +118,9 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
   const int pos0 = p.tok_pos[t0];
   const int* bt = p.block_table + (size_t)p.tok_req[t0] * p.bt_stride;
   const int hi_all = pos0 + n_tok;                              // keys lo_all <= k < hi_all may be seen
-  const int lo_all = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+  // the first position that position p sees (with `blocked` its own block of `window` positions, counted from 0)
+  auto first_seen = [&](int pos) { return p.window <= 0 ? 0 : p.blocked ? pos / p.window * p.window : pos - p.window + 1; };
+  const int lo_all = max(0, first_seen(pos0));
   const int t_lo = lo_all / GT_KEYS, t_hi = (hi_all + GT_KEYS - 1) / GT_KEYS, n_tiles = t_hi - t_lo;
 
   if (warp == 1) {
@@ -251,7 +253,7 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const int q4 = warp & 3, row = 32 * q4 + lane;
     const int tl = row / group, hh = row - tl * group;
     const bool rvalid = tl < n_tok;
-    const int rpos = pos0 + tl;
+    const int rpos = pos0 + tl, rfirst = first_seen(rpos), last_first = first_seen(pos0 + tpt - 1);
     const uint32_t lane_off = (uint32_t)(32 * q4) << 16;
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     const float c_in = CAPPED ? p.scale * 2.f * LOG2E / p.softcap : p.scale * LOG2E;
@@ -270,8 +272,8 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
       // which of the tile's columns this row may see: lo_c <= column <= hi_c; most tiles need no mask
       const int col0 = (t_lo + j) * GT_KEYS;
       const int hi_c = rvalid ? rpos - col0 : -1;
-      const int lo_c = (p.window > 0 ? rpos - p.window + 1 : 0) - col0;
-      const bool full = col0 + GT_KEYS - 1 <= pos0 && (p.window <= 0 || col0 + p.window > pos0 + tpt - 1);
+      const int lo_c = rfirst - col0;
+      const bool full = col0 + GT_KEYS - 1 <= pos0 && col0 >= last_first;
       float v[GT_KEYS];
 #pragma unroll
       for (int c = 0; c < GT_KEYS; c += 32) tmem_ld_32_issue(tmem_s + lane_off + (uint32_t)c, v + c);
@@ -496,7 +498,7 @@ int gb_gated_tcgen05_launch(const GatedTcgen05Launch& a, cudaStream_t stream) {
   p.block_table = a.block_table; p.bt_stride = a.bt_stride; p.page_size = a.page_size; p.n_pages = a.n_pages;
   p.tok_req = a.tok_req; p.tok_pos = a.tok_pos; p.q_start = a.q_start; p.gate = a.gate; p.ld_gate = a.ld_gate;
   p.out = a.out; p.out_f32 = a.out_f32; p.ldo = a.ldo; p.N = a.n; p.R = a.R; p.H = a.H; p.G = a.G; p.tpt = tpt; p.maps = a.maps;
-  p.window = a.window; p.sink = a.sink; p.scale = a.scale; p.softcap = a.softcap; p.sink_scores = a.sink_scores;
+  p.window = a.window; p.blocked = a.blocked; p.sink = a.sink; p.scale = a.scale; p.softcap = a.softcap; p.sink_scores = a.sink_scores;
   p.score_bias = a.score_bias; p.factor = a.factor; p.status = a.status;
   // (every request may end with a partly filled tile)
   const dim3 grid(a.G * a.maps, gb_div_up(a.n, tpt) + a.R);

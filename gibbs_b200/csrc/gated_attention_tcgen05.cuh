@@ -10,7 +10,7 @@ struct GatedTcgen05Launch {
   const int *tok_req, *tok_pos, *q_start;
   const float* gate; long long ld_gate;
   __nv_bfloat16* out; float* out_f32; long long ldo;      // one of the two
-  int n, R, H, G, dim, vdim, maps, window, sink;
+  int n, R, H, G, dim, vdim, maps, window, blocked, sink;
   float scale, softcap;
   const float* sink_scores;
   bool sigmoid;                    // weights sigmoid(score + score_bias[head]), the output times `factor`

@@ -470,17 +470,19 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
 
 
 # launches of more than 296 tiles of 64 rows: windows within a key tile and across tiles, groups that do not divide 128, pages of 8 to
-# 64, a single token beside portions, two maps, the edges of 64 keys, no softmax
-@pytest.mark.parametrize("heads,kvh,maps,vdim,ps,window,cap,sink,gate,sig,starts,lens", [
-    (16, 4, 1, 64, 16, 0, 30.0, True, True, False, [0, 63], [1000, 230]),
-    (32, 8, 1, 64, 16, 100, 30.0, True, False, False, [0, 1000, 64], [433, 1, 260]),
-    (24, 8, 1, 128, 8, 64, 0.0, False, False, False, [127, 65], [800, 7]),
-    (20, 4, 2, 128, 64, 1, 0.0, True, False, False, [0, 5], [300, 300]),
-    (16, 4, 2, 128, 32, 193, 0.0, False, False, False, [1000], [677]),
-    (16, 4, 1, 64, 16, 0, 0.0, False, False, True, [3, 0], [640, 700]),
-    (8, 8, 1, 64, 16, 40, 5.0, False, True, True, [0], [2500]),
+# 64, a single token beside portions, two maps, the edges of 64 keys, blocks of positions, no softmax
+@pytest.mark.parametrize("heads,kvh,maps,vdim,ps,window,cap,sink,gate,sig,starts,lens,blocked", [
+    (16, 4, 1, 64, 16, 0, 30.0, True, True, False, [0, 63], [1000, 230], False),
+    (32, 8, 1, 64, 16, 100, 30.0, True, False, False, [0, 1000, 64], [433, 1, 260], False),
+    (24, 8, 1, 128, 8, 64, 0.0, False, False, False, [127, 65], [800, 7], False),
+    (20, 4, 2, 128, 64, 1, 0.0, True, False, False, [0, 5], [300, 300], False),
+    (16, 4, 2, 128, 32, 193, 0.0, False, False, False, [1000], [677], False),
+    (16, 4, 1, 64, 16, 0, 0.0, False, False, True, [3, 0], [640, 700], False),
+    (8, 8, 1, 64, 16, 40, 5.0, False, True, True, [0], [2500], False),
+    (16, 4, 2, 128, 16, 100, 0.0, False, False, False, [150, 0], [500, 230], True), (32, 8, 1, 64, 16, 64, 20.0, True, True, False, [37], [700], True),
+    (16, 4, 2, 128, 32, 1024, 0.0, False, False, False, [0, 1000], [300, 377], True),
 ])
-def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens):
+def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
     from gibbs_b200.ops import hybrid
     torch.manual_seed(heads * 1000 + window)
     dk, n, group = 64, sum(lens), heads // kvh
@@ -496,7 +498,7 @@ def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, c
     # what no row sees is not finite: the rest of every last page, and what lies in front of a window
     for r, (a, b) in enumerate(zip(starts, lens)):
         at = torch.arange(need[r] * ps)
-        at = at[(at >= a + b) | (at <= (a - window if window else -1))]
+        at = at[(at >= a + b) | (at < (a // window * window if blocked else a - window + 1 if window else 0))]
         vp[bt[r][at // ps].long().cuda(), :, (at % ps).cuda()] = float("nan")
         kp[bt[r][at // ps].long().cuda(), :, (at % ps).cuda()] = float("inf")
     logits = torch.randn(n, heads * vdim, device="cuda") if gate else None
@@ -508,7 +510,7 @@ def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, c
                 [q.data_ptr(), kp.data_ptr(), vp.data_ptr(), tables.data_ptr(), bt.shape[1], ps, n_pages, tok_req.data_ptr(), pos.data_ptr(),
                  logits.data_ptr() if gate else 0, logits.stride(0) if gate else 0, out.data_ptr(), out.stride(0), n, heads, kvh, dk, vdim, window,
                  max(a + b for a, b in zip(starts, lens)), 0, len(lens), starts_.data_ptr(), score.data_ptr() if sink or sig else 0],
-                [scale, cap, factor if sig else 0.0], flags=(1 if sink else 0) | 2 | maps << 8)
+                [scale, cap, factor if sig else 0.0], flags=(1 if sink else 0) | 2 | (4 if blocked else 0) | maps << 8)
     assert (out[:, heads * maps * vdim:] == 7.0).all()
     got = out[:, :heads * maps * vdim].reshape(n, heads, maps, vdim).double()
     for r, (a, b) in enumerate(zip(starts, lens)):
@@ -516,7 +518,7 @@ def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, c
         pages = tables[r].long()[idx // ps]
         seen = idx[None] <= at[:, None]
         if window:
-            seen &= idx[None] > at[:, None] - window
+            seen &= idx[None] >= (at // window * window if blocked else at - window + 1)[:, None]
         k = kp[pages, :, idx % ps].double().reshape(a + b, kvh, maps, dk).repeat_interleave(group, 1)
         v = vp[pages, :, idx % ps].double().repeat_interleave(group, 1)
         v = torch.where(seen.any(0)[:, None, None], v, torch.zeros_like(v))
