@@ -758,7 +758,8 @@ GB_OP(gb_op_row_norm) {
     }
   }
   const size_t block_smem = sizeof(float) * ((size_t)(pend != nullptr ? ctx->pend_splits : 0) * dim + 2 * 512);
-  if (by_warps && n < NORM_FEW_ROWS && block_smem <= 160 * 1024) {
+  // (rows that bring pending sums at any number: a warp a row asks for its pieces' sums one after the other)
+  if (by_warps && (n < NORM_FEW_ROWS || pend != nullptr) && block_smem <= 160 * 1024) {
     // (whole warps; a thread without a piece adds zeros)
     const dim3 block(32 * gb_div_up(dim, 128));
 #define BLOCK_NORM(TO)                                                                                                     \
