@@ -466,12 +466,12 @@ __global__ void gelu_mul_rows_kernel(float* g, long long ld, const TT* __restric
 }
 
 // one block per (row, group)
-constexpr int GROUP_CACHE = 8;
+constexpr int GROUP_CACHE = 2;
 
 template <typename TO>
 __global__ void gated_group_norm_kernel(const float* y, long long ldy, const float* z, long long ldz,
                                         const float* __restrict__ gain, TO* out, long long ldo, int inner, int groups,
-                                        float eps) {
+                                        float eps, int pieces) {
   __shared__ float scratch[32];
   pdl_trigger();
   const int t = blockIdx.x, g = blockIdx.y;
@@ -479,33 +479,45 @@ __global__ void gated_group_norm_kernel(const float* y, long long ldy, const flo
   const float* yr = y + (size_t)t * ldy + c0;
   const float* zr = z + (size_t)t * ldz + c0;
   TO* o = out + (size_t)t * ldo + c0;
-  if (width <= GROUP_CACHE * (int)blockDim.x) {
-    // the group in registers; its gains are on hand before the kernel in front has finished (pinned, see gb_pin)
-    float v[GROUP_CACHE], a[GROUP_CACHE], b[GROUP_CACHE];
+  if (pieces) {
+    // rows of 16-byte pieces, up to GROUP_CACHE a thread, in registers; the gains are on hand before the kernel in front has
+    // finished (pinned, see gb_pin)
+    float4 v[GROUP_CACHE], a[GROUP_CACHE], b[GROUP_CACHE];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < GROUP_CACHE; ++i) {
-      const int d = threadIdx.x + i * blockDim.x;
-      v[i] = d < width ? gain[c0 + d] : 0.f;
+      const int d = 4 * (threadIdx.x + i * blockDim.x);
+      v[i] = d < width ? *reinterpret_cast<const float4*>(gain + c0 + d) : zero;
       gb_pin(v[i]);
     }
     pdl_wait();
 #pragma unroll
     for (int i = 0; i < GROUP_CACHE; ++i) {
-      const int d = threadIdx.x + i * blockDim.x;
-      a[i] = d < width ? ldcg_now(yr + d) : 0.f;
-      b[i] = d < width ? ldcg_now(zr + d) : 0.f;
+      const int d = 4 * (threadIdx.x + i * blockDim.x);
+      a[i] = d < width ? ldcg_now(reinterpret_cast<const float4*>(yr + d)) : zero;
+      b[i] = d < width ? ldcg_now(reinterpret_cast<const float4*>(zr + d)) : zero;
     }
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < GROUP_CACHE; ++i) {
-      a[i] *= hy_silu(b[i]);
-      ss += a[i] * a[i];
+      a[i].x *= hy_silu(b[i].x); a[i].y *= hy_silu(b[i].y); a[i].z *= hy_silu(b[i].z); a[i].w *= hy_silu(b[i].w);
+      ss += (a[i].x * a[i].x + a[i].y * a[i].y) + (a[i].z * a[i].z + a[i].w * a[i].w);
     }
     const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
 #pragma unroll
     for (int i = 0; i < GROUP_CACHE; ++i) {
-      const int d = threadIdx.x + i * blockDim.x;
-      if (d < width) o[d] = from_f32<TO>(a[i] * rstd * v[i]);
+      const int d = 4 * (threadIdx.x + i * blockDim.x);
+      if (d >= width) continue;
+      const float r0 = a[i].x * rstd * v[i].x, r1 = a[i].y * rstd * v[i].y, r2 = a[i].z * rstd * v[i].z, r3 = a[i].w * rstd * v[i].w;
+      if constexpr (sizeof(TO) == 2) {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(r0, r1), hi = __floats2bfloat162_rn(r2, r3);
+        uint2 w;
+        w.x = *reinterpret_cast<unsigned*>(&lo);
+        w.y = *reinterpret_cast<unsigned*>(&hi);
+        *reinterpret_cast<uint2*>(o + d) = w;
+      } else {
+        *reinterpret_cast<float4*>(o + d) = make_float4(r0, r1, r2, r3);
+      }
     }
     return;
   }
@@ -882,13 +894,17 @@ GB_OP(gb_op_gated_group_norm) {
   const int n = (int)a[8], inner = (int)a[9], groups = (int)a[10];
   if (n <= 0) return 0;
   if (groups <= 0 || inner % groups) GB_FAIL(GB_ERR_ARG, "gated_group_norm: %d columns in %d groups", inner, groups);
-  const dim3 grid(n, groups), block(norm_threads(inner / groups));
+  const int width = inner / groups, size = a[6] == GB_BF16 ? 2 : 4;
+  const dim3 grid(n, groups), block(norm_threads(width));
+  const int pieces = width % 4 == 0 && width <= 4 * GROUP_CACHE * (int)block.x && ((a[0] | a[2] | a[4] | 4 * a[1] | 4 * a[3]) & 15) == 0 &&
+                             a[7] % 4 == 0 && (a[5] & (4 * size - 1)) == 0
+                         ? 1 : 0;
   if (a[6] == GB_BF16)
     gb_launch(gated_group_norm_kernel<bf16>, grid, block, 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
-              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<bf16>(a[5]), a[7], inner, groups, (float)f[0]);
+              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<bf16>(a[5]), a[7], inner, groups, (float)f[0], pieces);
   else
     gb_launch(gated_group_norm_kernel<float>, grid, block, 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
-              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<float>(a[5]), a[7], inner, groups, (float)f[0]);
+              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), op_ptr<float>(a[5]), a[7], inner, groups, (float)f[0], pieces);
   GB_CHECK_LAUNCH("gated_group_norm");
   return 1;
 }
