@@ -441,7 +441,8 @@ __global__ void moe_experts_down_kernel(const TA* act, long long lda, const TW* 
 }
 
 __global__ void moe_combine_kernel(const float* out, long long ldo, const int* pair_row, const float* shared_gate,
-                                   const float* shared, long long lds, float* y, long long ldy, int width, int top) {
+                                   const float* shared, long long lds, int splits, size_t split_stride,
+                                   const float* __restrict__ shared_bias, float* y, long long ldy, int width, int top) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x;
@@ -449,21 +450,40 @@ __global__ void moe_combine_kernel(const float* out, long long ldo, const int* p
   for (int d = threadIdx.x; d < width; d += blockDim.x) {
     float v = 0.f;
     for (int k = 0; k < top; ++k) v += out[(size_t)pair_row[(size_t)t * top + k] * ldo + d];
-    if (shared) v += g * shared[(size_t)t * lds + d];
+    if (shared) {
+      float sh = splits > 0 ? 0.f : shared[(size_t)t * lds + d];
+      for (int u = 0; u < splits; ++u) sh += shared[u * split_stride + (size_t)t * lds + d];
+      v += g * (shared_bias ? sh + shared_bias[d] : sh);
+    }
     y[(size_t)t * ldy + d] = v;
   }
 }
 
 // The same arithmetic per value for rows of 16-byte pieces: the rows of four choices on their way together, a piece a thread.
 __global__ void moe_combine4_kernel(const float* out, long long ldo, const int* pair_row, const float* shared_gate,
-                                    const float* shared, long long lds, float* y, long long ldy, int width, int top) {
+                                    const float* shared, long long lds, int splits, size_t split_stride,
+                                    const float* __restrict__ shared_bias, float* y, long long ldy, int width, int top) {
   pdl_trigger();
   const int t = blockIdx.x, d = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
   pdl_wait();
   if (d >= width) return;
   const float g = shared_gate ? shared_gate[t] : 0.f;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 sh = shared ? ldcg_now(reinterpret_cast<const float4*>(shared + (size_t)t * lds + d)) : zero;
+  // (the shared expert's row, or the partial tiles [splits][rows][width] of the product that makes it, eight on their way together)
+  float4 sh = shared && splits == 0 ? ldcg_now(reinterpret_cast<const float4*>(shared + (size_t)t * lds + d)) : zero;
+  for (int u0 = 0; u0 < splits; u0 += 8) {
+    float4 q[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      q[u] = ldcg_now(reinterpret_cast<const float4*>(shared + (size_t)min(u0 + u, splits - 1) * split_stride + (size_t)t * lds + d));
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (u0 + u < splits) { sh.x += q[u].x; sh.y += q[u].y; sh.z += q[u].z; sh.w += q[u].w; }
+  }
+  if (splits > 0 && shared_bias) {
+    const float4 q = *reinterpret_cast<const float4*>(shared_bias + d);
+    sh.x += q.x; sh.y += q.y; sh.z += q.z; sh.w += q.w;
+  }
   float4 v = zero;
   for (int k0 = 0; k0 < top; k0 += 4) {
     float4 x[4];
@@ -764,16 +784,23 @@ GB_OP(gb_op_moe_experts) {
 GB_OP(gb_op_moe_combine) {
   const int n = (int)a[8], width = (int)a[9];
   if (n <= 0) return 0;
-  if (((a[0] | a[4] | a[6] | 4 * (a[1] | a[5] | a[7] | width)) & 15) == 0) {
+  // (a record with GB_OP_TAKES_PARTIALS: the shared expert's rows may be the partial tiles of the product in front)
+  const bool parts = a[4] != 0 && ctx->part_splits > 0;
+  const float* shared = parts ? ctx->part : op_ptr<const float>(a[4]);
+  const float* bias = parts ? ctx->part_bias : nullptr;
+  const long long lds = parts ? width : a[5];
+  const int splits = parts ? ctx->part_splits : 0;
+  const size_t stride = (size_t)n * width;
+  if (((a[0] | (long long)(uintptr_t)shared | (long long)(uintptr_t)bias | a[6] | 4 * (a[1] | lds | a[7] | width)) & 15) == 0) {
     const int threads = width <= 1024 ? 64 : 128;
     gb_launch(moe_combine4_kernel, dim3(n, gb_div_up(width, 4 * threads)), dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
-              op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), a[5], op_ptr<float>(a[6]), a[7],
+              op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), shared, lds, splits, stride, bias, op_ptr<float>(a[6]), a[7],
               width, (int)a[10]);
     GB_CHECK_LAUNCH("moe_combine (pieces)");
     return 1;
   }
   gb_launch(moe_combine_kernel, dim3(n), dim3(width <= 256 ? 64 : 256), 0, ctx->stream, op_ptr<const float>(a[0]), a[1],
-            op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), a[5], op_ptr<float>(a[6]), a[7],
+            op_ptr<const int>(a[2]), op_ptr<const float>(a[3]), shared, lds, splits, stride, bias, op_ptr<float>(a[6]), a[7],
             width, (int)a[10]);
   GB_CHECK_LAUNCH("moe_combine");
   return 1;

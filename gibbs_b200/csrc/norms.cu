@@ -309,6 +309,90 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
   }
 }
 
+// The same for rows of up to 2,048 values in 16-byte pieces: a block a row, a piece a thread, the gains on hand before the wait.
+// y may come as the partial tiles [splits][rows][dim] of the product that makes it (+ its bias): they are asked for in one trip
+// and added in their order, as the product's own reduction would.  A row's sums are formed by the same threads in the same
+// order whatever the number of rows.
+__global__ void __launch_bounds__(512)
+norm_add_block_kernel(float* x, long long ldx, const float* y, long long ldy, const float* __restrict__ gain, int dim, int kind, float eps,
+                      bf16* copy, ThenNorm then, const float* part, int splits, long long split_stride,
+                      const float* __restrict__ part_bias) {
+  extern __shared__ __align__(16) float tiles[];          // [splits][dim], then four rows of a number a thread
+  pdl_trigger();
+  const size_t r = blockIdx.x;
+  const int lane = threadIdx.x & 31, d = 4 * threadIdx.x;
+  const bool in = d < dim, second = then.gain != nullptr;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 g1 = in ? *reinterpret_cast<const float4*>(gain + d) : zero;
+  float4 g2 = in && second ? *reinterpret_cast<const float4*>(then.gain + d) : zero;
+  float4 pb = in && splits > 0 && part_bias ? *reinterpret_cast<const float4*>(part_bias + d) : zero;
+  gb_pin(g1);
+  gb_pin(g2);
+  gb_pin(pb);
+  float* sums = tiles + (size_t)splits * dim;
+  // a row's sum: every lane its pieces in ascending order, then the lanes
+  auto row_sum = [&](float mine, int turn) {
+    float* at = sums + turn * blockDim.x;
+    at[threadIdx.x] = mine;
+    __syncthreads();
+    float s = 0.f;
+    for (int i = lane; i < (int)blockDim.x; i += 32) s += at[i];
+    return warp_sum(s);
+  };
+  auto normed = [&](float4 v, int kd, float e, float4 g, int turn) {
+    const float mean = kd == NORM_LAYER ? row_sum((v.x + v.y) + (v.z + v.w), turn) / (float)dim : 0.f;
+    const float4 c = make_float4(v.x - mean, v.y - mean, v.z - mean, v.w - mean);
+    const float ss = row_sum(in ? (c.x * c.x + c.y * c.y) + (c.z * c.z + c.w * c.w) : 0.f, turn + 1);
+    const float rstd = 1.0f / sqrtf(ss / (float)dim + e);
+    return make_float4(c.x * rstd * g.x, c.y * rstd * g.y, c.z * rstd * g.z, c.w * rstd * g.w);
+  };
+  pdl_wait();
+  float4 v = zero, old = zero;
+  if (in) {
+    const float* from = part + r * dim + d;
+    for (int u = 0; u < splits; ++u) gb_cp_async_16(tiles + (size_t)u * dim + d, from + (size_t)u * split_stride);
+    old = ldcg_now(reinterpret_cast<const float4*>(x + r * ldx + d));
+    if (splits > 0) {
+      gb_cp_async_wait_all();
+      for (int u = 0; u < splits; ++u) {
+        const float4 q = *reinterpret_cast<const float4*>(tiles + (size_t)u * dim + d);
+        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+      }
+      if (part_bias) { v.x += pb.x; v.y += pb.y; v.z += pb.z; v.w += pb.w; }
+    } else {
+      v = ldcg_now(reinterpret_cast<const float4*>(y + r * ldy + d));
+    }
+  }
+  v = normed(v, kind, eps, g1, 0);
+  v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
+  auto pack = [](float4 q) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(q.x, q.y), hi = __floats2bfloat162_rn(q.z, q.w);
+    return make_uint2(*reinterpret_cast<unsigned*>(&lo), *reinterpret_cast<unsigned*>(&hi));
+  };
+  if (in) {
+    *reinterpret_cast<float4*>(x + r * ldx + d) = v;
+    if (copy) *reinterpret_cast<uint2*>(copy + r * dim + d) = pack(v);
+  }
+  if (!second) return;
+  if (!in) v = zero;
+  v = normed(v, then.kind, then.eps, g2, 2);
+  if (!in) return;
+  if (then.out_dtype == GB_BF16) *reinterpret_cast<uint2*>((bf16*)then.out + r * dim + d) = pack(v);
+  else *reinterpret_cast<float4*>((float*)then.out + r * dim + d) = v;
+}
+
+// y = the partial tiles' sum (+ bias), for rows that the kernel above does not take
+__global__ void norm_parts_kernel(const float* part, int splits, const float* __restrict__ bias, float* y, long long ldy, long long rows, int dim) {
+  pdl_trigger();
+  pdl_wait();
+  const long long total = rows * dim;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    float v = 0.f;
+    for (int u = 0; u < splits; ++u) v += part[(size_t)u * total + i];
+    y[(i / dim) * ldy + i % dim] = bias ? v + bias[i % dim] : v;
+  }
+}
+
 // x[t, :] += mult * (s1 * y1[t, :] + s2 * y2[t, :]): the residual sum of an arrangement whose sublayers read the same
 // normed rows and whose outputs are scaled channel by channel before they are added (y2, s2: optional).  `then`: the
 // norm in front of the NEXT layer, taken of the new rows while they are in registers.
@@ -835,6 +919,32 @@ GB_OP(gb_op_norm_add) {
   ThenNorm then = {op_ptr<const float>(a[9]), op_ptr<void>(a[10]), (int)a[11], (int)a[12], (float)f[1]};
   const bool second = then.gain != nullptr;
   if (second && then.kind != NORM_LAYER && then.kind != NORM_RMS) GB_FAIL(GB_ERR_ARG, "norm_add: second kind %d", then.kind);
+  // (a record with GB_OP_TAKES_PARTIALS: y may be the partial tiles of the product in front)
+  const float* part = ctx->part_splits > 0 ? ctx->part : nullptr;
+  const int splits = part != nullptr ? ctx->part_splits : 0;
+  const size_t smem = sizeof(float) * ((size_t)splits * dim + 4 * 512);
+  if (dim % 4 == 0 && dim <= 2048 && ((a[0] | a[2] | a[4] | a[9] | 4 * a[1] | 4 * a[3]) & 15) == 0 && (a[8] & 7) == 0 &&
+      (!second || (a[10] & (then.out_dtype == GB_BF16 ? 7 : 15)) == 0) && ((uintptr_t)part & 15) == 0 &&
+      (part == nullptr || ((uintptr_t)ctx->part_bias & 15) == 0) && smem <= 160 * 1024) {
+    static bool raised = false;
+    if (!raised) {
+      GB_CUDA(cudaFuncSetAttribute(norm_add_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+      raised = true;
+    }
+    gb_launch(norm_add_block_kernel, dim3(n), dim3(32 * gb_div_up(dim, 128)), smem, ctx->stream, op_ptr<float>(a[0]), a[1],
+              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]), then, part, splits,
+              (long long)n * dim, part != nullptr ? ctx->part_bias : nullptr);
+    GB_CHECK_LAUNCH("norm_add (a block a row)");
+    return 1;
+  }
+  int launched = 0;
+  if (part != nullptr) {
+    const long long total = (long long)n * dim;
+    gb_launch(norm_parts_kernel, dim3((int)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8)), dim3(256), 0, ctx->stream, part,
+              splits, ctx->part_bias, op_ptr<float>(a[2]), a[3], (long long)n, dim);
+    GB_CHECK_LAUNCH("norm_add (partial tiles)");
+    launched = 1;
+  }
   const bool fused = second && dim <= NORM_CACHE * threads;   // the row fits the registers
   ThenNorm none = {nullptr, nullptr, 0, 0, 0.f};
   // (us with the gains ahead and without, rows of 2048: 200 rows 3.2 and 4.2, 512 5.0 and 4.7, 2134 13.9 and 11.6; rows too long
@@ -844,7 +954,7 @@ GB_OP(gb_op_norm_add) {
             op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]),
             fused ? then : none);
   GB_CHECK_LAUNCH("norm_add");
-  if (!second || fused) return 1;
+  if (!second || fused) return launched + 1;
   // a row too long for the registers: the second norm as a kernel of its own
   if (then.out_dtype == GB_BF16)
     gb_launch(row_norm_kernel<bf16>, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], then.gain,
@@ -853,7 +963,7 @@ GB_OP(gb_op_norm_add) {
     gb_launch(row_norm_kernel<float>, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], then.gain,
               (float*)then.out, (const int*)nullptr, dim, then.kind, then.eps);
   GB_CHECK_LAUNCH("norm_add (second norm)");
-  return 2;
+  return launched + 2;
 }
 
 // a0 rows [g | u] (f32), a1 their stride, a2 out [n, inner], a3 out dtype, a4 its row stride, a5 rows, a6 inner;

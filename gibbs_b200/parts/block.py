@@ -132,6 +132,7 @@ class SandwichResidual(Block):
                 raise ValueError(f"the {role} must be a norm that can add into the stream (a RowNorm kind)")
 
     def _run(self, rn, x, caches, h_of):
+        rn.partial_branches = True                 # (the norm behind a sublayer adds up the partial tiles its last product leaves)
         hidden = x.shape[1]
         y = rn.buffer("branch", hidden, torch.float32)
         # a token input reads the stream through a product: in bfloat16 the norm that completes the

@@ -87,7 +87,7 @@ class ClampedGLU(BranchPart, FeedForward):
             rn.linear(h, self.gate_up, None, gu, role="glu_gate_up")
             rn.op("clamped_glu", [gu.data_ptr(), gu.stride(0), act.data_ptr(), ops.dtype_code(act.dtype), act.stride(0),
                                   rn.N, self.inner], [self.alpha, self.limit, self.up_add])
-        rn.linear(act, self.down, None, out, role="glu_down")
+        rn.branch_linear(act, self.down, None, out, role="glu_down")
 
 
 class RoutedGLU(BranchPart, FeedForward):
@@ -263,10 +263,13 @@ class RoutedGLU(BranchPart, FeedForward):
         sh = None
         if shared:
             sh = rn.buffer("moe_shared_out", d, torch.float32)
+            # (the kernel behind it adds the partial tiles its last product may leave)
+            leaves, rn.partial_branches = rn.partial_branches, True
             self.shared.run(rn, h, sh)
+            rn.partial_branches = leaves
         rn.op("moe_combine", [eout.data_ptr(), eout.stride(0), pair_row.data_ptr(), sg.data_ptr() if shared else 0,
                               sh.data_ptr() if shared else 0, sh.stride(0) if shared else 0, out.data_ptr(),
-                              out.stride(0), rn.N, d, top])
+                              out.stride(0), rn.N, d, top], flags=hybrid.TAKES_PARTIALS if shared else 0)
 
 
 class RoutedMLP(RoutedGLU):

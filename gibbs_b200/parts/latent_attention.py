@@ -161,7 +161,7 @@ class LatentAttention(BranchPart, Mixer):
                               o.data_ptr(), ops.dtype_code(o.dtype), o.stride(0), dv, rn.N, H, dv, r] +
               ([fused.data_ptr() + 4 * self.gate_col, fused.stride(0)] if self.gate_outputs else []),
               label="head_linear:values", flags=0 if USE_TENSOR_CORES else 1)
-        (rn.add_linear if accumulate else rn.linear)(o, self.o, None, out, role="latent_out")
+        rn.branch_linear(o, self.o, None, out, accumulate, role="latent_out")
 
 
 register_part("mixer", "latent_attention", LatentAttention)

@@ -113,7 +113,7 @@ class RowNorm(Norm):
             out = rn.buffer("normed", then.dim)
             a += [keep(rn, then.gain), out.data_ptr(), ops.dtype_code(out.dtype), then.KIND]
             f += [then.eps]
-        rn.op("norm_add", a, f, label="norm_add")
+        rn.op("norm_add", a, f, label="norm_add", flags=hybrid.TAKES_PARTIALS)
         return out
 
     def forward(self, x, out=None, rows=None):

@@ -82,7 +82,7 @@ class StateSpaceMixer(BranchPart, Mixer):
         rn.op("gated_group_norm", [y.data_ptr(), y.stride(0), u.data_ptr(), u.stride(0), keep(rn, self.gain),
                                    o.data_ptr(), ops.dtype_code(o.dtype), o.stride(0), rn.N, inner, self.norm_groups],
               [self.eps])
-        rn.linear(o, self.w_out, None, out, role="ssm_out")
+        rn.branch_linear(o, self.w_out, None, out, role="ssm_out")
 
 
 register_part("mixer", "state_space", StateSpaceMixer)
