@@ -88,8 +88,7 @@ enum { PREP_NORM_WHOLE = 1, PREP_Q_BF16 = 2, PREP_PAGES_BF16 = 4, PREP_NORM_HEAD
 __device__ __forceinline__ float prep_element(const float* x, const float* __restrict__ gain, bool gain_per_head,
                                               float rstd, int base, int d, int rot_dims, bool halves,
                                               const float* __restrict__ inv_freq, int pos, float mscale,
-                                              const float2* trig = nullptr, bool held = false,
-                                              float2 mine = make_float2(1.f, 0.f)) {
+                                              const float2* trig = nullptr) {
   const int gb = gain_per_head ? 0 : base;
   const float own = x[base + d] * rstd * (gain ? gain[gb + d] : 1.f);
   if (d >= rot_dims) return own;
@@ -99,10 +98,7 @@ __device__ __forceinline__ float prep_element(const float* x, const float* __res
   const int fi = halves ? (second ? d - half : d) : (d >> 1);
   const float other = x[base + partner] * rstd * (gain ? gain[gb + partner] : 1.f);
   float c, s;
-  if (held) {                                             // (the caller has this entry's cosine and sine in hand)
-    c = mine.x;
-    s = mine.y;
-  } else if (trig != nullptr) {
+  if (trig != nullptr) {
     c = trig[fi].x;
     s = trig[fi].y;
   } else {
@@ -120,12 +116,11 @@ __device__ __forceinline__ float prep_element(const float* x, const float* __res
 // FEW (steps of a few tokens): gridDim.y blocks share a token's heads, and the angles' cosines and sines (up to
 // PREP_PAIRS) are in shared memory before the product in front has finished.  Measured, 2 tokens of 32 + 8 heads of 64:
 // 6.1 us a launch in a decode step against 7.7 with one block a token.  (With many tokens a table per block was slower than
-// angles worked out by every head: the blocks that wait for it hold the SM.  There a lane keeps the cosines and sines of its
-// entries of a head, up to four, for all the heads its warp takes, and blocks are of eight warps, so that these are many.)
-constexpr int PREP_PAIRS = 128, PREP_FEW = 64, PREP_HELD = 4;
+// angles worked out by every head: the blocks that wait for it hold the SM.)
+constexpr int PREP_PAIRS = 128, PREP_FEW = 64;
 
 template <typename TC, typename TQ, bool FEW>
-__global__ void __launch_bounds__(512, FEW ? 3 : 2) qk_prep_kernel(const float* fused, long long ld, int k_col, int v_col, const float* __restrict__ q_gain,
+__global__ void __launch_bounds__(512, 3) qk_prep_kernel(const float* fused, long long ld, int k_col, int v_col, const float* __restrict__ q_gain,
                                const float* __restrict__ k_gain, const float* __restrict__ inv_freq, int rot_dims,
                                const int* tok_req, const int* tok_pos, const int* block_table, int bt_stride,
                                int page_size, TC* k_pages, TC* v_pages, int n_pages, int H, int G, int dim, int vdim,
@@ -157,24 +152,6 @@ __global__ void __launch_bounds__(512, FEW ? 3 : 2) qk_prep_kernel(const float* 
       trig = trig_table;
     }
   }
-  const bool held = !FEW && rot_dims <= 32 * PREP_HELD;
-  float2 mine[PREP_HELD];
-#pragma unroll
-  for (int i = 0; i < PREP_HELD; ++i) {
-    const int d = lane + 32 * i, half = rot_dims >> 1;
-    mine[i] = make_float2(1.f, 0.f);
-    if (held && d < rot_dims) {
-      const float ang = (float)pos * inv_freq[halves ? (d >= half ? d - half : d) : d >> 1];
-      mine[i] = make_float2(cosf(ang) * mscale, sinf(ang) * mscale);
-    }
-  }
-  // f(d, whether the lane holds entry d's cosine and sine, these) for the lane's entries of a head
-  auto each = [&](auto f) {
-#pragma unroll
-    for (int i = 0; i < PREP_HELD; ++i)
-      if (lane + 32 * i < dim) f(lane + 32 * i, held, mine[i]);
-    for (int d = lane + 32 * PREP_HELD; d < dim; d += 32) f(d, false, mine[0]);
-  };
   const int part = FEW ? blockIdx.y : 0, parts = FEW ? gridDim.y : 1;
   pdl_wait();
   const float* row = fused + (size_t)t * ld;
@@ -201,18 +178,17 @@ __global__ void __launch_bounds__(512, FEW ? 3 : 2) qk_prep_kernel(const float* 
     float post = temp;
     if (after) {
       float ss = 0.f;
-      each([&](int d, bool have, float2 cs) {
+      for (int d = lane; d < dim; d += 32) {
         const float v = prep_element(row, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
-                                     trig, have, cs);
+                                     trig);
         ss += v * v;
-      });
+      }
       post = temp / sqrtf(warp_sum(ss) / (float)dim + eps);
     }
-    each([&](int d, bool have, float2 cs) {
+    for (int d = lane; d < dim; d += 32)
       q_out[(size_t)t * ldq + h * dim + d] = from_f32<TQ>(post * prep_element(row, normed ? q_gain : nullptr, per_head, rstd,
                                                                               h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
-                                                                              trig, have, cs));
-    });
+                                                                              trig));
   }
   if (!writes) return;
   if (page < 0 || page >= n_pages) {
@@ -232,17 +208,16 @@ __global__ void __launch_bounds__(512, FEW ? 3 : 2) qk_prep_kernel(const float* 
     float post = 1.f;
     if (after) {
       float ss = 0.f;
-      each([&](int d, bool have, float2 cs) {
+      for (int d = lane; d < dim; d += 32) {
         const float v = prep_element(row + k_col, nullptr, true, 1.f, h * dim, d, rot_dims, halves, inv_freq, pos, mscale,
-                                     trig, have, cs);
+                                     trig);
         ss += v * v;
-      });
+      }
       post = 1.0f / sqrtf(warp_sum(ss) / (float)dim + eps);
     }
-    each([&](int d, bool have, float2 cs) {
+    for (int d = lane; d < dim; d += 32)
       dst[d] = from_f32<TC>(post * prep_element(row + k_col, normed ? k_gain : nullptr, per_head, rstd, h * dim, d, rot_dims,
-                                                halves, inv_freq, pos, mscale, trig, have, cs));
-    });
+                                                halves, inv_freq, pos, mscale, trig));
   }
   for (int i = threadIdx.x + part * blockDim.x; i < G * vdim; i += blockDim.x * parts) {
     const int g = i / vdim, d = i - g * vdim;
@@ -650,12 +625,11 @@ GB_OP(gb_op_qk_prep) {
   const long long ldq = (long long)H * maps * dim;
   const int mode = flags & (PREP_NORM_WHOLE | PREP_NORM_HEAD | PREP_ROT_HALVES | PREP_NORM_AFTER);
   const bool few = n <= PREP_FEW;
-  const int many_threads = threads > 256 && !(flags & PREP_NORM_WHOLE) ? 256 : threads;
   // (a warp a query head or two; the key heads and values come on top)
   const int parts = H * maps >= 4 * (threads / 32) ? 4 : gb_div_up(H * maps, threads / 32);
 #define PREP(TC, TQ)                                                                                                     \
   gb_launch(few ? qk_prep_kernel<TC, TQ, true> : qk_prep_kernel<TC, TQ, false>, few ? dim3(n, parts) : dim3(n),           \
-            dim3(few ? threads : many_threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2],                                     \
+            dim3(threads), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2],                                     \
             (int)a[3], op_ptr<const float>(a[4]), op_ptr<const float>(a[5]), op_ptr<const float>(a[6]), (int)a[7],        \
             op_ptr<const int>(a[8]), op_ptr<const int>(a[9]), op_ptr<const int>(a[10]), (int)a[11], (int)a[12],           \
             op_ptr<TC>(a[13]), op_ptr<TC>(a[14]), (int)a[15], H, G, dim, vdim, maps, mode, (float)f[0], (float)f[1], \
