@@ -243,8 +243,10 @@ constexpr int PAIR_STAGES = 6, PAIR_GROUPS = 2, PAIR_THREADS = 64 + PAIR_GROUPS 
 constexpr int PAIR_STAGE_BYTES = W_TILE_BYTES + PAIR_ROWS / 2 * BK * 2;
 constexpr int PAIR_STAGING_BYTES = 16 * 1024;                      // of a group: 32 token rows of 64 (g, u) in 32-bit
 constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_GROUPS * PAIR_STAGING_BYTES + 1024;
-// Rows an expert on average from which the pairs take a launch.  GIBBS_B200_MOE_PAIR_ROWS moves the line (for comparison runs).
-constexpr int PAIR_MIN_ROWS = 64;
+// Rows an expert on average from which the pairs take a launch.  Pairs against one CTA a tile, 32 experts of 2,048 x 2 x 1,024:
+// 52 / 53 us at 16 rows an expert, 53 / 58 at 32, 57 / 78 at 64, 63 / 111 at 128, 71 / 136 at 192, 101 / 169 at 256; below 32 the
+// two are within their noise and the narrow tiles leave less to pad.  GIBBS_B200_MOE_PAIR_ROWS moves the line (for comparison runs).
+constexpr int PAIR_MIN_ROWS = 32;
 constexpr int PAIR_MAX_EXPERTS = 128;                              // (by what shared memory is left)
 
 // Barrier of one group of epilogue warps; true for all of its threads when any of them brought true.
