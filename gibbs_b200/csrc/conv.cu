@@ -568,8 +568,9 @@ GB_API int gb_short_conv(const void* bcx, int dtype, long long ld, const float* 
     const bool vec = hidden % 8 == 0 && ld % 8 == 0 && slot_stride % 4 == 0 && ((uintptr_t)bcx & 15) == 0 &&
                      ((uintptr_t)out & 15) == 0 && ((uintptr_t)state & 15) == 0;
     if (vec && K <= 4) {
-      // (short runs while there are too few threads to fill the chip: four tokens a thread below 2,048)
-      const bool few = n_tokens < 2048;
+      // (short runs while there are too few threads to fill the chip.  us of runs of four and of eight, 2,048 channels: 128 tokens
+      // 1.8 and 2.1, 256 2.3 and 2.4, 512 2.7 and 2.8, 1,024 5.0 and 3.4, 2,048 8.3 and 6.3, 8,192 31 and 27)
+      const bool few = n_tokens < 768;
       // (a portion's last run may be partly filled: at most one per request beside the whole ones)
       const dim3 grid(n_tokens / (few ? 4 : 8) + n_requests, gb_div_up(hidden / 8, CONV_RUN_THREADS)), block(CONV_RUN_THREADS);
       auto kernel = K == 2 ? (few ? short_conv_run_kernel<2, 4> : short_conv_run_kernel<2, 8>)
