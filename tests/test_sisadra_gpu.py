@@ -614,12 +614,12 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
 @pytest.mark.parametrize("dim,kind,dtype,splits,bias", [(2048, 0, 1, 9, False), (2048, 1, 0, 16, True), (2044, 0, 1, 2, True), (1024, 0, 0, 0, False),
                                                         (132, 1, 1, 3, False), (128, 0, 1, 1, True), (4, 0, 0, 2, False)])
 def test_row_norm_of_few_rows_and_of_many_has_the_same_bits(dim, kind, dtype, splits, bias):
-    """The kernel with a block a row (below 64 rows) and the one with a warp a row, with sums of a product left to be added."""
+    """The kernel with a block a row (below 640 rows, and with sums of a product left to be added) and the one with a warp a row."""
     import ctypes
 
     from gibbs_b200.ops import _stream, device_status, hybrid
     torch.manual_seed(dim + splits)
-    dev, many = torch.device("cuda", torch.cuda.current_device()), 65
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 641
     x0, gain, add = torch.randn(many, dim, device=dev), torch.randn(dim, device=dev), torch.randn(dim, device=dev)
     pend = torch.randn(max(splits, 1), many, dim, device=dev)
 
@@ -646,9 +646,9 @@ def test_row_norm_of_few_rows_and_of_many_has_the_same_bits(dim, kind, dtype, sp
     # (a rounding of 2^-24 of what is in hand for every split and the bias)
     size = x0.abs() + pend[:splits].abs().sum(0) + add.abs()
     assert ((whole_x.double() - want).abs() <= (splits + 1) * 2.0 ** -24 * size.double()).all()
-    for n in (1, 2, 63):
+    for n in (1, 2, 639):
         x, out = run(n)
         assert torch.equal(x, whole_x[:n]) and torch.equal(out, whole[:n]), n
     if not splits:
-        rows = torch.tensor([64, 0, 7], dtype=torch.int32, device=dev)
+        rows = torch.tensor([640, 0, 7], dtype=torch.int32, device=dev)
         assert torch.equal(run(many, rows)[1], whole[rows.long()])
