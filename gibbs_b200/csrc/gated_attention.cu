@@ -378,8 +378,9 @@ sink_attention_kernel(const TQ* q, long long ldq, const TC* k_pages, const TC* v
 // One column of a (token, head)'s chunks: factor[s] * w[s][dv] over the chunks in order, sixteen requested at a time.
 // A chunk without keys (a negative factor) left no sum and is not read; one whose factor has become 0 is added all the same.
 template <bool WEIGHTED>
-__device__ __forceinline__ float sa_add_chunks(const float* w, size_t ld, int splits, const float* factor, int s0 = 0, float a = 0.f) {
-  for (; s0 < splits; s0 += 16) {
+__device__ __forceinline__ float sa_add_chunks(const float* w, size_t ld, int splits, const float* factor) {
+  float a = 0.f;
+  for (int s0 = 0; s0 < splits; s0 += 16) {
     float v[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) v[u] = s0 + u < splits && (!WEIGHTED || !(factor[s0 + u] < 0.f)) ? ldcg_now(w + (s0 + u) * ld) : 0.f;
@@ -395,15 +396,12 @@ __device__ __forceinline__ float sa_add_chunks(const float* w, size_t ld, int sp
 
 // One block per (token, head): the chunks' partial results (maximum, sum of weights, weighted sum), merged in
 // chunk order; the sink joins as a chunk of maximum 0, weight 1 and no values.  The chunks' factors are worked
-// out once in shared memory (2 x splits floats), then every thread has columns of its own; its first column's values of the first
-// SA_AHEAD chunks are asked for beside the maxima (a chunk without keys left no sum: what is read there is not used).  Bound by
-// the trip to L2.  Measured in decode steps of two tokens: 6.0 us a launch with 2 x 16 heads of 128 columns (25 with a warp per
+// out once in shared memory (2 x splits floats), then every thread has columns of its own.  Bound by the trips to
+// L2.  Measured in decode steps of two tokens: 6.0 us a launch with 2 x 16 heads of 128 columns (25 with a warp per
 // (token, head) that took one chunk after the other and its exponential again for every column), 4.8 with 32 heads of
 // 64 columns (7.8).
-constexpr int SA_AHEAD = 16;
-
 template <typename TO>
-__global__ void __launch_bounds__(256, 4) sink_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate, TO* out,
+__global__ void sink_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate, TO* out,
                                             long long ldo, int H, int vdim, int sink,
                                             const float* __restrict__ sink_scores, int maps) {
   extern __shared__ float chunk_factor[];                  // [splits] factors, [splits] sums of weights
@@ -414,22 +412,9 @@ __global__ void __launch_bounds__(256, 4) sink_attention_merge_kernel(const floa
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
   const size_t ld = (size_t)vdim + 2;
   const float* w = ws + (size_t)idx * splits * ld;
-  float z = sa_sink_score(sink_scores, h / maps);
-  gb_pin(z);
+  const float z = sa_sink_score(sink_scores, h / maps);
   pdl_wait();
-  const int mine = threadIdx.x;
-  const float m0 = mine < splits ? ldcg_now(w + (size_t)mine * ld) : 0.f, l0 = mine < splits ? ldcg_now(w + (size_t)mine * ld + 1) : 0.f;
-  const float gl = gate && mine < vdim ? ldcg_now(gate + (size_t)t * ld_gate + (size_t)h * vdim + mine) : 0.f;
-  float first[SA_AHEAD];
-  const float* at = w + 2 + mine;
-  const int ahead = mine < vdim ? splits : 0;
-#pragma unroll
-  for (int u = 0; u < SA_AHEAD; ++u, at += ld) first[u] = u < ahead ? ldcg_now(at) : 0.f;
-  if (mine < splits) {
-    chunk_factor[mine] = m0;
-    chunk_sum[mine] = l0;
-  }
-  for (int s = mine + blockDim.x; s < splits; s += blockDim.x) {
+  for (int s = threadIdx.x; s < splits; s += blockDim.x) {
     chunk_factor[s] = w[(size_t)s * ld];
     chunk_sum[s] = w[(size_t)s * ld + 1];
   }
@@ -444,21 +429,12 @@ __global__ void __launch_bounds__(256, 4) sink_attention_merge_kernel(const floa
   }
   __syncthreads();
   float L = sa_sink_weight(M, sink, z);
-#pragma unroll 8
   for (int s = 0; s < splits; ++s)
     if (!(chunk_factor[s] < 0.f)) L = fmaf(chunk_factor[s], chunk_sum[s], L);
   const float inv = 1.0f / L;
   for (int dv = threadIdx.x; dv < vdim; dv += blockDim.x) {
-    float a = 0.f;
-    int s0 = 0;
-    if (dv == mine) {
-#pragma unroll
-      for (int u = 0; u < SA_AHEAD; ++u)
-        if (u < splits && !(chunk_factor[u] < 0.f)) a = fmaf(chunk_factor[u], first[u], a);
-      s0 = SA_AHEAD;
-    }
-    if (s0 < splits) a = sa_add_chunks<true>(w + 2 + dv, ld, splits, chunk_factor, s0, a);
-    const float gt = gate ? hy_sigmoid(dv == mine ? gl : gate[(size_t)t * ld_gate + (size_t)h * vdim + dv]) : 1.f;
+    const float a = sa_add_chunks<true>(w + 2 + dv, ld, splits, chunk_factor);
+    const float gt = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + (size_t)h * vdim + dv]) : 1.f;
     out[(size_t)t * ldo + (size_t)h * vdim + dv] = from_f32<TO>(a * inv * gt);
   }
 }

@@ -548,70 +548,46 @@ latent_attention_kernel(const float* qp, const TC* pages, const int* block_table
 }
 
 // One block per (token, head): the chunks' partial results, merged in chunk order.  The chunks' weights
-// exp(m_s - M) are worked out once into shared memory.  Every thread asks for its first column of the first LM_AHEAD chunks
-// beside the maxima (a chunk without keys left no sum: what is read there is not used), for later ones sixteen at a time.  Bound
-// by the trip to L2.  Measured, 2 tokens x 16 heads,
+// exp(m_s - M) are worked out once into shared memory; then every thread has its columns and asks for
+// sixteen chunks' values at a time.  Bound by the trips to L2 (weights, then sums).  Measured, 2 tokens x 16 heads,
 // 32 chunks of 512: 6 us in a decode step, 37 to 40 with a warp per (token, head) that took one chunk after the other.
 constexpr int LM_CHUNKS = 96;                              // (the cuts give 64 at most, and with a window up to three more)
-constexpr int LM_AHEAD = 32;
 
-__global__ void __launch_bounds__(512, 2) latent_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate,
+__global__ void latent_attention_merge_kernel(const float* ws, int splits, const float* gate, long long ld_gate,
                                               float* out, long long ldo, int H, int r, const float* __restrict__ sink) {
-  __shared__ __align__(16) float es[LM_CHUNKS], els[LM_CHUNKS];
+  __shared__ float es[LM_CHUNKS];
   pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long idx = blockIdx.x;
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
   const size_t ld = (size_t)r + 2;
   const float* w = ws + (size_t)idx * splits * ld;
-  float z = sink ? sink[h] : 0.f;
-  gb_pin(z);
-  pdl_wait();
-  // (every warp takes the maxima for itself: lane s has chunks s, s + 32 and s + 64)
+  // (every warp takes the maxima and denominators for itself: lane s has chunks s, s + 32 and s + 64)
   float m[LM_CHUNKS / 32], l[LM_CHUNKS / 32], M = -INFINITY;
 #pragma unroll
   for (int i = 0; i < LM_CHUNKS / 32; ++i) {
     const int s = lane + 32 * i;
-    m[i] = s < splits ? ldcg_now(w + s * ld) : -INFINITY;
-    l[i] = s < splits ? ldcg_now(w + s * ld + 1) : 0.f;
+    m[i] = s < splits ? w[s * ld] : -INFINITY;
+    l[i] = s < splits ? w[s * ld + 1] : 0.f;
+    M = fmaxf(M, m[i]);
   }
-  const float gl = gate ? ldcg_now(gate + (size_t)t * ld_gate + h) : 0.f;
-  float first[LM_AHEAD];
-  const float* at = w + 2 + threadIdx.x;
-  const int ahead = (int)threadIdx.x < r ? splits : 0;
-#pragma unroll
-  for (int u = 0; u < LM_AHEAD; ++u, at += ld) first[u] = u < ahead ? ldcg_now(at) : 0.f;
-#pragma unroll
-  for (int i = 0; i < LM_CHUNKS / 32; ++i) M = fmaxf(M, m[i]);
   M = warp_max(M);
-  if (sink) M = fmaxf(M, z);
-  if (threadIdx.x < 32) {
+  if (sink) M = fmaxf(M, sink[h]);
+  float L = sink ? expf(sink[h] - M) : 0.f;
 #pragma unroll
-    for (int i = 0; i < LM_CHUNKS / 32; ++i) {
-      const float e = m[i] > -INFINITY ? expf(m[i] - M) : 0.f;
-      es[lane + 32 * i] = e;
-      els[lane + 32 * i] = e * l[i];
-    }
+  for (int i = 0; i < LM_CHUNKS / 32; ++i) {
+    const float e = m[i] > -INFINITY ? expf(m[i] - M) : 0.f, el = e * l[i];
+    for (int s = 32 * i; s < splits && s < 32 * i + 32; ++s) L += __shfl_sync(0xffffffffu, el, s & 31);      // in chunk order
+    if (threadIdx.x < 32) es[lane + 32 * i] = e;
   }
   __syncthreads();
-  float L = sink ? expf(z - M) : 0.f;
-  for (int s = 0; s < splits; s += 4) {                    // in chunk order (behind the last chunk: zeros)
-    const float4 e4 = *reinterpret_cast<const float4*>(els + s);
-    L = ((L + e4.x) + e4.y) + e4.z + e4.w;
-  }
-  const float g = gate ? hy_sigmoid(gl) : 1.f;
+  const float g = gate ? hy_sigmoid(gate[(size_t)t * ld_gate + h]) : 1.f;
   const float inv = g / L;
   float* dst = out + (size_t)t * ldo + (size_t)h * r;
   for (int d = threadIdx.x; d < r; d += blockDim.x) {
     float a = 0.f;
-    int s0 = 0;
-    if (d == (int)threadIdx.x) {
-#pragma unroll
-      for (int u = 0; u < LM_AHEAD; ++u)
-        if (es[u] != 0.f) a = fmaf(es[u], first[u], a);
-      s0 = LM_AHEAD;
-    }
-    for (; s0 < splits; s0 += 16) {
+    for (int s0 = 0; s0 < splits; s0 += 16) {
       float v[16];
 #pragma unroll
       for (int u = 0; u < 16; ++u) v[u] = s0 + u < splits && es[s0 + u] != 0.f ? ldcg_now(w + (s0 + u) * ld + 2 + d) : 0.f;
