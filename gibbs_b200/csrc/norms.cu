@@ -177,7 +177,7 @@ row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ ga
   }
 }
 
-// The same for few rows (a decode step): a block a row, a piece of four values a thread (dim <= 2048, a multiple of 4), the
+// The same for few rows (a decode step) and for rows with pending sums: a block a row, a piece of four values a thread (dim <= 2048, a multiple of 4), the
 // partial sums of all splits in one trip, the gain read before the wait.  The sums are added in the order of the kernel above
 // (a lane's pieces, then the lanes), so the bits are the same.
 // MANY (more rows with pending sums than blocks stay on the chip): the blocks walk the rows as in norm_add_block_kernel below.
@@ -339,6 +339,7 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
 }
 
 // The same for rows of up to 2,048 values in 16-byte pieces: a block a row, a piece a thread, the gains on hand before the wait.
+// (A decode step's product left its sum to a kernel of its own, 2.1 us, before the norm behind it, 3.0 us.)
 // y may come as the partial tiles [splits][rows][dim] of the product that makes it (+ its bias): they are asked for in one trip
 // and added in their order, as the product's own reduction would.  A row's sums are formed by the same threads in the same
 // order whatever the number of rows.
