@@ -180,16 +180,15 @@ row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ ga
 // The same for few rows (a decode step) and for rows with pending sums: a block a row, a piece of four values a thread (dim <= 2048, a multiple of 4), the
 // partial sums of all splits in one trip, the gain read before the wait.  The sums are added in the order of the kernel above
 // (a lane's pieces, then the lanes), so the bits are the same.
-// MANY (more rows with pending sums than blocks stay on the chip): the blocks walk the rows as in norm_add_block_kernel below.
-template <typename TO, bool MANY>
-__global__ void __launch_bounds__(512, MANY ? 3 : 4)
+template <typename TO>
+__global__ void __launch_bounds__(512)
 row_norm_block_kernel(const float* x, long long ldx, const float* __restrict__ gain, TO* out, const int* rows, int n_rows, int dim,
                       int kind, float eps, const float* pend, int pend_splits, const float* __restrict__ pend_bias) {
-  extern __shared__ __align__(16) float parts[];          // [splits, MANY: 2 x (splits + 1)][dim], then two rows of a number a thread
+  extern __shared__ __align__(16) float parts[];          // [splits][dim], then two rows of a number a thread
   pdl_trigger();
-  const int lane = threadIdx.x & 31, d = 4 * threadIdx.x;
+  const int r = blockIdx.x, lane = threadIdx.x & 31, d = 4 * threadIdx.x;
   const bool in = d < dim;
-  long long src = !MANY && rows ? rows[blockIdx.x] : blockIdx.x;
+  long long src = rows ? rows[r] : r;
   gb_pin(src);
   float* row = const_cast<float*>(x) + (size_t)src * ldx + d;
   float4 g = in ? *reinterpret_cast<const float4*>(gain + d) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -197,7 +196,23 @@ row_norm_block_kernel(const float* x, long long ldx, const float* __restrict__ g
   gb_pin(row);
   gb_pin(g);
   gb_pin(b);
-  float* sums = parts + (size_t)(MANY ? 2 * (pend_splits + 1) : pend_splits) * dim;
+  float* sums = parts + (size_t)pend_splits * dim;
+  pdl_wait();
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (in) {
+    const float* from = pend + (size_t)src * dim + d;
+    for (int u = 0; u < pend_splits; ++u) gb_cp_async_16(parts + (size_t)u * dim + d, from + (size_t)u * n_rows * dim);
+    v = ldcg_now(reinterpret_cast<const float4*>(row));
+    if (pend_splits > 0) {
+      gb_cp_async_wait_all();
+      for (int u = 0; u < pend_splits; ++u) {
+        const float4 q = *reinterpret_cast<const float4*>(parts + (size_t)u * dim + d);
+        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+      }
+      if (pend_bias) { v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+      *reinterpret_cast<float4*>(row) = v;
+    }
+  }
   // a row's sum: every lane its pieces in ascending order, then the lanes
   auto row_sum = [&](float mine, float* at) {
     at[threadIdx.x] = mine;
@@ -206,65 +221,21 @@ row_norm_block_kernel(const float* x, long long ldx, const float* __restrict__ g
     for (int i = lane; i < (int)blockDim.x; i += 32) s += at[i];
     return warp_sum(s);
   };
-  auto add_pending = [&](float4& v, const float* at) {
-    for (int u = 0; u < pend_splits; ++u) {
-      const float4 q = *reinterpret_cast<const float4*>(at + (size_t)u * dim + d);
-      v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-    }
-    if (pend_bias) { v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
-    *reinterpret_cast<float4*>(row) = v;
-  };
-  auto finish = [&](int r, float4 v) {
-    const float mean = kind == NORM_LAYER ? row_sum((v.x + v.y) + (v.z + v.w), sums) / (float)dim : 0.f;
-    const float a0 = v.x - mean, a1 = v.y - mean, a2 = v.z - mean, a3 = v.w - mean;
-    const float ss = row_sum(in ? (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3) : 0.f, sums + blockDim.x);
-    const float rstd = 1.0f / sqrtf(ss / (float)dim + eps);
-    if (!in) return;
-    TO* o = out + (size_t)r * dim + d;
-    const float r0 = a0 * rstd * g.x, r1 = a1 * rstd * g.y, r2 = a2 * rstd * g.z, r3 = a3 * rstd * g.w;
-    if constexpr (sizeof(TO) == 2) {
-      __nv_bfloat162 lo = __floats2bfloat162_rn(r0, r1), hi = __floats2bfloat162_rn(r2, r3);
-      uint2 w;
-      w.x = *reinterpret_cast<unsigned*>(&lo);
-      w.y = *reinterpret_cast<unsigned*>(&hi);
-      *reinterpret_cast<uint2*>(o) = w;
-    } else {
-      *reinterpret_cast<float4*>(o) = make_float4(r0, r1, r2, r3);
-    }
-  };
-  pdl_wait();
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if constexpr (MANY) {
-    auto ask = [&](int r, int turn) {
-      if (!in) return;
-      float* to = parts + (size_t)turn * (pend_splits + 1) * dim + d;
-      for (int u = 0; u < pend_splits; ++u) gb_cp_async_16(to + (size_t)u * dim, pend + ((size_t)u * n_rows + r) * dim + d);
-      gb_cp_async_16(to + (size_t)pend_splits * dim, x + (size_t)r * ldx + d);
-    };
-    ask(blockIdx.x, 0);
-    int turn = 0;
-    for (int r = blockIdx.x; r < n_rows; r += gridDim.x, turn ^= 1, row += (size_t)gridDim.x * ldx) {
-      gb_cp_async_wait_all();
-      if (in) {
-        const float* at = parts + (size_t)turn * (pend_splits + 1) * dim;
-        v = *reinterpret_cast<const float4*>(at + (size_t)pend_splits * dim + d);
-        add_pending(v, at);
-      }
-      if (r + (int)gridDim.x < n_rows) ask(r + gridDim.x, turn ^ 1);
-      finish(r, v);
-      __syncthreads();                                     // before the next row's sums land in the same place
-    }
+  const float mean = kind == NORM_LAYER ? row_sum((v.x + v.y) + (v.z + v.w), sums) / (float)dim : 0.f;
+  const float a0 = v.x - mean, a1 = v.y - mean, a2 = v.z - mean, a3 = v.w - mean;
+  const float ss = row_sum(in ? (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3) : 0.f, sums + blockDim.x);
+  const float rstd = 1.0f / sqrtf(ss / (float)dim + eps);
+  if (!in) return;
+  TO* o = out + (size_t)r * dim + d;
+  const float r0 = a0 * rstd * g.x, r1 = a1 * rstd * g.y, r2 = a2 * rstd * g.z, r3 = a3 * rstd * g.w;
+  if constexpr (sizeof(TO) == 2) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(r0, r1), hi = __floats2bfloat162_rn(r2, r3);
+    uint2 w;
+    w.x = *reinterpret_cast<unsigned*>(&lo);
+    w.y = *reinterpret_cast<unsigned*>(&hi);
+    *reinterpret_cast<uint2*>(o) = w;
   } else {
-    if (in) {
-      const float* from = pend + (size_t)src * dim + d;
-      for (int u = 0; u < pend_splits; ++u) gb_cp_async_16(parts + (size_t)u * dim + d, from + (size_t)u * n_rows * dim);
-      v = ldcg_now(reinterpret_cast<const float4*>(row));
-      if (pend_splits > 0) {
-        gb_cp_async_wait_all();
-        add_pending(v, parts);
-      }
-    }
-    finish(blockIdx.x, v);
+    *reinterpret_cast<float4*>(o) = make_float4(r0, r1, r2, r3);
   }
 }
 
@@ -343,15 +314,13 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
 // y may come as the partial tiles [splits][rows][dim] of the product that makes it (+ its bias): they are asked for in one trip
 // and added in their order, as the product's own reduction would.  A row's sums are formed by the same threads in the same
 // order whatever the number of rows.
-// MANY (more rows than blocks stay on the chip, y whole): the blocks walk the rows, the next row's copy to shared memory under way
-// while they meet at a row's barriers (two buffers; a thread reads what it copied itself) and the gains read once.
-template <bool MANY>
-__global__ void __launch_bounds__(512, 3)
+__global__ void __launch_bounds__(512)
 norm_add_block_kernel(float* x, long long ldx, const float* y, long long ldy, const float* __restrict__ gain, int dim, int kind, float eps,
                       bf16* copy, ThenNorm then, const float* part, int splits, long long split_stride,
-                      const float* __restrict__ part_bias, int n) {
-  extern __shared__ __align__(16) float tiles[];          // [splits, MANY: 2 x 2][dim], then four rows of a number a thread
+                      const float* __restrict__ part_bias) {
+  extern __shared__ __align__(16) float tiles[];          // [splits][dim], then four rows of a number a thread
   pdl_trigger();
+  const size_t r = blockIdx.x;
   const int lane = threadIdx.x & 31, d = 4 * threadIdx.x;
   const bool in = d < dim, second = then.gain != nullptr;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -361,7 +330,7 @@ norm_add_block_kernel(float* x, long long ldx, const float* y, long long ldy, co
   gb_pin(g1);
   gb_pin(g2);
   gb_pin(pb);
-  float* sums = tiles + (size_t)(MANY ? 4 : splits) * dim;
+  float* sums = tiles + (size_t)splits * dim;
   // a row's sum: every lane its pieces in ascending order, then the lanes
   auto row_sum = [&](float mine, int turn) {
     float* at = sums + turn * blockDim.x;
@@ -378,63 +347,39 @@ norm_add_block_kernel(float* x, long long ldx, const float* y, long long ldy, co
     const float rstd = 1.0f / sqrtf(ss / (float)dim + e);
     return make_float4(c.x * rstd * g.x, c.y * rstd * g.y, c.z * rstd * g.z, c.w * rstd * g.w);
   };
+  pdl_wait();
+  float4 v = zero, old = zero;
+  if (in) {
+    const float* from = part + r * dim + d;
+    for (int u = 0; u < splits; ++u) gb_cp_async_16(tiles + (size_t)u * dim + d, from + (size_t)u * split_stride);
+    old = ldcg_now(reinterpret_cast<const float4*>(x + r * ldx + d));
+    if (splits > 0) {
+      gb_cp_async_wait_all();
+      for (int u = 0; u < splits; ++u) {
+        const float4 q = *reinterpret_cast<const float4*>(tiles + (size_t)u * dim + d);
+        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+      }
+      if (part_bias) { v.x += pb.x; v.y += pb.y; v.z += pb.z; v.w += pb.w; }
+    } else {
+      v = ldcg_now(reinterpret_cast<const float4*>(y + r * ldy + d));
+    }
+  }
+  v = normed(v, kind, eps, g1, 0);
+  v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
   auto pack = [](float4 q) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(q.x, q.y), hi = __floats2bfloat162_rn(q.z, q.w);
     return make_uint2(*reinterpret_cast<unsigned*>(&lo), *reinterpret_cast<unsigned*>(&hi));
   };
-  auto finish = [&](size_t r, float4 old, float4 v) {
-    v = normed(v, kind, eps, g1, 0);
-    v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
-    if (in) {
-      *reinterpret_cast<float4*>(x + r * ldx + d) = v;
-      if (copy) *reinterpret_cast<uint2*>(copy + r * dim + d) = pack(v);
-    }
-    if (!second) return;
-    if (!in) v = zero;
-    v = normed(v, then.kind, then.eps, g2, 2);
-    if (!in) return;
-    if (then.out_dtype == GB_BF16) *reinterpret_cast<uint2*>((bf16*)then.out + r * dim + d) = pack(v);
-    else *reinterpret_cast<float4*>((float*)then.out + r * dim + d) = v;
-  };
-  pdl_wait();
-  float4 v = zero, old = zero;
-  if constexpr (MANY) {
-    auto ask = [&](int r, int b) {
-      if (!in) return;
-      gb_cp_async_16(tiles + (size_t)(2 * b) * dim + d, x + (size_t)r * ldx + d);
-      gb_cp_async_16(tiles + (size_t)(2 * b + 1) * dim + d, y + (size_t)r * ldy + d);
-    };
-    ask(blockIdx.x, 0);
-    int b = 0;
-    for (int r = blockIdx.x; r < n; r += gridDim.x, b ^= 1) {
-      gb_cp_async_wait_all();
-      if (in) {
-        old = *reinterpret_cast<const float4*>(tiles + (size_t)(2 * b) * dim + d);
-        v = *reinterpret_cast<const float4*>(tiles + (size_t)(2 * b + 1) * dim + d);
-      }
-      if (r + (int)gridDim.x < n) ask(r + gridDim.x, b ^ 1);
-      finish(r, old, v);
-      __syncthreads();                                     // before the next row's sums land in the same place
-    }
-  } else {
-    const size_t r = blockIdx.x;
-    if (in) {
-      const float* from = part + r * dim + d;
-      for (int u = 0; u < splits; ++u) gb_cp_async_16(tiles + (size_t)u * dim + d, from + (size_t)u * split_stride);
-      old = ldcg_now(reinterpret_cast<const float4*>(x + r * ldx + d));
-      if (splits > 0) {
-        gb_cp_async_wait_all();
-        for (int u = 0; u < splits; ++u) {
-          const float4 q = *reinterpret_cast<const float4*>(tiles + (size_t)u * dim + d);
-          v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-        }
-        if (part_bias) { v.x += pb.x; v.y += pb.y; v.z += pb.z; v.w += pb.w; }
-      } else {
-        v = ldcg_now(reinterpret_cast<const float4*>(y + r * ldy + d));
-      }
-    }
-    finish(r, old, v);
+  if (in) {
+    *reinterpret_cast<float4*>(x + r * ldx + d) = v;
+    if (copy) *reinterpret_cast<uint2*>(copy + r * dim + d) = pack(v);
   }
+  if (!second) return;
+  if (!in) v = zero;
+  v = normed(v, then.kind, then.eps, g2, 2);
+  if (!in) return;
+  if (then.out_dtype == GB_BF16) *reinterpret_cast<uint2*>((bf16*)then.out + r * dim + d) = pack(v);
+  else *reinterpret_cast<float4*>((float*)then.out + r * dim + d) = v;
 }
 
 // y = the partial tiles' sum (+ bias), for rows that the kernel above does not take
@@ -915,21 +860,17 @@ GB_OP(gb_op_row_norm) {
   // (rows that bring pending sums at any number: a warp a row asks for its pieces' sums one after the other)
   if (by_warps && (n < NORM_FEW_ROWS || pend != nullptr) && block_smem <= 160 * 1024) {
     // (whole warps; a thread without a piece adds zeros)
-    const int threads = 32 * gb_div_up(dim, 128), places = 148 * (1536 / threads), splits = pend != nullptr ? ctx->pend_splits : 0;
-    const size_t many_smem = sizeof(float) * (2 * (size_t)(splits + 1) * dim + 2 * threads);
-    const bool many = splits > 0 && n > places && many_smem <= 72 * 1024;
+    const dim3 block(32 * gb_div_up(dim, 128));
 #define BLOCK_NORM(TO)                                                                                                     \
     do {                                                                                                                  \
       static bool raised = false;                                                                                         \
       if (!raised) {                                                                                                      \
-        GB_CUDA(cudaFuncSetAttribute(row_norm_block_kernel<TO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); \
-        GB_CUDA(cudaFuncSetAttribute(row_norm_block_kernel<TO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024)); \
+        GB_CUDA(cudaFuncSetAttribute(row_norm_block_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); \
         raised = true;                                                                                                    \
       }                                                                                                                   \
-      gb_launch(many ? row_norm_block_kernel<TO, true> : row_norm_block_kernel<TO, false>, dim3(many ? places : n),        \
-                dim3(threads), many ? many_smem : block_smem, ctx->stream, op_ptr<const float>(a[0]), a[1],               \
+      gb_launch(row_norm_block_kernel<TO>, dim3(n), block, block_smem, ctx->stream, op_ptr<const float>(a[0]), a[1],      \
                 op_ptr<const float>(a[2]), op_ptr<TO>(a[3]), op_ptr<const int>(a[5]), n, dim, kind, (float)f[0], pend,    \
-                splits, pend != nullptr ? ctx->pend_bias : nullptr);                                                      \
+                pend != nullptr ? ctx->pend_splits : 0, pend != nullptr ? ctx->pend_bias : nullptr);                      \
     } while (0)
     if (a[4] == GB_BF16) BLOCK_NORM(bf16); else BLOCK_NORM(float);
 #undef BLOCK_NORM
@@ -990,15 +931,12 @@ GB_OP(gb_op_norm_add) {
       (part == nullptr || ((uintptr_t)ctx->part_bias & 15) == 0) && smem <= 160 * 1024) {
     static bool raised = false;
     if (!raised) {
-      GB_CUDA(cudaFuncSetAttribute(norm_add_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+      GB_CUDA(cudaFuncSetAttribute(norm_add_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
       raised = true;
     }
-    const int threads = 32 * gb_div_up(dim, 128), places = 148 * (1536 / threads);
-    const bool many = splits == 0 && n > places;
-    gb_launch(many ? norm_add_block_kernel<true> : norm_add_block_kernel<false>, dim3(many ? places : n), dim3(threads),
-              many ? sizeof(float) * 4 * (size_t)(dim + threads) : smem, ctx->stream, op_ptr<float>(a[0]), a[1],
+    gb_launch(norm_add_block_kernel, dim3(n), dim3(32 * gb_div_up(dim, 128)), smem, ctx->stream, op_ptr<float>(a[0]), a[1],
               op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]), then, part, splits,
-              (long long)n * dim, part != nullptr ? ctx->part_bias : nullptr, n);
+              (long long)n * dim, part != nullptr ? ctx->part_bias : nullptr);
     GB_CHECK_LAUNCH("norm_add (a block a row)");
     return 1;
   }
