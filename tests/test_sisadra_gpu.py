@@ -612,7 +612,8 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
 
 
 @pytest.mark.parametrize("dim,kind,dtype,splits,bias", [(2048, 0, 1, 9, False), (2048, 1, 0, 16, True), (2044, 0, 1, 2, True), (1024, 0, 0, 0, False),
-                                                        (132, 1, 1, 3, False), (128, 0, 1, 1, True), (4, 0, 0, 2, False)])
+                                                        (132, 1, 1, 3, False), (128, 0, 1, 1, True), (4, 0, 0, 2, False),
+                                                        (2048, 0, 1, 1, True), (2048, 1, 0, 3, False), (1540, 0, 1, 2, False)])
 def test_row_norm_of_few_rows_and_of_many_has_the_same_bits(dim, kind, dtype, splits, bias):
     """The kernel with a block a row (below 640 rows, and with sums of a product left to be added) and the one with a warp a row."""
     import ctypes
@@ -652,3 +653,52 @@ def test_row_norm_of_few_rows_and_of_many_has_the_same_bits(dim, kind, dtype, sp
     if not splits:
         rows = torch.tensor([640, 0, 7], dtype=torch.int32, device=dev)
         assert torch.equal(run(many, rows)[1], whole[rows.long()])
+
+
+@pytest.mark.parametrize("d,kind,second,splits,bias", [(2048, 1, True, 3, True), (2048, 0, False, 1, False), (2048, 1, False, 0, False), (2044, 0, True, 16, False),
+                                                       (132, 1, True, 2, True)])
+def test_norm_behind_a_sublayer_from_partial_tiles(d, kind, second, splits, bias):
+    """y whole, and as the partial tiles of its product, in steps of few rows and of many: the same bits (the tiles are added in
+    their order), and against 64 bits."""
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(d + splits)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 900
+    x0, gain, then, add = (torch.randn(*k, device=dev) for k in ((many, d), (d,), (d,), (d,)))
+    part = torch.randn(max(splits, 1), many, d, device=dev)
+    y0 = part[0].clone()
+    for u in range(1, splits):
+        y0 += part[u]
+    if bias:
+        y0 += add
+
+    def run(n, tiles):
+        x, y, parts = x0[:n].clone(), y0[:n].clone(), part[:, :n].contiguous()
+        h, copy = torch.zeros(n, d, device=dev, dtype=torch.bfloat16), torch.zeros(n, d, device=dev, dtype=torch.bfloat16)
+        if tiles:
+            y.fill_(float("nan"))
+        stream = _stream()
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), None, 0, None, 0, None, 0, None,
+                          parts.data_ptr() if tiles else None, splits if tiles else 0, add.data_ptr() if tiles and bias else None)
+        a = (ctypes.c_longlong * 24)(x.data_ptr(), d, y.data_ptr(), d, gain.data_ptr(), n, d, kind, copy.data_ptr(), then.data_ptr() if second else 0,
+                                     h.data_ptr() if second else 0, 1, kind)
+        assert hybrid._function("norm_add")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(1e-5, 1e-5), ctypes.c_int(hybrid.TAKES_PARTIALS if tiles else 0)) == 1
+        torch.cuda.synchronize()
+        assert torch.equal(copy, x.bfloat16())
+        return x, h
+
+    whole = run(many, False)
+    for n in (1, 444, 445, many):
+        for tiles in ((False, True) if splits else (False,)):
+            got = run(n, tiles)
+            assert torch.equal(got[0], whole[0][:n]) and torch.equal(got[1], whole[1][:n]), (n, tiles)
+
+    def norm(v, g):
+        v = v.double() - (v.double().mean(1, keepdim=True) if kind == 0 else 0.0)
+        return v / (v.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * g.double()
+    new = x0.double() + norm(y0, gain)
+    assert ((whole[0].double() - new).norm(dim=1) / new.norm(dim=1)).max() < 1e-6
+    if second:                                               # (half a place of bfloat16, 2^-8 of the value at most, and the 32-bit error)
+        want = norm(new, then)
+        assert ((whole[1].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
