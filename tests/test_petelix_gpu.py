@@ -469,7 +469,7 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     assert len(generated) == 5 and generated[0] == top["ids"][0]
 
 
-# launches of more than 296 tiles of 64 rows: windows within a key tile and across tiles, groups that do not divide 128, pages of 8 to
+# launches of 48 tiles of 64 rows (the smallest on tcgen05) and of many: windows within a key tile and across tiles, groups that do not divide 128, pages of 8 to
 # 64, a single token beside portions, two maps, the edges of 64 keys, blocks of positions, no softmax
 @pytest.mark.parametrize("heads,kvh,maps,vdim,ps,window,cap,sink,gate,sig,starts,lens,blocked", [
     (16, 4, 1, 64, 16, 0, 30.0, True, True, False, [0, 63], [1000, 230], False),
@@ -481,6 +481,8 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     (8, 8, 1, 64, 16, 40, 5.0, False, True, True, [0], [2500], False),
     (16, 4, 2, 128, 16, 100, 0.0, False, False, False, [150, 0], [500, 230], True), (32, 8, 1, 64, 16, 64, 20.0, True, True, False, [37], [700], True),
     (16, 4, 2, 128, 32, 1024, 0.0, False, False, False, [0, 1000], [300, 377], True),
+    (16, 4, 1, 64, 16, 0, 30.0, True, True, False, [0], [176], False), (32, 8, 1, 128, 16, 0, 0.0, False, False, False, [0, 0], [65, 1], False),
+    (8, 8, 1, 64, 16, 0, 0.0, False, False, True, [70], [321], False),
 ])
 def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
     from gibbs_b200.ops import hybrid
