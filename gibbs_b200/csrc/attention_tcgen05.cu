@@ -611,28 +611,33 @@ bool pages_map(CUtensorMap* out, const void* pages, long long rows, int hd, int 
   return true;
 }
 
-// CTAs that share a row tile's keys: as many as stay on the chip at two an SM.  Passes of 16 requests in portions of 512 tokens
-// (96 row tiles over contexts of up to 2,048), ms with 1, 2, 3 and 4 shares: 66.3, 65.1, 65.0, 65.7 (a layer's attention 37 -> 32
-// us); one prompt of 2,048 tokens (512 row tiles): 4.57, 4.64, 4.67, 4.74.  GIBBS_B200_ATTN_PARTS=1..4 overrides.
-int key_parts(long long ctas) {
+// CTAs that share a row tile's keys: none unless the longest context a row sees makes a share of MIN_PART_TILES key tiles for
+// two, and never more than the SMs hold at a time (`slots`): a second round of CTAs costs more than the shares give.  us without
+// shares and with them, 32 / 8 heads of 64: 100 tokens behind 8,000 keys 103 and 37, 20 behind 1,500 22.8 and 11.6; where two shares
+// would not fit, 1,000 tokens 22.2 and 27.9, 15 single tokens beside a portion of 500 28.9 and 36.6; heads of 128 on 128-key tiles (one
+// CTA an SM), 700 tokens 19.0 and 32.5; contexts too short for shares, eight portions of 100 tokens 12.8 and 20.6.
+// The shares, so the order in which a row's keys are added, depend on the number of tiles in the launch.  GIBBS_B200_ATTN_PARTS=1..4
+// overrides.
+int key_parts(long long ctas, long long slots, long long key_tiles) {
   static const int forced = [] {
     const char* e = getenv("GIBBS_B200_ATTN_PARTS");
     return e ? atoi(e) : 0;
   }();
   if (forced >= 1 && forced <= MAX_PARTS) return forced;
-  return ctas <= 74 ? 4 : (ctas <= 296 ? 2 : 1);
+  if (key_tiles < 2 * MIN_PART_TILES) return 1;
+  return 4 * ctas <= slots ? 4 : (2 * ctas <= slots ? 2 : 1);
 }
 
 template <int HD, int KEYS>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, int n_tiles,
-           cudaStream_t stream) {
+           long long max_keys, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
     GB_CUDA(cudaFuncSetAttribute(attention_tcgen05_kernel<HD, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg<HD, KEYS>::SMEM_BYTES));
     attr_set = true;
   }
-  const int parts = key_parts((long long)n_tiles * p.kv_heads);
+  const int parts = key_parts((long long)n_tiles * p.kv_heads, 148ll * Cfg<HD, KEYS>::CTAS, (max_keys + KEYS - 1) / KEYS);
   if (parts == 1) {
     gb_launch(attention_tcgen05_kernel<HD, KEYS>, dim3(p.kv_heads, n_tiles), dim3(192), Cfg<HD, KEYS>::SMEM_BYTES, stream,
               mq, mk, mv, p);
@@ -686,11 +691,12 @@ GB_API int gb_attention_tcgen05_supported(int heads, int kv_heads, int hd, int p
 
 // The arguments of gb_attention_tc (attention_tc.cu) without splits: q [n_tokens, heads*hd] bf16 with row
 // stride ldq, pages [n_pages, kv_heads, page_size, hd] bf16, out [n_tokens, heads*hd] bf16 with row stride ldo.
+// max_ctx: the longest context after the step (an upper bound), which only decides how many CTAs share a row tile's keys.
 // Returns the number of kernels launched, or a negative error code.
 GB_API int gb_attention_tcgen05(const void* q, long long ldq, const void* k_pages, const void* v_pages,
                                 const int* block_table, int bt_stride, int page_size, int n_pages, const int* q_start,
                                 const int* q_len, const int* start_pos, void* out, long long ldo, int n_requests,
-                                int n_tokens, int heads, int kv_heads, int hd, float scale, int window, int* status,
+                                int n_tokens, int heads, int kv_heads, int hd, float scale, int window, int max_ctx, int* status,
                                 cudaStream_t stream) {
   if (n_tokens <= 0 || n_requests <= 0) return 0;
   if (!gb_attention_tcgen05_supported(heads, kv_heads, hd, page_size, ldq, ldo))
@@ -720,11 +726,13 @@ GB_API int gb_attention_tcgen05(const void* q, long long ldq, const void* k_page
   // upper bound of the number of tiles: sum_r ceil(q_len_r / tpt) <= n_tokens / tpt + n_requests
   const long long n_tiles = ((long long)n_tokens + tpt - 1) / tpt + n_requests;
   if (n_tiles > 65535) GB_FAIL(GB_ERR_ARG, "gb_attention_tcgen05: %lld tiles in one launch", n_tiles);
+  // the keys that a tile of `tpt` tokens walks at most
+  const long long max_keys = window > 0 && window + tpt - 1 < max_ctx ? window + tpt - 1 : max_ctx;
   int rc;
   if (keys_per_tile(hd, page_size, n_tiles * kv_heads) == 64)
-    rc = hd == 64 ? launch<64, 64>(mq, mk, mv, p, (int)n_tiles, stream) : launch<128, 64>(mq, mk, mv, p, (int)n_tiles, stream);
+    rc = hd == 64 ? launch<64, 64>(mq, mk, mv, p, (int)n_tiles, max_keys, stream) : launch<128, 64>(mq, mk, mv, p, (int)n_tiles, max_keys, stream);
   else
-    rc = hd == 64 ? launch<64, 128>(mq, mk, mv, p, (int)n_tiles, stream) : launch<128, 128>(mq, mk, mv, p, (int)n_tiles, stream);
+    rc = hd == 64 ? launch<64, 128>(mq, mk, mv, p, (int)n_tiles, max_keys, stream) : launch<128, 128>(mq, mk, mv, p, (int)n_tiles, max_keys, stream);
   if (rc != GB_OK) return rc;
   GB_CHECK_LAUNCH("gb_attention_tcgen05");
   return 1;

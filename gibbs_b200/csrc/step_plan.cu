@@ -57,7 +57,7 @@ typedef int (*AttentionTcFn)(const void*, long long, const void*, const void*, c
                              float*, int*, cudaStream_t);
 typedef int (*AttentionTcgen05Fn)(const void*, long long, const void*, const void*, const int*, int, int, int,
                                   const int*, const int*, const int*, void*, long long, int, int, int, int, int, float,
-                                  int, int*, cudaStream_t);
+                                  int, int, int*, cudaStream_t);
 typedef int (*AttentionTcgen05SupportedFn)(int, int, int, int, long long, long long);
 typedef int (*SwigluFn)(const void*, void*, int, int, int, cudaStream_t);
 typedef int (*LinearDecodeFn)(const void*, long long, int, const float*, float, const int*, const float*, int,
@@ -342,8 +342,8 @@ int run_op(Walk& w, const PlanOp& o, bool force = false) {
         PLAN_CALL(w, F_ATTENTION_TCGEN05, ((AttentionTcgen05Fn)g_fn[F_ATTENTION_TCGEN05])(
             w.q, w.ldq, ptr<const void>(w, a[2]), ptr<const void>(w, a[3]), bt, (int)val(w, a[12]), page_size, (int)a[6],
             ptr<const int>(w, SYM_BIT | S_Q_START), ptr<const int>(w, SYM_BIT | S_Q_LEN),
-            ptr<const int>(w, SYM_BIT | S_START_POS), out, a[1], R, N, heads, kvh, hd, scale, (int)a[10], w.status,
-            w.stream));
+            ptr<const int>(w, SYM_BIT | S_START_POS), out, a[1], R, N, heads, kvh, hd, scale, (int)a[10],
+            (int)w.sym[S_MAXCTX], w.status, w.stream));
         return 0;
       }
       const int splits = small ? attention_splits(w, R, kvh, (int)w.sym[S_MAXCTX]) : 1;

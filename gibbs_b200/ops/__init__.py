@@ -749,7 +749,7 @@ def _attention_tc(q, heads, kv_heads, head_dim, k_pages, v_pages, block_table, s
             _c_int(block_table.shape[1]), _c_int(k_pages.shape[2]), _c_int(k_pages.shape[0]), _ptr(step.q_start),
             _ptr(step.q_len), _ptr(step.start_pos), _ptr(out), _c_ll(_rows(out, "out")), _c_int(step.n_requests),
             _c_int(n), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_float(scale), _c_int(window or 0),
-            _ptr(status), _stream())
+            _c_int(step.max_ctx_len), _ptr(status), _stream())
         if rc < 0:
             check(lib, rc)
         _launched(rc)
