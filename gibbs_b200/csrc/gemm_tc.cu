@@ -540,7 +540,7 @@ struct PairCfg {
   // tensor-memory loads, shared memory and stores on one warp a scheduler, and the last tile's is waited for.
   static constexpr int GROUPS = 2;
   static constexpr int THREADS = 64 + GROUPS * 128;
-  static constexpr int STAGING_BYTES = 16 * 1024;        // of a group: 32 token rows in 32-bit, or 64 in bfloat16
+  static constexpr int STAGING_BYTES = 16 * 1024;        // of a group: 32 token rows in 32-bit
   static constexpr int TMEM_COLS = 512;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + GROUPS * STAGING_BYTES + 1024;
 };
@@ -778,25 +778,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           }
           group_barrier(eg);
         } else if (hc > 0 && fast && p.mode == OUT_BF16) {
-          bf16* ob = reinterpret_cast<bf16*>(staging);
+          // Neighbouring lanes (weight rows n, n + 1) swap every other token's value, so that a lane stores two rows of one token: a
+          // store of a warp is two whole sectors of two tokens' rows, and nothing goes through shared memory, whose bandwidth the
+          // operands need.  us through shared memory with one group of epilogue warps, with two, and so: 8,000 x 8,192 x 1,024
+          // 109, 130, 108; 2,695 x 13,824 x 1,536 88, 97, 86; 8,000 x 6,144 x 2,048 140, 144, 138; 512 x 6,144 x 2,048 18.5, 21.5, 19.2.
+          const bool odd = lane & 1;
+          bf16* dst = (bf16*)p.out + (size_t)(m0 + h0 + odd) * p.ldo + (n & ~1);
 #pragma unroll 1
           for (int c0 = 0; c0 < hc; c0 += 32) {
             float v[32];
             tmem_ld_32(acc + (uint32_t)(h0 + c0), v);
+            if (last && c0 + 32 >= hc) {
+              tc_fence_before();
+              group_barrier(eg);
+              if (et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
+            }
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (c0 + j < hc) ob[(c0 + j) * BM + row] = __float2bfloat16_rn(apply_act(p.act, v[j] + b));
+            for (int j = 0; j < 32; ++j) v[j] += b;
+            if (p.act != ACT_NONE) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = apply_act(p.act, v[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+              const __nv_bfloat162 q2 = odd ? __floats2bfloat162_rn(other, v[j + 1]) : __floats2bfloat162_rn(v[j], other);
+              if (c0 + j + odd < hc) *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)(c0 + j) * p.ldo) = q2;
+            }
           }
-          tc_fence_before();
-          group_barrier(eg);
-          if (last && et == 0) mbar_arrive_leader(&tmem_empty_bar[a]);
-          bf16* dst = (bf16*)p.out + (size_t)(m0 + h0) * p.ldo + n0;
-          for (int idx = et; idx < hc * 16; idx += 128) {
-            const int mm = idx >> 4, piece = idx & 15;
-            *reinterpret_cast<uint4*>(dst + (size_t)mm * p.ldo + piece * 8) =
-                *reinterpret_cast<const uint4*>(ob + mm * BM + piece * 8);
-          }
-          group_barrier(eg);
         } else if (hc > 0 && fast && p.mode == OUT_F32) {
           // A plain 32-bit store needs no staging: a lane is a weight row, so one store of a warp
           // is 128 contiguous bytes of one token's row, a whole line.

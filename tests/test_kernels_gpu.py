@@ -126,6 +126,28 @@ def test_linear_tensor_cores(m, n, k):
     assert int(ops.device_status(DEV).item()) == 0
 
 
+# tiles of CTA pairs whose last rows are few, odd and none for one of the groups that store them; a function of the sums, a bias
+@pytest.mark.parametrize("m,n,k,act,use_bias", [(193, 8192, 64, "", False), (1281, 2048, 72, "", True), (2049, 2048, 200, "relu2", True),
+                                                (350, 4096, 1024, "gelu", False), (777, 2304, 64, "", True)])
+def test_bfloat16_products_of_many_rows_are_the_rounded_32_bit_ones(m, n, k, act, use_bias):
+    from gibbs_b200 import ops
+    torch.manual_seed(m + n)
+    a, w = torch.randn(m, k, device=DEV).bfloat16(), (torch.randn(n, k, device=DEV) / math.sqrt(k)).bfloat16()
+    bias = torch.randn(n, device=DEV) if use_bias else None
+    whole = torch.empty(m, n, device=DEV)
+    ops.linear_tc(a, w, bias, whole)
+    buf = torch.full((m + 2, n + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.linear_tc(a, w, bias, buf[:m, :n], act=ops.EPILOGUES[act] if act else 0)
+    assert (buf[m:] == 7.0).all() and (buf[:, n:] == 7.0).all()
+    if act == "relu2":
+        whole = whole.clamp(min=0.0) ** 2
+    if act == "gelu":                      # (the device's erff: 2 ulp, then half a place of bfloat16 either way)
+        want = torch.nn.functional.gelu(whole.double())
+        assert ((buf[:m, :n].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * whole.double().abs()).all()
+    else:
+        assert torch.equal(buf[:m, :n], whole.bfloat16())
+
+
 def test_linear_tensor_cores_strided_rows():
     """Operands that are column slices of wider rows (their row stride is not their width)."""
     from gibbs_b200 import ops
