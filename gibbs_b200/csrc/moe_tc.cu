@@ -238,16 +238,33 @@ moe_experts_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 // An expert's rows are cut evenly into ceil(rows / 256) tiles of a multiple of 32 rows: the width is the instruction's N and
 // known on the device only, so the token rows arrive in boxes of 16 (whole 8-row groups of the 128-byte swizzle).
 // Bound by what the tiles read from L2: one CTA of 128 x 128 reads 32 KB a k-block for 128 x 128 multiply-adds; here it is
-// 32 KB for 128 x 256, and experts of 257 rows take two tiles of 160 and not three of 128: 2,134 tokens, four of 32 experts of
+// 32 KB for 128 x 256, and experts of 257 rows take two tiles of 160 and not three of 128: 2,695 tokens, four of 32 experts of
 // 2,048 x 2 x 1,024 each, 121 -> 79 us a launch.
 constexpr int PAIR_STAGES = 6, PAIR_GROUPS = 2, PAIR_THREADS = 64 + PAIR_GROUPS * 128, PAIR_ROWS = 256, PAIR_BOX = 16;
 constexpr int PAIR_STAGE_BYTES = W_TILE_BYTES + PAIR_ROWS / 2 * BK * 2;
 constexpr int PAIR_STAGING_BYTES = 16 * 1024;                      // of a group: 32 token rows of 64 (g, u) in 32-bit
 constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + PAIR_GROUPS * PAIR_STAGING_BYTES + 1024;
-// Rows an expert on average from which the pairs take a launch.  Pairs against one CTA a tile, 32 experts of 2,048 x 2 x 1,024:
-// 52 / 53 us at 16 rows an expert, 53 / 58 at 32, 57 / 78 at 64, 63 / 111 at 128, 71 / 136 at 192, 101 / 169 at 256; below 32 the
-// two are within their noise and the narrow tiles leave less to pad.  GIBBS_B200_MOE_PAIR_ROWS moves the line (for comparison runs).
+// With few tiles the narrowest width at which the pairs take them in one round is used (a launch waits for one tile then, and a
+// tile's epilogue is as long as it is wide).
+//
+// Which launches the pairs take, by rows an expert on average and `tiles`, the experts' weight tiles of 256 rows.  Time on the
+// pairs over one CTA a tile, 4 to 128 experts of 256 x 128 to 2,048 x 1,024, even and uneven rows:
+//   GLU       0.5 to 1 from 32 rows; with 75 to 148 tiles (a second round that is half empty) 0.9 to 1.2 below 64 rows: not taken.  A few
+//             uneven launches of about one round remain at 1.04 to 1.17.
+//   function  0.3 to 1 from 32 rows
+//   plain     the other kernel's epilogue is as short, so only launches that fill the pairs gain: 0.65 to 1.0 from 128 tiles and 16,384 rows x
+//             weight tiles, or 30,720 at K of 1,024 and more; below that 1.1 to 1.5, and at K of 256 1.2 to 2.2 at any size
 constexpr int PAIR_MIN_ROWS = 32;
+bool takes_pairs(int mode, int pairs, int E, int weight_tiles, int K) {
+  // GIBBS_B200_MOE_PAIR_ROWS: from so many rows an expert, whatever the rest (for comparison runs)
+  static const int forced = [] { const char* e = getenv("GIBBS_B200_MOE_PAIR_ROWS"); return e ? atoi(e) : 0; }();
+  if (forced > 0) return (long long)pairs >= (long long)forced * E;
+  if ((long long)pairs < (long long)PAIR_MIN_ROWS * E) return false;
+  const long long tiles = (long long)weight_tiles * E, work = (long long)weight_tiles * pairs;
+  if (mode == 0) return tiles <= 74 || tiles > 148 || (long long)pairs >= 64ll * E;
+  if (mode == 1) return (K >= 512 && tiles >= 128 && work >= 16384) || (K >= 1024 && work >= 30720);
+  return true;
+}
 constexpr int PAIR_MAX_EXPERTS = 128;                              // (by what shared memory is left)
 
 // Barrier of one group of epilogue warps; true for all of its threads when any of them brought true.
@@ -258,6 +275,23 @@ __device__ __forceinline__ bool group_any(int group, bool v) {
   return r != 0;
 }
 __device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
+// A function of 32 finished sums: one switch for all of them.
+__device__ __forceinline__ void pair_act(float (&v)[32], int fn) {
+  switch (fn) {
+#define PAIR_ACT(kind)                                 \
+    case kind:                                         \
+      _Pragma("unroll") for (int j = 0; j < 32; ++j) v[j] = hy_act(v[j], kind); \
+      break
+    PAIR_ACT(ACT_GELU_ERF);
+    PAIR_ACT(ACT_GELU_TANH);
+    PAIR_ACT(ACT_SILU);
+    PAIR_ACT(ACT_RELU);
+    PAIR_ACT(ACT_RELU2);
+#undef PAIR_ACT
+    default: break;
+  }
+}
 
 __global__ void __launch_bounds__(PAIR_THREADS)
 moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -294,11 +328,29 @@ moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
     tmem_relinquish_pair();
   }
   pdl_wait();                                                       // the offsets and the rows come from the kernels before
+  const int weight_tiles = (p.rows_per_expert + 2 * BM - 1) / (2 * BM);
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   if (warp == 2) {
+    constexpr int PER_LANE = PAIR_MAX_EXPERTS / 32;
+    int lo[PER_LANE], rows[PER_LANE];
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const int e = lane + 32 * i;
+      lo[i] = e < E ? p.offsets[e] : 0;
+      rows[i] = e < E ? p.offsets[e + 1] - lo[i] : 0;
+    }
+    // the narrowest tiles that the pairs take in one round, whole ones where there are more
+    int cap = 32;
+    for (; cap < PAIR_ROWS; cap *= 2) {
+      int n = 0;
+#pragma unroll
+      for (int i = 0; i < PER_LANE; ++i) n += (rows[i] + cap - 1) / cap;
+      if (__reduce_add_sync(0xffffffffu, n) * weight_tiles <= n_pairs) break;
+    }
     int before = 0;
-    for (int e0 = 0; e0 < E; e0 += 32) {
-      const int e = e0 + lane, lo = e < E ? p.offsets[e] : 0, hi = e < E ? p.offsets[e + 1] : 0;
-      const int mine = (hi - lo + PAIR_ROWS - 1) / PAIR_ROWS;
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const int e = lane + 32 * i, mine = (rows[i] + cap - 1) / cap;
       int upto = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -306,10 +358,10 @@ moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
         if (lane >= o) upto += v;
       }
       if (e < E) {
-        row_at[e] = lo;
+        row_at[e] = lo[i];
         tile_at[e] = before + upto - mine;
         if (e + 1 == E) {
-          row_at[E] = hi;
+          row_at[E] = lo[i] + rows[i];
           tile_at[E] = before + upto;
         }
       }
@@ -321,9 +373,7 @@ moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
   cluster_sync_all();                                               // both CTAs' barriers are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
-  const int weight_tiles = (p.rows_per_expert + 2 * BM - 1) / (2 * BM);
   const int n_tiles = tile_at[E] * weight_tiles;
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
 
   struct Tile { int e, wt, r0, width, rows; };                      // expert, weight tile, first token row, N, rows that are the expert's
   auto tile_of = [&](int t) {
@@ -410,6 +460,7 @@ moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
     const int eg = (warp - 2) >> 2, et = threadIdx.x - 64 - 128 * eg;          // group, thread of the group
     const int q = warp & 3, row = 32 * q + lane;                               // lane of the accumulator = weight row of this CTA's 128
     uint8_t* staging = tiles + (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + (size_t)eg * PAIR_STAGING_BYTES;
+    const bool pieces = ((uintptr_t)p.out & 3) == 0 && p.ldo % 2 == 0 && p.n_valid % 2 == 0;      // (mode 2) stores of two values
     int tile_i = 0;
     for (int t = pair; t < n_tiles; t += n_pairs, ++tile_i) {
       const Tile tl = tile_of(t);
@@ -460,18 +511,31 @@ moe_experts_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
             }
           }
           group_barrier(eg);                                                   // (the pieces are rewritten by the next 32 rows)
-        } else if (w0 + row < p.n_valid) {
-          const int n = w0 + row;
-          if (p.mode == 1) {
-            float* dst = (float*)p.out + (size_t)(tl.r0 + h0) * p.ldo + n;     // a warp's store: 128 bytes of one token's row
+        } else if (p.mode == 1) {
+          if (w0 + row < p.n_valid) {
+            float* dst = (float*)p.out + (size_t)(tl.r0 + h0) * p.ldo + w0 + row;      // a warp's store: 128 bytes of one token's row
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < hc) dst[(size_t)j * p.ldo] = v[j];
-          } else {
-            bf16* dst = (bf16*)p.out + (size_t)(tl.r0 + h0) * p.ldo + n;
+          }
+        } else {
+          pair_act(v, p.fn);
+          if (pieces) {
+            // neighbouring lanes (weight rows n, n + 1) swap every other token's value: a store of a warp is two whole sectors of two
+            // tokens' rows
+            const bool odd = lane & 1;
+            bf16* dst = (bf16*)p.out + (size_t)(tl.r0 + h0 + odd) * p.ldo + w0 + (row & ~1);
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+              const __nv_bfloat162 two = odd ? __floats2bfloat162_rn(other, v[j + 1]) : __floats2bfloat162_rn(v[j], other);
+              if (j + odd < hc && w0 + row < p.n_valid) *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)j * p.ldo) = two;
+            }
+          } else if (w0 + row < p.n_valid) {
+            bf16* dst = (bf16*)p.out + (size_t)(tl.r0 + h0) * p.ldo + w0 + row;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (j < hc) dst[(size_t)j * p.ldo] = __float2bfloat16_rn(hy_act(v[j], p.fn));
+              if (j < hc) dst[(size_t)j * p.ldo] = __float2bfloat16_rn(v[j]);
           }
         }
       }
@@ -605,8 +669,7 @@ GB_OP(gb_op_moe_experts_tc) {
   // few rows an expert (decoding): narrow token tiles
   // (and wide ones where an expert has many: a tile's weights are read from L2 once for twice the tokens)
   const int BN = pairs <= 16 * E ? 16 : pairs < 192 * E ? 64 : 128;
-  static const int pair_rows = [] { const char* e = getenv("GIBBS_B200_MOE_PAIR_ROWS"); return e ? atoi(e) : PAIR_MIN_ROWS; }();
-  const bool on_pairs = (long long)pairs >= (long long)pair_rows * E && E <= PAIR_MAX_EXPERTS &&
+  const bool on_pairs = E <= PAIR_MAX_EXPERTS && takes_pairs(mode, pairs, E, gb_div_up(rows_per_expert, 2 * BM), K) &&
                         (mode != 0 || (a[8] % 4 == 0 && (a[7] & 7) == 0));
   if (!make_tmap(&tx, op_ptr<const void>(a[0]), a[2], K, a[1], on_pairs ? PAIR_BOX : BN))
     GB_FAIL(GB_ERR_CUDA, "moe_experts_tc: cuTensorMapEncodeTiled failed (rows)");
@@ -618,8 +681,8 @@ GB_OP(gb_op_moe_experts_tc) {
   p.total_kb = gb_div_up(K, BK);
   p.alpha = (float)f[0]; p.limit = (float)f[1]; p.up_add = (float)f[2];
   p.status = ctx->status;
-  if (on_pairs)                                                     // (rows / 256 + E: at most this many token tiles over all experts)
-    return launch_pairs(tw, tx, p, (long long)gb_div_up(rows_per_expert, 2 * BM) * (pairs / PAIR_ROWS + E), ctx->stream);
+  if (on_pairs)                                                     // (rows / 32 + E: at most this many token tiles over all experts)
+    return launch_pairs(tw, tx, p, (long long)gb_div_up(rows_per_expert, 2 * BM) * (pairs / 32 + E), ctx->stream);
   const int weight_tiles = gb_div_up(rows_per_expert, BM);
   const int row_tiles = gb_div_up(pairs, BN) + E;          // at most this many over all experts
   return BN == 16   ? launch<16>(tw, tx, p, weight_tiles, row_tiles, ctx->stream)

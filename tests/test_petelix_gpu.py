@@ -551,6 +551,22 @@ def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, c
     (5, 512, 256, 0, [1, 0, 3, 16, 17]), (40, 512, 256, 1, [0] * 38 + [2, 1]), (3, 136, 448, 0, [60, 0, 64]),
 ])
 def test_routed_experts_products_of_many_rows_and_of_few(E, K, out, mode, counts):
+    _routed_experts_product(E, K, out, mode, counts)
+
+
+# CTA pairs with tiles cut to 32, 64 and 128 rows because there are few, and whole ones on the other side of a round of 74; a function's outputs
+# stored two at a time and, where their number or stride is odd, one at a time; plain outputs at the line from which pairs take them and below it
+@pytest.mark.parametrize("E,K,out,mode,counts", [
+    (1, 64, 64, 0, [40]), (2, 72, 64, 0, [300, 1]), (8, 64, 128, 0, [0, 0, 700, 0, 0, 0, 0, 1]), (37, 64, 128, 0, [64] * 37), (38, 64, 256, 0, [70] * 38),
+    (3, 200, 321, 2, [64, 300, 200]), (1, 64, 2, 2, [33]), (5, 136, 130, 2, [31, 32, 33, 0, 257]), (4, 64, 1024, 2, [1000, 3, 0, 200]),
+    (128, 512, 130, 1, [128] * 126 + [129, 127]), (128, 512, 130, 1, [128] * 126 + [128, 127]), (64, 512, 448, 1, [0, 257] * 32),
+    (16, 1024, 512, 1, [960] * 16),
+])
+def test_routed_experts_products_at_the_edges_of_their_dispatch(E, K, out, mode, counts):
+    _routed_experts_product(E, K, out, mode, counts)
+
+
+def _routed_experts_product(E, K, out, mode, counts):
     from gibbs_b200.ops import hybrid
     torch.manual_seed(K + out)
     rows, per = sum(counts), (2 * out if mode == 0 else out)
