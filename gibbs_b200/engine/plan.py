@@ -69,6 +69,15 @@ def register_op(name: str, function) -> int:
     return rc
 
 
+def leave_tiles(record) -> bool:
+    """Tell a recorded product to leave the partial tiles of a split K to the operation recorded next; False for one that
+    does not run on the tensor cores, does not write 32-bit sums or adds into the stream."""
+    if record["op"] != P_LINEAR or record["a"][10] != 0 or record["a"][11] != 1 or record["a"][16] or record["flags"] & LF_RESIDUAL:
+        return False
+    record["flags"] = int(record["flags"]) | LF_PARTIALS
+    return True
+
+
 class TableRef:
     """Stands for 'the block table of group g of the current step' while a plan is built."""
 

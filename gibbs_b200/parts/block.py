@@ -132,9 +132,8 @@ class SandwichResidual(Block):
                 raise ValueError(f"the {role} must be a norm that can add into the stream (a RowNorm kind)")
 
     def _run(self, rn, x, caches, h_of):
-        rn.partial_branches = True                 # (the norm behind a sublayer adds up the partial tiles its last product leaves)
         hidden = x.shape[1]
-        y = rn.buffer("branch", hidden, torch.float32)
+        rn.last_read = y = rn.buffer("branch", hidden, torch.float32)      # (the norm behind a sublayer is the last to read its output)
         # a token input reads the stream through a product: in bfloat16 the norm that completes the
         # stream also leaves the rows in that type
         copy = None
@@ -300,11 +299,10 @@ class HyperResidual(Block):
         return False
 
     def _run(self, rn, x, caches):
-        rn.partial_branches = True                 # (the mixing adds up the partial tiles a sublayer's last product leaves)
         h, self._handed = self._handed, None
         if h is None:
             h = self.mixer_streams.read(rn, x, self.mixer_norm)
-        y = rn.buffer("branch", self.mixer_streams.dim, torch.float32)
+        rn.last_read = y = rn.buffer("branch", self.mixer_streams.dim, torch.float32)      # (the mixing is the last to read it)
         behind = None if self._next is None else (self._next.mixer_streams, self._next.mixer_norm)
         has_ffn = "ffn" in self.parts
         self.mixer.run(rn, h, y, self.caches_of("mixer", caches))

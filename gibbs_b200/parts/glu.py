@@ -249,27 +249,21 @@ class RoutedGLU(BranchPart, FeedForward):
             sh = None
             if self.shared is not None:
                 sh = rn.buffer("moe_shared_out", d, torch.float32)
-                # (the kernel behind it adds the partial tiles its last product may leave)
-                leaves, rn.partial_branches = rn.partial_branches, True
                 self.shared.run(rn, h, sh)
-                rn.partial_branches = leaves
             behind, normed_rows = then_operands(rn, then)
             rn.op("moe_combine_weighted", [eout.data_ptr(), eout.stride(0), pair_row.data_ptr(), idx.data_ptr(),
                                            wts.data_ptr(), h.data_ptr(), h.stride(0), ops.dtype_code(h.dtype),
                                            out.data_ptr(), out.stride(0), rn.N, d, top, E,
                                            0 if sh is None else sh.data_ptr(), 0 if sh is None else sh.stride(0), *behind],
-                  flags=(1 if accumulate else 0) | (0 if sh is None else hybrid.TAKES_PARTIALS))
+                  flags=(1 if accumulate else 0) | (0 if sh is None else rn.tiles_of(sh)))
             return normed_rows
         sh = None
         if shared:
             sh = rn.buffer("moe_shared_out", d, torch.float32)
-            # (the kernel behind it adds the partial tiles its last product may leave)
-            leaves, rn.partial_branches = rn.partial_branches, True
             self.shared.run(rn, h, sh)
-            rn.partial_branches = leaves
         rn.op("moe_combine", [eout.data_ptr(), eout.stride(0), pair_row.data_ptr(), sg.data_ptr() if shared else 0,
                               sh.data_ptr() if shared else 0, sh.stride(0) if shared else 0, out.data_ptr(),
-                              out.stride(0), rn.N, d, top], flags=hybrid.TAKES_PARTIALS if shared else 0)
+                              out.stride(0), rn.N, d, top], flags=rn.tiles_of(sh) if shared else 0)
 
 
 class RoutedMLP(RoutedGLU):

@@ -104,7 +104,8 @@ class RowNorm(Norm):
         """x += norm(y) * gain, for x the stream and y a sublayer's output (both float32).  ``copy``
         (bfloat16 [rows, dim], contiguous) also receives the new rows, for a product that reads
         the stream next.  ``then`` (another RowNorm: the norm in front of the next sublayer) is taken
-        of the new rows in the same kernel; its output is returned."""
+        of the new rows in the same kernel; its output is returned.  Where the arrangement says that nothing reads ``y``
+        afterwards (``rn.last_read``), the product that writes it may leave it in parts, which the kernel adds up."""
         a = [x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), keep(rn, self.gain), rn.N, self.dim, self.KIND,
              0 if copy is None else copy.data_ptr()]
         f = [self.eps]
@@ -113,7 +114,9 @@ class RowNorm(Norm):
             out = rn.buffer("normed", then.dim)
             a += [keep(rn, then.gain), out.data_ptr(), ops.dtype_code(out.dtype), then.KIND]
             f += [then.eps]
-        rn.op("norm_add", a, f, label="norm_add", flags=hybrid.TAKES_PARTIALS)
+        # (a kind with an add_normed of its own around this one may still read y)
+        last = rn.last_read is y and type(self).add_normed is RowNorm.add_normed
+        rn.op("norm_add", a, f, label="norm_add", flags=rn.tiles_of(y) if last else 0)
         return out
 
     def forward(self, x, out=None, rows=None):

@@ -59,12 +59,19 @@ class Runner:
         (``hybrid.TAKES_PARTIALS``): a plan may leave the sums of a split K in parts."""
         self.linear(x, weight, bias, out, role=role)
 
-    # set by an arrangement whose next kernel reads a sublayer's output and can add up partial tiles itself
-    partial_branches = False
+    # set by an arrangement in front of the operation that takes a sublayer's output: that tensor, which nothing reads afterwards
+    last_read = None
 
     def branch_linear(self, x, weight, bias, out, accumulate: bool = False, role: str = "") -> None:
-        """A sublayer's last product: written into ``out``, or added (``add_linear``)."""
+        """A sublayer's last product: written into ``out``, or added (``add_linear``).  A plan may still be told to leave
+        its sums in parts (``tiles_of``)."""
         (self.add_linear if accumulate else self.linear)(x, weight, bias, out, role=role)
+
+    def tiles_of(self, y) -> int:
+        """Flags for an operation that is recorded next, reads ``y`` as the last to do so and can add up partial tiles:
+        ``hybrid.TAKES_PARTIALS`` where the record directly in front is the ``branch_linear`` that writes ``y`` (which
+        is told to leave them), 0 where ``y`` is whole."""
+        return 0
 
     def op(self, name: str, a, f=(), label: str = "", flags: int = 0) -> None:
         raise NotImplementedError
@@ -121,6 +128,7 @@ class Planned(Runner):
     def __init__(self, plan):
         from ..engine import plan as P
         self.plan, self.rt = plan, plan.rt
+        self._branch = (None, None)          # what the latest branch_linear writes, and its record
         self.N, self.R, self.W = P.sym(P.S_N), P.sym(P.S_R), P.sym(P.S_W)
         self.token_ids, self.tok_req, self.tok_pos = P.sym(P.S_TOKEN_IDS), P.sym(P.S_TOK_REQ), P.sym(P.S_TOK_POS)
         self.q_start, self.q_len, self.start_pos = P.sym(P.S_Q_START), P.sym(P.S_Q_LEN), P.sym(P.S_START_POS)
@@ -154,9 +162,15 @@ class Planned(Runner):
         self.plan.linear(x, weight, bias, out, "plain", role=role or "plain", partials="always")
 
     def branch_linear(self, x, weight, bias, out, accumulate=False, role=""):
-        if accumulate or not self.partial_branches:
-            return super().branch_linear(x, weight, bias, out, accumulate, role)
-        self.partial_linear(x, weight, bias, out, role)
+        super().branch_linear(x, weight, bias, out, accumulate, role)
+        if not accumulate:
+            self._branch = (out, self.plan.ops[-1])
+
+    def tiles_of(self, y):
+        out, record = self._branch
+        if out is not y or self.plan.ops[-1] is not record:
+            return 0                # (a part that works on y behind its product, or has another product behind it)
+        return hybrid.TAKES_PARTIALS if self._P.leave_tiles(record) else 0
 
     def op(self, name, a, f=(), label="", flags=0):
         self.plan.emit(hybrid.plan_id(name), list(a), list(f), flags=flags, label=label or name)
@@ -189,7 +203,9 @@ def stream_tensor(x) -> torch.Tensor:
 class BranchPart:
     """Mixin for mixers and feed-forwards written against a ``Runner``: ``run(rn, h, out,
     caches)`` WRITES the sublayer's output into ``out`` (float32 [rows, hidden]), so that an
-    arrangement can put a norm between the sublayer and the residual sum.  In an arrangement
+    arrangement can put a norm between the sublayer and the residual sum.  (A last product recorded
+    with ``branch_linear`` may be left in parts, when nothing was recorded behind it and the operation that takes
+    ``out`` says that it adds them.)  In an arrangement
     that adds sublayers straight into the stream, ``forward`` adds ``out`` to it."""
     writes_branch = True
     # True for a part whose ``run`` takes ``accumulate=True`` and then ADDS its output into ``out``: in an
