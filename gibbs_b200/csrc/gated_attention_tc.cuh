@@ -500,8 +500,10 @@ int run_attention_tc(const GbPlanCtx* ctx, const long long* a, const double* f, 
   int rc;
   // portions without chunks of keys, where the other kernel takes them.  us there and here, 32 / 8 heads of 64, prompts of
   // 64 tokens 8.3 and 8.6 (sigmoids 8.6 and 8.1), 96 10 and 11 (10 and 10), 256 15 and 19 (14 and 17), 512 25 and 39 (21 and 35),
-  // 1,536 68 and 133 (51 and 116); behind a context of 2,048 less their own, 64 tokens 66 and 94 (53 and 81)
-  if (!narrow && p.splits == 1 && tiles * G * maps >= 48 && p.keep_first == 0) {
+  // 1,536 68 and 133 (51 and 116); behind a context of 2,048 less their own, 64 tokens 66 and 94 (53 and 81).
+  // Steps whose every portion fills less than 16 of a tile's 128 rows stay here (64 requests of 2 tokens at 100 keys 24 and 22; of 8, 24 and 32)
+  const long long longest = ctx->sym != nullptr && ctx->sym[GB_SYM_MAX_PORTION] > 0 ? ctx->sym[GB_SYM_MAX_PORTION] : n;
+  if (!narrow && p.splits == 1 && tiles * G * maps >= 48 && p.keep_first == 0 && longest * group >= 16) {
     const GatedTcgen05Launch b = {p.q, p.k_pages, p.v_pages, p.block_table, p.bt_stride, p.page_size, p.n_pages, p.tok_req,
                                   p.tok_pos, p.q_start, p.gate, p.ld_gate, p.out, p.out_f32, p.ldo, n, R, H, G, dim, vdim, maps,
                                   p.window, p.blocked, p.sink, p.scale, p.softcap, p.sink_scores, SIG, score_bias, factor, p.status};

@@ -103,17 +103,27 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
   }
-  // which request's which tile, from the last to the first (a prompt's last tiles see the most keys: they start first)
-  int tile = (int)blockIdx.y, t0 = -1, n_tok = 0;
-  for (int r = p.R - 1; r >= 0; --r) {
-    const int qs = p.q_start[r], qe = r + 1 < p.R ? p.q_start[r + 1] : p.N;
+  // which request's which tile, from the last to the first (a prompt's last tiles see the most keys: they start first); every warp
+  // looks at 32 requests at a time
+  int t0 = -1, n_tok = 0;
+  for (int r0 = 0, before = 0; r0 < p.R && t0 < 0; r0 += 32) {
+    const int r = p.R - 1 - r0 - lane;
+    const int qs = r >= 0 ? p.q_start[r] : 0, qe = r < 0 ? 0 : r + 1 < p.R ? p.q_start[r + 1] : p.N;
     const int nt = (qe - qs + tpt - 1) / tpt;
-    if (tile < nt) {
-      t0 = qs + (nt - 1 - tile) * tpt;
-      n_tok = min(tpt, qe - t0);
-      break;
+    int upto = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
     }
-    tile -= nt;
+    const unsigned hit = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.y);
+    if (hit) {
+      // (its first tile is the request's last)
+      const int src = __ffs(hit) - 1, from_end = before + __shfl_sync(0xffffffffu, upto, src) - (int)blockIdx.y;
+      t0 = __shfl_sync(0xffffffffu, qs, src) + (from_end - 1) * tpt;
+      n_tok = min(tpt, __shfl_sync(0xffffffffu, qe, src) - t0);
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
   }
   if (t0 < 0) return;
   const int pos0 = p.tok_pos[t0];

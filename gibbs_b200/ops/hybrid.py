@@ -54,8 +54,13 @@ def _function(name: str):
     return fn
 
 
-def call(name: str, a, f=(), flags: int = 0, device=None) -> int:
-    """Launch one operation now, on the current stream."""
+def step_symbols(n_tokens: int, n_requests: int, n_wanted: int, max_portion: int, max_context: int):
+    """The counts of a step as an operation launched with ``call`` sees them (gb_plan_op.h; the addresses are 0)."""
+    return (ctypes.c_longlong * 32)(n_tokens, n_requests, n_wanted, max_portion, max_context)
+
+
+def call(name: str, a, f=(), flags: int = 0, device=None, symbols=None) -> int:
+    """Launch one operation now, on the current stream.  ``symbols`` (``step_symbols``): the step it belongs to."""
     fn = _function(name)
     if len(a) > 24 or len(f) > 3:
         raise ValueError("an operation has 24 integer and 3 floating-point operands")
@@ -65,7 +70,8 @@ def call(name: str, a, f=(), flags: int = 0, device=None) -> int:
     fa = (ctypes.c_double * 3)(*[float(v) for v in f])
     status = device_status(device if device is not None else torch.device("cuda", torch.cuda.current_device()))
     stream = _stream()
-    ctx = _Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, status.data_ptr(), None, 0, None, 0, None, 0,
+    ctx = _Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, status.data_ptr(),
+               None if symbols is None else ctypes.cast(symbols, ctypes.c_void_p), 0 if symbols is None else 32, None, 0, None, 0,
                None, None, 0, None)                # (called directly, nothing is ever pending)
     rc = fn(ctypes.byref(ctx), ia, fa, ctypes.c_int(flags))
     if rc < 0:

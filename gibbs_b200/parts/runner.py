@@ -91,6 +91,7 @@ class Eager(Runner):
         self.N, self.R, self.W = step.n_tokens, step.n_requests, step.n_want
         self.max_context = max(int(step.max_ctx_len), 1)
         self.max_portion = int(getattr(step, "max_q_len", 0))
+        self._symbols = hybrid.step_symbols(self.N, self.R, self.W, self.max_portion, self.max_context)
         for k in ("token_ids", "tok_req", "tok_pos", "q_start", "q_len", "start_pos", "want_rows"):
             setattr(self, k, getattr(step, k).data_ptr())
 
@@ -114,7 +115,7 @@ class Eager(Runner):
         ops.linear_tc(x[:self.N] if x.shape[0] != self.N else x, weight, bias, out, act=ops.EPILOGUES[act])
 
     def op(self, name, a, f=(), label="", flags=0):
-        hybrid.call(name, a, f, flags=flags, device=self.rt.device)
+        hybrid.call(name, a, f, flags=flags, device=self.rt.device, symbols=self._symbols)
 
     def table(self, view):
         bt = view.block_table

@@ -485,6 +485,20 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     (8, 8, 1, 64, 16, 0, 0.0, False, False, True, [70], [321], False),
 ])
 def test_tensor_core_attention_of_portions(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
+    _portions_against_float64(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked)
+
+
+# more requests than a warp has lanes, short portions beside long ones
+@pytest.mark.parametrize("heads,kvh,vdim,window,sig,starts,lens", [
+    (16, 4, 64, 0, False, [40 * (r % 5) for r in range(70)], [1 + 7 * r % 50 for r in range(70)]),
+    (8, 8, 128, 30, False, [r for r in range(33)], [130 - 4 * r for r in range(32)] + [1]),
+    (32, 8, 64, 0, True, [0] * 32 + [500], [40] * 32 + [77]),
+])
+def test_tensor_core_attention_of_many_portions(heads, kvh, vdim, window, sig, starts, lens):
+    _portions_against_float64(heads, kvh, 1, vdim, 16, window, 0.0, False, False, sig, starts, lens, False)
+
+
+def _portions_against_float64(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
     from gibbs_b200.ops import hybrid
     torch.manual_seed(heads * 1000 + window)
     dk, n, group = 64, sum(lens), heads // kvh
