@@ -12,13 +12,15 @@
 //                   in tensor memory is rescaled only when the maximum has grown by more than 8 (a factor of 256).
 //
 // Three CTAs fit on an SM at values of 64 (73 KB of shared memory, 128 tensor-memory columns, 112 registers a thread), two at
-// 128: while one is in its softmax the others' products run.  2,134 tokens, 32 / 8 heads of 64, soft cap, window of 1,024: 187 us a
+// 128: while one is in its softmax the others' products run.  2,695 tokens, 32 / 8 heads of 64, soft cap, window of 1,024: 187 us a
 // layer on the mma.sync kernel, 123 here; with sigmoids 128 and 55.  Bound by the special functions of the softmax warps (three a
 // score under a soft cap, 16 a cycle and SM) and by the chain of a key tile.
 //
 // The arithmetic of a weight (scores times log2(e), the hardware's 2^x and 1/x) is that of gated_attention_tc.cuh.
 // A weight of zero does not keep what is not finite out of a product, so the values of positions that no row of the tile
-// sees (the rest of the last page, pages the window has passed) are zeroed in shared memory before they are multiplied.
+// sees (the rest of the last page, pages the window has passed) are zeroed in shared memory before they are multiplied.  Of the
+// others a row may meet one that only another row sees: a row whose result is not finite is worked out again by itself, over its own
+// keys.  (Looking at the values of every key tile that not all rows see whole cost 5 to 8 % of a launch.)
 // Every wait is bounded; a wait that runs out sets *status and the CTA drains and returns.
 #include <mutex>
 
@@ -43,6 +45,7 @@ struct GtParams {
   float scale, softcap;
   const float* sink_scores;
   const float* score_bias; float factor;
+  const bf16 *q, *k_pages, *v_pages;     // (for rows that are worked out again)
   int* status;
 };
 
@@ -66,10 +69,53 @@ __device__ __forceinline__ float gt_rcp(float x) {
   return y;
 }
 
+// One row (a token's query head) again, by itself and over the keys first .. last that it sees, in 32-bit: sum[0 .. DV - 1] its weighted
+// sum, m and l its maximum and its sum of weights.  For rows whose result is not finite, which another row's value may have done.
+template <int DV, bool CAPPED, bool SIG>
+__device__ __noinline__ void gt_row(float* sum, float& m, float& l, const GtParams& p, const int* bt, int g, int mp, const bf16* q, int first,
+                                    int last, float c_in, float c_mul, float c_add, float bias) {
+  m = -INFINITY;
+  l = 0.f;
+  for (int d = 0; d < DV; ++d) sum[d] = 0.f;
+  for (int key = max(first, 0); key <= last; ++key) {
+    int page = bt[key / p.page_size];
+    if (page < 0 || page >= p.n_pages) page = 0;                // (as its tile was brought)
+    const size_t at = ((size_t)page * p.G + g) * p.page_size + key % p.page_size;
+    const __nv_bfloat162* k = reinterpret_cast<const __nv_bfloat162*>(p.k_pages + (at * p.maps + mp) * GT_DK);
+    const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(p.v_pages + at * DV);
+    float s0 = 0.f, s1 = 0.f;
+    for (int d = 0; d < GT_DK / 2; ++d) {
+      const float2 x = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(q)[d]), y = __bfloat1622float2(k[d]);
+      s0 = fmaf(x.x, y.x, s0);
+      s1 = fmaf(x.y, y.y, s1);
+    }
+    float s = (s0 + s1) * c_in;
+    if (CAPPED) s = fmaf(c_mul, gt_rcp(gt_ex2(s) + 1.f), c_add);
+    float w;
+    if (SIG) {
+      w = gt_rcp(1.f + gt_ex2(-(s + bias)));
+    } else {
+      if (s > m) {
+        const float c = m == -INFINITY ? 0.f : gt_ex2(m - s);
+        l *= c;
+        for (int d = 0; d < DV; ++d) sum[d] *= c;
+        m = s;
+      }
+      w = gt_ex2(s - (m == -INFINITY ? 0.f : m));
+      l += w;
+    }
+    for (int d = 0; d < DV / 2; ++d) {
+      const float2 y = __bfloat1622float2(v[d]);
+      sum[2 * d] = fmaf(w, y.x, sum[2 * d]);
+      sum[2 * d + 1] = fmaf(w, y.y, sum[2 * d + 1]);
+    }
+  }
+}
+
 template <int DV, bool CAPPED, bool SIG>
 __global__ void __launch_bounds__(192) __maxnreg__((GtCfg<DV>::REGS))
 sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                              const __grid_constant__ CUtensorMap map_v, const GtParams p) {
+                              const __grid_constant__ CUtensorMap map_v, const __grid_constant__ GtParams p) {
   pdl_trigger();
   using C = GtCfg<DV>;
   constexpr int VSUB = DV / 64;                                 // 64-column sub-tiles of a V tile
@@ -271,6 +317,7 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const float c_mul = -2.f * p.softcap * LOG2E, c_add = p.softcap * LOG2E;
     const float bias = SIG && p.score_bias && rvalid ? p.score_bias[g * group + hh] * LOG2E : 0.f;
     float m_used = -INFINITY, l_run = 0.f;
+    float total[DV];                                            // a row that is worked out again, in local memory
     bool alive = true;
     for (int j = 0; j < n_tiles; ++j) {
       if (!__all_sync(0xffffffffu, mbar_wait(&s_full, j & 1) && !abort_flag)) {
@@ -398,30 +445,47 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     if (alive) {
       pdl_wait();                                               // (long over; the gate's logits come from a kernel before)
       const int h = (g * group + hh) * p.maps + mp, t = t0 + tl;
-      float f = p.factor;
-      if (!SIG) {
-        const float m = m_used * LN2;                           // natural units (-inf stays)
+      auto scale_of = [&](float m2, float l) {
+        if (SIG) return p.factor;
+        const float m = m2 * LN2;                               // natural units (-inf stays)
         const float z = p.sink_scores && rvalid ? p.sink_scores[g * group + hh] : 0.f;
         const float M = p.sink ? fmaxf(m, z) : m;
         const float e = expf(m - M);
-        f = e * (1.0f / fmaf(e, l_run, p.sink ? expf(z - M) : 0.f));
-      }
+        return e * (1.0f / fmaf(e, l, p.sink ? expf(z - M) : 0.f));
+      };
       const float* gt = p.gate ? p.gate + (size_t)t * p.ld_gate + (size_t)h * DV : nullptr;
       const size_t at = (size_t)t * p.ldo + (size_t)h * DV;
+      auto store = [&](int c0, float (&o)[16], float f) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] *= gt ? f * hy_sigmoid(gt[c0 + i]) : f;
+        if (p.out_f32) {
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) *reinterpret_cast<float2*>(p.out_f32 + at + c0 + i) = make_float2(o[i], o[i + 1]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) *reinterpret_cast<__nv_bfloat162*>(p.out + at + c0 + i) = __floats2bfloat162_rn(o[i], o[i + 1]);
+        }
+      };
+      const float f = scale_of(m_used, l_run);
+      float check = 0.f;                                        // (x * 0 is a zero or not a number)
 #pragma unroll 1
       for (int c0 = 0; c0 < DV; c0 += 16) {
         float o[16];
         tmem_ld_16(tmem_o + lane_off + (uint32_t)c0, o);
-        if (rvalid) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] *= gt ? f * hy_sigmoid(gt[c0 + i]) : f;
-          if (p.out_f32) {
+        for (int i = 0; i < 16; ++i) check = fmaf(o[i], 0.f, check);
+        if (rvalid) store(c0, o, f);
+      }
+      if (rvalid && !(check == 0.f)) {
+        float m, l;
+        gt_row<DV, CAPPED, SIG>(total, m, l, p, bt, g, mp, p.q + ((size_t)t * p.H * p.maps + h) * GT_DK, rfirst, rpos, c_in, c_mul, c_add, bias);
+        const float fr = scale_of(m, l);
+#pragma unroll 1
+        for (int c0 = 0; c0 < DV; c0 += 16) {
+          float o[16];
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) *reinterpret_cast<float2*>(p.out_f32 + at + c0 + i) = make_float2(o[i], o[i + 1]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; i += 2) *reinterpret_cast<__nv_bfloat162*>(p.out + at + c0 + i) = __floats2bfloat162_rn(o[i], o[i + 1]);
-          }
+          for (int i = 0; i < 16; ++i) o[i] = total[c0 + i];
+          store(c0, o, fr);
         }
       }
     }
@@ -510,7 +574,7 @@ int gb_gated_tcgen05_launch(const GatedTcgen05Launch& a, cudaStream_t stream) {
   p.tok_req = a.tok_req; p.tok_pos = a.tok_pos; p.q_start = a.q_start; p.gate = a.gate; p.ld_gate = a.ld_gate;
   p.out = a.out; p.out_f32 = a.out_f32; p.ldo = a.ldo; p.N = a.n; p.R = a.R; p.H = a.H; p.G = a.G; p.tpt = tpt; p.maps = a.maps;
   p.window = a.window; p.blocked = a.blocked; p.sink = a.sink; p.scale = a.scale; p.softcap = a.softcap; p.sink_scores = a.sink_scores;
-  p.score_bias = a.score_bias; p.factor = a.factor; p.status = a.status;
+  p.score_bias = a.score_bias; p.factor = a.factor; p.q = a.q; p.k_pages = a.k_pages; p.v_pages = a.v_pages; p.status = a.status;
   // (every request may end with a partly filled tile)
   const dim3 grid(a.G * a.maps, gb_div_up(a.n, tpt) + a.R);
   const bool capped = a.softcap > 0.f;

@@ -498,6 +498,63 @@ def test_tensor_core_attention_of_many_portions(heads, kvh, vdim, window, sig, s
     _portions_against_float64(heads, kvh, 1, vdim, 16, window, 0.0, False, False, sig, starts, lens, False)
 
 
+class _Pages:
+    """One request's keys and values on shuffled pages, and the attention of its last ``n`` tokens (or of some of them)."""
+
+    def __init__(self, heads, kvh, vdim, start, n, one_sign=False):
+        self.heads, self.kvh, self.vdim, self.start, self.n, self.ps, ctx = heads, kvh, vdim, start, n, 16, start + n
+        self.n_pages = -(-ctx // self.ps) + 2
+        self.table = torch.randperm(self.n_pages)[:self.n_pages - 2].int().cuda()[None].contiguous()
+        self.q = (torch.randn(n, heads * 64, device="cuda") * 0.5).bfloat16()
+        self.k = torch.randn(self.n_pages, kvh, self.ps, 64, device="cuda").bfloat16()
+        v = torch.randn(self.n_pages, kvh, self.ps, vdim, device="cuda")
+        self.v = (1 + v.abs() if one_sign else v).bfloat16()
+
+    def at(self, positions):
+        """(pages, rows) of positions."""
+        i = torch.as_tensor(positions, device="cuda")
+        return self.table[0].long()[i // self.ps], i % self.ps
+
+    def attend(self, window=0, sig=False, blocked=False, first=0, n=None, v=None, cap=0.0):
+        from gibbs_b200.ops import hybrid
+        n, v = self.n - first if n is None else n, self.v if v is None else v
+        i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+        out = torch.empty(n, self.heads * self.vdim, device="cuda")
+        q, bias = self.q[first:first + n].contiguous(), torch.zeros(self.heads, device="cuda")
+        req, pos, at = i32([0] * n), i32(list(range(self.start + first, self.start + first + n))), i32([0])
+        hybrid.call("sigmoid_attention_tc" if sig else "sink_attention_tc",
+                    [q.data_ptr(), self.k.data_ptr(), v.data_ptr(), self.table.data_ptr(), self.table.shape[1], self.ps, self.n_pages, req.data_ptr(),
+                     pos.data_ptr(), 0, 0, out.data_ptr(), out.stride(0), n, self.heads, self.kvh, 64, self.vdim, window, self.start + self.n, 0, 1,
+                     at.data_ptr(), bias.data_ptr() if sig else 0], [0.125, cap, 1.0 if sig else 0.0], flags=2 | (4 if blocked else 0) | 1 << 8)
+        return out.reshape(n, self.heads, self.vdim)
+
+
+# portions whose own later tokens, and positions that a window has passed for some rows, have values that are not finite
+@pytest.mark.parametrize("vdim,start,n,window,sig,blocked,odd", [
+    (64, 0, 400, 0, False, False, [17, 63, 64, 200, 399]), (128, 100, 300, 0, True, False, [130, 131, 250]), (64, 5, 500, 70, False, False, [3, 40, 300]),
+    (128, 5, 500, 200, False, False, [150, 504]), (64, 0, 400, 128, True, True, [130, 255, 256]), (64, 4500, 300, 0, False, False, [4490, 4600, 4700]),
+])
+def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(vdim, start, n, window, sig, blocked, odd):
+    torch.manual_seed(vdim + n)
+    a = _Pages(16, 4, vdim, start, n)
+    want = a.attend(window, sig, blocked)
+    v = a.v.clone()
+    what = [float("inf"), float("nan"), float("-inf")]
+    for i, pos in enumerate(odd):
+        page, row = a.at(pos)
+        v[page, i % 4, row, 7 * i % vdim] = what[i % 3]
+    got = a.attend(window, sig, blocked, v=v)
+    pos = torch.arange(start, start + n, device="cuda")
+    first = pos * 0 if not window else pos // window * window if blocked else pos - window + 1
+    touched = torch.zeros(n, 16, vdim, dtype=torch.bool, device="cuda")
+    for i, o in enumerate(odd):
+        touched[(pos >= o) & (first <= o), 4 * (i % 4):4 * (i % 4) + 4, 7 * i % vdim] = True
+    assert not torch.isfinite(got[touched]).any()
+    # (rows that met such a value are worked out again, in 32-bit and in another order: what the weights' 16 bits and the sums allow twice)
+    size = a.attend(window, sig, blocked, v=a.v.abs())
+    assert ((got - want).abs() <= 2.0 ** -14.5 * size + 1e-6)[~touched].all()
+
+
 def _portions_against_float64(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
     from gibbs_b200.ops import hybrid
     torch.manual_seed(heads * 1000 + window)
