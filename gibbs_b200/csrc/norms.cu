@@ -113,8 +113,7 @@ __global__ void norm_pending_add_kernel(float* __restrict__ x, long long ldx, co
 }
 
 // One warp a row, the row in registers as V4 pieces of four values a lane (dim <= 128 * V4, a multiple of 4, rows
-// 16-byte aligned): no block-wide sums, 16-byte loads and packed stores.  Which kernel runs depends on the row's
-// length and alignment only, never on the number of rows.
+// 16-byte aligned): no block-wide sums, 16-byte loads and packed stores.
 template <typename TO, int V4, bool PEND>
 __global__ void __launch_bounds__(128)
 row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ gain, TO* out, const int* rows, int n, int dim,
@@ -177,7 +176,7 @@ row_norm_warp_kernel(const float* x, long long ldx, const float* __restrict__ ga
   }
 }
 
-// The same for few rows (a decode step) and for rows with pending sums: a block a row, a piece of four values a thread (dim <= 2048, a multiple of 4), the
+// The same with a block a row, for few rows (a decode step) and for most with pending sums: a piece of four values a thread, the
 // partial sums of all splits in one trip, the gain read before the wait.  The sums are added in the order of the kernel above
 // (a lane's pieces, then the lanes), so the bits are the same.
 template <typename TO>
@@ -837,8 +836,8 @@ GB_OP(gb_op_row_norm) {
   const size_t out_bytes = a[4] == GB_BF16 ? 2 : 4;
   const bool by_warps = dim % 4 == 0 && dim <= 2048 && a[1] % 4 == 0 && (a[0] & 15) == 0 && (a[2] & 15) == 0 &&
                         (a[3] & (4 * out_bytes - 1)) == 0;
-  // sums a product left to be added into the stream (a record with GB_OP_TAKES_PENDING): the kernel with a warp a row
-  // adds them while it reads its rows, when these are all of the stream's rows; else they are added first
+  // sums a product left to be added into the stream (a record with GB_OP_TAKES_PENDING): the kernels for rows of 16-byte
+  // pieces add them while they read their rows, when these are all of the stream's rows; else they are added first
   const float* pend = (flags & GB_OP_TAKES_PENDING) && ctx->pend_splits > 0 ? ctx->pend : nullptr;
   int launched = 0;
   if (pend != nullptr) {
@@ -857,8 +856,11 @@ GB_OP(gb_op_row_norm) {
     }
   }
   const size_t block_smem = sizeof(float) * ((size_t)(pend != nullptr ? ctx->pend_splits : 0) * dim + 2 * 512);
-  // (rows that bring pending sums at any number: a warp a row asks for its pieces' sums one after the other)
-  if (by_warps && (n < NORM_FEW_ROWS || pend != nullptr) && block_smem <= 160 * 1024) {
+  // A block a row, or a warp a row (the same bits).  Narrow rows leave a block little to do: from 8,000 rows of 64 with pending sums, 10.4 us
+  // and 4.7.  Without pending sums below NORM_FEW_ROWS; with them, which a warp asks for one after the other, at any number of rows above
+  // 1,024 (2,695 rows of 2,048 and four tiles 21 and 35 us), below that to 2,048 rows (2,695 rows of 1,024 8.8 and 7.7, 1,024 rows 5.2 and 6.9).
+  const bool by_blocks = dim > 256 && n < (pend == nullptr ? NORM_FEW_ROWS : dim > 1024 ? 1 << 30 : 2048);
+  if (by_warps && by_blocks && block_smem <= 160 * 1024) {
     // (whole warps; a thread without a piece adds zeros)
     const dim3 block(32 * gb_div_up(dim, 128));
 #define BLOCK_NORM(TO)                                                                                                     \

@@ -702,3 +702,37 @@ def test_norm_behind_a_sublayer_from_partial_tiles(d, kind, second, splits, bias
     if second:                                               # (half a place of bfloat16, 2^-8 of the value at most, and the 32-bit error)
         want = norm(new, then)
         assert ((whole[1].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+# rows that bring sums of a product on either side of the lines between a block and a warp a row: narrow ones, 2,048 rows of up to 1,024 values
+@pytest.mark.parametrize("dim,kind,splits", [(256, 1, 4), (260, 0, 2), (512, 1, 3), (1024, 0, 1), (64, 1, 16), (1028, 0, 2)])
+def test_row_norm_with_pending_sums_has_the_same_bits_at_any_number_of_rows(dim, kind, splits):
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(dim + splits)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 2049
+    x0, gain, add = torch.randn(many, dim, device=dev), torch.randn(dim, device=dev), torch.randn(dim, device=dev)
+    pend = torch.randn(splits, many, dim, device=dev)
+
+    def run(n):
+        x, parts, out = x0[:n].clone(), pend[:, :n].contiguous(), torch.full((n, dim), 7.0, device=dev)
+        sym, stream = (ctypes.c_longlong * 32)(n), _stream()
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), ctypes.cast(sym, ctypes.c_void_p),
+                          32, x.data_ptr(), dim, parts.data_ptr(), splits, add.data_ptr(), None, 0, None)
+        a = (ctypes.c_longlong * 24)(x.data_ptr(), dim, gain.data_ptr(), out.data_ptr(), 0, 0, n, dim, kind)
+        assert hybrid._function("row_norm")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(1e-6), ctypes.c_int(hybrid.TAKES_PENDING)) == 1
+        torch.cuda.synchronize()
+        return x, out
+
+    whole_x, whole = run(many)
+    want = x0.clone()
+    for u in range(splits):
+        want += pend[u]
+    assert torch.equal(whole_x, want + add)
+    v = whole_x.double() - (whole_x.double().mean(1, keepdim=True) if kind == 0 else 0.0)
+    exact = v / (v.pow(2).mean(1, keepdim=True) + 1e-6).sqrt() * gain.double()
+    assert ((whole.double() - exact).norm(dim=1) / exact.norm(dim=1)).max() < 1e-6
+    for n in (1, 639, 640, 2047, 2048):
+        x, out = run(n)
+        assert torch.equal(x, whole_x[:n]) and torch.equal(out, whole[:n]), n
