@@ -239,7 +239,7 @@ row_norm_block_kernel(const float* x, long long ldx, const float* __restrict__ g
 }
 
 // AHEAD: the gains are on hand before the kernel in front has finished (pinned, see gb_pin): read behind the sums, each was a
-// trip to L2 of its own (2 rows of 2048 in a decode step: 6.3 us; 2.8 so).  They cost registers, so blocks an SM, which a launch
+// trip to L2 of its own (2 rows of 2,048 in a decode step, which the kernel below takes now: 6.3 us; 2.8 so).  They cost registers, so blocks an SM, which a launch
 // of many rows needs more.
 template <bool AHEAD>
 __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long long ldy, const float* __restrict__ gain,
@@ -308,77 +308,114 @@ __global__ void norm_add_kernel(float* x, long long ldx, const float* y, long lo
   }
 }
 
-// The same for rows of up to 2,048 values in 16-byte pieces: a block a row, a piece a thread, the gains on hand before the wait.
+// The same for rows of up to 2,048 values in 16-byte pieces: a block a row, PIECES of them a thread (a piece's number is
+// threadIdx.x + i * blockDim.x), the gains on hand before the wait.
 // (A decode step's product left its sum to a kernel of its own, 2.1 us, before the norm behind it, 3.0 us.)
 // y may come as the partial tiles [splits][rows][dim] of the product that makes it (+ its bias): they are asked for in one trip
-// and added in their order, as the product's own reduction would.  A row's sums are formed by the same threads in the same
-// order whatever the number of rows.
-__global__ void __launch_bounds__(512)
+// and added in their order, as the product's own reduction would.  A row's sums are formed in the same order whatever PIECES is:
+// every lane of a warp adds the pieces lane, lane + 32, ... in ascending order, then the lanes are added.
+template <int PIECES>
+__global__ void __launch_bounds__(512 / PIECES)
 norm_add_block_kernel(float* x, long long ldx, const float* y, long long ldy, const float* __restrict__ gain, int dim, int kind, float eps,
                       bf16* copy, ThenNorm then, const float* part, int splits, long long split_stride,
                       const float* __restrict__ part_bias) {
-  extern __shared__ __align__(16) float tiles[];          // [splits][dim], then four rows of a number a thread
+  extern __shared__ __align__(16) float tiles[];          // [splits][dim], then four rows of a number a piece
   pdl_trigger();
   const size_t r = blockIdx.x;
-  const int lane = threadIdx.x & 31, d = 4 * threadIdx.x;
-  const bool in = d < dim, second = then.gain != nullptr;
+  const int lane = threadIdx.x & 31, threads = blockDim.x, pieces = PIECES * threads;
+  const bool second = then.gain != nullptr;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 g1 = in ? *reinterpret_cast<const float4*>(gain + d) : zero;
-  float4 g2 = in && second ? *reinterpret_cast<const float4*>(then.gain + d) : zero;
-  float4 pb = in && splits > 0 && part_bias ? *reinterpret_cast<const float4*>(part_bias + d) : zero;
-  gb_pin(g1);
-  gb_pin(g2);
-  gb_pin(pb);
-  float* sums = tiles + (size_t)splits * dim;
-  // a row's sum: every lane its pieces in ascending order, then the lanes
-  auto row_sum = [&](float mine, int turn) {
-    float* at = sums + turn * blockDim.x;
-    at[threadIdx.x] = mine;
-    __syncthreads();
-    float s = 0.f;
-    for (int i = lane; i < (int)blockDim.x; i += 32) s += at[i];
-    return warp_sum(s);
-  };
-  auto normed = [&](float4 v, int kd, float e, float4 g, int turn) {
-    const float mean = kd == NORM_LAYER ? row_sum((v.x + v.y) + (v.z + v.w), turn) / (float)dim : 0.f;
-    const float4 c = make_float4(v.x - mean, v.y - mean, v.z - mean, v.w - mean);
-    const float ss = row_sum(in ? (c.x * c.x + c.y * c.y) + (c.z * c.z + c.w * c.w) : 0.f, turn + 1);
-    const float rstd = 1.0f / sqrtf(ss / (float)dim + e);
-    return make_float4(c.x * rstd * g.x, c.y * rstd * g.y, c.z * rstd * g.z, c.w * rstd * g.w);
-  };
-  pdl_wait();
-  float4 v = zero, old = zero;
-  if (in) {
-    const float* from = part + r * dim + d;
-    for (int u = 0; u < splits; ++u) gb_cp_async_16(tiles + (size_t)u * dim + d, from + (size_t)u * split_stride);
-    old = ldcg_now(reinterpret_cast<const float4*>(x + r * ldx + d));
-    if (splits > 0) {
-      gb_cp_async_wait_all();
-      for (int u = 0; u < splits; ++u) {
-        const float4 q = *reinterpret_cast<const float4*>(tiles + (size_t)u * dim + d);
-        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-      }
-      if (part_bias) { v.x += pb.x; v.y += pb.y; v.z += pb.z; v.w += pb.w; }
-    } else {
-      v = ldcg_now(reinterpret_cast<const float4*>(y + r * ldy + d));
+  int d[PIECES];
+  float4 g1[PIECES], g2[PIECES], pb[PIECES];
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    d[i] = 4 * (threadIdx.x + i * threads);
+    g1[i] = d[i] < dim ? *reinterpret_cast<const float4*>(gain + d[i]) : zero;
+    g2[i] = d[i] < dim && second ? *reinterpret_cast<const float4*>(then.gain + d[i]) : zero;
+    pb[i] = d[i] < dim && splits > 0 && part_bias ? *reinterpret_cast<const float4*>(part_bias + d[i]) : zero;
+    if (PIECES == 1) {                                    // (several pieces would hold registers that a launch of many rows needs more)
+      gb_pin(g1[i]);
+      gb_pin(g2[i]);
+      gb_pin(pb[i]);
     }
   }
-  v = normed(v, kind, eps, g1, 0);
-  v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w);
+  float* sums = tiles + (size_t)splits * dim;
+  auto row_sum = [&](const float (&mine)[PIECES], int turn) {
+    float* at = sums + turn * pieces;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) at[threadIdx.x + i * threads] = mine[i];
+    __syncthreads();
+    float s = 0.f;
+    for (int i = lane; i < pieces; i += 32) s += at[i];
+    return warp_sum(s);
+  };
+  float4 v[PIECES], old[PIECES];
+  // v = to + norm(v) * g
+  auto normed = [&](int kd, float e, const float4 (&g)[PIECES], const float4 (&to)[PIECES], int turn) {
+    float one[PIECES];
+    float mean = 0.f;
+    if (kd == NORM_LAYER) {
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) one[i] = (v[i].x + v[i].y) + (v[i].z + v[i].w);
+      mean = row_sum(one, turn) / (float)dim;
+    }
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      v[i] = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
+      one[i] = d[i] < dim ? fmaf(v[i].x, v[i].x, __fmul_rn(v[i].y, v[i].y)) + fmaf(v[i].z, v[i].z, __fmul_rn(v[i].w, v[i].w)) : 0.f;
+    }
+    const float rstd = 1.0f / sqrtf(row_sum(one, turn + 1) / (float)dim + e);
+    // (written out, so that no choice of the compiler's between one rounding and two differs with PIECES)
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i)
+      v[i] = make_float4(fmaf(__fmul_rn(v[i].x, rstd), g[i].x, to[i].x), fmaf(__fmul_rn(v[i].y, rstd), g[i].y, to[i].y),
+                         fmaf(__fmul_rn(v[i].z, rstd), g[i].z, to[i].z), fmaf(__fmul_rn(v[i].w, rstd), g[i].w, to[i].w));
+  };
   auto pack = [](float4 q) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(q.x, q.y), hi = __floats2bfloat162_rn(q.z, q.w);
     return make_uint2(*reinterpret_cast<unsigned*>(&lo), *reinterpret_cast<unsigned*>(&hi));
   };
-  if (in) {
-    *reinterpret_cast<float4*>(x + r * ldx + d) = v;
-    if (copy) *reinterpret_cast<uint2*>(copy + r * dim + d) = pack(v);
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    v[i] = old[i] = zero;
+    if (d[i] >= dim) continue;
+    const float* from = part + r * dim + d[i];
+    for (int u = 0; u < splits; ++u) gb_cp_async_16(tiles + (size_t)u * dim + d[i], from + (size_t)u * split_stride);
+    if (splits == 0) v[i] = ldcg_now(reinterpret_cast<const float4*>(y + r * ldy + d[i]));
+    old[i] = ldcg_now(reinterpret_cast<const float4*>(x + r * ldx + d[i]));
+  }
+  if (splits > 0) {
+    gb_cp_async_wait_all();
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+      if (d[i] >= dim) continue;
+      for (int u = 0; u < splits; ++u) {
+        const float4 q = *reinterpret_cast<const float4*>(tiles + (size_t)u * dim + d[i]);
+        v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w;
+      }
+      if (part_bias) { v[i].x += pb[i].x; v[i].y += pb[i].y; v[i].z += pb[i].z; v[i].w += pb[i].w; }
+    }
+  }
+  normed(kind, eps, g1, old, 0);
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    old[i] = zero;
+    if (d[i] < dim) {
+      *reinterpret_cast<float4*>(x + r * ldx + d[i]) = v[i];
+      if (copy) *reinterpret_cast<uint2*>(copy + r * dim + d[i]) = pack(v[i]);
+    } else {
+      v[i] = zero;
+    }
   }
   if (!second) return;
-  if (!in) v = zero;
-  v = normed(v, then.kind, then.eps, g2, 2);
-  if (!in) return;
-  if (then.out_dtype == GB_BF16) *reinterpret_cast<uint2*>((bf16*)then.out + r * dim + d) = pack(v);
-  else *reinterpret_cast<float4*>((float*)then.out + r * dim + d) = v;
+  normed(then.kind, then.eps, g2, old, 2);
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    if (d[i] >= dim) continue;
+    if (then.out_dtype == GB_BF16) *reinterpret_cast<uint2*>((bf16*)then.out + r * dim + d[i]) = pack(v[i]);
+    else *reinterpret_cast<float4*>((float*)then.out + r * dim + d[i]) = v[i];
+  }
 }
 
 // y = the partial tiles' sum (+ bias), for rows that the kernel above does not take
@@ -931,14 +968,22 @@ GB_OP(gb_op_norm_add) {
   if (dim % 4 == 0 && dim <= 2048 && ((a[0] | a[2] | a[4] | a[9] | 4 * a[1] | 4 * a[3]) & 15) == 0 && (a[8] & 7) == 0 &&
       (!second || (a[10] & (then.out_dtype == GB_BF16 ? 7 : 15)) == 0) && ((uintptr_t)part & 15) == 0 &&
       (part == nullptr || ((uintptr_t)ctx->part_bias & 15) == 0) && smem <= 160 * 1024) {
-    static bool raised = false;
-    if (!raised) {
-      GB_CUDA(cudaFuncSetAttribute(norm_add_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-      raised = true;
-    }
-    gb_launch(norm_add_block_kernel, dim3(n), dim3(32 * gb_div_up(dim, 128)), smem, ctx->stream, op_ptr<float>(a[0]), a[1],
-              op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]), then, part, splits,
-              (long long)n * dim, part != nullptr ? ctx->part_bias : nullptr);
+#define NORM_ADD(PIECES)                                                                                                            \
+    do {                                                                                                                            \
+      static bool raised = false;                                                                                                   \
+      if (!raised) {                                                                                                                \
+        GB_CUDA(cudaFuncSetAttribute(norm_add_block_kernel<PIECES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));     \
+        raised = true;                                                                                                              \
+      }                                                                                                                             \
+      gb_launch(norm_add_block_kernel<PIECES>, dim3(n), dim3(32 * gb_div_up(dim, 128 * PIECES)), smem, ctx->stream,                 \
+                op_ptr<float>(a[0]), a[1], op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0],      \
+                op_ptr<bf16>(a[8]), then, part, splits, (long long)n * dim, part != nullptr ? ctx->part_bias : nullptr);            \
+    } while (0)
+    // (us of a piece a thread, four a thread, and of the kernel below, which serves the other rows; with the second norm: 2,695 rows of 2,048
+    // 21.6, 16.7, 21.2, 8,000 64.7, 52.4, 60.8, 1,024 10.1, 8.4, 12.7; 2,134 rows of 1,024 9.6, 8.4, 12.6, 1,500 7.8, 7.8, 11.1; 8,000 of 128
+    // 10.4, 11.8, 13.1)
+    if (dim > 512 && (long long)n * dim >= 1 << 21) NORM_ADD(4); else NORM_ADD(1);
+#undef NORM_ADD
     GB_CHECK_LAUNCH("norm_add (a block a row)");
     return 1;
   }
@@ -952,8 +997,8 @@ GB_OP(gb_op_norm_add) {
   }
   const bool fused = second && dim <= NORM_CACHE * threads;   // the row fits the registers
   ThenNorm none = {nullptr, nullptr, 0, 0, 0.f};
-  // (us with the gains ahead and without, rows of 2048: 200 rows 3.2 and 4.2, 512 5.0 and 4.7, 2134 13.9 and 11.6; rows too long
-  // for the registers read them at the end either way)
+  // (rows that are no 16-byte pieces, or longer than 2,048.  us with the gains ahead and without, measured at rows of 2,048: 200 rows
+  // 3.2 and 4.2, 512 5.0 and 4.7, 2,134 13.9 and 11.6; rows too long for the registers read them at the end either way)
   const bool ahead = n <= 296 && dim <= NORM_CACHE * threads;
   gb_launch(ahead ? norm_add_kernel<true> : norm_add_kernel<false>, dim3(n), dim3(threads), 0, ctx->stream, op_ptr<float>(a[0]), a[1],
             op_ptr<const float>(a[2]), a[3], op_ptr<const float>(a[4]), dim, kind, (float)f[0], op_ptr<bf16>(a[8]),

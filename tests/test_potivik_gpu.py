@@ -916,3 +916,53 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     out = capsys.readouterr().out
     generated = [int(t) for t in out.split("Output:\n")[1].splitlines()[0].split(",")]
     assert len(generated) == 5 and generated[0] == top["ids"][0]
+
+
+# the paths beside the block kernel: rows longer than 2,048 or no multiple of 4, y in wider rows, tiles added up into y first
+@pytest.mark.parametrize("d,kind,second,splits,bias,pad", [(2052, 1, True, 3, True, 0), (4096, 0, True, 16, False, 8), (4096, 1, False, 0, False, 0),
+                                                           (130, 0, True, 2, True, 6), (2050, 1, False, 1, False, 2), (1027, 1, True, 0, False, 1)])
+def test_norm_behind_a_sublayer_of_rows_that_no_block_takes_whole(d, kind, second, splits, bias, pad):
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(d)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 299
+    x0, gain, then, add = (torch.randn(*k, device=dev) for k in ((many, d), (d,), (d,), (d,)))
+    part = torch.randn(max(splits, 1), many, d, device=dev)
+    y0 = part[0].clone()
+    for u in range(1, splits):
+        y0 += part[u]
+    if bias and splits:
+        y0 += add
+
+    def run(n, tiles):
+        x, parts = x0[:n].clone(), part[:, :n].contiguous()
+        y = torch.full((n, d + pad), float("nan"), device=dev)
+        if not tiles:
+            y[:, :d] = y0[:n]
+        h, copy = torch.zeros(n, d, device=dev), torch.zeros(n, d, device=dev, dtype=torch.bfloat16)
+        stream = _stream()
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), None, 0, None, 0, None, 0, None,
+                          parts.data_ptr() if tiles else None, splits if tiles else 0, add.data_ptr() if tiles and bias else None)
+        a = (ctypes.c_longlong * 24)(x.data_ptr(), d, y.data_ptr(), d + pad, gain.data_ptr(), n, d, kind, copy.data_ptr(), then.data_ptr() if second else 0,
+                                     h.data_ptr() if second else 0, 0, kind)
+        rc = hybrid._function("norm_add")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(1e-5, 1e-5), ctypes.c_int(hybrid.TAKES_PARTIALS if tiles else 0))
+        assert rc == 1 + int(tiles) + int(second and d > 2048)
+        torch.cuda.synchronize()
+        assert torch.equal(copy, x.bfloat16()) and (y[:, d:].isnan().all())
+        return x, h
+
+    whole = run(many, False)
+    for n in (1, 296, 297, many):                            # (either side of the rule for gains ahead)
+        for tiles in ((False, True) if splits else (False,)):
+            got = run(n, tiles)
+            assert torch.equal(got[0], whole[0][:n]) and torch.equal(got[1], whole[1][:n]), (n, tiles)
+
+    def norm(v, g):
+        v = v.double() - (v.double().mean(1, keepdim=True) if kind == 0 else 0.0)
+        return v / (v.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * g.double()
+    new = x0.double() + norm(y0, gain)
+    assert ((whole[0].double() - new).norm(dim=1) / new.norm(dim=1)).max() < 1e-6
+    if second:
+        want = norm(new, then)
+        assert ((whole[1].double() - want).norm(dim=1) / want.norm(dim=1)).max() < 1e-6

@@ -736,3 +736,38 @@ def test_row_norm_with_pending_sums_has_the_same_bits_at_any_number_of_rows(dim,
     for n in (1, 639, 640, 2047, 2048):
         x, out = run(n)
         assert torch.equal(x, whole_x[:n]) and torch.equal(out, whole[:n]), n
+
+
+# one piece a thread and four
+@pytest.mark.parametrize("d,kind,second,splits,edge", [(2048, 1, True, 0, 1024), (2048, 0, False, 3, 1024), (1540, 0, True, 1, 1362), (516, 1, True, 2, 4065),
+                                                       (1024, 0, True, 0, 2048)])
+def test_norm_behind_a_sublayer_has_the_same_bits_at_any_number_of_rows(d, kind, second, splits, edge):
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(d)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), edge + 3
+    x0, gain, then = (torch.randn(*k, device=dev) for k in ((many, d), (d,), (d,)))
+    part = torch.randn(max(splits, 1), many, d, device=dev)
+
+    def run(n):
+        x, parts = x0[:n].clone(), part[:, :n].contiguous()
+        h, copy = torch.zeros(n, d, device=dev, dtype=torch.bfloat16), torch.zeros(n, d, device=dev, dtype=torch.bfloat16)
+        stream = _stream()
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), None, 0, None, 0, None, 0, None,
+                          parts.data_ptr() if splits else None, splits, None)
+        a = (ctypes.c_longlong * 24)(x.data_ptr(), d, parts.data_ptr(), d, gain.data_ptr(), n, d, kind, copy.data_ptr(), then.data_ptr() if second else 0,
+                                     h.data_ptr() if second else 0, 1, kind)
+        assert hybrid._function("norm_add")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(1e-5, 1e-5), ctypes.c_int(hybrid.TAKES_PARTIALS if splits else 0)) == 1
+        torch.cuda.synchronize()
+        assert torch.equal(copy, x.bfloat16())
+        return x, h
+
+    assert (edge - 1) * d < 1 << 21 <= edge * d
+    x, h = run(many)
+    norm = lambda v, g: (v - (v.mean(1, keepdim=True) if kind == 0 else 0.0)) / ((v - (v.mean(1, keepdim=True) if kind == 0 else 0.0)).pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * g.double()
+    want = x0.double() + norm(part[:max(splits, 1)].double().sum(0), gain)
+    assert ((x.double() - want).norm(dim=1) / want.norm(dim=1)).max() < 1e-6
+    for n in (1, edge - 1, edge):
+        got = run(n)
+        assert torch.equal(got[0], x[:n]) and torch.equal(got[1], h[:n]), n
