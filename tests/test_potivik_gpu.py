@@ -966,3 +966,40 @@ def test_norm_behind_a_sublayer_of_rows_that_no_block_takes_whole(d, kind, secon
     if second:
         want = norm(new, then)
         assert ((whole[1].double() - want).norm(dim=1) / want.norm(dim=1)).max() < 1e-6
+
+
+# rows in 16-byte pieces (blocks for few rows and for many) and value by value; no shared expert, one that is whole, and one as partial tiles
+@pytest.mark.parametrize("width,top", [(1024, 2), (2048, 1), (260, 5), (130, 3), (2048, 8)])
+@pytest.mark.parametrize("splits,bias", [(-1, False), (0, False), (1, True), (9, False), (3, True)])
+def test_experts_outputs_are_summed_with_a_shared_expert_in_tiles(width, top, splits, bias):
+    import ctypes
+
+    from gibbs_b200.ops import _stream, device_status, hybrid
+    torch.manual_seed(width + top)
+    dev, many = torch.device("cuda", torch.cuda.current_device()), 700
+    e, gate = torch.randn(many * top, width, device=dev), torch.rand(many, device=dev)
+    part, add = torch.randn(max(splits, 1), many, width, device=dev), torch.randn(width, device=dev)
+    shared = part[0].clone()
+    for u in range(1, splits):
+        shared += part[u]
+    if splits > 0 and bias:
+        shared += add
+    for n in (1, 591, 592, many):
+        pair = torch.randperm(n * top, device=dev).int()
+        parts, whole, y = part[:, :n].contiguous(), shared[:n].clone(), torch.full((n, width + 4), 7.0, device=dev)
+        if splits > 0:
+            whole.fill_(float("nan"))
+        stream = _stream()
+        ctx = hybrid._Ctx(stream.value if isinstance(stream, ctypes.c_void_p) else stream, device_status(dev).data_ptr(), None, 0, None, 0, None, 0, None,
+                          parts.data_ptr() if splits > 0 else None, max(splits, 0), add.data_ptr() if splits > 0 and bias else None)
+        a = (ctypes.c_longlong * 24)(e.data_ptr(), width, pair.data_ptr(), gate.data_ptr() if splits >= 0 else 0, whole.data_ptr() if splits >= 0 else 0,
+                                     width, y.data_ptr(), width + 4, n, width, top)
+        assert hybrid._function("moe_combine")(ctypes.byref(ctx), a, (ctypes.c_double * 3)(), ctypes.c_int(hybrid.TAKES_PARTIALS if splits > 0 else 0)) == 1
+        torch.cuda.synchronize()
+        assert (y[:, width:] == 7.0).all()
+        rows = e[pair.long()].reshape(n, top, width).double()
+        want, size = rows.sum(1), rows.abs().sum(1)
+        if splits >= 0:
+            want, size = want + gate[:n, None].double() * shared[:n].double(), size + gate[:n, None].double() * shared[:n].double().abs()
+        # (a rounding for every addition; the shared row's own sums are those of the reference)
+        assert ((y[:, :width].double() - want).abs() <= (top + 2) * 2.0 ** -24 * size).all(), n
