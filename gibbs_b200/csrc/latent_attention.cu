@@ -24,7 +24,7 @@ namespace {
 enum { STATUS_BAD_PAGE_WRITE = 1, STATUS_BAD_PAGE_READ = 2 };
 
 // one block per token: warp 0 writes the cache row, the others rotate the heads' queries
-template <typename TC>
+template <typename TC, int ROT, int LAT>                   // rotated pairs and latent entries a lane holds
 __global__ void latent_prep_kernel(const float* fused, long long ld, int dkv_col, const float* queries, long long ldq,
                                    const float* __restrict__ gain,
                                    const float* __restrict__ inv_freq, int rot_dims, const int* tok_req,
@@ -37,15 +37,18 @@ __global__ void latent_prep_kernel(const float* fused, long long ld, int dkv_col
   const int half = rot_dims >> 1;
   // The angles, the page and the gains are known before the kernel in front has finished (pinned, see gb_pin); behind the wait
   // all of a row's values are asked for before the first is used.
-  constexpr int ROT = 2, LAT = 16, HEADS = 3;              // rotated pairs and latent entries a lane holds; heads a warp takes at a time
+  constexpr int HEADS = 3;                                 // heads a warp takes at a time
   const bool rot_here = half <= 32 * ROT, lat_here = r <= 32 * LAT;
   float c[ROT], s[ROT], g[LAT];
 #pragma unroll
   for (int i = 0; i < ROT; ++i) {
     const int j = lane + 32 * i;
-    const float ang = rot_here && j < half ? (float)pos * inv_freq[j] : 0.f;
-    c[i] = cosf(ang);
-    s[i] = sinf(ang);
+    c[i] = s[i] = 0.f;
+    if (rot_here && 32 * i < half) {                       // (the same in a whole warp: what no lane needs is not worked out)
+      const float ang = j < half ? (float)pos * inv_freq[j] : 0.f;
+      c[i] = cosf(ang);
+      s[i] = sinf(ang);
+    }
     gb_pin(c[i]);
     gb_pin(s[i]);
   }
@@ -79,7 +82,10 @@ __global__ void latent_prep_kernel(const float* fused, long long ld, int dkv_col
       if (lat_here) {
         float x[LAT];
 #pragma unroll
-        for (int i = 0; i < LAT; ++i) x[i] = lane + 32 * i < r ? ldcg_now(lat + lane + 32 * i) : 0.f;
+        for (int i = 0; i < LAT; ++i) {
+          x[i] = 0.f;
+          if (32 * i < r && lane + 32 * i < r) x[i] = ldcg_now(lat + lane + 32 * i);
+        }
 #pragma unroll
         for (int i = 0; i < LAT; ++i)
           if (lane + 32 * i < r) ss += x[i] * x[i];
@@ -114,6 +120,7 @@ __global__ void latent_prep_kernel(const float* fused, long long ld, int dkv_col
   if (warps > 1 && warp == 0) return;
   const float* q0 = queries + (size_t)t * ldq + dn;        // a head's rotated part lies dn behind its first entry
   float* o0 = qp + (size_t)t * H * (r + dr) + r;
+  if (dr == 0) return;
   for (int h0 = warp - w0; h0 < H; h0 += HEADS * step) {
     float u[HEADS][ROT], v[HEADS][ROT];
 #pragma unroll
@@ -750,13 +757,23 @@ GB_OP(gb_op_latent_prep) {
   if (n <= 0) return 0;
   if (a[5] % 2 || a[5] > a[17]) GB_FAIL(GB_ERR_ARG, "latent_prep: %lld rotated dimensions of %lld", a[5], a[17]);
   const int warps = H + 1 < 8 ? H + 1 : 8;
-#define PREP(TC)                                                                                                       \
-  gb_launch(latent_prep_kernel<TC>, dim3(n), dim3(32 * warps), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2], \
+#define PREP(TC, ROT, LAT)                                                                                                 \
+  gb_launch(latent_prep_kernel<TC, ROT, LAT>, dim3(n), dim3(32 * warps), 0, ctx->stream, op_ptr<const float>(a[0]), a[1], (int)a[2], \
             a[20] ? op_ptr<const float>(a[20]) : op_ptr<const float>(a[0]), a[20] ? a[21] : a[1], op_ptr<const float>(a[3]), \
             op_ptr<const float>(a[4]), (int)a[5], op_ptr<const int>(a[6]),                   \
             op_ptr<const int>(a[7]), op_ptr<const int>(a[8]), (int)a[9], (int)a[10], op_ptr<TC>(a[11]), (int)a[12], H,  \
             (int)a[16], (int)a[17], (int)a[18], op_ptr<float>(a[19]), (float)f[0], ctx->status)
-  if (a[13] == GB_BF16) PREP(bf16); else PREP(float);
+#define PREP_LAT(TC, ROT)                                                                                   \
+  do {                                                                                                      \
+    if (a[18] <= 128) PREP(TC, ROT, 4); else if (a[18] <= 256) PREP(TC, ROT, 8); else PREP(TC, ROT, 16);   \
+  } while (0)
+#define PREP_ROT(TC)                                            \
+  do {                                                          \
+    if (a[5] <= 64) PREP_LAT(TC, 1); else PREP_LAT(TC, 2);      \
+  } while (0)
+  if (a[13] == GB_BF16) PREP_ROT(bf16); else PREP_ROT(float);
+#undef PREP_ROT
+#undef PREP_LAT
 #undef PREP
   GB_CHECK_LAUNCH("latent_prep");
   return 1;

@@ -771,3 +771,37 @@ def test_norm_behind_a_sublayer_has_the_same_bits_at_any_number_of_rows(d, kind,
     for n in (1, edge - 1, edge):
         got = run(n)
         assert torch.equal(got[0], x[:n]) and torch.equal(got[1], h[:n]), n
+
+
+# latents of one to sixteen values a lane and longer, rotated parts of none, up to 64, up to 128 and more entries
+@pytest.mark.parametrize("H,dn,dr,rot,r", [(1, 3, 2, 2, 1), (4, 16, 64, 64, 128), (3, 8, 80, 66, 136), (16, 128, 64, 64, 512), (2, 5, 128, 128, 256),
+                                           (16, 64, 0, 0, 264), (3, 4, 160, 160, 600), (9, 8, 7, 0, 40)])
+def test_latent_preparation(H, dn, dr, rot, r):
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(r + dr)
+    n, ps, first, F = 37, 8, 5, H * (dn + dr) + r + dr
+    blocks = -(-(first + n) // ps)
+    fused, gain, inv = torch.randn(n, F, device="cuda"), torch.randn(r, device="cuda"), torch.rand(rot // 2 + 1, device="cuda")
+    pages, qp = torch.full((blocks, ps, r + dr), 7.0, device="cuda"), torch.full((n, H, r + dr), 7.0, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    bt, req, pos = i32([list(range(blocks))[::-1]]), i32([0] * n), i32(list(range(first, first + n)))
+    hybrid.call("latent_prep", [fused.data_ptr(), F, H * (dn + dr), gain.data_ptr(), inv.data_ptr(), rot, req.data_ptr(), pos.data_ptr(), bt.data_ptr(),
+                                blocks, ps, pages.data_ptr(), blocks, 0, n, H, dn, dr, r, qp.data_ptr()], [1e-5])
+    angle = (pos.float()[:, None] * inv[:rot // 2]).double()          # (the angle itself is a 32-bit product)
+    c, s = angle.cos(), angle.sin()
+
+    def turned(v):
+        v = v.double().clone()
+        a, b = v[..., 0:rot:2].clone(), v[..., 1:rot:2].clone()
+        shape = [n] + [1] * (v.dim() - 2) + [rot // 2]
+        v[..., 0:rot:2], v[..., 1:rot:2] = a * c.reshape(shape) - b * s.reshape(shape), b * c.reshape(shape) + a * s.reshape(shape)
+        return v
+
+    lat = fused[:, H * (dn + dr):H * (dn + dr) + r].double()
+    want = torch.cat([lat / (lat.pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * gain.double(), turned(fused[:, H * (dn + dr) + r:])], 1)
+    flat = pages[bt[0].long()].reshape(-1, r + dr)
+    # (sines and cosines to 2 ulp, sums of products of numbers up to 6; a latent's sum of squares and its root)
+    assert ((flat[first:first + n].double() - want).abs() <= 1e-5 + 1e-6 * want.abs()).all()
+    assert (flat[:first] == 7.0).all() and (flat[first + n:] == 7.0).all()
+    q = turned(fused[:, :H * (dn + dr)].reshape(n, H, dn + dr)[:, :, dn:])
+    assert ((qp[:, :, r:].double() - q).abs() <= 1e-5).all() and (qp[:, :, :r] == 7.0).all()
