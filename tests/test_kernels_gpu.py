@@ -244,6 +244,13 @@ def test_short_conv_of_portions_and_the_state_they_leave(hidden, k, lens):
     assert torch.equal(st.cpu(), want_state)
 
 
+# rows of 8 to 64 groups of eight channels: eight, four, two runs and one a block, a last block that is partly filled
+@pytest.mark.parametrize("hidden,k,lens", [(8, 3, [1, 5, 9]), (72, 4, [3, 800]), (136, 2, [1, 2, 3] * 12), (256, 4, [1, 9, 790, 2]), (264, 3, [770, 13]),
+                                           (512, 3, [5] * 40)])
+def test_short_conv_of_portions_of_narrow_rows(hidden, k, lens):
+    test_short_conv_of_portions_and_the_state_they_leave(hidden, k, lens)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("hidden,k,use_bias", [(96, 4, True), (200, 2, False), (2048, 3, False)])
 def test_short_conv_one_token_per_request(dtype, hidden, k, use_bias):
