@@ -504,9 +504,10 @@ int run_attention_tc(const GbPlanCtx* ctx, const long long* a, const double* f, 
   // Steps whose every portion fills less than 16 of a tile's 128 rows stay here (64 requests of 2 tokens at 100 keys 24 and 22; of 8, 24 and 32)
   const long long longest = ctx->sym != nullptr && ctx->sym[GB_SYM_MAX_PORTION] > 0 ? ctx->sym[GB_SYM_MAX_PORTION] : n;
   if (!narrow && p.splits == 1 && tiles * G * maps >= 48 && p.keep_first == 0 && longest * group >= 16) {
+    const int seen = p.window > 0 && p.window + 128 < a[19] ? p.window + 128 : (int)a[19];
     const GatedTcgen05Launch b = {p.q, p.k_pages, p.v_pages, p.block_table, p.bt_stride, p.page_size, p.n_pages, p.tok_req,
                                   p.tok_pos, p.q_start, p.gate, p.ld_gate, p.out, p.out_f32, p.ldo, n, R, H, G, dim, vdim, maps,
-                                  p.window, p.blocked, p.sink, p.scale, p.softcap, p.sink_scores, SIG, score_bias, factor, p.status};
+                                  p.window, p.blocked, p.sink, p.scale, p.softcap, p.sink_scores, SIG, score_bias, factor, seen, p.status};
     if (gb_gated_tcgen05_takes(b)) return gb_gated_tcgen05_launch(b, ctx->stream);
   }
   const dim3 grid(tiles, G * maps, p.splits);

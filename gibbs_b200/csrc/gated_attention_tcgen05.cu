@@ -33,6 +33,11 @@ namespace {
 using namespace sm100;
 
 constexpr int GT_ROWS = 128, GT_KEYS = 64, GT_RING = 3, GT_DK = 64;
+// LONG: every GT_FOLD key tiles O moves from tensor memory to a sum beside it.  The tensor core truncates its sums, so one over a long context
+// is off by the more the longer it is, here as on mma.sync (relative error of values of one sign, 64-entry heads: 4,096 keys 1.4e-5, 8,192
+// 3.8e-5 on both, 32,768 2.0e-4; with LONG 1.5e-5 at all of these).  A kernel of its own, because the code for it costs the others 2 to
+// 5 % of a launch.
+constexpr int GT_FOLD = 64;
 constexpr int GT_TIMEOUT = 40;
 enum { GT_BAD_PAGE_READ = 2 };
 
@@ -67,6 +72,20 @@ __device__ __forceinline__ float gt_rcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// total[0 .. DV - 1] = total * 2^(total[DV] - m) + O * corr, total[DV] = m; the first time without what was there.
+template <int DV, bool SIG>
+__device__ __noinline__ void gt_fold(float* total, bool more, float corr, float m, uint32_t tmem_row) {
+  const float f = !more ? 0.f : SIG ? 1.f : total[DV] == -INFINITY ? 0.f : gt_ex2(total[DV] - m);
+#pragma unroll 1
+  for (int c0 = 0; c0 < DV; c0 += 16) {
+    float o[16];
+    tmem_ld_16(tmem_row + (uint32_t)c0, o);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) total[c0 + i] = more ? fmaf(total[c0 + i], f, o[i] * corr) : o[i] * corr;
+  }
+  total[DV] = m;
 }
 
 // One row (a token's query head) again, by itself and over the keys first .. last that it sees, in 32-bit: sum[0 .. DV - 1] its weighted
@@ -112,7 +131,7 @@ __device__ __noinline__ void gt_row(float* sum, float& m, float& l, const GtPara
   }
 }
 
-template <int DV, bool CAPPED, bool SIG>
+template <int DV, bool CAPPED, bool SIG, bool LONG>
 __global__ void __launch_bounds__(192) __maxnreg__((GtCfg<DV>::REGS))
 sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ GtParams p) {
@@ -294,7 +313,7 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
           if (VSUB > 1) db = (db & ~((uint64_t)0x3FFF << 16)) | ((uint64_t)((GT_KEYS * 128) >> 4) << 16);
 #pragma unroll
           for (int term = 0; term < 2; ++term)
-            umma_bf16(tmem_o, smem_desc_sw128(sp + (size_t)term * C::P_BYTES) + 2 * k, db, idesc_o, (uint32_t)((j | k | term) != 0));
+            umma_bf16(tmem_o, smem_desc_sw128(sp + (size_t)term * C::P_BYTES) + 2 * k, db, idesc_o, (uint32_t)(((LONG ? j % GT_FOLD : j) | k | term) != 0));
         }
         umma_commit(&kv_empty[s]);
         umma_commit(&o_full);
@@ -317,7 +336,8 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
     const float c_mul = -2.f * p.softcap * LOG2E, c_add = p.softcap * LOG2E;
     const float bias = SIG && p.score_bias && rvalid ? p.score_bias[g * group + hh] * LOG2E : 0.f;
     float m_used = -INFINITY, l_run = 0.f;
-    float total[DV];                                            // a row that is worked out again, in local memory
+    // In local memory: with LONG, O of the tiles in front and the maximum it is relative to; a row that is worked out again.
+    float total[DV + 1];
     bool alive = true;
     for (int j = 0; j < n_tiles; ++j) {
       if (!__all_sync(0xffffffffu, mbar_wait(&s_full, j & 1) && !abort_flag)) {
@@ -384,7 +404,8 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         break;
       }
       tc_fence_after();
-      if (!SIG && j > 0 && __any_sync(0xffffffffu, grow)) {
+      const bool fold = LONG && j > 0 && j % GT_FOLD == 0;
+      if (!SIG && j > 0 && !fold && __any_sync(0xffffffffu, grow)) {
 #pragma unroll 1
         for (int c0 = 0; c0 < DV; c0 += 16) {
           float o[16];
@@ -410,6 +431,10 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         uint8_t* dst = sp + (size_t)row * 128 + ((chunk ^ (row & 7)) << 4);
         *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         *reinterpret_cast<uint4*>(dst + C::P_BYTES) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      if (fold) {
+        gt_fold<DV, SIG>(total, j > GT_FOLD, corr, m_used, tmem_o + lane_off);
+        tc_fence_before();                                      // (the next product starts a new sum in O)
       }
       if (col0 + GT_KEYS > hi_all || col0 < lo_all) {
         // values of positions that nobody here sees: zeros
@@ -467,13 +492,18 @@ sink_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const _
         }
       };
       const float f = scale_of(m_used, l_run);
+      const bool folded = LONG && n_tiles > GT_FOLD;
+      const float f_total = !folded ? 0.f : SIG ? 1.f : total[DV] == -INFINITY ? 0.f : gt_ex2(total[DV] - m_used);
       float check = 0.f;                                        // (x * 0 is a zero or not a number)
 #pragma unroll 1
       for (int c0 = 0; c0 < DV; c0 += 16) {
         float o[16];
         tmem_ld_16(tmem_o + lane_off + (uint32_t)c0, o);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) check = fmaf(o[i], 0.f, check);
+        for (int i = 0; i < 16; ++i) {
+          if (folded) o[i] = fmaf(total[c0 + i], f_total, o[i]);
+          check = fmaf(o[i], 0.f, check);
+        }
         if (rvalid) store(c0, o, f);
       }
       if (rvalid && !(check == 0.f)) {
@@ -535,15 +565,15 @@ bool pages_map(CUtensorMap* map, const void* pages, long long rows, int width, i
   return encode(map, pages, 2, dims, strides, box);
 }
 
-template <int DV, bool CAPPED, bool SIG>
+template <int DV, bool CAPPED, bool SIG, bool LONG>
 int launch_gt(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const GtParams& p, dim3 grid, cudaStream_t stream) {
   static bool raised = false;
   if (!raised) {
-    GB_CUDA((cudaFuncSetAttribute(sink_attention_tcgen05_kernel<DV, CAPPED, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GB_CUDA((cudaFuncSetAttribute(sink_attention_tcgen05_kernel<DV, CAPPED, SIG, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   GtCfg<DV>::SMEM_BYTES)));
     raised = true;
   }
-  gb_launch(sink_attention_tcgen05_kernel<DV, CAPPED, SIG>, grid, dim3(192), GtCfg<DV>::SMEM_BYTES, stream, mq, mk, mv, p);
+  gb_launch(sink_attention_tcgen05_kernel<DV, CAPPED, SIG, LONG>, grid, dim3(192), GtCfg<DV>::SMEM_BYTES, stream, mq, mk, mv, p);
   GB_CHECK_LAUNCH("sink_attention_tcgen05");
   return 1;
 }
@@ -578,9 +608,11 @@ int gb_gated_tcgen05_launch(const GatedTcgen05Launch& a, cudaStream_t stream) {
   // (every request may end with a partly filled tile)
   const dim3 grid(a.G * a.maps, gb_div_up(a.n, tpt) + a.R);
   const bool capped = a.softcap > 0.f;
-#define GT(DV)                                                                                                        \
-  (a.sigmoid ? (capped ? launch_gt<DV, true, true>(mq, mk, mv, p, grid, stream) : launch_gt<DV, false, true>(mq, mk, mv, p, grid, stream)) \
-             : (capped ? launch_gt<DV, true, false>(mq, mk, mv, p, grid, stream) : launch_gt<DV, false, false>(mq, mk, mv, p, grid, stream)))
+  const bool is_long = a.longest > GT_FOLD * GT_KEYS;
+#define GT_AS(DV, CAPPED, SIG) \
+  (is_long ? launch_gt<DV, CAPPED, SIG, true>(mq, mk, mv, p, grid, stream) : launch_gt<DV, CAPPED, SIG, false>(mq, mk, mv, p, grid, stream))
+#define GT(DV) (a.sigmoid ? (capped ? GT_AS(DV, true, true) : GT_AS(DV, false, true)) : (capped ? GT_AS(DV, true, false) : GT_AS(DV, false, false)))
   return a.vdim == 64 ? GT(64) : GT(128);
 #undef GT
+#undef GT_AS
 }

@@ -15,6 +15,7 @@ struct GatedTcgen05Launch {
   const float* sink_scores;
   bool sigmoid;                    // weights sigmoid(score + score_bias[head]), the output times `factor`
   const float* score_bias; float factor;
+  int longest;                     // positions that a tile walks at most
   int* status;
 };
 

@@ -555,6 +555,30 @@ def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(vdim, start
     assert ((got - want).abs() <= 2.0 ** -14.5 * size + 1e-6)[~touched].all()
 
 
+# contexts of thousands of keys, values of one sign, so that truncated sums show: no further off than the kernel of 64-row tiles, which fewer tokens
+# at a time bring into play
+@pytest.mark.parametrize("vdim,sig,cap", [(64, False, 0.0), (128, False, 20.0), (64, True, 0.0), (128, True, 0.0)])
+@pytest.mark.parametrize("ctx", [2048, 4096, 8192, 16300])
+def test_long_contexts_lose_no_precision(vdim, sig, cap, ctx):
+    torch.manual_seed(ctx + vdim)
+    n = 256
+    a = _Pages(16, 4, vdim, ctx - n, n, one_sign=True)
+    got, other = a.attend(0, sig, cap=cap), torch.cat([a.attend(0, sig, first=t, n=64, cap=cap) for t in range(0, n, 64)])
+    err = [0.0, 0.0]
+    page, row = a.at(list(range(ctx)))
+    k, v = (x[page, :, row].double().repeat_interleave(4, 1) for x in (a.k, a.v))
+    for t in range(0, n, 64):
+        s = torch.einsum("thd,khd->thk", a.q[t:t + 64].double().reshape(64, 16, 64), k) * 0.125
+        s = cap * torch.tanh(s / cap) if cap else s
+        seen = torch.arange(ctx, device="cuda")[None] <= torch.arange(ctx - n + t, ctx - n + t + 64, device="cuda")[:, None]
+        w = torch.sigmoid(s).masked_fill(~seen[:, None], 0.0) if sig else torch.softmax(s.masked_fill(~seen[:, None], -math.inf), 2)
+        want = torch.einsum("thk,khd->thd", w, v)
+        for i, x in enumerate((got, other)):
+            err[i] += ((x[t:t + 64].double() - want) / want).pow(2).mean().item() / (n // 64)
+    err = [e ** 0.5 for e in err]
+    assert err[0] <= 1.001 * err[1] and err[0] < 2e-5, err
+
+
 def _portions_against_float64(heads, kvh, maps, vdim, ps, window, cap, sink, gate, sig, starts, lens, blocked):
     from gibbs_b200.ops import hybrid
     torch.manual_seed(heads * 1000 + window)
