@@ -1003,3 +1003,19 @@ def test_experts_outputs_are_summed_with_a_shared_expert_in_tiles(width, top, sp
             want, size = want + gate[:n, None].double() * shared[:n].double(), size + gate[:n, None].double() * shared[:n].double().abs()
         # (a rounding for every addition; the shared row's own sums are those of the reference)
         assert ((y[:, :width].double() - want).abs() <= (top + 2) * 2.0 ** -24 * size).all(), n
+
+
+# a value a thread below 512 columns a group, pieces from there, rows that are not aligned
+@pytest.mark.parametrize("inner,groups,pad", [(64, 1, 0), (1016, 2, 0), (1024, 2, 0), (2048, 1, 0), (2052, 1, 0), (1024, 2, 1), (3072, 4, 4)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_gated_group_norm(inner, groups, pad, bf16):
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(inner)
+    n, ld = 7, inner + pad
+    y, z, gain = torch.randn(n, ld, device=DEV), torch.randn(n, ld, device=DEV), torch.randn(inner, device=DEV)
+    out = torch.full((n, inner + 8), 7.0, device=DEV, dtype=torch.bfloat16 if bf16 else torch.float32)
+    hybrid.call("gated_group_norm", [y.data_ptr(), ld, z.data_ptr(), ld, gain.data_ptr(), out.data_ptr(), 1 if bf16 else 0, inner + 8, n, inner, groups], [1e-5])
+    v = (y[:, :inner].double() * torch.nn.functional.silu(z[:, :inner].double())).reshape(n, groups, -1)
+    want = (v / (v.pow(2).mean(2, keepdim=True) + 1e-5).sqrt()).reshape(n, inner) * gain.double()
+    # (32-bit: expf, a sum of squares and its root; bfloat16: half a place)
+    assert ((out[:, :inner].double() - want).abs() <= (2.0 ** -8 if bf16 else 2e-6) * want.abs() + 1e-7).all() and (out[:, inner:] == 7.0).all()
