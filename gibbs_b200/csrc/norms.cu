@@ -694,10 +694,10 @@ __global__ void act_rows4_kernel(const float* x, long long ld, TO* out, long lon
   }
 }
 
-// one warp per (row, head); values of up to 32 * HN_VR entries stay in registers
+// one warp per (row, head); values of up to 32 * VR entries stay in registers
 constexpr int HN_VR = 8;
 
-template <typename TO>
+template <typename TO, int VR>
 __global__ void head_norm_kernel(const float* x, long long ldx, long long xh, const float* x2,
                                  const float* __restrict__ gain, const float* gate, long long ld_gate, TO* out,
                                  long long ldo, int n, int H, int vdim, float eps, float lambda, float factor,
@@ -710,9 +710,9 @@ __global__ void head_norm_kernel(const float* x, long long ldx, long long xh, co
   const int t = (int)(idx / H), h = (int)(idx - (long long)t * H);
   const size_t at = (size_t)t * ldx + (size_t)h * xh;
   // the gains before the wait (pinned, see gb_pin), the gate's logits with the row
-  float v[HN_VR], g[HN_VR], z[HN_VR];
+  float v[VR], g[VR], z[VR];
 #pragma unroll
-  for (int i = 0; i < HN_VR; ++i) {
+  for (int i = 0; i < VR; ++i) {
     const int d = lane + 32 * i;
     g[i] = gain && d < vdim ? gain[gain_whole ? h * vdim + d : d] : 1.f;
     gb_pin(g[i]);
@@ -721,20 +721,20 @@ __global__ void head_norm_kernel(const float* x, long long ldx, long long xh, co
   float ss = 0.f;
   const float div = den ? fmaxf(fabsf(den[idx]), floor_[idx]) + lambda : 1.f;
 #pragma unroll
-  for (int i = 0; i < HN_VR; ++i) {
+  for (int i = 0; i < VR; ++i) {
     const int d = lane + 32 * i;
     v[i] = d < vdim ? ldcg_now(x + at + d) : 0.f;
     z[i] = gate && d < vdim ? ldcg_now(gate + (size_t)t * ld_gate + (size_t)h * vdim + d) : 0.f;
   }
 #pragma unroll
-  for (int i = 0; i < HN_VR; ++i) {
+  for (int i = 0; i < VR; ++i) {
     const int d = lane + 32 * i;
     if (d < vdim) v[i] = x2 ? v[i] - lambda * x2[at + d] : den ? v[i] / div : v[i];
     ss += v[i] * v[i];
   }
   const float rstd = factor / sqrtf(warp_sum(ss) / (float)vdim + eps);
 #pragma unroll
-  for (int i = 0; i < HN_VR; ++i) {
+  for (int i = 0; i < VR; ++i) {
     const int d = lane + 32 * i;
     if (d >= vdim) continue;
     float o = v[i] * rstd;
@@ -1147,14 +1147,17 @@ GB_OP(gb_op_head_norm) {
   if (vdim > 32 * HN_VR) GB_FAIL(GB_ERR_ARG, "head_norm: heads of %d values (at most %d)", vdim, 32 * HN_VR);
   if (a[13] && (a[3] || !a[14])) GB_FAIL(GB_ERR_ARG, "head_norm: a divisor comes with a floor and without a second operand");
   const dim3 grid(gb_div_up((long long)n * H, 4)), block(128);
-  if (a[8] == GB_BF16)
-    gb_launch(head_norm_kernel<bf16>, grid, block, 0, ctx->stream, op_ptr<const float>(a[0]), a[1], a[2],
-              op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), op_ptr<const float>(a[5]), a[6], op_ptr<bf16>(a[7]), a[9],
-              n, H, vdim, (float)f[0], (float)f[1], (float)f[2], op_ptr<const float>(a[13]), op_ptr<const float>(a[14]), flags & 1, (flags >> 1) & 1);
-  else
-    gb_launch(head_norm_kernel<float>, grid, block, 0, ctx->stream, op_ptr<const float>(a[0]), a[1], a[2],
-              op_ptr<const float>(a[3]), op_ptr<const float>(a[4]), op_ptr<const float>(a[5]), a[6], op_ptr<float>(a[7]), a[9],
-              n, H, vdim, (float)f[0], (float)f[1], (float)f[2], op_ptr<const float>(a[13]), op_ptr<const float>(a[14]), flags & 1, (flags >> 1) & 1);
+#define HEAD_NORM(TO, VR)                                                                                                       \
+  gb_launch(head_norm_kernel<TO, VR>, grid, block, 0, ctx->stream, op_ptr<const float>(a[0]), a[1], a[2], op_ptr<const float>(a[3]), \
+            op_ptr<const float>(a[4]), op_ptr<const float>(a[5]), a[6], op_ptr<TO>(a[7]), a[9], n, H, vdim, (float)f[0], (float)f[1], \
+            (float)f[2], op_ptr<const float>(a[13]), op_ptr<const float>(a[14]), flags & 1, (flags >> 1) & 1)
+#define HEAD_NORM_VR(TO)                                                                                   \
+  do {                                                                                                     \
+    if (vdim <= 64) HEAD_NORM(TO, 2); else if (vdim <= 128) HEAD_NORM(TO, 4); else HEAD_NORM(TO, HN_VR);   \
+  } while (0)
+  if (a[8] == GB_BF16) HEAD_NORM_VR(bf16); else HEAD_NORM_VR(float);
+#undef HEAD_NORM_VR
+#undef HEAD_NORM
   GB_CHECK_LAUNCH("head_norm");
   return 1;
 }

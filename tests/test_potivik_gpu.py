@@ -1019,3 +1019,23 @@ def test_gated_group_norm(inner, groups, pad, bf16):
     want = (v / (v.pow(2).mean(2, keepdim=True) + 1e-5).sqrt()).reshape(n, inner) * gain.double()
     # (32-bit: expf, a sum of squares and its root; bfloat16: half a place)
     assert ((out[:, :inner].double() - want).abs() <= (2.0 ** -8 if bf16 else 2e-6) * want.abs() + 1e-7).all() and (out[:, inner:] == 7.0).all()
+
+
+# heads of up to 64, 128 and 256 values
+@pytest.mark.parametrize("vdim", [1, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("second,gated,whole,silu", [(False, True, False, False), (True, False, True, False), (False, False, False, False), (True, True, True, True)])
+def test_head_norm(vdim, second, gated, whole, silu):
+    from gibbs_b200.ops import hybrid
+    torch.manual_seed(vdim)
+    n, H, eps, lam, factor = 5, 3, 1e-5, 0.3, 1.5
+    x, x2, gate = (torch.randn(n, H * vdim, device=DEV) for _ in range(3))
+    gain, out = torch.randn(H * vdim if whole else vdim, device=DEV), torch.empty(n, H * vdim, device=DEV)
+    hybrid.call("head_norm", [x.data_ptr(), H * vdim, vdim, x2.data_ptr() if second else 0, gain.data_ptr(), gate.data_ptr() if gated else 0, H * vdim,
+                              out.data_ptr(), 0, H * vdim, n, H, vdim], [eps, lam, factor], flags=(1 if whole else 0) | (2 if silu else 0))
+    v = (x.double() - lam * x2.double() if second else x.double()).reshape(n, H, vdim)
+    want = v / (v.pow(2).mean(2, keepdim=True) + eps).sqrt() * factor * gain.double().reshape(-1, vdim)
+    if gated:
+        g = gate.double().reshape(n, H, vdim)
+        want = want * (torch.nn.functional.silu(g) if silu else torch.sigmoid(g))
+    # (lambda is a 32-bit number here; a difference of two rounded numbers, then as above)
+    assert ((out.reshape(n, H, vdim).double() - want).abs() <= 4e-6 * want.abs() + 2e-6).all()
