@@ -875,6 +875,13 @@ def test_short_conv_from_partial_tiles_equals_the_two_kernel_way(hidden, k, spli
         assert torch.equal(st_a, st_b)
 
 
+# rows that are no multiple of four channels, and filters of more than four taps: a channel a thread
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden,k,splits,use_bias", [(97, 3, 5, True), (1030, 2, 2, False), (30, 4, 16, True), (96, 6, 3, True)])
+def test_short_conv_from_partial_tiles_of_rows_without_pieces(hidden, k, splits, use_bias):
+    test_short_conv_from_partial_tiles_equals_the_two_kernel_way(hidden, k, splits, use_bias)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("heads,kvh,hd,rd,adjacent,norm,splits,write_kv",
                          [(4, 2, 16, 16, False, True, 2, True), (3, 1, 32, 16, True, False, 5, True),

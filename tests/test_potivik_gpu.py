@@ -918,6 +918,33 @@ def test_command_line_from_a_configuration_to_tokens(tmp_path, capsys):
     assert len(generated) == 5 and generated[0] == top["ids"][0]
 
 
+@pytest.mark.parametrize("H,r,dr,spans", [(16, 320, 32, [(3, 560)]), (4, 448, 32, [(40, 1100)]), (4, 480, 0, [(0, 640), (17, 515)]), (16, 264, 0, [(0, 300)])])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_portions_without_a_window_on_the_kernel_for_wide_latents(H, r, dr, spans, with_sink):
+    """Key tiles whole and in two halves (portions of 512 tokens and more, few row tiles), against 64 bits."""
+    call = LatentCalls(H, r, dr, blocks=96)
+    torch.manual_seed(r)
+    n, longest = sum(k for _, k in spans), max(p + k for p, k in spans)
+    q, gate = torch.randn(n, H, r + dr, device=DEV).bfloat16().float(), torch.randn(n, H, device=DEV)
+    sink = torch.randn(H, device=DEV) if with_sink else None
+    one, two = (call(q, gate, sink, spans, 0, longest, chunks=c).reshape(n, H, r).double() for c in (False, True))
+    rows, at = call.pages[call.table.long()].reshape(-1, r + dr).double(), 0
+    for first, k in spans:
+        mine = slice(at, at + k)
+        at += k
+        sc = torch.einsum("nhd,ld->nhl", q[mine].double(), rows[:first + k]) * (r + dr) ** -0.5
+        sc.masked_fill_((torch.arange(first + k, device=DEV) > torch.arange(first, first + k, device=DEV)[:, None])[:, None], -math.inf)
+        if with_sink:
+            sc = torch.cat([sc, sink.double()[None, :, None].expand(k, H, 1)], 2)
+        w = torch.softmax(sc, 2)[:, :, :first + k]
+        gates = torch.sigmoid(gate[mine].double())[..., None]
+        want, size = (w @ rows[:first + k, :r]) * gates, (w @ rows[:first + k, :r].abs()) * gates
+        # weights of 16 bits (2^-17 each), scores of some units formed in 32-bit sums of up to 576 terms (2^-16 of a weight), sums that the
+        # tensor core truncates
+        for got in (one, two):
+            assert ((got[mine] - want).abs() <= 2.0 ** -14 * size + 1e-7).all()
+
+
 # the paths beside the block kernel: rows longer than 2,048 or no multiple of 4, y in wider rows, tiles added up into y first
 @pytest.mark.parametrize("d,kind,second,splits,bias,pad", [(2052, 1, True, 3, True, 0), (4096, 0, True, 16, False, 8), (4096, 1, False, 0, False, 0),
                                                            (130, 0, True, 2, True, 6), (2050, 1, False, 1, False, 2), (1027, 1, True, 0, False, 1)])
