@@ -30,8 +30,11 @@ namespace {
 using namespace sm100;
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
-// (stages: as many as leave room for two blocks an SM)
-template <int BN> constexpr int stages_of() { return BN <= 16 ? 6 : BN <= 64 ? 4 : 3; }
+// (stages: as many as leave room for two blocks an SM; narrow tiles with four leave room for three, which launches of more blocks than two an SM
+// need: us with six and with four, 32 experts, 128 rows of 512 x 2 x 2,048 33.5 and 27.9, 32 rows of 2,048 x 2 x 1,024 37.8 and 32.6; 8 rows of these 12.9 and
+// 14.4)
+template <int BN> constexpr int stages_of() { return BN <= 64 ? 4 : 3; }
+constexpr int FEW_STAGES = 6;
 constexpr int W_TILE_BYTES = BM * BK * 2;
 constexpr int STATUS_TIMEOUT = 24;
 
@@ -48,11 +51,10 @@ struct GroupedParams {
 
 __device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-template <int BN>
+template <int BN, int STAGES>
 __global__ void __launch_bounds__(192)
 moe_experts_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                       const GroupedParams p) {
-  constexpr int STAGES = stages_of<BN>();
   constexpr int X_TILE_BYTES = BN * BK * 2, STAGE_BYTES = W_TILE_BYTES + X_TILE_BYTES;
   constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
   pdl_trigger();
@@ -595,16 +597,16 @@ struct WKeyHash {
 std::mutex g_wmap_mutex;
 std::unordered_map<WKey, CUtensorMap, WKeyHash> g_wmaps;   // weights do not move: their maps are made once
 
-template <int BN>
+template <int BN, int STAGES = stages_of<BN>()>
 int launch(const CUtensorMap& tw, const CUtensorMap& tx, const GroupedParams& p, int weight_tiles, int row_tiles,
            cudaStream_t stream) {
-  constexpr int SMEM = stages_of<BN>() * (W_TILE_BYTES + BN * BK * 2) + 1024;
+  constexpr int SMEM = STAGES * (W_TILE_BYTES + BN * BK * 2) + 1024;
   static bool raised = false;
   if (!raised) {
-    GB_CUDA(cudaFuncSetAttribute(moe_experts_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    GB_CUDA((cudaFuncSetAttribute(moe_experts_tc_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM)));
     raised = true;
   }
-  gb_launch(moe_experts_tc_kernel<BN>, dim3(weight_tiles, row_tiles), dim3(192), SMEM, stream, tw, tx, p);
+  gb_launch(moe_experts_tc_kernel<BN, STAGES>, dim3(weight_tiles, row_tiles), dim3(192), SMEM, stream, tw, tx, p);
   GB_CHECK_LAUNCH("moe_experts_tc");
   return 1;
 }
@@ -685,7 +687,10 @@ GB_OP(gb_op_moe_experts_tc) {
     return launch_pairs(tw, tx, p, (long long)gb_div_up(rows_per_expert, 2 * BM) * (pairs / 32 + E), ctx->stream);
   const int weight_tiles = gb_div_up(rows_per_expert, BM);
   const int row_tiles = gb_div_up(pairs, BN) + E;          // at most this many over all experts
-  return BN == 16   ? launch<16>(tw, tx, p, weight_tiles, row_tiles, ctx->stream)
+  // (blocks that find rows, at most: whole tiles and a partly filled one for every expert that has any)
+  const bool few = (long long)weight_tiles * (pairs / BN + (pairs < E ? pairs : E)) <= 2 * 148;
+  return BN == 16   ? (few ? launch<16, FEW_STAGES>(tw, tx, p, weight_tiles, row_tiles, ctx->stream)
+                           : launch<16>(tw, tx, p, weight_tiles, row_tiles, ctx->stream))
          : BN == 64 ? launch<64>(tw, tx, p, weight_tiles, row_tiles, ctx->stream)
                     : launch<128>(tw, tx, p, weight_tiles, row_tiles, ctx->stream);
 }
