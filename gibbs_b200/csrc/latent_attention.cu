@@ -862,7 +862,7 @@ GB_OP(gb_op_latent_attention) {
   float* ws = op_ptr<float>(a[19]);
   if (ws == nullptr || (long long)n * H * splits > gb_latent_attention_workspace_rows()) splits = 1;
   // bfloat16 pages, a window or single tokens: tensor cores with whole queries and weights (latent_attention_tc.cu).
-  // Measured at 16 heads, 512 + 64 entries, window 1024 (with the merge): portions of 1801 and 333 tokens 0.84 ms against 3.66 on
+  // Measured at 16 heads, 512 + 64 entries, window 1024 (with the merge): portions of 1801 and 333 tokens 0.77 ms against 3.66 on
   // the kernel below, two single tokens at 1801 and 900 keys 16 us against 60.
   if (a[22] && gb_latent_attention_split_takes(n, (int)a[21], H, r, dr, a[2] == GB_BF16, op_ptr<const void>(a[1]),
                                                op_ptr<const void>(a[0]), op_ptr<const void>(a[11]), a[12]) &&

@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(RP > 256 ? 256 : 128, 1) latent_attention_tc_k
 // The same for latents wider than 256 whose rows leave room for the weights in shared memory: 16 warps, four groups of 16 rows x
 // four slices.  For S a slice is 16 of a key tile's 64 keys (every score once, where the kernel above works every score out in
 // both groups of warps), for O a quarter of the latent's columns; maxima and the weights' two terms go through shared memory
-// between the four warps of a row group, which meet at a barrier of their own.  Bound by mma.sync as below: portions of 1,801 and
-// 894 tokens, latent of 512, 475 us a launch and 583 with the kernel above.
+// between the four warps of a row group, which meet at a barrier of their own.  Bound by waiting, as below: portions of 1,801 and
+// 894 tokens, 16 heads, latent of 512, 475 us a launch and 583 with the kernel above.
 constexpr int LTW_SLICES = 4, LTW_THREADS = 128 * LTW_SLICES, LTW_OC = 128, LTW_PLD = 72;
 
 size_t ltw_smem(int stride) {
@@ -567,9 +567,11 @@ template <int RP> int ltc_launch(const LtcParams& p, int tiles, int R, cudaStrea
 //  columns.  Key tiles lie at multiples of 32, so a row's sums are grouped by its position alone, whatever the rows
 //  beside it.  With `splits`, blockIdx.y takes a chunk of keys, a multiple of `chunk` from position 0, and leaves (maximum,
 //  sum, weighted sum) per row for the merge kernel.
-//  Bound by mma.sync: a step of 32 rows x 32 keys takes about 9,600 cycles at 512 + 64 entries, 400 products on each of the SM's
-//  four schedulers at the 19 to 24 cycles that one takes there; the operand reads from shared memory need 2,700.  Sixteen warps and
-//  the tiles with the most keys first: portions of 1,801 and 333 tokens, 64 heads, 1,067 -> 958 us; two single tokens 12.6 -> 9.5.
+//  Bound by waiting: a step of 32 rows x 32 keys takes about 9,600 cycles at 512 + 64 entries.  Its 408 products on each of the SM's
+//  four schedulers need 3,300 (independent mma.sync.m16n8k16 issue one in 8.0 cycles a scheduler, with 4 to 16 warps; one behind
+//  another in 20), its operand reads from shared memory 2,700; scores, softmax and weighted sum follow one another, with barriers
+//  between.  Sixteen warps and the tiles with the most keys first: portions of 1,801 and 894 tokens, 16 heads, 1,067 -> 957 us; two
+//  single tokens 12.6 -> 9.5.
 constexpr int LTX_ROWS = 32, LTX_KEYS = 32, LTX_SLICES = 8, LTX_WARPS = 2 * LTX_SLICES, LTX_SLD = 32, LTX_PLD = 40;
 
 struct LtxParams {
