@@ -612,20 +612,27 @@ bool pages_map(CUtensorMap* out, const void* pages, long long rows, int hd, int 
 }
 
 // CTAs that share a row tile's keys: none unless the longest context a row sees makes a share of MIN_PART_TILES key tiles for
-// two, and never more than the SMs hold at a time (`slots`): a second round of CTAs costs more than the shares give.  us without
-// shares and with them, 32 / 8 heads of 64: 100 tokens behind 8,000 keys 103 and 37, 20 behind 1,500 22.8 and 11.6; where two shares
-// would not fit, 1,000 tokens 22.2 and 27.9, 15 single tokens beside a portion of 500 28.9 and 36.6; heads of 128 on 128-key tiles (one
-// CTA an SM), 700 tokens 19.0 and 32.5; contexts too short for shares, eight portions of 100 tokens 12.8 and 20.6.
-// The shares, so the order in which a row's keys are added, depend on the number of tiles in the launch.  GIBBS_B200_ATTN_PARTS=1..4
-// overrides.
-int key_parts(long long ctas, long long slots, long long key_tiles) {
+// two.  Four or two where all of them are on the chip at a time: a second round of CTAs costs more than the shares give, except
+// where one CTA's walk of a long context (LONG_TILES) is what the launch waits for.  us without shares and with them, caches cold:
+//   all at a time, 32 / 8 heads of 64: 100 tokens behind 8,000 keys 115 and 37, 20 behind 1,500 29 and 13
+//   a second round, 24 / 8 heads of 64, a portion of 500 beside 12 tokens at 2,060 keys (208 CTAs): behind 1,024 keys 44 and 45, 1,536 44 and
+//   48, 4,000 67 and 65, 7,500 111 and 87; beside 15 at 500 (232 CTAs), behind 4,000 and 7,500: 68 and 55, 112 and 78; 32 / 8, 256 CTAs
+//   behind 4,000 at worst 65 and 67
+//   not taken: 32 / 8, 1,000 tokens 21 and 26; eight portions of 100 tokens 11 and 19; heads of 128 on 128-key tiles (one CTA an SM), 700
+//   tokens 18 and 31, 512 behind 4,000 73 and 79
+// The shares, so the order in which a row's keys are added, depend on the number of tiles in the launch and its longest context.
+// GIBBS_B200_ATTN_PARTS=1..4 overrides.
+constexpr int LONG_TILES = 32;
+int key_parts(long long ctas, int ctas_per_sm, long long key_tiles) {
   static const int forced = [] {
     const char* e = getenv("GIBBS_B200_ATTN_PARTS");
     return e ? atoi(e) : 0;
   }();
   if (forced >= 1 && forced <= MAX_PARTS) return forced;
   if (key_tiles < 2 * MIN_PART_TILES) return 1;
-  return 4 * ctas <= slots ? 4 : (2 * ctas <= slots ? 2 : 1);
+  const long long slots = 148ll * ctas_per_sm;
+  if (4 * ctas <= slots) return 4;
+  return 2 * ctas <= slots || (ctas_per_sm > 1 && ctas <= slots && key_tiles >= LONG_TILES) ? 2 : 1;
 }
 
 template <int HD, int KEYS>
@@ -637,7 +644,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
                                  Cfg<HD, KEYS>::SMEM_BYTES));
     attr_set = true;
   }
-  const int parts = key_parts((long long)n_tiles * p.kv_heads, 148ll * Cfg<HD, KEYS>::CTAS, (max_keys + KEYS - 1) / KEYS);
+  const int parts = key_parts((long long)n_tiles * p.kv_heads, Cfg<HD, KEYS>::CTAS, (max_keys + KEYS - 1) / KEYS);
   if (parts == 1) {
     gb_launch(attention_tcgen05_kernel<HD, KEYS>, dim3(p.kv_heads, n_tiles), dim3(192), Cfg<HD, KEYS>::SMEM_BYTES, stream,
               mq, mk, mv, p);

@@ -657,7 +657,7 @@ def test_attention_tensor_cores(heads, kvh, hd, ps, window, before, q_lens):
 @pytest.mark.parametrize("heads,kvh,hd,ps,window,before,lens", [
     (24, 8, 64, 16, 0, [1500, 700, 3000, 90], [400, 1, 1, 1]), (4, 4, 64, 128, 0, [1100], [10]), (2, 1, 64, 16, 0, [0], [1000]),
     (12, 2, 128, 32, 900, [1200, 0], [150, 43]), (16, 2, 128, 16, 0, [4000], [20]), (32, 8, 64, 16, 0, [0], [1500]),
-    (8, 2, 64, 8, 500, [2000], [130]),
+    (8, 2, 64, 8, 500, [2000], [130]), (24, 8, 64, 16, 0, [500] * 15 + [4100], [1] * 15 + [497]),
 ])
 def test_attention_of_portions_over_long_contexts(heads, kvh, hd, ps, window, before, lens):
     from gibbs_b200 import ops
